@@ -167,10 +167,6 @@ struct GemmArgs {
     const float *gv_rope_cos = nullptr, *gv_rope_sin = nullptr;
     const int *gv_rope_pos = nullptr, *gv_rope_step_d = nullptr; int64_t gv_rope_pos_step = 0;
     int gv_rope_cols = 0, gv_hd = 0;
-    // nearest-row search instead of a stored product (tensor-core engine only): for every x row, the
-    // W row n minimising colnorm[n] - 2 x.W_n, kept as min over packed (ordered distance << 32 | n).
-    const float *argmin_colnorm = nullptr;
-    unsigned long long *argmin_best = nullptr;
     // fused QKV projection, head dim 64 (fp16-pair engine with 128-column tiles only): the per-head RMSNorm and
     // the rotary embedding of the query / key heads (what qk_post() does in a pass of its own) are applied in the
     // epilogue, where a thread holds the 64 columns of one head of its row. Columns [0, qk_heads * 64) are heads

@@ -337,7 +337,6 @@ static inline bool al16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 bool gemm_h3_supported(const GemmArgs &a) {
     int64_t ldx = a.ldx ? a.ldx : a.K, ldy = a.ldy ? a.ldy : (a.glu ? a.N / 2 : a.N);
-    if (a.argmin_best) return false;                                // nearest-row search stays on the TF32 kernel
     if (a.M <= 16 || a.N < 32 || a.K < 32) return false;           // up to 16 rows: the weight-streaming GEMV kernel
     if ((a.K & 7) || (ldx & 7)) return false;                       // fp16 rows: TMA strides are multiples of 16 bytes
     if (a.x_lo && a.x_fmt != SPLIT_H16) return false;
@@ -383,7 +382,6 @@ void gemm_h3(const GemmArgs &a) {
     ep.bias = a.bias; ep.res = a.res; ep.ldres = a.ldres ? a.ldres : a.N;
     ep.y = a.y; ep.y_lo = a.y_lo; ep.y_fmt = a.y_fmt; ep.ldy = a.ldy ? a.ldy : (a.glu ? a.N / 2 : a.N);
     ep.M = a.M; ep.N = a.N; ep.act = a.act; ep.glu = a.glu; ep.err = tc_err_flag();
-    ep.colnorm = nullptr; ep.best = nullptr;
     ep.qk_heads = a.qk_heads; ep.qk_H = a.qk_H; ep.qk_qw = a.qk_qw; ep.qk_kw = a.qk_kw; ep.qk_cos = a.qk_cos; ep.qk_sin = a.qk_sin; ep.qk_pos = a.qk_pos;
     ep.acc_scale = H16_X_UNSCALE * H16_X_UNSCALE;                  // weights split per call carry the activations' factor
     int skip_w2 = 0;

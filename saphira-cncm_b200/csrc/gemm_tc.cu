@@ -141,88 +141,11 @@ __global__ void __launch_bounds__(TC_THREADS) k_gemm_tc(const __grid_constant__ 
             ok = mbar_wait(afull0 + 8 * acc, use & 1u, ep.err, 3);
             tc_fence_after();
             if (!ok) break;
-            float bestd = INFINITY; int bestn = 0x7fffffff;
-            if (ep.best) {
-                // Nearest row. The tile has one k-block (K = 64 for the codebook search), so this loop is the kernel:
-                // the next 32 columns are on their way out of tensor memory while these are compared, the column
-                // norms come as float4, and four independent running minima (columns j mod 4) break the
-                // compare-select chain; they merge at the end by (distance, index), which keeps the first minimum.
-                const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-                float bd[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-                int bn[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
-                uint32_t ra[32], rb[32];
-                tmem_ld32_issue(trow, ra);
-                tmem_ld_wait();
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 64) {
-                    if (c0 + 32 < BN) tmem_ld32_issue(trow + (uint32_t)(c0 + 32), rb);
-                    {
-                        const int nb = n0 + c0;
-                        if (nb + 32 <= ep.N) {
-#pragma unroll
-                            for (int j = 0; j < 32; j += 4) {
-                                const float4 cn = *(const float4 *)(ep.colnorm + nb + j);
-                                const float cc[4] = {cn.x, cn.y, cn.z, cn.w};
-#pragma unroll
-                                for (int e = 0; e < 4; e++) {
-                                    const float d = fmaf(-2.0f, __uint_as_float(ra[j + e]), cc[e]);
-                                    if (d < bd[e]) { bd[e] = d; bn[e] = nb + j + e; }
-                                }
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; j++) {
-                                const int n = nb + j;
-                                if (n < ep.N) {
-                                    const float d = fmaf(-2.0f, __uint_as_float(ra[j]), ep.colnorm[n]);
-                                    if (d < bd[j & 3]) { bd[j & 3] = d; bn[j & 3] = n; }
-                                }
-                            }
-                        }
-                    }
-                    tmem_ld_wait();
-                    if (c0 + 64 < BN) tmem_ld32_issue(trow + (uint32_t)(c0 + 64), ra);
-                    if (c0 + 32 < BN) {
-                        const int nb = n0 + c0 + 32;
-                        if (nb + 32 <= ep.N) {
-#pragma unroll
-                            for (int j = 0; j < 32; j += 4) {
-                                const float4 cn = *(const float4 *)(ep.colnorm + nb + j);
-                                const float cc[4] = {cn.x, cn.y, cn.z, cn.w};
-#pragma unroll
-                                for (int e = 0; e < 4; e++) {
-                                    const float d = fmaf(-2.0f, __uint_as_float(rb[j + e]), cc[e]);
-                                    if (d < bd[e]) { bd[e] = d; bn[e] = nb + j + e; }
-                                }
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; j++) {
-                                const int n = nb + j;
-                                if (n < ep.N) {
-                                    const float d = fmaf(-2.0f, __uint_as_float(rb[j]), ep.colnorm[n]);
-                                    if (d < bd[j & 3]) { bd[j & 3] = d; bn[j & 3] = n; }
-                                }
-                            }
-                        }
-                    }
-                    tmem_ld_wait();
-                }
-#pragma unroll
-                for (int e = 0; e < 4; e++)
-                    if (bd[e] < bestd || (bd[e] == bestd && bn[e] < bestn)) { bestd = bd[e]; bestn = bn[e]; }
-            } else {
-#pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 32) {
-                    uint32_t r[32];
-                    tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + c0), r);
-                    tc_epilogue_chunk(ep, r, m, n0, c0);
-                }
-            }
-            if (ep.best && m < ep.M && bestn != 0x7fffffff) {
-                unsigned u = __float_as_uint(bestd);
-                u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);           // order-preserving float -> uint
-                atomicMin(ep.best + m, ((unsigned long long)u << 32) | (unsigned)bestn);
+            for (int c0 = 0; c0 < BN; c0 += 32) {
+                uint32_t r[32];
+                tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + c0), r);
+                tc_epilogue_chunk(ep, r, m, n0, c0);
             }
             tc_fence_before();
             __syncwarp();
@@ -392,7 +315,7 @@ bool gemm_tc_supported(const GemmArgs &a) {
     int64_t ldx = a.ldx ? a.ldx : a.K, ldy = a.ldy ? a.ldy : (a.glu ? a.N / 2 : a.N);
     if (a.M <= 16 || a.N < 32 || a.K < 32) return false;           // up to 16 rows: the weight-streaming GEMV kernel
     if ((a.K & 3) || (ldx & 3)) return false;                       // TMA strides: multiples of 16 bytes
-    if (!al16(a.x) || !al16(a.W) || (!a.argmin_best && !al16(a.y)) || (a.bias && !al16(a.bias)) || (a.res && !al16(a.res))) return false;
+    if (!al16(a.x) || !al16(a.W) || !al16(a.y) || (a.bias && !al16(a.bias)) || (a.res && !al16(a.res))) return false;
     if (a.glu && ((a.N & 1) || (ldy & 1))) return false;
     return true;
 }
@@ -421,7 +344,7 @@ void gemm_tc(const GemmArgs &a) {
     ep.bias = a.bias; ep.res = a.res; ep.ldres = a.ldres ? a.ldres : a.N;
     ep.y = a.y; ep.y_lo = a.y_lo; ep.y_fmt = a.y_fmt; ep.ldy = a.ldy ? a.ldy : (a.glu ? a.N / 2 : a.N);
     ep.M = a.M; ep.N = a.N; ep.act = a.act; ep.glu = a.glu; ep.err = tc_err_flag();
-    ep.colnorm = a.argmin_colnorm; ep.best = a.argmin_best; ep.tma_store = 0;
+    ep.tma_store = 0;
     int64_t ldx = a.ldx ? a.ldx : a.K;
     const bool x3 = ctx().gemm_mode >= 2;
     if (!x3) {
@@ -570,7 +493,7 @@ extern "C" int ncmb_linear_fwd_noalloc(const float *x, const float *W, const flo
     encode_map_now(&ma, xhi, batch, K, K, TC_BM, false); encode_map_now(&mal, xlo, batch, K, K, TC_BM, true);
     encode_map_now(&mb, whi, M, K, K, 128, false); encode_map_now(&mbl, wlo, M, K, K, 128, true);
     TcEpi ep{};
-    ep.bias = b; ep.res = nullptr; ep.ldres = M; ep.y = y; ep.y_lo = nullptr; ep.y_fmt = SPLIT_TF32; ep.tma_store = 0; ep.ldy = M; ep.colnorm = nullptr; ep.best = nullptr; ep.M = batch; ep.N = M; ep.act = ACT_NONE; ep.glu = 0;
+    ep.bias = b; ep.res = nullptr; ep.ldres = M; ep.y = y; ep.y_lo = nullptr; ep.y_fmt = SPLIT_TF32; ep.tma_store = 0; ep.ldy = M; ep.M = batch; ep.N = M; ep.act = ACT_NONE; ep.glu = 0;
     ep.err = err_of[dev];
     launch_tc<128, 3, true>(a, ep, &ma, &mb, &mal, &mbl);
     return 0;

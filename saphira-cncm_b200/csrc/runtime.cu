@@ -3,6 +3,7 @@
 // B200 build: weights live in one HBM slab per file instead of one cudaMalloc per
 // tensor, and every copy goes through the library's stream.
 #include "common.cuh"
+#include "nearest.cuh"
 
 #include <algorithm>
 #include <map>
@@ -159,6 +160,7 @@ Tensor *tensor_alloc(int ndim, const int64_t *shape) {
 static void forget_copies_of(const void *p, size_t bytes) {
     gemm_h3_forget_range(p, bytes);
     gemm_tc_forget_range(p, bytes);
+    nearest_forget_range(p, bytes);
 }
 
 void tensor_free(Tensor *t) {
@@ -509,6 +511,7 @@ int weights_load(WeightStore *ws, const char *path) {
 void weights_free(WeightStore *ws) {
     if (!ws || !ws->items) return;
     gemm_tc_forget_weights();
+    nearest_forget_weights();
     gemm_h3_forget_weights();        // cached hi/lo splits point at memory that is about to go away
     cudaStreamSynchronize(stream());
     auto it = slab_of_store().find(ws->items);
@@ -659,7 +662,7 @@ int ncmb_gemm_tc_check(void) { ensure_device(); return gemm_tc_check(); }
 void ncmb_set_rng_mode(int mode) { ensure_device(); ctx().rng_mode = mode; }
 void ncmb_set_row_offset(long long off) { ctx().row_offset = off; }
 long long ncmb_launch_count(void) { return ctx().launches; }
-void ncmb_forget_weight_copies(void) { gemm_tc_forget_weights(); gemm_h3_forget_weights(); }
+void ncmb_forget_weight_copies(void) { gemm_tc_forget_weights(); gemm_h3_forget_weights(); nearest_forget_weights(); }
 int ncmb_weights_are_bf16(const WeightStore *ws) { return ws && ws->items && bf16_stores().count(ws->items) ? 1 : 0; }
 void ncmb_mem_info(unsigned long long *free_bytes, unsigned long long *total_bytes) {
     ensure_device();

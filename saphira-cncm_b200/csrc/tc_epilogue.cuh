@@ -14,7 +14,6 @@ struct TcEpi {
     float *y; float *y_lo; int64_t ldy;
     int y_fmt;                                          // SPLIT_TF32 / SPLIT_H16 when y_lo is set
     int64_t M; int N; int act; int glu;
-    const float *colnorm; unsigned long long *best;     // nearest-row mode
     int *err;
     int tma_store;                                      // fp32 result tiles leave through shared memory and TMA stores
     // per-head RMSNorm + rotary embedding of a fused QKV projection (head dim 64), see GemmArgs

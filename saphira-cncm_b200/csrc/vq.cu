@@ -4,9 +4,10 @@
 // Phi blend, argmin over a materialised [rows][V] distance matrix). Here every
 // tensor stays token-major [B][L][D] in HBM: the resampling kernels take strides,
 // so no [B][L][D] <-> [B][D][L] transposes are issued, and the nearest-code search
-// keeps a running (distance, index) minimum instead of writing distances out.
+// (nearest.cu) keeps running minima instead of writing distances out.
 #include "common.cuh"
 #include "vq.cuh"
+#include "nearest.cuh"
 
 namespace ncmb {
 
@@ -23,118 +24,6 @@ __global__ void k_gather_codes(const float *__restrict__ E, const int *__restric
 }
 __global__ void k_sub_inplace(float *__restrict__ y, const float *__restrict__ x, int64_t n) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) y[i] -= x[i];
-}
-
-// ---- nearest code: argmin_j |x_r - E_j|^2, strict < so the lowest index wins ties
-// (reference src/vq.c:440-441). 16 rows per CTA; the codebook streams through shared
-// memory in 128-code tiles; thread j of a tile owns code j for all 16 rows. ----
-constexpr int NR_ROWS = 16, NR_TILE = 128;
-__global__ void __launch_bounds__(NR_TILE) k_nearest(const float *__restrict__ x, const float *__restrict__ E,
-                                                     int64_t rows, int V, int D, int *__restrict__ idx_out,
-                                                     int out_tlen, int out_stride, int out_off) {
-    extern __shared__ float sm[];
-    float *xs = sm;                         // [NR_ROWS][D]
-    float *es = xs + NR_ROWS * D;           // [NR_TILE][D + 1]
-    const int tid = threadIdx.x;
-    const int64_t r0 = (int64_t)blockIdx.x * NR_ROWS;
-    for (int i = tid; i < NR_ROWS * D; i += NR_TILE) {
-        int64_t r = r0 + i / D;
-        xs[i] = r < rows ? x[r * D + (i % D)] : 0.f;
-    }
-    float best[NR_ROWS]; int bi[NR_ROWS];
-#pragma unroll
-    for (int r = 0; r < NR_ROWS; r++) { best[r] = INFINITY; bi[r] = 0x7fffffff; }
-    for (int j0 = 0; j0 < V; j0 += NR_TILE) {
-        __syncthreads();
-        for (int i = tid; i < NR_TILE * D; i += NR_TILE) {
-            int j = i / D, c = i % D;
-            es[j * (D + 1) + c] = (j0 + j < V) ? E[(int64_t)(j0 + j) * D + c] : 0.f;
-        }
-        __syncthreads();
-        int j = j0 + tid;
-        if (j < V) {
-            float acc[NR_ROWS];
-#pragma unroll
-            for (int r = 0; r < NR_ROWS; r++) acc[r] = 0.f;
-            const float *er = es + tid * (D + 1);
-            for (int c = 0; c < D; c++) {
-                float e = er[c];
-#pragma unroll
-                for (int r = 0; r < NR_ROWS; r++) { float d = xs[r * D + c] - e; acc[r] = fmaf(d, d, acc[r]); }
-            }
-#pragma unroll
-            for (int r = 0; r < NR_ROWS; r++) if (acc[r] < best[r]) { best[r] = acc[r]; bi[r] = j; }
-        }
-    }
-    __syncthreads();                         // the code tile is dead: reuse it for the cross-thread reduction
-    float *bval = es;                        // [NR_ROWS][NR_TILE]
-    int *bidx = (int *)(es + NR_ROWS * NR_TILE);
-#pragma unroll
-    for (int r = 0; r < NR_ROWS; r++) { bval[r * NR_TILE + tid] = best[r]; bidx[r * NR_TILE + tid] = bi[r]; }
-    __syncthreads();
-    if (tid < NR_ROWS) {
-        int64_t r = r0 + tid;
-        if (r < rows) {
-            float bv = INFINITY; int bj = 0x7fffffff;
-            for (int t = 0; t < NR_TILE; t++) {
-                float v = bval[tid * NR_TILE + t]; int j = bidx[tid * NR_TILE + t];
-                if (v < bv || (v == bv && j < bj)) { bv = v; bj = j; }
-            }
-            if (bj == 0x7fffffff) bj = 0;
-            int64_t b = r / out_tlen; int t = (int)(r % out_tlen);
-            idx_out[b * out_stride + out_off + t] = bj;
-        }
-    }
-}
-
-// ---- tensor-core route: |x - e|^2 = |x|^2 - 2 x.e + |e|^2, and |x|^2 does not change the argmin, so
-// the search is a [rows x V x D] GEMM whose epilogue keeps min_n(|e_n|^2 - 2 x.e_n) per row and never
-// writes the products. Three-pass TF32 keeps the dot products fp32-grade. ----
-__global__ void k_row_sqnorm(const float *__restrict__ E, int V, int D, float *__restrict__ out) {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= V) return;
-    float s = 0.f;
-    for (int c = 0; c < D; c++) { float e = E[(int64_t)v * D + c]; s = fmaf(e, e, s); }
-    out[v] = s;
-}
-__global__ void k_unpack_best(const unsigned long long *__restrict__ best, int64_t rows, int *__restrict__ idx_out,
-                              int out_tlen, int out_stride, int out_off) {
-    int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    int64_t b = r / out_tlen; int t = (int)(r % out_tlen);
-    idx_out[b * out_stride + out_off + t] = (int)(best[r] & 0xffffffffull);
-}
-
-static bool vq_nearest_tc(const float *x, const float *E, int64_t rows, int V, int D, int *idx_out, int out_tlen, int out_stride, int out_off) {
-    static Workspace ws;
-    GemmArgs g;
-    g.x = x; g.ldx = D; g.W = E; g.M = rows; g.N = V; g.K = D;
-    size_t need = (size_t)rows * 8 + (size_t)V * 4 + 1024;
-    if (need > ws.cap) ws.reserve(need + need / 4);
-    ws.reset();
-    unsigned long long *best = ws.get<unsigned long long>(rows);
-    float *cn = ws.get<float>(V);
-    g.argmin_best = best; g.argmin_colnorm = cn;
-    if (ctx().gemm_mode < 1 || !gemm_tc_supported(g)) return false;
-    CUDA_CHECK(cudaMemsetAsync(best, 0xff, (size_t)rows * 8, stream()));
-    LAUNCH(k_row_sqnorm, (unsigned)cdiv(V, 128), 128, 0, E, V, D, cn);
-    {
-        StaticWeights sw;                       // codebooks are model weights: cache their hi / lo split
-        gemm_tc(g);
-    }
-    LAUNCH(k_unpack_best, (unsigned)cdiv(rows, 256), 256, 0, best, rows, idx_out, out_tlen, out_stride, out_off);
-    return true;
-}
-
-void vq_nearest(const float *x, const float *E, int64_t rows, int V, int D, int *idx_out, int out_tlen, int out_stride, int out_off) {
-    if (rows <= 0) return;
-    if (rows >= 1024 && vq_nearest_tc(x, E, rows, V, D, idx_out, out_tlen, out_stride, out_off)) return;
-    size_t es_fl = (size_t)NR_TILE * (D + 1);
-    if (es_fl < 2 * (size_t)NR_ROWS * NR_TILE) es_fl = 2 * (size_t)NR_ROWS * NR_TILE;
-    size_t smem = sizeof(float) * ((size_t)NR_ROWS * D + es_fl);
-    if (smem > 48 * 1024) fatal("vq_nearest: D=%d too large for this kernel", D);
-    ProfScope ps(NCMB_K_VQ, 3.0 * (double)rows * V * D, 4.0 * (double)rows * (D + 1));
-    LAUNCH(k_nearest, grid1d(rows, NR_ROWS), NR_TILE, smem, x, E, rows, V, D, idx_out, out_tlen, out_stride, out_off);
 }
 
 static unsigned ew(int64_t n) {
@@ -255,7 +144,7 @@ void vq_encode_dev(VQState *v, const float *z, int B, int *idx_dev, float *scrat
     for (int lv = 0; lv < v->n_levels; lv++) {
         int tlen = v->levels[lv];
         down_for_quant_dev(v, z_rest, B, L, lv, down, scratch, scratch + n);
-        vq_nearest(down, v->E[lv], (int64_t)B * tlen, v->vocabs[lv], D, idx_dev, tlen, total, off);
+        nearest_codes(down, v->E[lv], (int64_t)B * tlen, v->vocabs[lv], D, idx_dev, tlen, total, off);
         if (lv + 1 < v->n_levels) {
             vq_increment_dev(v, idx_dev + off, total, 0, lv, B, up, scratch);
             ProfScope ps(NCMB_K_VQ);
@@ -412,7 +301,7 @@ void ncmb_vq_encode_dev(VQState *vq, const float *z_dev, int B, int *idx_dev) {
 }
 void ncmb_vq_nearest_dev(VQState *vq, int level, const float *x_dev, long long n, int *idx_dev) {
     ensure_device();
-    vq_nearest(x_dev, vq->E[level], n, vq->vocabs[level], vq->D, idx_dev, 1, 1, 0);
+    nearest_codes(x_dev, vq->E[level], n, vq->vocabs[level], vq->D, idx_dev, 1, 1, 0);
 }
 
 } // extern "C"

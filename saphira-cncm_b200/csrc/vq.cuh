@@ -23,6 +23,5 @@ void vq_increment_dev(VQState *v, const int *codes_dev, int stride, int rowmod, 
 void vq_next_input_dev(VQState *v, const int *codes_dev, int stride, int rowmod, int level, float *z_hat, float *x_out, int B, float *scratch /*5n*/);
 void vq_encode_dev(VQState *v, const float *z, int B, int *idx_dev, float *scratch /*7n*/);
 void vq_zhat_final_dev(VQState *v, const int *idx_dev, int B, float *z_hat, float **snapshots, float *scratch /*5n*/);
-void vq_nearest(const float *x, const float *E, int64_t rows, int V, int D, int *idx_out, int out_tlen, int out_stride, int out_off);
 int *vq_codes_to_dev(VQState *v, const int *host, size_t n);
 } // namespace ncmb
