@@ -22,8 +22,69 @@ __global__ void k_gather_codes(const float *__restrict__ E, const int *__restric
         out[i] = E[(int64_t)code * D + d];
     }
 }
-__global__ void k_sub_inplace(float *__restrict__ y, const float *__restrict__ x, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) y[i] -= x[i];
+__global__ void k_axpy_inplace(float *__restrict__ y, const float *__restrict__ x, float a, int64_t n) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) y[i] = __fadd_rn(y[i], a * x[i]);
+}
+
+// One level's contribution in one pass over z: dst = src + sign * up, and next = the mean of dst over the L / tnext positions of
+// each step of the next level (its quantizer input), where up is the level's codes brought to length L by linear interpolation
+// (align_corners = False; constant when the level has one step), or read from `up_in`. Four channels per thread; src == null is
+// zero. One read and one write of z (memory bound) where gather, interpolation, update and mean were passes of their own.
+struct LevelStep {
+    const float *E; const int *codes; int stride, rowmod, tlen, V;
+    const float *up_in, *src; float *dst, *next;
+    float sign; int L, D, tnext; int64_t n4;                 // n4 = B * tnext * D / 4 threads
+};
+__global__ void __launch_bounds__(256) k_level_step(LevelStep a) {
+    extern __shared__ double ls_tab[];                       // [L] weights of the lower step, then [L] lower and upper steps
+    int *i0 = (int *)(ls_tab + a.L), *i1 = i0 + a.L;
+    const bool flat = a.tlen == 1 || a.L == 1;               // the mean of the level's steps, at every position
+    if (!a.up_in && !flat) {
+        for (int t = threadIdx.x; t < a.L; t += blockDim.x) {
+            const double src = (t + 0.5) * ((double)a.tlen / a.L) - 0.5;
+            const int s0 = (int)floor(src);
+            ls_tab[t] = src - s0;
+            i0[t] = s0 < 0 ? 0 : (s0 >= a.tlen ? a.tlen - 1 : s0);
+            i1[t] = s0 + 1 < 0 ? 0 : (s0 + 1 >= a.tlen ? a.tlen - 1 : s0 + 1);
+        }
+        __syncthreads();
+    }
+    const int D4 = a.D >> 2, w = a.L / a.tnext;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n4; i += (int64_t)gridDim.x * blockDim.x) {
+        const int d = (int)(i % D4) * 4; const int64_t bt = i / D4; const int tn = (int)(bt % a.tnext); const int64_t b = bt / a.tnext;
+        const int *cb = a.codes + (a.rowmod > 0 ? b % a.rowmod : b) * a.stride;
+        auto code_row = [&](int j) {
+            int c = cb[j];
+            c = c < 0 ? 0 : (c >= a.V ? a.V - 1 : c);
+            return *(const float4 *)(a.E + (int64_t)c * a.D + d);
+        };
+        float4 one = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!a.up_in && flat) {
+            for (int j = 0; j < a.tlen; j++) { const float4 v = code_row(j); one.x += v.x; one.y += v.y; one.z += v.z; one.w += v.w; }
+            const float c = (float)a.tlen;
+            one = make_float4(one.x / c, one.y / c, one.z / c, one.w / c);
+        }
+        float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int t = tn * w; t < (tn + 1) * w; t++) {
+            const int64_t at = (b * a.L + t) * a.D + d;
+            float4 u = one;
+            if (a.up_in) u = *(const float4 *)(a.up_in + at);
+            else if (!flat) {
+                const double w1 = ls_tab[t], w0 = 1.0 - w1;
+                const float4 p = code_row(i0[t]), q = code_row(i1[t]);
+                u.x = (float)(w0 * (double)p.x + w1 * (double)q.x); u.y = (float)(w0 * (double)p.y + w1 * (double)q.y);
+                u.z = (float)(w0 * (double)p.z + w1 * (double)q.z); u.w = (float)(w0 * (double)p.w + w1 * (double)q.w);
+            }
+            float4 z = a.src ? *(const float4 *)(a.src + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+            z.x = __fadd_rn(z.x, a.sign * u.x); z.y = __fadd_rn(z.y, a.sign * u.y); z.z = __fadd_rn(z.z, a.sign * u.z); z.w = __fadd_rn(z.w, a.sign * u.w);
+            *(float4 *)(a.dst + at) = z;
+            m.x += z.x; m.y += z.y; m.z += z.z; m.w += z.w;
+        }
+        if (a.next) {
+            const float c = (float)w;
+            *(float4 *)(a.next + (b * a.tnext + tn) * a.D + d) = make_float4(m.x / c, m.y / c, m.z / c, m.w / c);
+        }
+    }
 }
 
 static unsigned ew(int64_t n) {
@@ -90,10 +151,12 @@ static void down_for_quant_dev(VQState *v, const float *z, int B, int Lin, int l
     } else {
         interp_area(z, nlc(D, Lin), out, nlc(D, tlen), B, D, Lin, tlen);
     }
-    if (v->has_all && level >= 1 && level <= v->n_levels - 2 && v->drefW[level]) {
-        conv1d(out, nlc(D, tlen), v->drefW[level], v->drefB[level], tmp1, nlc(D, tlen), B, D, D, tlen, 3, 1, 1, out, 0.f);
-        CUDA_CHECK(cudaMemcpyAsync(out, tmp1, (size_t)B * tlen * D * 4, cudaMemcpyDeviceToDevice, stream()));
-    }
+}
+// the refining convolution of an inner level's quantizer input
+static void down_refine_dev(VQState *v, int level, int B, float *out, float *tmp1) {
+    int D = v->D, tlen = v->levels[level];
+    conv1d(out, nlc(D, tlen), v->drefW[level], v->drefB[level], tmp1, nlc(D, tlen), B, D, D, tlen, 3, 1, 1, out, 0.f);
+    CUDA_CHECK(cudaMemcpyAsync(out, tmp1, (size_t)B * tlen * D * 4, cudaMemcpyDeviceToDevice, stream()));
 }
 
 static int phi_index(const VQState *v, int level) {       // reference src/vq.c:212-221
@@ -127,28 +190,59 @@ void vq_increment_dev(VQState *v, const int *codes_dev, int stride, int rowmod, 
 
 size_t vq_scratch_floats(const VQState *v, int B) { return 4 * (size_t)B * v->L * v->D + 64; }
 
+// dst = src + sign * (level's increment), next (optional) = dst at the length of the next level. `up` (B*L*D floats) and
+// scratch (4 x that) are used by the increments that are not a plain interpolation of the codes.
+static void level_step(VQState *v, const int *codes, int stride, int rowmod, int level, int B, const float *src, float *dst, float sign,
+                       int tnext, float *next, float *up, float *scratch) {
+    const int D = v->D, L = v->L;
+    const bool refined = v->has_all && level >= 1 && level <= v->n_levels - 2 && v->urefW[level];
+    const bool plain = !(level == 0 && v->has_l1) && !v->resi && !refined && D % 4 == 0;
+    if (!plain) vq_increment_dev(v, codes, stride, rowmod, level, B, up, scratch);
+    const bool tiles = next && L % tnext == 0;
+    if (D % 4) {                                              // rows that are not whole float4s: one pass per operation
+        const size_t n = (size_t)B * L * D;
+        if (src != dst) {
+            if (src) CUDA_CHECK(cudaMemcpyAsync(dst, src, n * 4, cudaMemcpyDeviceToDevice, stream()));
+            else CUDA_CHECK(cudaMemsetAsync(dst, 0, n * 4, stream()));
+        }
+        ProfScope ps(NCMB_K_VQ);
+        LAUNCH(k_axpy_inplace, ew((int64_t)n), 256, 0, dst, up, sign, (int64_t)n);
+    } else {
+        LevelStep a{};
+        a.E = v->E[level]; a.codes = codes; a.stride = stride; a.rowmod = rowmod; a.tlen = v->levels[level]; a.V = v->vocabs[level];
+        a.up_in = plain ? nullptr : up; a.src = src; a.dst = dst; a.next = tiles ? next : nullptr;
+        a.sign = sign; a.L = L; a.D = D; a.tnext = tiles ? tnext : L; a.n4 = (int64_t)B * a.tnext * (D / 4);
+        ProfScope ps(NCMB_K_VQ);
+        LAUNCH(k_level_step, ew(a.n4), 256, (size_t)L * 16, a);
+        if (tiles) return;
+    }
+    if (next) interp_area(dst, nlc(D, L), next, nlc(D, tnext), B, D, L, tnext);
+}
+
 void vq_next_input_dev(VQState *v, const int *codes_dev, int stride, int rowmod, int level, float *z_hat, float *x_out, int B, float *scratch) {
-    size_t n = (size_t)B * v->L * v->D;
-    float *up = scratch + 4 * n;           // caller provides 5n floats
-    vq_increment_dev(v, codes_dev, stride, rowmod, level, B, up, scratch);
-    add_inplace(z_hat, up, (int64_t)n);
-    interp_area(z_hat, nlc(v->D, v->L), x_out, nlc(v->D, v->levels[level + 1]), B, v->D, v->L, v->levels[level + 1]);
+    float *up = scratch + 4 * (size_t)B * v->L * v->D;        // caller provides 5n floats
+    level_step(v, codes_dev, stride, rowmod, level, B, z_hat, z_hat, 1.0f, v->levels[level + 1], x_out, up, scratch);
 }
 
 void vq_encode_dev(VQState *v, const float *z, int B, int *idx_dev, float *scratch) {
-    int D = v->D, L = v->L, total = vq_total_codes(v);
-    size_t n = (size_t)B * L * D;
+    const int D = v->D, L = v->L, total = vq_total_codes(v);
+    const size_t n = (size_t)B * L * D;
     float *z_rest = scratch + 5 * n, *down = scratch + 6 * n, *up = scratch + 4 * n;   // caller provides 7n floats
-    CUDA_CHECK(cudaMemcpyAsync(z_rest, z, n * 4, cudaMemcpyDeviceToDevice, stream()));
+    const float *cur = z;
     int off = 0;
     for (int lv = 0; lv < v->n_levels; lv++) {
-        int tlen = v->levels[lv];
-        down_for_quant_dev(v, z_rest, B, L, lv, down, scratch, scratch + n);
-        nearest_codes(down, v->E[lv], (int64_t)B * tlen, v->vocabs[lv], D, idx_dev, tlen, total, off);
+        const int tlen = v->levels[lv];
+        const bool refined = v->has_all && lv >= 1 && lv <= v->n_levels - 2 && v->drefW[lv];
+        const float *q = down;
+        if (lv == 0) down_for_quant_dev(v, cur, B, L, lv, down, scratch, scratch + n);
+        else if (refined) down_refine_dev(v, lv, B, down, scratch);
+        else if (tlen == L) q = cur;                          // the mean over one position is the position
+        nearest_codes(q, v->E[lv], (int64_t)B * tlen, v->vocabs[lv], D, idx_dev, tlen, total, off);
         if (lv + 1 < v->n_levels) {
-            vq_increment_dev(v, idx_dev + off, total, 0, lv, B, up, scratch);
-            ProfScope ps(NCMB_K_VQ);
-            LAUNCH(k_sub_inplace, ew((int64_t)n), 256, 0, z_rest, up, (int64_t)n);
+            const int tn = v->levels[lv + 1];
+            const bool next_refined = v->has_all && lv + 1 <= v->n_levels - 2 && v->drefW[lv + 1];
+            level_step(v, idx_dev + off, total, 0, lv, B, cur, z_rest, -1.0f, tn, tn == L && !next_refined ? nullptr : down, up, scratch);
+            cur = z_rest;
         }
         off += tlen;
     }
@@ -158,11 +252,9 @@ void vq_zhat_final_dev(VQState *v, const int *idx_dev, int B, float *z_hat, floa
     int total = vq_total_codes(v);
     size_t n = (size_t)B * v->L * v->D;
     float *up = scratch + 4 * n;
-    CUDA_CHECK(cudaMemsetAsync(z_hat, 0, n * 4, stream()));
     int base = 0;
     for (int lv = 0; lv < v->n_levels; lv++) {
-        vq_increment_dev(v, idx_dev + base, total, 0, lv, B, up, scratch);
-        add_inplace(z_hat, up, (int64_t)n);
+        level_step(v, idx_dev + base, total, 0, lv, B, lv ? z_hat : nullptr, z_hat, 1.0f, v->L, nullptr, up, scratch);
         if (snapshots && snapshots[lv] && snapshots[lv] != z_hat)
             CUDA_CHECK(cudaMemcpyAsync(snapshots[lv], z_hat, n * 4, cudaMemcpyDeviceToDevice, stream()));
         base += v->levels[lv];
@@ -283,13 +375,10 @@ void vq_idx_to_ncm_input(VQState *vq, const int *idx, int B, float *x_out) {
     int *cd = vq_codes_to_dev(vq, idx, (size_t)B * total);
     float *scr = vq_scratch(vq, B, 7);
     float *up = scr + 4 * n, *z_hat = scr + 5 * n, *chunk = scr + 6 * n;
-    CUDA_CHECK(cudaMemsetAsync(z_hat, 0, n * 4, stream()));
     int base = 0, off = 0;
     for (int li = 0; li < vq->n_levels - 1; li++) {
         int nlen = vq->levels[li + 1];
-        vq_increment_dev(vq, cd + base, total, 0, li, B, up, scr);
-        add_inplace(z_hat, up, (int64_t)n);
-        interp_area(z_hat, nlc(D, L), chunk, nlc(D, nlen), B, D, L, nlen);
+        level_step(vq, cd + base, total, 0, li, B, li ? z_hat : nullptr, z_hat, 1.0f, nlen, chunk, up, scr);
         CUDA_CHECK(cudaMemcpy2DAsync(x_out + (size_t)off * D, (size_t)T * D * 4, chunk, (size_t)nlen * D * 4,
                                      (size_t)nlen * D * 4, B, cudaMemcpyDeviceToDevice, stream()));
         base += vq->levels[li]; off += nlen;
