@@ -4,6 +4,7 @@
 #include "common.cuh"
 #include "vq.cuh"
 #include "vqvae.cuh"
+#include "vae_fused.cuh"
 
 namespace ncmb {
 
@@ -78,10 +79,16 @@ void vqvae_decode_dev(VQVAEState *v, const float *zhat, float *logits, int B) {
     v->work.reset();
     float *x = v->work.get<float>(n * D);
     BlockBufs bufs = vae_bufs(v->work, n, D, Hh);
-    CUDA_CHECK(cudaMemcpyAsync(x, zhat, (size_t)n * D * 4, cudaMemcpyDeviceToDevice, stream()));
-    if (c->dec_positional) add_rows_bcast(x, v->dec_wpe, B, T * D);
-    for (auto &w : v->dec) vae_run_block(v, w, x, B, T, 0, bufs);
-    layernorm(x, v->dec_lnf, nullptr, bufs.ln, n, D, 1e-6f);
+    if (vae_stack_supported(v->dec, D, c->vq_n_layers, T, 0)) {
+        VaeStackIO io;
+        io.x = zhat; io.wpe = c->dec_positional ? v->dec_wpe : nullptr; io.lnf = v->dec_lnf; io.y = bufs.ln;
+        vae_stack(v->dec, c->vq_n_layers, B, T, io);
+    } else {
+        CUDA_CHECK(cudaMemcpyAsync(x, zhat, (size_t)n * D * 4, cudaMemcpyDeviceToDevice, stream()));
+        if (c->dec_positional) add_rows_bcast(x, v->dec_wpe, B, T * D);
+        for (auto &w : v->dec) vae_run_block(v, w, x, B, T, 0, bufs);
+        layernorm(x, v->dec_lnf, nullptr, bufs.ln, n, D, 1e-6f);
+    }
     GemmArgs g;
     g.x = bufs.ln; g.ldx = D; g.W = v->dec_out; g.y = logits; g.ldy = V; g.M = n; g.N = V; g.K = D;
     gemm(g);
@@ -98,6 +105,13 @@ void decode_tokens_dev(VQVAEState *v, const int *codes_dev, int B, int *tokens_d
     float *zh = v->dec_ws.get<float>(n);
     float *lg = v->dec_ws.get<float>((size_t)B * L * Vp);
     vq_zhat_final_dev(vq, codes_dev, B, zh, nullptr, scr);
+    const NCMConfig *c = &v->cfg;
+    if (Vp <= 64 && c->vq_compression <= 1 && c->vq_context_length == L && vae_stack_supported(v->dec, D, c->vq_n_layers, L, 0)) {
+        VaeStackIO io;                                         // a small vocabulary is decided inside the same kernel
+        io.x = zh; io.wpe = c->dec_positional ? v->dec_wpe : nullptr; io.lnf = v->dec_lnf; io.out_w = v->dec_out; io.V = Vp; io.tok = tokens_dev;
+        vae_stack(v->dec, c->vq_n_layers, B, L, io);
+        return;
+    }
     vqvae_decode_dev(v, zh, lg, B);
     argmax_rows(lg, (int64_t)B * L, Vp, tokens_dev);
 }
@@ -171,6 +185,13 @@ void vqvae_encode_z(VQVAEState *v, const int *ids, float *z, int B) {
     float *t1 = v->work.get<float>(n * D), *t2 = v->work.get<float>(n * D);
     BlockBufs bufs = vae_bufs(v->work, n, D, Hh);
     upload(ids_dev, ids, (size_t)n * sizeof(int));
+    if (c->enc_conv_layers == 0 && c->vq_compression <= 1 && c->pre_quant_groupnorm <= 0 && vae_stack_supported(v->enc, D, c->vq_n_layers, T, c->enc_attn_window)) {
+        VaeStackIO io;
+        io.ids = ids_dev; io.wte = v->enc_wte; io.wpe = c->enc_positional ? v->enc_wpe : nullptr; io.y = z;
+        io.lnf = wneed(ws, "tok.encoder.ln_e.weight")->data;
+        vae_stack(v->enc, c->vq_n_layers, B, T, io);
+        return;
+    }
     embed_rows(v->enc_wte, ids_dev, x, n, D);
     if (c->enc_positional) add_rows_bcast(x, v->enc_wpe, B, T * D);
     for (int i = 0; i < c->enc_conv_layers; i++) {
