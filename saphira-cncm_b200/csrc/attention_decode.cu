@@ -32,7 +32,6 @@ struct AttnDecDev {
     const int *q_start, *k_start, *k_len;
     const int *step_d; int64_t len_step;
     int H, Hkv, max_split, cps;
-    int hs;                            // warp-per-chunk kernel: warps that share a chunk's (query, head) pairs
     float scale;
     float *part; unsigned *count;
 };
@@ -254,113 +253,153 @@ __global__ void __launch_bounds__(AD_THREADS) k_attention_decode(AttnDecDev a) {
     if (tid == 0) a.count[row * a.Hkv + kvh] = 0;          // ready for the next launch
 }
 
-// ---- head dim 64: one WARP per (32-key chunk, group of heads) ----
-// The kernel above gives every 32-key chunk a CTA, three block-wide barriers per chunk, and merges all chunk
-// partials of a row through global memory; at one sequence that chain of barriers and L2 round trips is the kernel
-// (16 us per layer for 800 cached keys of the 14-query-head / 2-kv-head shape). Here a warp works alone on 32 keys
-// and up to GMW of the kv group's (query, head) pairs: the lane holding key j forms that key's scores (q broadcast
-// from shared memory), the softmax statistics of the chunk are warp shuffles, and for O += P V the lanes switch to
-// owning two output dimensions each while the probabilities travel by shuffle -- K and V rows are requested
-// before anything is computed and no barrier is needed until the warps' partials (maximum, sum, context) meet in
-// shared memory. A kv group with more pairs than one warp takes is shared out over `hs` warps per chunk (they read
-// the same K and V rows, out of L1), so a warp's arithmetic stays short. A CTA covers `blockDim / 32 / hs` chunks;
-// one partial per CTA goes to global memory, and only when the row needs more than one CTA.
-constexpr int ADW_MAXC = 8;            // chunks per CTA at most
+// ---- head dim 64, up to eight (query, head) pairs per kv head: lanes share keys, loads straight to registers ----
+// Eight lanes hold a key: lane (kg, dp) keeps dims 4 dp .. and 32 + 4 dp .. of key kg of a group of four, so a warp's load of
+// four keys (or values) is eight full 128-byte lines, and the same lane needs the same dims of the query (in registers for
+// all GM pairs) and of the context (accumulated in registers). The eight partial dot products of a key meet by a
+// reduce-scatter that leaves pair dp's score in lane dp (seven shuffles for eight pairs instead of twenty-four), the softmax
+// runs on those, and the probabilities travel back by one shuffle per pair and key. Nothing goes through shared memory until a
+// warp's keys are done. A warp takes runs of 16 keys: the values of a run and the keys of the next are requested before the
+// run's arithmetic. The warps of a CTA interleave runs; a row is cut over CTAs only while there are too few (row, kv head)
+// pairs to fill the GPU, and the last CTA of a pair to finish merges.
+//
+// Bound: the K|V cache read once. Per key and kv head about 35 warp instructions at eight pairs.
+constexpr int ADG_RUN = 16;            // keys of a run: four groups of four
+constexpr int ADG_MAXW = 8;            // warps of a CTA at most
 
-template <int GMW>
-__global__ void __launch_bounds__(256) k_attention_dec_warp(AttnDecDev a) {
-    constexpr int HD = 64, GA = AD_MAXG;
-    __shared__ __align__(16) float qs[GA][HD];
-    __shared__ float pm[ADW_MAXC][GA], pl[ADW_MAXC][GA], wg[ADW_MAXC][GA];
-    __shared__ __align__(8) float po[ADW_MAXC][GA][HD];
-    __shared__ float Mg[GA], Lg[GA];
+template <int GM>
+__global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a) {
+    constexpr int HD = 64, NI = ADG_RUN / 4;
+    constexpr int HSH = GM == 8 ? 0 : GM == 4 ? 1 : GM == 2 ? 2 : 3;          // lane dp holds pair dp >> HSH after the reduction
+    __shared__ float pm[ADG_MAXW][GM], pl[ADG_MAXW][GM], wg[ADG_MAXW][GM];
+    __shared__ __align__(16) float po[ADG_MAXW][GM][HD];
+    __shared__ float Mg[GM], Lg[GM];
     __shared__ int s_last;
     const int row = blockIdx.z, kvh = blockIdx.y, sp = blockIdx.x;
     const int Gh = a.H / a.Hkv;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int hs = a.hs, cpc = (blockDim.x >> 5) / hs;        // warps per chunk, chunks per CTA
-    const int cw = warp / hs, hg = warp - cw * hs;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int kg = lane >> 3, dp = lane & 7;
     pdl_launch_dependents();
     pdl_wait();
     const int *lens = a.k_len ? a.k_len + (a.step_d ? (int64_t)(*a.step_d) * a.len_step : 0) : nullptr;
     const int k00 = a.k_start[row], n1s = lens ? lens[row] : a.k_start[row + 1] - k00;
     const int k20 = a.k2_start ? a.k2_start[row] : 0, n2s = a.k2_start ? a.k2_start[row + 1] - k20 : 0;
     const int n1 = n1s + n2s;
-    const int per_cta = cpc * 32;
-    const int nsplit = (n1 + per_cta - 1) / per_cta;
+    const int per_cta = a.cps * nw * ADG_RUN;                                 // keys a CTA takes
+    const int nsplit = max(1, (n1 + per_cta - 1) / per_cta);
     if (sp >= nsplit) return;
-    const int kw = sp * per_cta + cw * 32;                    // first key of this warp's chunk
     const int q0 = a.q_start[row], nq = a.q_start[row + 1] - q0;
-    const int G = Gh * nq;                                    // virtual heads: vh = g * nq + qi
-    const int g0 = hg * GMW;                                  // this warp's heads: [g0, g0 + GMW) below G
-    auto krow = [&](int j) -> const float * {
-        return j < n1s ? a.k + (int64_t)(k00 + j) * a.ldk : a.k2 + (int64_t)(k20 + j - n1s) * a.ldk2;
-    };
-    auto vrow = [&](int j) -> const float * {
-        return j < n1s ? a.v + (int64_t)(k00 + j) * a.ldk : a.v2 + (int64_t)(k20 + j - n1s) * a.ldk2;
-    };
-    for (int i = tid; i < G * HD; i += blockDim.x) {
-        const int vh = i / HD, d = i % HD;
-        qs[vh][d] = a.q[(int64_t)(q0 + vh % nq) * a.ldq + (kvh * Gh + vh / nq) * HD + d];
+    const int G = Gh * nq;                                                    // virtual heads: vh = g * nq + qi
+    const int first = sp * per_cta + warp * ADG_RUN, step = nw * ADG_RUN, last = min(n1, (sp + 1) * per_cta);
+    float q[GM][8];
+#pragma unroll
+    for (int g = 0; g < GM; g++) {
+        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+        if (g < G) {
+            const float *qp = a.q + (int64_t)(q0 + g % nq) * a.ldq + (kvh * Gh + g / nq) * HD + 4 * dp;
+            lo = *(const float4 *)qp; hi = *(const float4 *)(qp + 32);
+        }
+        q[g][0] = lo.x * a.scale; q[g][1] = lo.y * a.scale; q[g][2] = lo.z * a.scale; q[g][3] = lo.w * a.scale;
+        q[g][4] = hi.x * a.scale; q[g][5] = hi.y * a.scale; q[g][6] = hi.z * a.scale; q[g][7] = hi.w * a.scale;
     }
-    // every load of the chunk is requested now: the lane's key row, and for the context step the two dimensions
-    // (2 lane, 2 lane + 1) of all 32 value rows
-    const bool valid = kw + lane < n1;
-    float4 kr[HD / 4];
-    {
-        const float4 *kp = (const float4 *)(krow(valid ? kw + lane : 0) + kvh * HD);
+    float4 kf[NI][2], vf[NI][2];
+    auto load = [&](float4 (&f)[NI][2], const float *s1, int64_t ld1, const float *s2, int64_t ld2, int j0) {
 #pragma unroll
-        for (int i = 0; i < HD / 4; i++) kr[i] = valid ? kp[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    float2 vv[32];
+        for (int i = 0; i < NI; i++) {
+            const int j = j0 + 4 * i + kg;
+            if (j < last) {
+                const float *p = (j < n1s ? s1 + (int64_t)(k00 + j) * ld1 : s2 + (int64_t)(k20 + j - n1s) * ld2) + kvh * HD + 4 * dp;
+                f[i][0] = *(const float4 *)p; f[i][1] = *(const float4 *)(p + 32);
+            } else f[i][0] = f[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    float acc[GM][8], m = -INFINITY, l = 0.f;
 #pragma unroll
-    for (int jj = 0; jj < 32; jj++)
-        vv[jj] = (kw + jj < n1) ? *(const float2 *)(vrow(kw + jj) + kvh * HD + 2 * lane) : make_float2(0.f, 0.f);
-    __syncthreads();
-    float s[GMW];
+    for (int g = 0; g < GM; g++)
 #pragma unroll
-    for (int gi = 0; gi < GMW; gi++) {
-        s[gi] = 0.f;
-        const int g = g0 + gi;
-        if (g < G) {                                          // warp-uniform
-            float dot = 0.f;
+        for (int d = 0; d < 8; d++) acc[g][d] = 0.f;
+    if (first < last) load(kf, a.k, a.ldk, a.k2, a.ldk2, first);
+    for (int j0 = first; j0 < last; j0 += step) {
+        load(vf, a.v, a.ldk, a.v2, a.ldk2, j0);
+        float s[NI];
 #pragma unroll
-            for (int i = 0; i < HD / 4; i++) {
-                const float4 t = *(const float4 *)&qs[g][4 * i];   // one address for the whole warp: a broadcast
-                dot = fmaf(kr[i].x, t.x, dot); dot = fmaf(kr[i].y, t.y, dot); dot = fmaf(kr[i].z, t.z, dot); dot = fmaf(kr[i].w, t.w, dot);
+        for (int i = 0; i < NI; i++) {
+            const float4 c0 = kf[i][0], c1 = kf[i][1];
+            float v[GM];
+#pragma unroll
+            for (int g = 0; g < GM; g++) {
+                float t = q[g][0] * c0.x;
+                t = fmaf(q[g][1], c0.y, t); t = fmaf(q[g][2], c0.z, t); t = fmaf(q[g][3], c0.w, t);
+                t = fmaf(q[g][4], c1.x, t); t = fmaf(q[g][5], c1.y, t); t = fmaf(q[g][6], c1.z, t); t = fmaf(q[g][7], c1.w, t);
+                v[g] = t;
             }
-            const float sc = valid ? dot * a.scale : -INFINITY;
-            float m = sc;
+            int o = 4;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            const float p = (sc == -INFINITY) ? 0.f : expf(sc - m);
-            float l = p;
+            for (int w = GM / 2; w > 0; w >>= 1, o >>= 1) {                   // halve the pairs a lane keeps
+                const bool up = (dp & o) != 0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-            s[gi] = p;
-            if (lane == 0) { pm[cw][g] = m; pl[cw][g] = l; }
+                for (int g = 0; g < w; g++) {
+                    const float give = up ? v[g] : v[g + w], keep = up ? v[g + w] : v[g];
+                    v[g] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            }
+            for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            s[i] = (j0 + 4 * i + kg < last) ? v[0] : -INFINITY;
+        }
+        if (j0 + step < last) load(kf, a.k, a.ldk, a.k2, a.ldk2, j0 + step);
+        float mx = s[0];
+#pragma unroll
+        for (int i = 1; i < NI; i++) mx = fmaxf(mx, s[i]);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        mx = fmaxf(mx, m);                                                    // at least one key of the run exists: finite
+        const float al = m == -INFINITY ? 0.f : expf(m - mx);
+        l *= al;
+        m = mx;
+#pragma unroll
+        for (int i = 0; i < NI; i++) { s[i] = expf(s[i] - m); l += s[i]; }
+        if (__any_sync(0xffffffffu, al != 1.0f)) {
+#pragma unroll
+            for (int g = 0; g < GM; g++) {
+                const float r = __shfl_sync(0xffffffffu, al, g << HSH);
+#pragma unroll
+                for (int d = 0; d < 8; d++) acc[g][d] *= r;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+            const float4 c0 = vf[i][0], c1 = vf[i][1];
+#pragma unroll
+            for (int g = 0; g < GM; g++) {
+                const float p = __shfl_sync(0xffffffffu, s[i], (lane & 24) | (g << HSH));
+                acc[g][0] = fmaf(p, c0.x, acc[g][0]); acc[g][1] = fmaf(p, c0.y, acc[g][1]); acc[g][2] = fmaf(p, c0.z, acc[g][2]); acc[g][3] = fmaf(p, c0.w, acc[g][3]);
+                acc[g][4] = fmaf(p, c1.x, acc[g][4]); acc[g][5] = fmaf(p, c1.y, acc[g][5]); acc[g][6] = fmaf(p, c1.z, acc[g][6]); acc[g][7] = fmaf(p, c1.w, acc[g][7]);
+            }
         }
     }
-    float2 acc[GMW];
+    // the four key groups of the warp, then the warps
+    l += __shfl_xor_sync(0xffffffffu, l, 8);
+    l += __shfl_xor_sync(0xffffffffu, l, 16);
 #pragma unroll
-    for (int gi = 0; gi < GMW; gi++) acc[gi] = make_float2(0.f, 0.f);
+    for (int g = 0; g < GM; g++)
 #pragma unroll
-    for (int jj = 0; jj < 32; jj++) {
+        for (int d = 0; d < 8; d++) {
+            acc[g][d] += __shfl_xor_sync(0xffffffffu, acc[g][d], 8);
+            acc[g][d] += __shfl_xor_sync(0xffffffffu, acc[g][d], 16);
+        }
+    if (kg == 0) {
+        if ((dp & ((1 << HSH) - 1)) == 0) { pm[warp][dp >> HSH] = m; pl[warp][dp >> HSH] = l; }
 #pragma unroll
-        for (int gi = 0; gi < GMW; gi++) {
-            const float pj = __shfl_sync(0xffffffffu, s[gi], jj);
-            acc[gi].x = fmaf(pj, vv[jj].x, acc[gi].x); acc[gi].y = fmaf(pj, vv[jj].y, acc[gi].y);
+        for (int g = 0; g < GM; g++) {
+            *(float4 *)&po[warp][g][4 * dp] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+            *(float4 *)&po[warp][g][32 + 4 * dp] = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
         }
     }
-#pragma unroll
-    for (int gi = 0; gi < GMW; gi++)
-        if (g0 + gi < G) *(float2 *)&po[cw][g0 + gi][2 * lane] = acc[gi];
     __syncthreads();
-    // ---- the chunks' partials meet: maximum and weights per head, then the context columns ----
     if (tid < G) {
         float M = -INFINITY, L = 0.f;
-        for (int w = 0; w < cpc; w++) M = fmaxf(M, pm[w][tid]);
-        for (int w = 0; w < cpc; w++) {
+        for (int w = 0; w < nw; w++) M = fmaxf(M, pm[w][tid]);
+        for (int w = 0; w < nw; w++) {
             const float e = (pm[w][tid] == -INFINITY) ? 0.f : expf(pm[w][tid] - M);
             wg[w][tid] = e; L = fmaf(pl[w][tid], e, L);
         }
@@ -371,7 +410,7 @@ __global__ void __launch_bounds__(256) k_attention_dec_warp(AttnDecDev a) {
     for (int i = tid; i < G * HD; i += blockDim.x) {
         const int g = i / HD, d = i % HD;
         float O = 0.f;
-        for (int w = 0; w < cpc; w++) O = fmaf(po[w][g][d], wg[w][g], O);
+        for (int w = 0; w < nw; w++) O = fmaf(po[w][g][d], wg[w][g], O);
         if (nsplit == 1) {
             const float L = Lg[g];
             const float r = L > 0.f ? O / L : 0.f;
@@ -703,117 +742,16 @@ bool attention_decode_supported(const AttnArgs &a) {
     return true;
 }
 
-void attention_decode(const AttnArgs &a) {
+// The device arguments of a call whose rows are cut over max_split CTAs of cps chunks (or runs per warp), with the partial
+// buffer and the completion counters it needs.
+static AttnDecDev decode_args(const AttnArgs &a, int max_split, int cps) {
     static float *part = nullptr; static size_t part_cap = 0;
     static unsigned *count = nullptr; static size_t count_cap = 0;
-    // Keys of a row are shared out in 32-key chunks. With few (row, kv head) pairs every chunk gets a CTA of its own
-    // (a batch-1 decode step has nothing else to fill the GPU with); with many pairs a CTA walks several chunks,
-    // so that the fixed cost per CTA (query load, partials through L2, the merge) is paid about 8 x SMs times
-    // and not once per chunk.
-    const int max_chunks = (int)cdiv(a.max_k1 + a.max_k2, AD_KEYS);
-    const int64_t pairs = (int64_t)a.rows * a.Hkv;
-    static const bool warp_kernel = !getenv("NCM_B200_OLD_ATTN_DEC");
-    const bool warp_always = getenv("NCM_B200_ATTN_DEC_WARP") != nullptr;       // read per call: tests run both kernels on the same inputs
-    // The warp-per-chunk kernel for few (row, kv head) pairs, where the older kernel is a chain of barriers and a long
-    // merge: a warp takes up to two (query, head) pairs (more make its serial arithmetic the kernel: seven per warp
-    // measured 1.10 -> 1.16 ms per token on the Qwen2 shape), two or four chunks per CTA, and all CTAs must be resident at
-    // once. With hundreds of pairs the older kernel's higher occupancy wins (GPT-2 at 64 sequences: 1.44 against
-    // 1.94 ms per step).
-    const int gq_w = (a.H / a.Hkv) * a.max_q;
-    // many (query, head) pairs per kv group and enough (row, kv head) pairs to fill the GPU with warps: the
-    // tensor-core kernel (read per call: the tests run every kernel on the same inputs)
-    const char *mma_s = getenv("NCM_B200_ATTN_DEC_MMA");
-    const int mma_env = mma_s ? atoi(mma_s) : -1;
-    auto al16 = [](const void *q) { return ((uintptr_t)q & 15) == 0; };
-    const bool mma_takes = a.hd == 64 && gq_w <= AD_MAXG && ((a.ldk1 & 3) == 0) && (!a.k2 || (a.ldk2 & 3) == 0) && ((a.ldq & 3) == 0) &&
-                           al16(a.q) && al16(a.k1) && al16(a.v1) && (!a.k2 || (al16(a.k2) && al16(a.v2)));
-    // (measured: the 4-token level of config 2 -- 16 pairs per group, 9 chunks -- 2.99 -> 2.44 ms over its 12 layers; the
-    // Qwen2 batched-decode shape -- 7 pairs, 16 - 32 chunks -- at 256 sequences 42 936 -> 44 923 tokens/s, at 32
-    // sequences 12 821 -> 12 661: with few (row, kv head) pairs the CTA-per-chunk kernels spread a row over more SMs)
-    static const int mma_min_g = getenv("NCM_B200_ATTN_DEC_MMA_MIN_G") ? atoi(getenv("NCM_B200_ATTN_DEC_MMA_MIN_G")) : 12;
-    static const int mma_max_ch = getenv("NCM_B200_ATTN_DEC_MMA_MAX_CHUNKS") ? atoi(getenv("NCM_B200_ATTN_DEC_MMA_MAX_CHUNKS")) : 16;
-    const bool mma_pays = (gq_w >= mma_min_g && max_chunks <= mma_max_ch && pairs * 4 >= (int64_t)ctx().sm_count) ||
-                          (gq_w >= 6 && pairs >= 2 * (int64_t)ctx().sm_count);
-    if (mma_takes && (mma_env == 1 || (mma_env != 0 && mma_pays))) {
-        // chunks per warp: as few CTAs per (row, kv head) as still give every SM about eight warps
-        const int64_t want_ctas = std::max<int64_t>(1, cdiv((int64_t)ctx().sm_count * 2, pairs));
-        int cpw = (int)cdiv(max_chunks, ADM_WARPS * want_ctas);
-        if (cpw < 1) cpw = 1;
-        if (cpw > 16) cpw = 16;
-        const int max_split = (int)cdiv(max_chunks, ADM_WARPS * cpw);
-        if (max_split <= AD_MAXSPLIT) {
-            size_t need = (size_t)a.rows * a.Hkv * max_split * AD_MAXG * (a.hd + 2);
-            if (need > part_cap) {
-                if (part) { CUDA_CHECK(cudaStreamSynchronize(stream())); dev_free(part); }
-                part = (float *)dev_alloc(need * 4); part_cap = need;
-            }
-            size_t nc = (size_t)a.rows * a.Hkv;
-            if (nc > count_cap) {
-                if (count) { CUDA_CHECK(cudaStreamSynchronize(stream())); dev_free(count); }
-                count = (unsigned *)dev_alloc(nc * 4); count_cap = nc;
-                CUDA_CHECK(cudaMemsetAsync(count, 0, nc * 4, stream()));
-            }
-            AttnDecDev d;
-            d.q = a.q; d.ldq = a.ldq; d.k = a.k1; d.v = a.v1; d.ldk = a.ldk1;
-            d.k2 = a.k2; d.v2 = a.v2; d.ldk2 = a.ldk2; d.k2_start = a.k2 ? a.k2_start : nullptr; d.out = a.out; d.out_lo = a.out_lo; d.out_fmt = a.out_fmt; d.ldo = a.ldo;
-            d.q_start = a.q_start; d.k_start = a.k1_start; d.k_len = a.k1_len;
-            d.step_d = a.step_d; d.len_step = a.k1_len_step;
-            d.H = a.H; d.Hkv = a.Hkv; d.max_split = max_split; d.cps = cpw; d.hs = 1;
-            d.scale = 1.0f / sqrtf((float)a.hd);
-            d.part = part; d.count = count;
-            dim3 grid((unsigned)max_split, (unsigned)a.Hkv, (unsigned)a.rows);
-            ProfScope ps(NCMB_K_ATTN, 4.0 * (double)a.total_q * a.avg_keys * a.H * a.hd, 0);
-            LAUNCH_PDL(k_attention_dec_mma, grid, ADM_WARPS * 32, 0, d);
-            return;
-        }
-    }
-    const int gmw = gq_w <= 1 ? 1 : (gq_w <= 8 ? 2 : 4);
-    const int hs = (int)cdiv(gq_w, gmw);                                         // 1, 2, 3 or 4 warps per chunk
-    const int cpc = hs <= 2 ? 4 : 2;                                             // chunks per CTA (128 or 64 keys): at most eight warps
-    const int max_split_w = (int)cdiv(max_chunks, cpc);
-    const bool warp_pays = warp_always || pairs * max_split_w <= 2 * (int64_t)ctx().sm_count;
-    if (warp_kernel && warp_pays && a.hd == 64 && hs * cpc <= 8 && max_split_w <= AD_MAXSPLIT &&
-        ((a.ldk1 & 3) == 0) && (!a.k2 || (a.ldk2 & 3) == 0)) {
-        const int max_split = max_split_w;
-        size_t need = (size_t)a.rows * a.Hkv * max_split * AD_MAXG * (a.hd + 2);
-        if (need > part_cap) {
-            if (part) { CUDA_CHECK(cudaStreamSynchronize(stream())); dev_free(part); }
-            part = (float *)dev_alloc(need * 4); part_cap = need;
-        }
-        size_t nc = (size_t)a.rows * a.Hkv;
-        if (nc > count_cap) {
-            if (count) { CUDA_CHECK(cudaStreamSynchronize(stream())); dev_free(count); }
-            count = (unsigned *)dev_alloc(nc * 4); count_cap = nc;
-            CUDA_CHECK(cudaMemsetAsync(count, 0, nc * 4, stream()));
-        }
-        AttnDecDev d;
-        d.q = a.q; d.ldq = a.ldq; d.k = a.k1; d.v = a.v1; d.ldk = a.ldk1;
-        d.k2 = a.k2; d.v2 = a.v2; d.ldk2 = a.ldk2; d.k2_start = a.k2 ? a.k2_start : nullptr; d.out = a.out; d.out_lo = a.out_lo; d.out_fmt = a.out_fmt; d.ldo = a.ldo;
-        d.q_start = a.q_start; d.k_start = a.k1_start; d.k_len = a.k1_len;
-        d.step_d = a.step_d; d.len_step = a.k1_len_step;
-        d.H = a.H; d.Hkv = a.Hkv; d.max_split = max_split; d.cps = cpc; d.hs = hs;
-        d.scale = 1.0f / sqrtf((float)a.hd);
-        d.part = part; d.count = count;
-        dim3 grid((unsigned)max_split, (unsigned)a.Hkv, (unsigned)a.rows);
-        ProfScope ps(NCMB_K_ATTN, 4.0 * (double)a.total_q * a.avg_keys * a.H * a.hd, 0);
-        const int threads = hs * cpc * 32;
-        if (gmw == 1) LAUNCH_PDL((k_attention_dec_warp<1>), grid, threads, 0, d);
-        else if (gmw == 2) LAUNCH_PDL((k_attention_dec_warp<2>), grid, threads, 0, d);
-        else LAUNCH_PDL((k_attention_dec_warp<4>), grid, threads, 0, d);
-        return;
-    }
-    static const int per_sm = getenv("NCM_B200_ATTN_DEC_PER_SM") ? atoi(getenv("NCM_B200_ATTN_DEC_PER_SM")) : 8;
-    int want_split = (int)std::min<int64_t>(max_chunks, cdiv((int64_t)ctx().sm_count * per_sm, pairs));
-    if (want_split < 1) want_split = 1;
-    static const int cps_env = getenv("NCM_B200_ATTN_DEC_CPS") ? atoi(getenv("NCM_B200_ATTN_DEC_CPS")) : 0;
-    const int cps = cps_env > 0 ? std::min(cps_env, max_chunks) : (int)cdiv(max_chunks, want_split);
-    const int max_split = (int)cdiv(max_chunks, cps);
-    size_t need = (size_t)a.rows * a.Hkv * max_split * AD_MAXG * (a.hd + 2);
+    const size_t need = (size_t)a.rows * a.Hkv * max_split * AD_MAXG * (a.hd + 2), nc = (size_t)a.rows * a.Hkv;
     if (need > part_cap) {
         if (part) { CUDA_CHECK(cudaStreamSynchronize(stream())); dev_free(part); }
         part = (float *)dev_alloc(need * 4); part_cap = need;
     }
-    size_t nc = (size_t)a.rows * a.Hkv;
     if (nc > count_cap) {
         if (count) { CUDA_CHECK(cudaStreamSynchronize(stream())); dev_free(count); }
         count = (unsigned *)dev_alloc(nc * 4); count_cap = nc;
@@ -827,6 +765,71 @@ void attention_decode(const AttnArgs &a) {
     d.H = a.H; d.Hkv = a.Hkv; d.max_split = max_split; d.cps = cps;
     d.scale = 1.0f / sqrtf((float)a.hd);
     d.part = part; d.count = count;
+    return d;
+}
+
+void attention_decode(const AttnArgs &a) {
+    // Keys of a row are shared out in 32-key chunks. With few (row, kv head) pairs every chunk gets a CTA of its own
+    // (a batch-1 decode step has nothing else to fill the GPU with); with many pairs a CTA walks several chunks,
+    // so that the fixed cost per CTA (query load, partials through L2, the merge) is paid about 8 x SMs times
+    // and not once per chunk.
+    const int max_chunks = (int)cdiv(a.max_k1 + a.max_k2, AD_KEYS);
+    const int64_t pairs = (int64_t)a.rows * a.Hkv;
+    const int gq_w = (a.H / a.Hkv) * a.max_q;
+    // many (query, head) pairs per kv group and enough (row, kv head) pairs to fill the GPU with warps: the
+    // tensor-core kernel (read per call: the tests run every kernel on the same inputs)
+    const char *mma_s = getenv("NCM_B200_ATTN_DEC_MMA");
+    const int mma_env = mma_s ? atoi(mma_s) : -1;
+    auto al16 = [](const void *q) { return ((uintptr_t)q & 15) == 0; };
+    const bool mma_takes = a.hd == 64 && gq_w <= AD_MAXG && ((a.ldk1 & 3) == 0) && (!a.k2 || (a.ldk2 & 3) == 0) && ((a.ldq & 3) == 0) &&
+                           al16(a.q) && al16(a.k1) && al16(a.v1) && (!a.k2 || (al16(a.k2) && al16(a.v2)));
+    const bool gqa_takes = mma_takes && gq_w <= 8 && mma_env != 1;
+    // (measured: the 4-token level of config 2 -- 16 pairs per group, 9 chunks -- 2.99 -> 2.44 ms over its 12 layers; the
+    // Qwen2 batched-decode shape -- 7 pairs, 16 - 32 chunks -- at 256 sequences 42 936 -> 44 923 tokens/s, at 32
+    // sequences 12 821 -> 12 661: with few (row, kv head) pairs the CTA-per-chunk kernels spread a row over more SMs)
+    static const int mma_min_g = getenv("NCM_B200_ATTN_DEC_MMA_MIN_G") ? atoi(getenv("NCM_B200_ATTN_DEC_MMA_MIN_G")) : 12;
+    static const int mma_max_ch = getenv("NCM_B200_ATTN_DEC_MMA_MAX_CHUNKS") ? atoi(getenv("NCM_B200_ATTN_DEC_MMA_MAX_CHUNKS")) : 16;
+    const bool mma_pays = (gq_w >= mma_min_g && max_chunks <= mma_max_ch && pairs * 4 >= (int64_t)ctx().sm_count) ||
+                          (gq_w >= 6 && pairs >= 2 * (int64_t)ctx().sm_count);
+    if (mma_takes && (mma_env == 1 || (mma_env != 0 && !gqa_takes && mma_pays))) {
+        // chunks per warp: as few CTAs per (row, kv head) as still give every SM about eight warps
+        const int64_t want_ctas = std::max<int64_t>(1, cdiv((int64_t)ctx().sm_count * 2, pairs));
+        int cpw = (int)cdiv(max_chunks, ADM_WARPS * want_ctas);
+        if (cpw < 1) cpw = 1;
+        if (cpw > 16) cpw = 16;
+        const int max_split = (int)cdiv(max_chunks, ADM_WARPS * cpw);
+        if (max_split <= AD_MAXSPLIT) {
+            AttnDecDev d = decode_args(a, max_split, cpw);
+            dim3 grid((unsigned)max_split, (unsigned)a.Hkv, (unsigned)a.rows);
+            ProfScope ps(NCMB_K_ATTN, 4.0 * (double)a.total_q * a.avg_keys * a.H * a.hd, 0);
+            LAUNCH_PDL(k_attention_dec_mma, grid, ADM_WARPS * 32, 0, d);
+            return;
+        }
+    }
+    if (gqa_takes) {
+        // Enough (row, kv head) pairs to fill the SMs: four warps take all keys of a pair. Fewer: eight warps, and the row is cut
+        // over as many CTAs as give every SM one, at least a run of keys per warp.
+        const int runs = (int)cdiv(a.max_k1 + a.max_k2, ADG_RUN);
+        const int nw = pairs >= 2 * (int64_t)ctx().sm_count ? std::min(4, runs) : std::min(ADG_MAXW, runs);
+        int split = (int)std::max<int64_t>(1, std::min<int64_t>(ctx().sm_count / pairs, cdiv(runs, nw)));
+        if (split > AD_MAXSPLIT) split = AD_MAXSPLIT;
+        const int cps = (int)cdiv(runs, (int64_t)nw * split);
+        AttnDecDev d = decode_args(a, (int)cdiv(runs, (int64_t)nw * cps), cps);
+        dim3 grid((unsigned)d.max_split, (unsigned)a.Hkv, (unsigned)a.rows);
+        ProfScope ps(NCMB_K_ATTN, 4.0 * (double)a.total_q * a.avg_keys * a.H * a.hd, 0);
+        if (gq_w <= 1) LAUNCH_PDL((k_attention_dec_gqa<1>), grid, nw * 32, 0, d);
+        else if (gq_w <= 2) LAUNCH_PDL((k_attention_dec_gqa<2>), grid, nw * 32, 0, d);
+        else if (gq_w <= 4) LAUNCH_PDL((k_attention_dec_gqa<4>), grid, nw * 32, 0, d);
+        else LAUNCH_PDL((k_attention_dec_gqa<8>), grid, nw * 32, 0, d);
+        return;
+    }
+    static const int per_sm = getenv("NCM_B200_ATTN_DEC_PER_SM") ? atoi(getenv("NCM_B200_ATTN_DEC_PER_SM")) : 8;
+    int want_split = (int)std::min<int64_t>(max_chunks, cdiv((int64_t)ctx().sm_count * per_sm, pairs));
+    if (want_split < 1) want_split = 1;
+    static const int cps_env = getenv("NCM_B200_ATTN_DEC_CPS") ? atoi(getenv("NCM_B200_ATTN_DEC_CPS")) : 0;
+    const int cps = cps_env > 0 ? std::min(cps_env, max_chunks) : (int)cdiv(max_chunks, want_split);
+    const int max_split = (int)cdiv(max_chunks, cps);
+    AttnDecDev d = decode_args(a, max_split, cps);
     dim3 grid((unsigned)max_split, (unsigned)a.Hkv, (unsigned)a.rows);
     ProfScope ps(NCMB_K_ATTN, 4.0 * (double)a.total_q * a.avg_keys * a.H * a.hd, 0);
     const int gq = (a.H / a.Hkv) * a.max_q;

@@ -306,6 +306,13 @@ struct BlockWeights {
     const void *next_w = nullptr; size_t next_w_bytes = 0;
     int Hh = 0, gated = 0, act = ACT_GELU;
 };
+// a norm as its consumer needs it: kind 0 none, 1 LayerNorm, 2 RMSNorm
+struct NormSpec { int kind = 0; const float *w = nullptr, *b = nullptr; float eps = 0.f; };
+static inline NormSpec ln1_of(const BlockWeights &w) { return NormSpec{w.norm == NORM_RMS ? 2 : 1, w.ln1w, w.norm == NORM_RMS ? nullptr : w.ln1b, w.norm == NORM_RMS ? 1e-6f : w.eps}; }
+// Few rows (gemm_few.cu): a chain of blocks hands the normed row over as an fp16 pair, because the kernel that closes a block
+// adds the slices of its last product and holds whole rows. `on` is set by the chain's owner; run_block() writes the pair of
+// `next` applied to its output and sets ready.
+struct FewChain { bool on = false, ready = false; NormSpec next; void *y1 = nullptr, *y2 = nullptr; };
 struct BlockBufs { float *ln, *qkv, *ctx, *mlp, *h; };   // [n][C], [n][C+2kvd], [n][C], [n][Hh or 2Hh], [n][Hh]
 struct AttnPlan {
     const int *q_start = nullptr, *k1_start = nullptr, *k1_len = nullptr, *k2_start = nullptr;
@@ -323,8 +330,10 @@ struct AttnPlan {
     // after the K/V of this pass are final (norm + rope applied) they are stored here:
     float *kv_store = nullptr; int64_t kv_pitch = 0;   // row pitch in floats; rows = tokens, width 2*kvd
     int kv_rows_per_seq = 0; int64_t kv_seq_pitch = 0; // > 0: token t of sequence s goes to s*kv_seq_pitch + t*kv_pitch
+    FewChain *few = nullptr;             // few-row chain, or null
     int kv_only = 0;                     // stop after the K/V of this pass are stored (last layer of a cache fill)
 };
+bool few_chain_supported(int64_t ntok, int C, int H, int nkv, const BlockWeights &w);
 void run_block(float *x, int64_t ntok, int C, int H, int nkv, const BlockWeights &w, const BlockBufs &b, const AttnPlan &p);
 void apply_norm(const float *x, const float *w, const float *b, float *y, int64_t rows, int C, int kind, float eps);
 void apply_norm_split(const float *x, const float *w, const float *b, float *y, float *y_lo, int64_t rows, int C, int kind, float eps, int fmt);

@@ -1,0 +1,43 @@
+// Products of a weight matrix with few rows (gemm_few.cu): decode steps and the first levels of a generate.
+#pragma once
+#include "common.cuh"
+
+namespace ncmb {
+
+// y = act(x W^T + bias) for 5 to 256 rows of x (given as an fp16 pair), weights as fp16 pairs in the cache of the fp16-pair
+// engine. With `part` set, K may be cut into slices whose raw sums go to part[slice][row][N] (no bias, no activation); the
+// consumer adds them in slice order. Otherwise the result is stored: fp32 (y_lo null) or as an fp16 pair; glu: W holds
+// interleaved gate / up rows and y has N / 2 columns.
+struct FewGemm {
+    const void *x1, *x2; int64_t ldx;        // halfs
+    const float *W; int M, N, K;
+    const float *bias = nullptr; int act = ACT_NONE, glu = 0;
+    float *y = nullptr, *y_lo = nullptr; int64_t ldy = 0;
+    float *part = nullptr; int max_slices = 1;
+};
+constexpr int FEW_MAX_ROWS = 256;
+bool gemm_few_supported(int64_t M, int N, int K);
+int gemm_few_slices(int M, int N, int K, int max_slices);      // slices gemm_few() will use for a call with `part`
+void gemm_few(const FewGemm &g);
+
+// x[row] += bias + sum_s part[s][row] (S slices of rows x C), then norm(x) as an fp16 pair (ln_kind 0: no norm; 1 LayerNorm;
+// 2 RMSNorm). S = 0: only the norm.
+void few_reduce_norm(float *x, const float *part, int S, const float *bias, int rows, int C, int ln_kind, const float *ln_w, const float *ln_b,
+                     float eps, void *y1, void *y2);
+
+// q | k | v = bias + sum_s part[s][row], rotated (tables may be null), q to q[row * ldq], k | v to q as well (kv_self) and / or
+// to the cache row kv + (row / rps) * seq_pitch + (row % rps) * pitch + *step_d * step
+struct FewQkv {
+    const float *part; int S, rows, H, Hkv; const float *bias;
+    const float *cos_t = nullptr, *sin_t = nullptr; const int *pos = nullptr, *step_d = nullptr; int64_t pos_step = 0;
+    float *q; int64_t ldq; int kv_self = 0;
+    float *kv = nullptr; int rps = 1; int64_t seq_pitch = 0, pitch = 0, step = 0;
+    int hd = 64;
+};
+void few_reduce_qkv(const FewQkv &a);
+
+// the fp16 pair of a static weight matrix [N][K], its scale and whether the second half is all zero (gemm_h3.cu)
+struct H3Weights { const unsigned short *v1, *v2; float scale; bool v2_zero; };
+H3Weights gemm_h3_weights(const float *W, int64_t n);
+
+} // namespace ncmb

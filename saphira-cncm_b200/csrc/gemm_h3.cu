@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "tc_common.cuh"
 #include "tc_epilogue.cuh"
+#include "gemm_few.cuh"
 
 #include <algorithm>
 #include <unordered_map>
@@ -313,6 +314,19 @@ static void split_h16_weights(const float *W, unsigned short *v1, unsigned short
 // [8192, 16384): small weights stay clear of the fp16 subnormals); w2_zero: no element needed its second half
 struct ShadowH { unsigned short *v1, *v2; int64_t n; float scale; bool w2_zero; };
 static std::unordered_map<const float *, ShadowH> &shadow_h() { static std::unordered_map<const float *, ShadowH> c; return c; }
+// the cached pair of a static weight matrix of n elements, formed on first use
+H3Weights gemm_h3_weights(const float *W, int64_t n) {
+    auto &sc = shadow_h();
+    auto it = sc.find(W);
+    if (it == sc.end() || it->second.n != n) {
+        if (it != sc.end()) dev_free(it->second.v1);
+        unsigned short *buf = (unsigned short *)dev_alloc((size_t)2 * n * 2);
+        float scale = 1.0f; bool w2_zero = false;
+        split_h16_weights(W, buf, buf + n, n, &scale, &w2_zero);
+        it = sc.insert_or_assign(W, ShadowH{buf, buf + n, n, scale, w2_zero}).first;
+    }
+    return H3Weights{it->second.v1, it->second.v2, it->second.scale, it->second.w2_zero};
+}
 static Workspace &split_ws_h() { static Workspace w; return w; }
 
 // Drops the cached fp16 pairs of weights (call when weight memory is freed or rewritten).
@@ -402,18 +416,10 @@ void gemm_h3(const GemmArgs &a) {
     }
     const unsigned short *w1, *w2;
     if (cache_w) {
-        auto &sc = shadow_h();
-        auto it = sc.find(a.W);
-        if (it == sc.end() || it->second.n != nw) {
-            if (it != sc.end()) dev_free(it->second.v1);
-            unsigned short *buf = (unsigned short *)dev_alloc((size_t)2 * nw * 2);
-            float scale = 1.0f; bool w2_zero = false;
-            split_h16_weights(a.W, buf, buf + nw, nw, &scale, &w2_zero);
-            it = sc.insert_or_assign(a.W, ShadowH{buf, buf + nw, nw, scale, w2_zero}).first;
-        }
-        w1 = it->second.v1; w2 = it->second.v2;
-        ep.acc_scale = H16_X_UNSCALE / it->second.scale;
-        skip_w2 = it->second.w2_zero ? 1 : 0;
+        const H3Weights hw = gemm_h3_weights(a.W, nw);
+        w1 = hw.v1; w2 = hw.v2;
+        ep.acc_scale = H16_X_UNSCALE / hw.scale;
+        skip_w2 = hw.v2_zero ? 1 : 0;
     } else {
         unsigned short *p1 = ws.get<unsigned short>(nw), *p2 = ws.get<unsigned short>(nw);
         split_h16(a.W, a.K, p1, p2, a.N, a.K);

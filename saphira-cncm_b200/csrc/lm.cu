@@ -6,6 +6,7 @@
 #include "common.cuh"
 #include "lm_mega.cuh"
 #include "tc_common.cuh"
+#include "gemm_few.cuh"
 
 #include <algorithm>
 #include <string>
@@ -207,6 +208,7 @@ struct LMRun {
     float *mg_part = nullptr; unsigned *mg_count = nullptr, *mg_bar = nullptr; MegaLayer *mg_layers = nullptr;                      // kernel launches one replay of the captured step stands for
     unsigned long long *amax_d = nullptr;
     double *uni_cur = nullptr;
+    FewChain few;                 // the decode step's few-row chain
     // likelihood runs: next-token target and result per token row
     int64_t nll_rows = 0; int *tgt_d = nullptr; double *nll_d = nullptr;
 };
@@ -258,8 +260,17 @@ void lm_embed(LMRun &r, const int *ids_d, const int *pos_d, int64_t n) {
     }
 }
 
-void lm_head(LMRun &r, const float *h, int64_t rows, float *logits) {
+NormSpec lm_last_norm(const NcmbLM *m) { return NormSpec{m->is_qwen ? 2 : 1, m->lnfw, m->is_qwen ? nullptr : m->lnfb, m->is_qwen ? 1e-6f : 1e-5f}; }
+
+// few: the rows' final norm as a pair, when a few-row chain left it behind
+void lm_head(LMRun &r, const float *h, int64_t rows, float *logits, const FewChain *few = nullptr) {
     NcmbLM *m = r.m;
+    if (few && few->on && few->ready) {
+        FewGemm g{few->y1, few->y2, m->C, m->wte, (int)rows, m->V, m->C};
+        g.y = logits; g.ldy = m->V;
+        gemm_few(g);
+        return;
+    }
     GemmArgs g;
     g.x = h; g.ldx = m->C; g.W = m->wte; g.W16 = m->wte16; g.y = logits; g.ldy = m->V; g.M = rows; g.N = m->V; g.K = m->C;
     g.ln_kind = m->is_qwen ? 2 : 1; g.ln_w = m->lnfw; g.ln_b = m->lnfb; g.ln_eps = m->is_qwen ? 1e-6f : 1e-5f;
@@ -330,9 +341,13 @@ void lm_decode_step(LMRun &r, const int *ids_d) {
     p.total_q = r.B; p.avg_keys = (r.np + r.cap) / 2.0;
     p.kv_pitch = 2 * kvd; p.kv_rows_per_seq = 1; p.kv_seq_pitch = (int64_t)r.cap * 2 * kvd;
     p.kv_store_step = 2 * kvd;
+    r.few = FewChain();
+    r.few.on = few_chain_supported(r.B, m->C, m->H, m->nkv, m->blocks[0]) && gemm_few_supported(r.B, m->V, m->C);
+    p.few = &r.few;
     for (int li = 0; li < m->NL; li++) {
         p.k1 = r.kv[li]; p.v1 = r.kv[li] + kvd;
         p.kv_store = r.kv[li] + sh * 2 * kvd;
+        r.few.next = li + 1 < m->NL ? ln1_of(m->blocks[li + 1]) : lm_last_norm(m);
         run_block(r.x, r.B, m->C, m->H, m->nkv, m->blocks[li], r.bufs, p);
     }
 }
@@ -519,7 +534,7 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
         long long l0 = ctx().launches;
         if (capture) CUDA_CHECK(cudaStreamBeginCapture(gs, cudaStreamCaptureModeThreadLocal));
         lm_decode_step(r, r.ids_d);
-        lm_head(r, r.x, B, r.logits);
+        lm_head(r, r.x, B, r.logits, &r.few);
         if (capture) {
             lm_sample(r, temp, top_k, top_p, n_new);
             CUDA_CHECK(cudaStreamEndCapture(gs, &graph));

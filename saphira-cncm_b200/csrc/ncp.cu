@@ -17,6 +17,7 @@
 //    kernel per level; the reference's RNG stream is pre-drawn on the host in its
 //    (level, row, position) order so sampled codes match it draw for draw.
 #include "common.cuh"
+#include "gemm_few.cuh"
 #include "vq.cuh"
 #include "vqvae.cuh"
 
@@ -267,8 +268,18 @@ extern "C" VQState *ncp_vq(NCPState *m) { return m->vq; }
 
 // ------------------------------------------------------------------ shared pieces
 
-static void head_logits(NCPState *m, int k, const float *x, int64_t rows, float *lg, float *tmp) {
+// ln_f of the stack's output x, then head k. few: the normed rows as a pair, when a few-row chain left them behind.
+static void final_logits(NCPState *m, int k, const float *x, int64_t rows, const BlockBufs &bufs, float *lg, const FewChain &few) {
     const HeadW &h = m->heads[k];
+    if (few.on && few.ready && !h.proj && gemm_few_supported(rows, h.V, m->C)) {
+        FewGemm g{few.y1, few.y2, m->C, h.W, (int)rows, h.V, m->C};
+        g.bias = h.b; g.y = lg; g.ldy = h.V;
+        gemm_few(g);
+        return;
+    }
+    layernorm(x, m->lnfw, m->lnfb, bufs.ln, rows, m->C, 1e-6f);
+    x = bufs.ln;
+    float *tmp = bufs.ctx;
     GemmArgs g;
     if (h.proj) {
         g.x = x; g.ldx = m->C; g.W = h.proj; g.bias = h.projb; g.y = tmp; g.ldy = h.Dd; g.M = rows; g.N = h.Dd; g.K = m->C;
@@ -282,6 +293,11 @@ static void head_logits(NCPState *m, int k, const float *x, int64_t rows, float 
     }
 }
 
+static bool chain_on(const NCPState *m, int64_t n) { return !m->blocks.empty() && few_chain_supported(n, m->C, m->H, m->nkv, m->blocks[0]); }
+static NormSpec next_norm(const NCPState *m, int li) {
+    return li + 1 < m->NL ? ln1_of(m->blocks[li + 1]) : NormSpec{1, m->lnfw, m->lnfb, 1e-6f};
+}
+
 // Fills the per-layer K/V cache from the compacted prefix tokens in g->xpre.
 static void prefix_pass(NCPGen *g) {
     NCPState *m = g->m;
@@ -292,7 +308,11 @@ static void prefix_pass(NCPGen *g) {
     if (m->cfg.use_rope) { p.cos_t = m->gcos[0]; p.sin_t = m->gsin[0]; }
     p.total_q = g->ntok; p.avg_keys = g->Bm ? (double)g->ntok / g->Bm : 0;
     p.kv_pitch = 2 * m->nkv * m->hd;
+    FewChain few;
+    few.on = chain_on(m, g->ntok);
+    p.few = &few;
     for (int li = 0; li < m->NL; li++) {
+        few.next = next_norm(m, li);
         p.kv_store = g->kv[li];
         p.kv_only = (li == m->NL - 1);            // the last layer's prefix outputs are never read
         run_block(g->xpre, g->ntok, m->C, m->H, m->nkv, m->blocks[li], g->bufs, p);
@@ -315,12 +335,15 @@ static void level_pass(NCPGen *g, float *x, int Lc, int hi, int lev_slot) {
     p.pos = g->lev_pos_d[lev_slot];
     if (m->cfg.use_rope) { p.cos_t = m->gcos[hi]; p.sin_t = m->gsin[hi]; }
     p.total_q = n; p.avg_keys = (g->Bm ? (double)g->ntok / g->Bm : 0) + Lc;
+    FewChain few;
+    few.on = chain_on(m, n);
+    p.few = &few;
     for (int li = 0; li < m->NL; li++) {
         p.k1 = g->kv[li]; p.v1 = g->kv[li] + kvd;
+        few.next = next_norm(m, li);
         run_block(x, n, m->C, m->H, m->nkv, m->blocks[li], g->bufs, p);
     }
-    layernorm(x, m->lnfw, m->lnfb, g->bufs.ln, n, m->C, 1e-6f);
-    head_logits(m, hi, g->bufs.ln, n, g->logits, g->bufs.ctx);
+    final_logits(m, hi, x, n, g->bufs, g->logits, few);
 }
 
 // The same for the teacher-forced forward with the block-causal pattern (reference src/ncp.c:361-404: a target
@@ -342,14 +365,17 @@ static void level_pass_causal(NCPGen *g, float *x, int Lc, int hi, int lev_slot,
     if (m->cfg.use_rope) { p.cos_t = m->gcos[hi]; p.sin_t = m->gsin[hi]; }
     p.total_q = n; p.avg_keys = (g->Bm ? (double)g->ntok / g->Bm : 0) + off + Lc;
     p.kv_pitch = 2 * kvd; p.kv_rows_per_seq = Lc; p.kv_seq_pitch = (int64_t)m->T * 2 * kvd;
+    FewChain few;
+    few.on = chain_on(m, n);
+    p.few = &few;
     for (int li = 0; li < m->NL; li++) {
         p.k1 = lvlkv[li]; p.v1 = lvlkv[li] + kvd;
         p.k2 = g->kv[li]; p.v2 = g->kv[li] + kvd;
         p.kv_store = lvlkv[li] + (size_t)off * 2 * kvd;
+        few.next = next_norm(m, li);
         run_block(x, n, m->C, m->H, m->nkv, m->blocks[li], g->bufs, p);
     }
-    layernorm(x, m->lnfw, m->lnfb, g->bufs.ln, n, m->C, 1e-6f);
-    head_logits(m, hi, g->bufs.ln, n, g->logits, g->bufs.ctx);
+    final_logits(m, hi, x, n, g->bufs, g->logits, few);
 }
 
 // x += conv(x) as the reference's GENERATE path computes it: the conv output stays in
@@ -530,8 +556,8 @@ static void gen_l0(NCPGen *g) {
         if (!c->query_level0) { fprintf(stderr, "generate(idx=None) requires query_level0 or predict_level0\n"); exit(1); }
         if (!m->l0q) { fprintf(stderr, "missing weight gen.l0_queries\n"); exit(1); }
         // q0 = l0_queries broadcast over rows
-        for (int b = 0; b < Bm; b++)
-            CUDA_CHECK(cudaMemcpyAsync(g->xout + (size_t)b * l0len * D, m->l0q, (size_t)l0len * D * 4, cudaMemcpyDeviceToDevice, stream()));
+        CUDA_CHECK(cudaMemsetAsync(g->xout, 0, (size_t)Bm * l0len * D * 4, stream()));
+        add_rows_bcast(g->xout, m->l0q, Bm, l0len * D);
         if (c->puc_enabled) puc_generate(m, 0, g->xout, g->xtmp, Bm, l0len, 3);
         GemmArgs a;
         a.x = g->xout; a.ldx = D; a.W = m->wteW; a.bias = m->wteB; a.y = g->xlev; a.ldy = C; a.M = (int64_t)Bm * l0len; a.N = C; a.K = D;

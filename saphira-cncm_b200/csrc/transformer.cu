@@ -5,7 +5,9 @@
 // SDPA; here the fused QKV projection is consumed in place by the attention kernel
 // and the residual adds ride in the GEMM epilogues.
 #include "common.cuh"
+#include "gemm_few.cuh"
 
+#include <algorithm>
 #include <stdarg.h>
 
 namespace ncmb {
@@ -74,8 +76,84 @@ unsigned short *dev_bf16_exact(const float *w, int64_t n) {
 // Scratch for the lo halves of the block's GEMM inputs in three-pass mode (ln, ctx, hidden).
 static Workspace &block_lo_ws() { static Workspace w; return w; }
 
+// The attention call of a block whose q (and, for own-pass keys, k | v) sit in b.qkv.
+static void block_attention(const BlockBufs &b, const AttnPlan &p, int64_t ntok, int C, int H, int nkv, float *ctx_lo, int fmt) {
+    const int hd = C / H, kvd = nkv * hd, Wq = C + 2 * kvd;
+    float *kp = b.qkv + C, *vp = b.qkv + C + kvd;
+    AttnArgs a;
+    a.q = b.qkv; a.ldq = Wq;
+    if (p.k1) { a.k1 = p.k1; a.v1 = p.v1; a.ldk1 = p.ldk1; }
+    else { a.k1 = kp; a.v1 = vp; a.ldk1 = Wq; }
+    a.k1_start = p.k1_start; a.k1_len = p.k1_len;
+    if (p.self_is_k2) { a.k2 = kp; a.v2 = vp; a.ldk2 = Wq; a.k2_start = p.k2_start ? p.k2_start : p.q_start; }
+    else if (p.k2) { a.k2 = p.k2; a.v2 = p.v2; a.ldk2 = p.ldk2; a.k2_start = p.k2_start; }
+    a.out = b.ctx; a.out_lo = ctx_lo; a.out_fmt = fmt; a.ldo = C;
+    a.q_start = p.q_start;
+    a.rows = p.rows; a.H = H; a.Hkv = nkv; a.hd = hd; a.max_q = p.max_q;
+    a.causal = p.causal; a.causal_off = p.causal_off; a.window = p.window;
+    a.total_q = p.total_q; a.avg_keys = p.avg_keys;
+    a.max_k1 = p.max_k1; a.max_k2 = p.self_is_k2 ? p.max_q : (p.k2 ? p.max_k2 : 0);
+    a.step_d = p.step_d; a.k1_len_step = p.k1_len_step;
+    a.q_total = ntok; a.k1_total = p.k1 ? p.k1_total : ntok; a.k2_total = p.self_is_k2 ? ntok : (p.k2 ? p.k2_total : 0);
+    attention(a);
+}
+
+// Slices of K a product of M rows may be cut into: every slice is written and read once more (8 bytes per output), which for
+// many rows costs more than the idle SMs it avoids.
+static int few_max_slices(int64_t M) { return M <= 64 ? 24 : (M <= 128 ? 8 : 4); }
+
+bool few_chain_supported(int64_t ntok, int C, int H, int nkv, const BlockWeights &w) {
+    static const bool off = getenv("NCM_B200_NO_FEW") != nullptr;
+    const int hd = C / H;
+    return !off && gemm_few_supported(ntok, C + 2 * nkv * hd, C) && gemm_few_supported(ntok, w.Hh, w.Hh) && C % 8 == 0 && C <= 4096 && hd % 2 == 0 &&
+           !w.qnw && !w.knw && (!w.gated || w.fcw_il);
+}
+
+// One block for a few rows: four products on the weight-streaming kernel, and what lies between them folded into the kernels
+// that add the slices of the first, second and last -- eight launches, where the general path takes eleven to thirteen.
+static void run_block_few(float *x, int64_t ntok, int C, int H, int nkv, const BlockWeights &w, const BlockBufs &b, const AttnPlan &p) {
+    FewChain &fc = *p.few;
+    const int hd = C / H, kvd = nkv * hd, Wq = C + 2 * kvd, M = (int)ntok, ms = few_max_slices(ntok);
+    static Workspace ws;
+    const int Sq = gemm_few_slices(M, Wq, C, ms), So = gemm_few_slices(M, C, C, ms), Sd = gemm_few_slices(M, C, w.Hh, ms);
+    const size_t part_fl = (size_t)M * std::max((size_t)Sq * Wq, (size_t)std::max(So, Sd) * C);
+    const size_t need = part_fl * 4 + (size_t)M * (2 * C + w.Hh) * 4 + 4096;
+    if (need > ws.cap) { ws.reserve(need + need / 4); fc.ready = false; }
+    ws.reset();
+    // (the chain's pair comes first: it lies in the same place for every block, written by the previous block's last kernel)
+    unsigned short *n1 = ws.get<unsigned short>((size_t)M * C), *n2 = ws.get<unsigned short>((size_t)M * C);
+    float *part = ws.get<float>(part_fl);
+    float *ctx_lo = ws.get<float>((size_t)M * C / 2 + 8), *h_lo = ws.get<float>((size_t)M * w.Hh / 2 + 8);
+    if (!fc.ready) few_reduce_norm(x, nullptr, 0, nullptr, M, C, ln1_of(w).kind, w.ln1w, ln1_of(w).b, ln1_of(w).eps, n1, n2);
+    const NormSpec ln2{ln1_of(w).kind, w.ln2w, w.norm == NORM_RMS ? nullptr : w.ln2b, ln1_of(w).eps};
+    FewGemm g{n1, n2, C, w.qkvw, M, Wq, C};
+    g.part = part; g.max_slices = ms;
+    gemm_few(g);
+    FewQkv q{part, Sq, M, H, nkv, w.qkvb};
+    q.cos_t = p.cos_t; q.sin_t = p.sin_t; q.pos = p.pos; q.step_d = p.step_d; q.pos_step = p.pos_step;
+    q.q = b.qkv; q.ldq = Wq; q.kv_self = (!p.k1 || p.self_is_k2 || p.kv_store == nullptr) ? 1 : 0;
+    q.kv = p.kv_store; q.rps = p.kv_rows_per_seq > 0 ? p.kv_rows_per_seq : M; q.seq_pitch = p.kv_seq_pitch; q.pitch = p.kv_pitch; q.step = p.kv_store_step;
+    q.hd = hd;
+    few_reduce_qkv(q);
+    if (p.kv_only) return;
+    block_attention(b, p, ntok, C, H, nkv, ctx_lo, SPLIT_H16);
+    g = FewGemm{b.ctx, ctx_lo, C, w.ow, M, C, C};
+    g.part = part; g.max_slices = ms;
+    gemm_few(g);
+    few_reduce_norm(x, part, So, w.ob, M, C, ln2.kind, ln2.w, ln2.b, ln2.eps, n1, n2);
+    g = FewGemm{n1, n2, C, w.gated ? w.fcw_il : w.fcw, M, w.gated ? 2 * w.Hh : w.Hh, C};
+    g.bias = w.gated ? w.fcb_il : w.fcb; g.act = w.act; g.glu = w.gated; g.y = b.h; g.y_lo = h_lo; g.ldy = w.Hh;
+    gemm_few(g);
+    g = FewGemm{b.h, h_lo, w.Hh, w.pw, M, C, w.Hh};
+    g.part = part; g.max_slices = ms;
+    gemm_few(g);
+    few_reduce_norm(x, part, Sd, w.pb, M, C, fc.next.kind, fc.next.w, fc.next.b, fc.next.eps, n1, n2);
+    fc.ready = fc.next.kind != 0; fc.y1 = n1; fc.y2 = n2;
+}
+
 void run_block(float *x, int64_t ntok, int C, int H, int nkv, const BlockWeights &w, const BlockBufs &b, const AttnPlan &p) {
     if (ntok <= 0) return;
+    if (p.few && p.few->on) { run_block_few(x, ntok, C, H, nkv, w, b, p); return; }
     const int hd = C / H, kvd = nkv * hd, Wq = C + 2 * kvd;
     // In three-pass mode the producers of GEMM inputs (norms, attention, MLP activation) write
     // TF32 hi / lo pairs directly, so no separate split pass runs between kernels.
@@ -134,7 +212,7 @@ void run_block(float *x, int64_t ntok, int C, int H, int nkv, const BlockWeights
         g.qk_applied = &qk_done;
     }
     gemm(g);
-    float *qp = b.qkv, *kp = b.qkv + C, *vp = b.qkv + C + kvd;
+    float *qp = b.qkv, *kp = b.qkv + C;
     if (!qk_done) qk_post(qp, Wq, H, kp, Wq, nkv, hd, ntok, w.qnw, w.knw, p.cos_t, p.sin_t, p.pos, p.step_d, p.pos_step);
     if (p.kv_store && !kv_written) {
         int width4 = 2 * kvd / 4;
@@ -145,22 +223,7 @@ void run_block(float *x, int64_t ntok, int C, int H, int nkv, const BlockWeights
                p.kv_rows_per_seq, p.kv_seq_pitch, ntok, width4, p.step_d, p.kv_store_step);
     }
     if (p.kv_only) return;
-    AttnArgs a;
-    a.q = qp; a.ldq = Wq;
-    if (p.k1) { a.k1 = p.k1; a.v1 = p.v1; a.ldk1 = p.ldk1; }
-    else { a.k1 = kp; a.v1 = vp; a.ldk1 = Wq; }
-    a.k1_start = p.k1_start; a.k1_len = p.k1_len;
-    if (p.self_is_k2) { a.k2 = kp; a.v2 = vp; a.ldk2 = Wq; a.k2_start = p.k2_start ? p.k2_start : p.q_start; }
-    else if (p.k2) { a.k2 = p.k2; a.v2 = p.v2; a.ldk2 = p.ldk2; a.k2_start = p.k2_start; }
-    a.out = b.ctx; a.out_lo = ctx_lo; a.out_fmt = fmt; a.ldo = C;
-    a.q_start = p.q_start;
-    a.rows = p.rows; a.H = H; a.Hkv = nkv; a.hd = hd; a.max_q = p.max_q;
-    a.causal = p.causal; a.causal_off = p.causal_off; a.window = p.window;
-    a.total_q = p.total_q; a.avg_keys = p.avg_keys;
-    a.max_k1 = p.max_k1; a.max_k2 = p.self_is_k2 ? p.max_q : (p.k2 ? p.max_k2 : 0);
-    a.step_d = p.step_d; a.k1_len_step = p.k1_len_step;
-    a.q_total = ntok; a.k1_total = p.k1 ? p.k1_total : ntok; a.k2_total = p.self_is_k2 ? ntok : (p.k2 ? p.k2_total : 0);
-    attention(a);
+    block_attention(b, p, ntok, C, H, nkv, ctx_lo, fmt);
     // x += ctx Wo^T + bo
     g = GemmArgs();
     g.x_fmt = fmt;
