@@ -16,10 +16,27 @@
 // so one captured CUDA graph serves every decode step.
 #include "common.cuh"
 #include "split.cuh"
+#include "gemm_few.cuh"
 
 #include <algorithm>
 
 namespace ncmb {
+
+// programmatic dependent launch (see launch_pdl) of clusters of nc CTAs along x
+template <typename... KArgs, typename... Args>
+static void launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, int nc, Args... args) {
+    static const bool off = getenv("NCM_B200_NO_PDL") != nullptr;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.stream = stream();
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (nc > 1) { at[n].id = cudaLaunchAttributeClusterDimension; at[n].val.clusterDim.x = (unsigned)nc; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1; n++; }
+    if (!off) { at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[n].val.programmaticStreamSerializationAllowed = 1; n++; }
+    cfg.attrs = at; cfg.numAttrs = n;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+    if (e != cudaSuccess) fatal("decode attention: launch failed: %s", cudaGetErrorString(e));
+    ctx().launches++;
+}
 
 constexpr int AD_KEYS = 32, AD_THREADS = 128, AD_MAXSPLIT = 64;   // up to 2048 keys per row
 constexpr int AD_MAXG = 16;        // (query, head) pairs of one kv group handled together: G * queries per row <= 16
@@ -31,7 +48,7 @@ struct AttnDecDev {
     float *out; float *out_lo; int out_fmt; int64_t ldo;
     const int *q_start, *k_start, *k_len;
     const int *step_d; int64_t len_step;
-    int H, Hkv, max_split, cps;
+    int H, Hkv, rows, max_split, cps;
     float scale;
     float *part; unsigned *count;
 };
@@ -254,88 +271,160 @@ __global__ void __launch_bounds__(AD_THREADS) k_attention_decode(AttnDecDev a) {
 }
 
 // ---- head dim 64, up to eight (query, head) pairs per kv head: lanes share keys, loads straight to registers ----
-// Eight lanes hold a key: lane (kg, dp) keeps dims 4 dp .. and 32 + 4 dp .. of key kg of a group of four, so a warp's load of
-// four keys (or values) is eight full 128-byte lines, and the same lane needs the same dims of the query (in registers for
-// all GM pairs) and of the context (accumulated in registers). The eight partial dot products of a key meet by a
-// reduce-scatter that leaves pair dp's score in lane dp (seven shuffles for eight pairs instead of twenty-four), the softmax
-// runs on those, and the probabilities travel back by one shuffle per pair and key. Nothing goes through shared memory until a
-// warp's keys are done. A warp takes runs of 16 keys: the values of a run and the keys of the next are requested before the
-// run's arithmetic. The warps of a CTA interleave runs; a row is cut over CTAs only while there are too few (row, kv head)
-// pairs to fill the GPU, and the last CTA of a pair to finish merges.
+// LPK lanes hold a key: with sixteen (more than four pairs) a lane keeps four dims, with eight it keeps eight, of the key, of
+// the query (in registers for all GM pairs) and of the context (accumulated in registers); a warp's loads are full 128-byte
+// lines. The partial dot products of a key meet by a reduce-scatter that leaves one pair's score in a lane (eight shuffles for
+// eight pairs), the softmax runs on those, and the probabilities travel back by one shuffle per pair and key. Nothing goes
+// through shared memory until a warp's keys are done. A warp takes runs of four loads (8 or 16 keys): the values of a run and
+// the keys of the next are requested before the run's arithmetic. The CTAs of a cluster share the keys of a (row, kv head) pair,
+// their warps interleaving runs, and merge over distributed shared memory.
 //
-// Bound: the K|V cache read once. Per key and kv head about 35 warp instructions at eight pairs.
-constexpr int ADG_RUN = 16;            // keys of a run: four groups of four
+// FUSED (decode steps): q, k and v of the new token arrive as the slices of the QKV product. Every CTA adds what its heads
+// need, rotates it, keeps the new key and value in shared memory and the first CTA of the cluster appends them to the cache.
+// The cached keys and values of a warp's first run are requested before the kernel waits for that product; the reduce_norm
+// kernel in front of the product starts its successor only after its own wait, so the cache and the step counter are final.
+//
+// Bound: the K|V cache read once; for few rows the chain product -> sums -> scores -> merge.
+constexpr int ADG_NI = 4;              // loads of a run per lane
 constexpr int ADG_MAXW = 8;            // warps of a CTA at most
+constexpr int ADG_MAXC = 8;            // CTAs of a cluster at most
 
-template <int GM>
-__global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a) {
-    constexpr int HD = 64, NI = ADG_RUN / 4;
-    constexpr int HSH = GM == 8 ? 0 : GM == 4 ? 1 : GM == 2 ? 2 : 3;          // lane dp holds pair dp >> HSH after the reduction
+struct AttnFused {                     // see FewQkv: slices of the QKV product of a decode step, one token per row
+    const float *part; int S; const float *bias;
+    const float *cos_t, *sin_t; const int *pos; int64_t pos_step;
+    float *kv; int64_t seq_pitch, step;      // cache position of the new token: kv + row * seq_pitch + *step_d * step, k | v of all kv heads
+};
+
+__device__ __forceinline__ float ld_cluster(const float *p, unsigned rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+    return v;
+}
+
+template <int GM, bool FUSED>
+__global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a, AttnFused f) {
+    constexpr int HD = 64, LPK = GM > 4 ? 16 : 8, DPL = HD / LPK, NF = DPL / 4, KPI = 32 / LPK, NI = ADG_NI, RUN = NI * KPI;
+    constexpr int LOG = GM == 8 ? 3 : GM == 4 ? 2 : GM == 2 ? 1 : 0, HSH = (LPK == 16 ? 4 : 3) - LOG;   // lane dp holds pair dp >> HSH
     __shared__ float pm[ADG_MAXW][GM], pl[ADG_MAXW][GM], wg[ADG_MAXW][GM];
     __shared__ __align__(16) float po[ADG_MAXW][GM][HD];
-    __shared__ float Mg[GM], Lg[GM];
-    __shared__ int s_last;
-    const int row = blockIdx.z, kvh = blockIdx.y, sp = blockIdx.x;
+    __shared__ __align__(16) float co[GM][HD];               // the CTA's context, maximum and sum, read by the cluster
+    __shared__ float cm[GM], cl[GM], cw[ADG_MAXC][GM];
+    __shared__ __align__(16) float qn[FUSED ? GM + 2 : 1][HD];   // the new token's queries, key, value
+    const int rank = blockIdx.x, nc = gridDim.x;             // one cluster per (row, kv head)
+    const int row = blockIdx.z, kvh = blockIdx.y;
     const int Gh = a.H / a.Hkv;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
-    const int kg = lane >> 3, dp = lane & 7;
+    const int kg = lane / LPK, dp = lane % LPK;
     pdl_launch_dependents();
-    pdl_wait();
-    const int *lens = a.k_len ? a.k_len + (a.step_d ? (int64_t)(*a.step_d) * a.len_step : 0) : nullptr;
+    if (!FUSED) pdl_wait();
+    const int64_t st = a.step_d ? (int64_t)*a.step_d : 0;
+    const int *lens = a.k_len ? a.k_len + st * a.len_step : nullptr;
     const int k00 = a.k_start[row], n1s = lens ? lens[row] : a.k_start[row + 1] - k00;
     const int k20 = a.k2_start ? a.k2_start[row] : 0, n2s = a.k2_start ? a.k2_start[row + 1] - k20 : 0;
-    const int n1 = n1s + n2s;
-    const int per_cta = a.cps * nw * ADG_RUN;                                 // keys a CTA takes
-    const int nsplit = max(1, (n1 + per_cta - 1) / per_cta);
-    if (sp >= nsplit) return;
-    const int q0 = a.q_start[row], nq = a.q_start[row + 1] - q0;
-    const int G = Gh * nq;                                                    // virtual heads: vh = g * nq + qi
-    const int first = sp * per_cta + warp * ADG_RUN, step = nw * ADG_RUN, last = min(n1, (sp + 1) * per_cta);
-    float q[GM][8];
-#pragma unroll
-    for (int g = 0; g < GM; g++) {
-        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-        if (g < G) {
-            const float *qp = a.q + (int64_t)(q0 + g % nq) * a.ldq + (kvh * Gh + g / nq) * HD + 4 * dp;
-            lo = *(const float4 *)qp; hi = *(const float4 *)(qp + 32);
-        }
-        q[g][0] = lo.x * a.scale; q[g][1] = lo.y * a.scale; q[g][2] = lo.z * a.scale; q[g][3] = lo.w * a.scale;
-        q[g][4] = hi.x * a.scale; q[g][5] = hi.y * a.scale; q[g][6] = hi.z * a.scale; q[g][7] = hi.w * a.scale;
-    }
-    float4 kf[NI][2], vf[NI][2];
-    auto load = [&](float4 (&f)[NI][2], const float *s1, int64_t ld1, const float *s2, int64_t ld2, int j0) {
+    const int n1 = n1s + n2s, cached = FUSED ? n1 - 1 : n1;
+    const int q0 = a.q_start[row], nq = FUSED ? 1 : a.q_start[row + 1] - q0;
+    const int G = Gh * nq;                                   // virtual heads: vh = g * nq + qi
+    const int first = (warp * nc + rank) * RUN, step = nw * nc * RUN;
+    float4 kf[NI][NF], vf[NI][NF];
+    // dims of a lane: 4 dp .. (and 32 + 4 dp .. where it holds eight)
+    auto load = [&](float4 (&r)[NI][NF], const float *s1, int64_t ld1, const float *s2, int64_t ld2, int j0) {
 #pragma unroll
         for (int i = 0; i < NI; i++) {
-            const int j = j0 + 4 * i + kg;
-            if (j < last) {
-                const float *p = (j < n1s ? s1 + (int64_t)(k00 + j) * ld1 : s2 + (int64_t)(k20 + j - n1s) * ld2) + kvh * HD + 4 * dp;
-                f[i][0] = *(const float4 *)p; f[i][1] = *(const float4 *)(p + 32);
-            } else f[i][0] = f[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int j = j0 + KPI * i + kg;
+            const float *p = nullptr;
+            if (j < cached) p = (j < n1s ? s1 + (int64_t)(k00 + j) * ld1 : s2 + (int64_t)(k20 + j - n1s) * ld2) + kvh * HD + 4 * dp;
+#pragma unroll
+            for (int h = 0; h < NF; h++) r[i][h] = p ? *(const float4 *)(p + 32 * h) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
-    float acc[GM][8], m = -INFINITY, l = 0.f;
+    if (first < cached) {
+        load(kf, a.k, a.ldk, a.k2, a.ldk2, first);
+        load(vf, a.v, a.ldk, a.v2, a.ldk2, first);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NI; i++)
+#pragma unroll
+            for (int h = 0; h < NF; h++) kf[i][h] = vf[i][h] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if constexpr (FUSED) {
+        pdl_wait();
+        const int Wq = (a.H + 2 * a.Hkv) * HD;
+        for (int it = tid; it < (Gh + 2) * (HD / 2); it += blockDim.x) {
+            const int hh = it / (HD / 2), d = it % (HD / 2);
+            const int h = hh < Gh ? kvh * Gh + hh : (hh == Gh ? a.H + kvh : a.H + a.Hkv + kvh);
+            const float *p = f.part + (int64_t)row * Wq + h * HD + d;
+            const int64_t ps = (int64_t)a.rows * Wq;
+            float v0 = 0.f, v1 = 0.f;
+            for (int s = 0; s < f.S; s += 8) {
+                float t0[8], t1[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (s + u < f.S) { t0[u] = __ldcg(p + (s + u) * ps); t1[u] = __ldcg(p + (s + u) * ps + HD / 2); }
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (s + u < f.S) { v0 += t0[u]; v1 += t1[u]; }
+            }
+            if (f.bias) { v0 += __ldg(f.bias + h * HD + d); v1 += __ldg(f.bias + h * HD + d + HD / 2); }
+            if (f.cos_t && hh <= Gh) {
+                const int64_t at = (int64_t)f.pos[st * f.pos_step + row] * HD + d;
+                const float y0 = __fadd_rn(__fmul_rn(v0, f.cos_t[at]), __fmul_rn(-v1, f.sin_t[at]));
+                const float y1 = __fadd_rn(__fmul_rn(v1, f.cos_t[at + HD / 2]), __fmul_rn(v0, f.sin_t[at + HD / 2]));
+                v0 = y0; v1 = y1;
+            }
+            const int slot = hh < Gh ? hh : GM + hh - Gh;
+            qn[slot][d] = v0; qn[slot][d + HD / 2] = v1;
+            if (hh >= Gh && rank == 0) {
+                float *kv = f.kv + (int64_t)row * f.seq_pitch + st * f.step + (h - a.H) * HD + d;
+                kv[0] = v0; kv[HD / 2] = v1;
+            }
+        }
+        __syncthreads();
+    }
+    float q[GM][DPL];
 #pragma unroll
     for (int g = 0; g < GM; g++)
 #pragma unroll
-        for (int d = 0; d < 8; d++) acc[g][d] = 0.f;
-    if (first < last) load(kf, a.k, a.ldk, a.k2, a.ldk2, first);
-    for (int j0 = first; j0 < last; j0 += step) {
-        load(vf, a.v, a.ldk, a.v2, a.ldk2, j0);
+        for (int h = 0; h < NF; h++) {
+            float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (g < G) {
+                if (FUSED) t = *(const float4 *)&qn[FUSED ? g : 0][4 * dp + 32 * h];
+                else t = *(const float4 *)(a.q + (int64_t)(q0 + g % nq) * a.ldq + (kvh * Gh + g / nq) * HD + 4 * dp + 32 * h);
+            }
+            q[g][4 * h] = t.x * a.scale; q[g][4 * h + 1] = t.y * a.scale; q[g][4 * h + 2] = t.z * a.scale; q[g][4 * h + 3] = t.w * a.scale;
+        }
+    float acc[GM][DPL], m = -INFINITY, l = 0.f;
+#pragma unroll
+    for (int g = 0; g < GM; g++)
+#pragma unroll
+        for (int d = 0; d < DPL; d++) acc[g][d] = 0.f;
+    for (int j0 = first; j0 < n1; j0 += step) {
+        if constexpr (FUSED) {                                // the new token's key and value
+#pragma unroll
+            for (int i = 0; i < NI; i++)
+                if (j0 + KPI * i + kg == cached) {
+#pragma unroll
+                    for (int h = 0; h < NF; h++) { kf[i][h] = *(const float4 *)&qn[GM][4 * dp + 32 * h]; vf[i][h] = *(const float4 *)&qn[GM + 1][4 * dp + 32 * h]; }
+                }
+        }
         float s[NI];
 #pragma unroll
         for (int i = 0; i < NI; i++) {
-            const float4 c0 = kf[i][0], c1 = kf[i][1];
             float v[GM];
 #pragma unroll
             for (int g = 0; g < GM; g++) {
-                float t = q[g][0] * c0.x;
-                t = fmaf(q[g][1], c0.y, t); t = fmaf(q[g][2], c0.z, t); t = fmaf(q[g][3], c0.w, t);
-                t = fmaf(q[g][4], c1.x, t); t = fmaf(q[g][5], c1.y, t); t = fmaf(q[g][6], c1.z, t); t = fmaf(q[g][7], c1.w, t);
+                float t = 0.f;
+#pragma unroll
+                for (int h = 0; h < NF; h++) {
+                    t = fmaf(q[g][4 * h], kf[i][h].x, t); t = fmaf(q[g][4 * h + 1], kf[i][h].y, t);
+                    t = fmaf(q[g][4 * h + 2], kf[i][h].z, t); t = fmaf(q[g][4 * h + 3], kf[i][h].w, t);
+                }
                 v[g] = t;
             }
-            int o = 4;
+            int o = LPK / 2;
 #pragma unroll
-            for (int w = GM / 2; w > 0; w >>= 1, o >>= 1) {                   // halve the pairs a lane keeps
+            for (int w = GM / 2; w > 0; w >>= 1, o >>= 1) {   // halve the pairs a lane keeps
                 const bool up = (dp & o) != 0;
 #pragma unroll
                 for (int g = 0; g < w; g++) {
@@ -343,16 +432,17 @@ __global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a) {
                     v[g] = keep + __shfl_xor_sync(0xffffffffu, give, o);
                 }
             }
-            for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-            s[i] = (j0 + 4 * i + kg < last) ? v[0] : -INFINITY;
-        }
-        if (j0 + step < last) load(kf, a.k, a.ldk, a.k2, a.ldk2, j0 + step);
-        float mx = s[0];
 #pragma unroll
-        for (int i = 1; i < NI; i++) mx = fmaxf(mx, s[i]);
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-        mx = fmaxf(mx, m);                                                    // at least one key of the run exists: finite
+            for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+            s[i] = (j0 + KPI * i + kg < n1) ? v[0] : -INFINITY;
+        }
+        const bool more = j0 + step < n1;
+        if (more) load(kf, a.k, a.ldk, a.k2, a.ldk2, j0 + step);
+        float mx = m;
+#pragma unroll
+        for (int i = 0; i < NI; i++) mx = fmaxf(mx, s[i]);
+#pragma unroll
+        for (int o = LPK; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));   // a run has at least one key: finite
         const float al = m == -INFINITY ? 0.f : expf(m - mx);
         l *= al;
         m = mx;
@@ -363,37 +453,39 @@ __global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a) {
             for (int g = 0; g < GM; g++) {
                 const float r = __shfl_sync(0xffffffffu, al, g << HSH);
 #pragma unroll
-                for (int d = 0; d < 8; d++) acc[g][d] *= r;
+                for (int d = 0; d < DPL; d++) acc[g][d] *= r;
             }
         }
 #pragma unroll
         for (int i = 0; i < NI; i++) {
-            const float4 c0 = vf[i][0], c1 = vf[i][1];
 #pragma unroll
             for (int g = 0; g < GM; g++) {
-                const float p = __shfl_sync(0xffffffffu, s[i], (lane & 24) | (g << HSH));
-                acc[g][0] = fmaf(p, c0.x, acc[g][0]); acc[g][1] = fmaf(p, c0.y, acc[g][1]); acc[g][2] = fmaf(p, c0.z, acc[g][2]); acc[g][3] = fmaf(p, c0.w, acc[g][3]);
-                acc[g][4] = fmaf(p, c1.x, acc[g][4]); acc[g][5] = fmaf(p, c1.y, acc[g][5]); acc[g][6] = fmaf(p, c1.z, acc[g][6]); acc[g][7] = fmaf(p, c1.w, acc[g][7]);
+                const float p = __shfl_sync(0xffffffffu, s[i], (lane & ~(LPK - 1)) | (g << HSH));
+#pragma unroll
+                for (int h = 0; h < NF; h++) {
+                    acc[g][4 * h] = fmaf(p, vf[i][h].x, acc[g][4 * h]); acc[g][4 * h + 1] = fmaf(p, vf[i][h].y, acc[g][4 * h + 1]);
+                    acc[g][4 * h + 2] = fmaf(p, vf[i][h].z, acc[g][4 * h + 2]); acc[g][4 * h + 3] = fmaf(p, vf[i][h].w, acc[g][4 * h + 3]);
+                }
             }
         }
+        if (more) load(vf, a.v, a.ldk, a.v2, a.ldk2, j0 + step);
     }
-    // the four key groups of the warp, then the warps
-    l += __shfl_xor_sync(0xffffffffu, l, 8);
-    l += __shfl_xor_sync(0xffffffffu, l, 16);
+    // the key groups of the warp, then the warps, then the CTAs of the cluster
 #pragma unroll
-    for (int g = 0; g < GM; g++)
+    for (int o = LPK; o < 32; o <<= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, o);
 #pragma unroll
-        for (int d = 0; d < 8; d++) {
-            acc[g][d] += __shfl_xor_sync(0xffffffffu, acc[g][d], 8);
-            acc[g][d] += __shfl_xor_sync(0xffffffffu, acc[g][d], 16);
-        }
+        for (int g = 0; g < GM; g++)
+#pragma unroll
+            for (int d = 0; d < DPL; d++) acc[g][d] += __shfl_xor_sync(0xffffffffu, acc[g][d], o);
+    }
     if (kg == 0) {
         if ((dp & ((1 << HSH) - 1)) == 0) { pm[warp][dp >> HSH] = m; pl[warp][dp >> HSH] = l; }
 #pragma unroll
-        for (int g = 0; g < GM; g++) {
-            *(float4 *)&po[warp][g][4 * dp] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
-            *(float4 *)&po[warp][g][32 + 4 * dp] = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
-        }
+        for (int g = 0; g < GM; g++)
+#pragma unroll
+            for (int h = 0; h < NF; h++)
+                *(float4 *)&po[warp][g][4 * dp + 32 * h] = make_float4(acc[g][4 * h], acc[g][4 * h + 1], acc[g][4 * h + 2], acc[g][4 * h + 3]);
     }
     __syncthreads();
     if (tid < G) {
@@ -403,63 +495,46 @@ __global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a) {
             const float e = (pm[w][tid] == -INFINITY) ? 0.f : expf(pm[w][tid] - M);
             wg[w][tid] = e; L = fmaf(pl[w][tid], e, L);
         }
-        Mg[tid] = M; Lg[tid] = L;
+        cm[tid] = M; cl[tid] = L;
     }
     __syncthreads();
-    float *mine = a.part + ((int64_t)(row * a.Hkv + kvh) * a.max_split + sp) * AD_MAXG * (HD + 2);
+    auto store = [&](int g, int d, float r) {
+        const int64_t at = (int64_t)(q0 + g % nq) * a.ldo + (kvh * Gh + g / nq) * HD + d;
+        if (a.out_lo) store_split1(a.out, a.out_lo, at, r, a.out_fmt);
+        else a.out[at] = r;
+    };
     for (int i = tid; i < G * HD; i += blockDim.x) {
         const int g = i / HD, d = i % HD;
         float O = 0.f;
         for (int w = 0; w < nw; w++) O = fmaf(po[w][g][d], wg[w][g], O);
-        if (nsplit == 1) {
-            const float L = Lg[g];
-            const float r = L > 0.f ? O / L : 0.f;
-            const int64_t at = (int64_t)(q0 + g % nq) * a.ldo + (kvh * Gh + g / nq) * HD + d;
-            if (a.out_lo) store_split1(a.out, a.out_lo, at, r, a.out_fmt);
-            else a.out[at] = r;
-        } else {
-            mine[g * (HD + 2) + 2 + d] = O;
-            if (d == 0) { mine[g * (HD + 2)] = Mg[g]; mine[g * (HD + 2) + 1] = Lg[g]; }
-        }
+        if (nc == 1) store(g, d, cl[g] > 0.f ? O / cl[g] : 0.f);
+        else co[g][d] = O;
     }
-    if (nsplit == 1) return;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-        unsigned old = atomicAdd(a.count + row * a.Hkv + kvh, 1u);
-        s_last = (old == (unsigned)(nsplit - 1));
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // the last CTA of the (row, kv head) merges the CTAs' partials (a handful: 64 to 256 keys each); the weights of a
-    // partial are recomputed where they are used (an exponential per load) rather than staged
-    const float *base = a.part + (int64_t)(row * a.Hkv + kvh) * a.max_split * AD_MAXG * (HD + 2);
+    if (nc == 1) return;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (tid < G) {
-        float M = -INFINITY, L = 0.f;
-        for (int x = 0; x < nsplit; x++) M = fmaxf(M, __ldcg(base + ((int64_t)x * AD_MAXG + tid) * (HD + 2)));
-        for (int x = 0; x < nsplit; x++) {
-            const float *ps = base + ((int64_t)x * AD_MAXG + tid) * (HD + 2);
-            L = fmaf(__ldcg(ps + 1), expf(__ldcg(ps) - M), L);
+        float mc[ADG_MAXC], M = -INFINITY, L = 0.f;
+#pragma unroll
+        for (int c = 0; c < ADG_MAXC; c++) { mc[c] = c < nc ? ld_cluster(&cm[tid], c) : -INFINITY; M = fmaxf(M, mc[c]); }
+#pragma unroll
+        for (int c = 0; c < ADG_MAXC; c++) {
+            const float e = mc[c] == -INFINITY ? 0.f : expf(mc[c] - M);
+            cw[c][tid] = e;
+            if (c < nc) L = fmaf(ld_cluster(&cl[tid], c), e, L);
         }
-        Mg[tid] = M; Lg[tid] = L;
+        wg[0][tid] = L > 0.f ? 1.0f / L : 0.f;
     }
     __syncthreads();
-    for (int i = tid; i < G * HD; i += blockDim.x) {
+    // every CTA closes its share of the pair's outputs
+    for (int i = rank * blockDim.x + tid; i < G * HD; i += nc * blockDim.x) {
         const int g = i / HD, d = i % HD;
-        const float M = Mg[g];
         float O = 0.f;
-        for (int x = 0; x < nsplit; x++) {
-            const float *ps = base + ((int64_t)x * AD_MAXG + g) * (HD + 2);
-            O = fmaf(__ldcg(ps + 2 + d), expf(__ldcg(ps) - M), O);
-        }
-        const float L = Lg[g];
-        const float r = L > 0.f ? O / L : 0.f;
-        const int64_t at = (int64_t)(q0 + g % nq) * a.ldo + (kvh * Gh + g / nq) * HD + d;
-        if (a.out_lo) store_split1(a.out, a.out_lo, at, r, a.out_fmt);
-        else a.out[at] = r;
+#pragma unroll
+        for (int c = 0; c < ADG_MAXC; c++)
+            if (c < nc) O = fmaf(ld_cluster(&co[g][d], c), cw[c][g], O);
+        store(g, d, O * wg[0][g]);
     }
-    if (tid == 0) a.count[row * a.Hkv + kvh] = 0;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // co is read by the others
 }
 
 // ---- head dim 64, many (query, head) pairs per kv group: one WARP per run of 32-key chunks, products on mma.sync ----
@@ -757,7 +832,7 @@ static AttnDecDev decode_args(const AttnArgs &a, int max_split, int cps) {
         count = (unsigned *)dev_alloc(nc * 4); count_cap = nc;
         CUDA_CHECK(cudaMemsetAsync(count, 0, nc * 4, stream()));
     }
-    AttnDecDev d;
+    AttnDecDev d{};
     d.q = a.q; d.ldq = a.ldq; d.k = a.k1; d.v = a.v1; d.ldk = a.ldk1;
     d.k2 = a.k2; d.v2 = a.v2; d.ldk2 = a.ldk2; d.k2_start = a.k2 ? a.k2_start : nullptr; d.out = a.out; d.out_lo = a.out_lo; d.out_fmt = a.out_fmt; d.ldo = a.ldo;
     d.q_start = a.q_start; d.k_start = a.k1_start; d.k_len = a.k1_len;
@@ -766,6 +841,43 @@ static AttnDecDev decode_args(const AttnArgs &a, int max_split, int cps) {
     d.scale = 1.0f / sqrtf((float)a.hd);
     d.part = part; d.count = count;
     return d;
+}
+
+static bool al16(const void *q) { return ((uintptr_t)q & 15) == 0; }
+static bool gqa_shape(const AttnArgs &a) {
+    return a.hd == 64 && (a.H / a.Hkv) * a.max_q <= 8 && (a.ldk1 & 3) == 0 && (!a.k2 || (a.ldk2 & 3) == 0) && al16(a.k1) && al16(a.v1) && (!a.k2 || (al16(a.k2) && al16(a.v2)));
+}
+
+// CTAs of a (row, kv head) pair: with enough pairs to fill the SMs one of four warps; with fewer, eight warps each and a cluster
+// that gives every SM about a CTA, at least a run of keys per warp.
+static void attention_gqa(const AttnArgs &a, const AttnFused &f, bool fused) {
+    const int64_t pairs = (int64_t)a.rows * a.Hkv;
+    const int gq = (a.H / a.Hkv) * a.max_q, gm = gq <= 1 ? 1 : gq <= 2 ? 2 : gq <= 4 ? 4 : 8, sms = ctx().sm_count;
+    const int runs = (int)cdiv(a.max_k1 + a.max_k2, ADG_NI * (gm == 8 ? 2 : 4));
+    const int nw = std::min(pairs >= 2 * (int64_t)sms ? 4 : ADG_MAXW, runs);
+    int nc = 1;
+    while (nc < ADG_MAXC && pairs * nc * 2 <= 2 * (int64_t)sms && nw * nc < runs) nc *= 2;
+    AttnDecDev d{};
+    d.q = a.q; d.ldq = a.ldq; d.k = a.k1; d.v = a.v1; d.ldk = a.ldk1;
+    d.k2 = a.k2; d.v2 = a.v2; d.ldk2 = a.ldk2; d.k2_start = a.k2 ? a.k2_start : nullptr; d.out = a.out; d.out_lo = a.out_lo; d.out_fmt = a.out_fmt; d.ldo = a.ldo;
+    d.q_start = a.q_start; d.k_start = a.k1_start; d.k_len = a.k1_len;
+    d.step_d = a.step_d; d.len_step = a.k1_len_step;
+    d.H = a.H; d.Hkv = a.Hkv; d.rows = a.rows; d.scale = 1.0f / sqrtf((float)a.hd);
+    const dim3 grid((unsigned)nc, (unsigned)a.Hkv, (unsigned)a.rows);
+    ProfScope ps(NCMB_K_ATTN, 4.0 * (double)a.total_q * a.avg_keys * a.H * a.hd, 0);
+#define GQA_LAUNCH(GM_) do { if (fused) launch_pdl_cluster(k_attention_dec_gqa<GM_, true>, grid, dim3(nw * 32), nc, d, f); \
+                             else launch_pdl_cluster(k_attention_dec_gqa<GM_, false>, grid, dim3(nw * 32), nc, d, f); } while (0)
+    if (gm == 1) GQA_LAUNCH(1);
+    else if (gm == 2) GQA_LAUNCH(2);
+    else if (gm == 4) GQA_LAUNCH(4);
+    else GQA_LAUNCH(8);
+#undef GQA_LAUNCH
+}
+
+bool attention_fused_supported(const AttnArgs &a) { return gqa_shape(a) && a.max_q == 1 && !a.k2 && a.k1_len && !a.causal && !a.window && a.max_k1 > 0; }
+void attention_fused(const AttnArgs &a, const FewQkv &q) {
+    AttnFused f{q.part, q.S, q.bias, q.cos_t, q.sin_t, q.pos, q.pos_step, q.kv, q.seq_pitch, q.step};
+    attention_gqa(a, f, true);
 }
 
 void attention_decode(const AttnArgs &a) {
@@ -780,10 +892,9 @@ void attention_decode(const AttnArgs &a) {
     // tensor-core kernel (read per call: the tests run every kernel on the same inputs)
     const char *mma_s = getenv("NCM_B200_ATTN_DEC_MMA");
     const int mma_env = mma_s ? atoi(mma_s) : -1;
-    auto al16 = [](const void *q) { return ((uintptr_t)q & 15) == 0; };
     const bool mma_takes = a.hd == 64 && gq_w <= AD_MAXG && ((a.ldk1 & 3) == 0) && (!a.k2 || (a.ldk2 & 3) == 0) && ((a.ldq & 3) == 0) &&
                            al16(a.q) && al16(a.k1) && al16(a.v1) && (!a.k2 || (al16(a.k2) && al16(a.v2)));
-    const bool gqa_takes = mma_takes && gq_w <= 8 && mma_env != 1;
+    const bool gqa_takes = gqa_shape(a) && ((a.ldq & 3) == 0) && al16(a.q) && mma_env != 1;
     // (measured: the 4-token level of config 2 -- 16 pairs per group, 9 chunks -- 2.99 -> 2.44 ms over its 12 layers; the
     // Qwen2 batched-decode shape -- 7 pairs, 16 - 32 chunks -- at 256 sequences 42 936 -> 44 923 tokens/s, at 32
     // sequences 12 821 -> 12 661: with few (row, kv head) pairs the CTA-per-chunk kernels spread a row over more SMs)
@@ -806,23 +917,7 @@ void attention_decode(const AttnArgs &a) {
             return;
         }
     }
-    if (gqa_takes) {
-        // Enough (row, kv head) pairs to fill the SMs: four warps take all keys of a pair. Fewer: eight warps, and the row is cut
-        // over as many CTAs as give every SM one, at least a run of keys per warp.
-        const int runs = (int)cdiv(a.max_k1 + a.max_k2, ADG_RUN);
-        const int nw = pairs >= 2 * (int64_t)ctx().sm_count ? std::min(4, runs) : std::min(ADG_MAXW, runs);
-        int split = (int)std::max<int64_t>(1, std::min<int64_t>(ctx().sm_count / pairs, cdiv(runs, nw)));
-        if (split > AD_MAXSPLIT) split = AD_MAXSPLIT;
-        const int cps = (int)cdiv(runs, (int64_t)nw * split);
-        AttnDecDev d = decode_args(a, (int)cdiv(runs, (int64_t)nw * cps), cps);
-        dim3 grid((unsigned)d.max_split, (unsigned)a.Hkv, (unsigned)a.rows);
-        ProfScope ps(NCMB_K_ATTN, 4.0 * (double)a.total_q * a.avg_keys * a.H * a.hd, 0);
-        if (gq_w <= 1) LAUNCH_PDL((k_attention_dec_gqa<1>), grid, nw * 32, 0, d);
-        else if (gq_w <= 2) LAUNCH_PDL((k_attention_dec_gqa<2>), grid, nw * 32, 0, d);
-        else if (gq_w <= 4) LAUNCH_PDL((k_attention_dec_gqa<4>), grid, nw * 32, 0, d);
-        else LAUNCH_PDL((k_attention_dec_gqa<8>), grid, nw * 32, 0, d);
-        return;
-    }
+    if (gqa_takes) { attention_gqa(a, AttnFused{}, false); return; }
     static const int per_sm = getenv("NCM_B200_ATTN_DEC_PER_SM") ? atoi(getenv("NCM_B200_ATTN_DEC_PER_SM")) : 8;
     int want_split = (int)std::min<int64_t>(max_chunks, cdiv((int64_t)ctx().sm_count * per_sm, pairs));
     if (want_split < 1) want_split = 1;

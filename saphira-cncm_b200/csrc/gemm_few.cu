@@ -26,7 +26,7 @@ constexpr int fw_stages(int NT, bool W2) {
     int s = (110 * 1024) / fw_stage(NT, W2);
     return s > 4 ? 4 : (s < 2 ? 2 : s);
 }
-constexpr int fw_threads(int NT) { return NT >= 64 ? 320 : 192; }
+constexpr int FW_THREADS = 320;          // producer warp, MMA warp, eight epilogue warps (two per TMEM quadrant)
 constexpr size_t fw_smem(int NT, bool W2) { return 1024 + (size_t)fw_stages(NT, W2) * fw_stage(NT, W2) + (2 * fw_stages(NT, W2) + 1) * 8 + 16; }
 
 struct FewDev {
@@ -38,16 +38,20 @@ struct FewDev {
     int *err;
 };
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+// eight columns each of two accumulators
+__device__ __forceinline__ void tmem_ld8x2(uint32_t ta, uint32_t tb, uint32_t *a, uint32_t *b) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n\t"
                  "tcgen05.wait::ld.sync.aligned;"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
+                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]),
+                   "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7])
+                 : "r"(ta), "r"(tb) : "memory");
 }
+// silu through ex2.approx / rcp.approx, as in the fp16-pair engine's gated epilogue; the other activations as everywhere
+__device__ __forceinline__ float fw_act(float v, int act) { return act == ACT_SILU ? __fdividef(v, 1.0f + __expf(-v)) : tc_act(v, act); }
 
 template <int NT, bool W2>
-__global__ void __launch_bounds__(fw_threads(NT)) k_gemm_few(const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmW2,
+__global__ void __launch_bounds__(FW_THREADS) k_gemm_few(const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmW2,
                                                             const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2, FewDev a) {
     constexpr int ST = fw_stages(NT, W2), STAGE = fw_stage(NT, W2), WB = FW_WTILE * (W2 ? 2 : 1), XT = fw_xtile(NT);
     constexpr int COLS = 2 * NT;                             // W1 x1 (+ W2 x1) in the first NT columns, W1 x2 in the rest
@@ -129,43 +133,46 @@ __global__ void __launch_bounds__(fw_threads(NT)) k_gemm_few(const __grid_consta
             umma_commit(done);
         }
     } else {
-        constexpr int HALVES = NT >= 64 ? 2 : 1;             // with 64 tokens and more, two warps share a TMEM quadrant's columns
-        const int q = warp & 3, t_half = (warp - 2) >> 2;
+        const int q = warp & 3, t_half = (warp - 2) >> 2;    // two warps share a quadrant's columns, eight tokens at a time
         const int n = n0 + q * 32 + lane;                    // this thread's weight row = output column
         const float b = (a.bias && n < a.N) ? a.bias[n] : 0.f;
         pdl_wait();                                          // earlier readers of y / part have finished
         const bool ok = mbar_wait(done, 0, a.err, 54);
         tc_fence_after();
-        const int64_t srow = (int64_t)blockIdx.y * a.M + m0;
-        for (int t0 = t_half * (NT / HALVES); ok && t0 < (t_half + 1) * (NT / HALVES) && t0 < rows; t0 += 16) {
-            uint32_t r[16], r2[16];
-            tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)t0, r);
-            tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(NT + t0), r2);
+        const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+        for (int t0 = t_half * 8; ok && t0 < rows; t0 += 16) {
+            uint32_t r[8], r2[8];
+            tmem_ld8x2(trow + (uint32_t)t0, trow + (uint32_t)(NT + t0), r, r2);
+            float v[8];
 #pragma unroll
-            for (int t = 0; t < 16; t++) {
-                float v = (__uint_as_float(r[t]) + __uint_as_float(r2[t])) * a.acc_scale;
-                const bool on = t0 + t < rows && n < a.N;
-                if (a.part) {
-                    if (on) a.part[(srow + t0 + t) * a.N + n] = v;
-                    continue;
-                }
-                v += b;
-                if (a.glu) {                                 // even lanes hold gates, odd lanes the up row of the same unit
-                    const float u = __shfl_down_sync(0xffffffffu, v, 1);
-                    v = __fmul_rn(tc_act(v, a.act), u);
-                    if (on && !(lane & 1)) {
-                        const int64_t at = (int64_t)(m0 + t0 + t) * a.ldy + (n >> 1);
-                        if (a.y_lo) store_split1(a.y, a.y_lo, at, v, SPLIT_H16);
-                        else a.y[at] = v;
+            for (int t = 0; t < 8; t++) v[t] = (__uint_as_float(r[t]) + __uint_as_float(r2[t])) * a.acc_scale + b;
+            if (a.part) {
+                float *p = a.part + ((int64_t)blockIdx.y * a.M + m0 + t0) * a.N + n;
+#pragma unroll
+                for (int t = 0; t < 8; t++)
+                    if (t0 + t < rows && n < a.N) p[(int64_t)t * a.N] = v[t];
+            } else if (a.glu) {
+                // even lanes hold a unit's gate, odd lanes its up row: the pair exchanges so that each has both of one of two tokens
+                const bool odd = lane & 1;
+                const int64_t at = (int64_t)(m0 + t0 + (odd ? 1 : 0)) * a.ldy + (n >> 1);
+#pragma unroll
+                for (int t = 0; t < 8; t += 2) {
+                    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[t] : v[t + 1], 1);
+                    const float o = __fmul_rn(fw_act(odd ? got : v[t], a.act), odd ? v[t + 1] : got);
+                    if (t0 + t + (odd ? 1 : 0) < rows && n < a.N) {
+                        if (a.y_lo) store_split1(a.y, a.y_lo, at + t * a.ldy, o, SPLIT_H16);
+                        else a.y[at + t * a.ldy] = o;
                     }
-                    continue;
                 }
-                v = tc_act(v, a.act);
-                if (on) {
-                    const int64_t at = (int64_t)(m0 + t0 + t) * a.ldy + n;
-                    if (a.y_lo) store_split1(a.y, a.y_lo, at, v, SPLIT_H16);
-                    else a.y[at] = v;
-                }
+            } else {
+                const int64_t at = (int64_t)(m0 + t0) * a.ldy + n;
+#pragma unroll
+                for (int t = 0; t < 8; t++)
+                    if (t0 + t < rows && n < a.N) {
+                        const float o = fw_act(v[t], a.act);
+                        if (a.y_lo) store_split1(a.y, a.y_lo, at + t * a.ldy, o, SPLIT_H16);
+                        else a.y[at + t * a.ldy] = o;
+                    }
             }
         }
     }
@@ -180,14 +187,16 @@ __global__ void __launch_bounds__(fw_threads(NT)) k_gemm_few(const __grid_consta
 // ---- what follows a sliced product in a block ----
 // One CTA per row: the slices' sums, bias and residual, then the norm of the row as an fp16 pair for the next product. The row
 // stays in registers between the two (C up to 4096).
-constexpr int FR_T = 256, FR_V = 4;
+constexpr int FR_T = 256, FR_V = 4, FR_IN = 12;
 __global__ void __launch_bounds__(FR_T) k_few_reduce_norm(float *__restrict__ x, const float *__restrict__ part, int S, const float *__restrict__ bias, int rows, int C,
                                                          int ln_kind, const float *__restrict__ ln_w, const float *__restrict__ ln_b, float eps,
                                                          unsigned short *__restrict__ y1, unsigned short *__restrict__ y2) {
     __shared__ float red[2][FR_T / 32];
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c4n = C >> 2;
-    pdl_launch_dependents();
+    // the successor may start only once everything before this kernel is complete: attention reads the cache and the step
+    // counter before it waits for the product that follows here
     pdl_wait();
+    pdl_launch_dependents();
     float4 v[FR_V];
 #pragma unroll
     for (int i = 0; i < FR_V; i++) {
@@ -200,15 +209,15 @@ __global__ void __launch_bounds__(FR_T) k_few_reduce_norm(float *__restrict__ x,
             const int64_t step = (int64_t)rows * C;
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
             int s = 0;
-            for (; s + 4 <= S; s += 4) {
-                const float4 p0 = __ldcg((const float4 *)(p + s * step)), p1 = __ldcg((const float4 *)(p + (s + 1) * step));
-                const float4 p2 = __ldcg((const float4 *)(p + (s + 2) * step)), p3 = __ldcg((const float4 *)(p + (s + 3) * step));
-                a.x += p0.x; a.y += p0.y; a.z += p0.z; a.w += p0.w;
-                a.x += p1.x; a.y += p1.y; a.z += p1.z; a.w += p1.w;
-                a.x += p2.x; a.y += p2.y; a.z += p2.z; a.w += p2.w;
-                a.x += p3.x; a.y += p3.y; a.z += p3.z; a.w += p3.w;
+            for (; s < S; s += FR_IN) {                          // FR_IN slices in flight (absent ones are not added)
+                float4 t[FR_IN];
+#pragma unroll
+                for (int u = 0; u < FR_IN; u++)
+                    if (s + u < S) t[u] = __ldcg((const float4 *)(p + (s + u) * step));
+#pragma unroll
+                for (int u = 0; u < FR_IN; u++)
+                    if (s + u < S) { a.x += t[u].x; a.y += t[u].y; a.z += t[u].z; a.w += t[u].w; }
             }
-            for (; s < S; s++) { const float4 p0 = __ldcg((const float4 *)(p + s * step)); a.x += p0.x; a.y += p0.y; a.z += p0.z; a.w += p0.w; }
             if (bias) { const float4 b = __ldg((const float4 *)(bias + c * 4)); a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
             v[i] = make_float4(a.x + r.x, a.y + r.y, a.z + r.z, a.w + r.w);
             *(float4 *)(x + (int64_t)row * C + c * 4) = v[i];
@@ -293,12 +302,12 @@ __global__ void __launch_bounds__(256) k_few_reduce_qkv(FewQkv a) {
 bool gemm_few_supported(int64_t M, int N, int K) {
     return ctx().gemm_mode >= 3 && M >= 5 && M <= FEW_MAX_ROWS && N >= 32 && K >= 32 && (K & 7) == 0;
 }
-// Slices of K: as many as give every SM one CTA, each at least one 64-wide step; a slice more costs another read of the rows in
+// Slices of K: as many as give every SM one CTA, each at least two 64-wide steps; a slice more costs another read of the rows in
 // the kernel that adds them, so a long row count takes fewer.
 int gemm_few_slices(int M, int N, int K, int max_slices) {
     const int tiles = (int)(cdiv(N, 128) * cdiv(M, 128)), nkb = (int)cdiv(K, 64);
     int s = std::max(1, ctx().sm_count / tiles);
-    s = std::min(std::min(s, nkb), max_slices);
+    s = std::min(std::min(s, std::max(1, nkb / 2)), max_slices);
     const int kb_per = (int)cdiv(nkb, s);
     return (int)cdiv(nkb, kb_per);
 }
@@ -309,7 +318,7 @@ static void launch_few(const FewGemm &g, const FewDev &d, const H3Weights &w, in
     if (!set) { CUDA_CHECK(cudaFuncSetAttribute((k_gemm_few<NT, W2>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fw_smem(NT, W2))); set = true; }
     const CUtensorMap mw1 = tc_get_map_h16(w.v1, g.N, g.K, g.K, 128), mw2 = tc_get_map_h16(w.v2, g.N, g.K, g.K, 128);
     const CUtensorMap mx1 = tc_get_map_h16(g.x1, g.M, g.K, g.ldx, NT), mx2 = tc_get_map_h16(g.x2, g.M, g.K, g.ldx, NT);
-    LAUNCH_PDL((k_gemm_few<NT, W2>), dim3((unsigned)cdiv(g.N, 128), (unsigned)slices, (unsigned)cdiv(g.M, NT)), fw_threads(NT), fw_smem(NT, W2), mw1, mw2, mx1, mx2, d);
+    LAUNCH_PDL((k_gemm_few<NT, W2>), dim3((unsigned)cdiv(g.N, 128), (unsigned)slices, (unsigned)cdiv(g.M, NT)), FW_THREADS, fw_smem(NT, W2), mw1, mw2, mx1, mx2, d);
 }
 
 void gemm_few(const FewGemm &g) {

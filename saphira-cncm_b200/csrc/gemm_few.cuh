@@ -36,6 +36,11 @@ struct FewQkv {
 };
 void few_reduce_qkv(const FewQkv &a);
 
+// Decode attention that takes q and the new token's k | v from the slices itself and appends k | v to the cache
+// (attention_decode.cu): one query per row, cached keys only, head dim 64, up to eight query heads per kv head.
+bool attention_fused_supported(const AttnArgs &a);
+void attention_fused(const AttnArgs &a, const FewQkv &q);
+
 // the fp16 pair of a static weight matrix [N][K], its scale and whether the second half is all zero (gemm_h3.cu)
 struct H3Weights { const unsigned short *v1, *v2; float scale; bool v2_zero; };
 H3Weights gemm_h3_weights(const float *W, int64_t n);

@@ -77,7 +77,7 @@ unsigned short *dev_bf16_exact(const float *w, int64_t n) {
 static Workspace &block_lo_ws() { static Workspace w; return w; }
 
 // The attention call of a block whose q (and, for own-pass keys, k | v) sit in b.qkv.
-static void block_attention(const BlockBufs &b, const AttnPlan &p, int64_t ntok, int C, int H, int nkv, float *ctx_lo, int fmt) {
+static AttnArgs attention_args(const BlockBufs &b, const AttnPlan &p, int64_t ntok, int C, int H, int nkv, float *ctx_lo, int fmt) {
     const int hd = C / H, kvd = nkv * hd, Wq = C + 2 * kvd;
     float *kp = b.qkv + C, *vp = b.qkv + C + kvd;
     AttnArgs a;
@@ -95,7 +95,7 @@ static void block_attention(const BlockBufs &b, const AttnPlan &p, int64_t ntok,
     a.max_k1 = p.max_k1; a.max_k2 = p.self_is_k2 ? p.max_q : (p.k2 ? p.max_k2 : 0);
     a.step_d = p.step_d; a.k1_len_step = p.k1_len_step;
     a.q_total = ntok; a.k1_total = p.k1 ? p.k1_total : ntok; a.k2_total = p.self_is_k2 ? ntok : (p.k2 ? p.k2_total : 0);
-    attention(a);
+    return a;
 }
 
 // Slices of K a product of M rows may be cut into: every slice is written and read once more (8 bytes per output), which for
@@ -110,7 +110,7 @@ bool few_chain_supported(int64_t ntok, int C, int H, int nkv, const BlockWeights
 }
 
 // One block for a few rows: four products on the weight-streaming kernel, and what lies between them folded into the kernels
-// that add the slices of the first, second and last -- eight launches, where the general path takes eleven to thirteen.
+// that add the slices of the first, second and last -- seven launches for a decode step, eight otherwise, where the general path takes eleven to thirteen.
 static void run_block_few(float *x, int64_t ntok, int C, int H, int nkv, const BlockWeights &w, const BlockBufs &b, const AttnPlan &p) {
     FewChain &fc = *p.few;
     const int hd = C / H, kvd = nkv * hd, Wq = C + 2 * kvd, M = (int)ntok, ms = few_max_slices(ntok);
@@ -134,9 +134,13 @@ static void run_block_few(float *x, int64_t ntok, int C, int H, int nkv, const B
     q.q = b.qkv; q.ldq = Wq; q.kv_self = (!p.k1 || p.self_is_k2 || p.kv_store == nullptr) ? 1 : 0;
     q.kv = p.kv_store; q.rps = p.kv_rows_per_seq > 0 ? p.kv_rows_per_seq : M; q.seq_pitch = p.kv_seq_pitch; q.pitch = p.kv_pitch; q.step = p.kv_store_step;
     q.hd = hd;
-    few_reduce_qkv(q);
-    if (p.kv_only) return;
-    block_attention(b, p, ntok, C, H, nkv, ctx_lo, SPLIT_H16);
+    const AttnArgs at = attention_args(b, p, ntok, C, H, nkv, ctx_lo, SPLIT_H16);
+    if (!q.kv_self && p.kv_rows_per_seq == 1 && p.rows == M && attention_fused_supported(at)) attention_fused(at, q);
+    else {
+        few_reduce_qkv(q);
+        if (p.kv_only) return;
+        attention(at);
+    }
     g = FewGemm{b.ctx, ctx_lo, C, w.ow, M, C, C};
     g.part = part; g.max_slices = ms;
     gemm_few(g);
@@ -223,7 +227,7 @@ void run_block(float *x, int64_t ntok, int C, int H, int nkv, const BlockWeights
                p.kv_rows_per_seq, p.kv_seq_pitch, ntok, width4, p.step_d, p.kv_store_step);
     }
     if (p.kv_only) return;
-    block_attention(b, p, ntok, C, H, nkv, ctx_lo, fmt);
+    attention(attention_args(b, p, ntok, C, H, nkv, ctx_lo, fmt));
     // x += ctx Wo^T + bo
     g = GemmArgs();
     g.x_fmt = fmt;
