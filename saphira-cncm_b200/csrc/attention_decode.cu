@@ -24,10 +24,10 @@ namespace ncmb {
 
 // programmatic dependent launch (see launch_pdl) of clusters of nc CTAs along x
 template <typename... KArgs, typename... Args>
-static void launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, int nc, Args... args) {
+static void launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int nc, Args... args) {
     static const bool off = getenv("NCM_B200_NO_PDL") != nullptr;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = block; cfg.stream = stream();
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream();
     cudaLaunchAttribute at[2];
     int n = 0;
     if (nc > 1) { at[n].id = cudaLaunchAttributeClusterDimension; at[n].val.clusterDim.x = (unsigned)nc; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1; n++; }
@@ -275,8 +275,9 @@ __global__ void __launch_bounds__(AD_THREADS) k_attention_decode(AttnDecDev a) {
 // the query (in registers for all GM pairs) and of the context (accumulated in registers); a warp's loads are full 128-byte
 // lines. The partial dot products of a key meet by a reduce-scatter that leaves one pair's score in a lane (eight shuffles for
 // eight pairs), the softmax runs on those, and the probabilities travel back by one shuffle per pair and key. Nothing goes
-// through shared memory until a warp's keys are done. A warp takes runs of four loads (8 or 16 keys): the values of a run and
-// the keys of the next are requested before the run's arithmetic. The CTAs of a cluster share the keys of a (row, kv head) pair,
+// between lanes through shared memory until a warp's keys are done. A warp takes runs of four loads (8 or 16 keys); each lane
+// keeps the loads of its next runs in flight with cp.async into slots of its own (a longer register file, no
+// barrier): holding a run ahead in registers left 48 KB in flight per SM and a third of the bandwidth. The CTAs of a cluster share the keys of a (row, kv head) pair,
 // their warps interleaving runs, and merge over distributed shared memory.
 //
 // FUSED (decode steps): q, k and v of the new token arrive as the slices of the QKV product. Every CTA adds what its heads
@@ -286,7 +287,8 @@ __global__ void __launch_bounds__(AD_THREADS) k_attention_decode(AttnDecDev a) {
 //
 // Bound: the K|V cache read once; for few rows the chain product -> sums -> scores -> merge.
 constexpr int ADG_NI = 4;              // loads of a run per lane
-constexpr int ADG_MAXW = 8;            // warps of a CTA at most
+constexpr int adg_depth(int GM) { return GM > 4 ? 4 : 2; }   // runs in flight per warp, the current one included (16 KB per warp either way)
+constexpr int ADG_MAXW = 4;            // warps of a CTA at most
 constexpr int ADG_MAXC = 8;            // CTAs of a cluster at most
 
 struct AttnFused {                     // see FewQkv: slices of the QKV product of a decode step, one token per row
@@ -294,6 +296,14 @@ struct AttnFused {                     // see FewQkv: slices of the QKV product 
     const float *cos_t, *sin_t; const int *pos; int64_t pos_step;
     float *kv; int64_t seq_pitch, step;      // cache position of the new token: kv + row * seq_pitch + *step_d * step, k | v of all kv heads
 };
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool on) {      // off: the slot is zeroed
+    const int n = on ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+// a slot holds NI loads of keys and NI of values per lane, 16 bytes each (twice where a lane keeps eight dims)
+constexpr size_t adg_smem(int GM, int nw) { return (size_t)nw * adg_depth(GM) * 2 * ADG_NI * (GM > 4 ? 1 : 2) * 512; }
 
 __device__ __forceinline__ float ld_cluster(const float *p, unsigned rank) {
     uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
@@ -304,8 +314,9 @@ __device__ __forceinline__ float ld_cluster(const float *p, unsigned rank) {
 }
 
 template <int GM, bool FUSED>
-__global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a, AttnFused f) {
-    constexpr int HD = 64, LPK = GM > 4 ? 16 : 8, DPL = HD / LPK, NF = DPL / 4, KPI = 32 / LPK, NI = ADG_NI, RUN = NI * KPI;
+__global__ void __launch_bounds__(ADG_MAXW * 32) k_attention_dec_gqa(AttnDecDev a, AttnFused f) {
+    extern __shared__ __align__(16) float4 adg_ring[];
+    constexpr int HD = 64, LPK = GM > 4 ? 16 : 8, DPL = HD / LPK, NF = DPL / 4, KPI = 32 / LPK, NI = ADG_NI, RUN = NI * KPI, DEPTH = adg_depth(GM);
     constexpr int LOG = GM == 8 ? 3 : GM == 4 ? 2 : GM == 2 ? 1 : 0, HSH = (LPK == 16 ? 4 : 3) - LOG;   // lane dp holds pair dp >> HSH
     __shared__ float pm[ADG_MAXW][GM], pl[ADG_MAXW][GM], wg[ADG_MAXW][GM];
     __shared__ __align__(16) float po[ADG_MAXW][GM][HD];
@@ -327,57 +338,72 @@ __global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a, AttnFus
     const int q0 = a.q_start[row], nq = FUSED ? 1 : a.q_start[row + 1] - q0;
     const int G = Gh * nq;                                   // virtual heads: vh = g * nq + qi
     const int first = (warp * nc + rank) * RUN, step = nw * nc * RUN;
-    float4 kf[NI][NF], vf[NI][NF];
+    float4 *ring = adg_ring + (size_t)warp * DEPTH * 2 * NI * NF * 32 + lane;        // [slot][keys | values][load][half][lane]
     // dims of a lane: 4 dp .. (and 32 + 4 dp .. where it holds eight)
-    auto load = [&](float4 (&r)[NI][NF], const float *s1, int64_t ld1, const float *s2, int64_t ld2, int j0) {
+    int jl = first;                                          // first key of the next run to request
+    auto request = [&](int slot) {
+        float4 *dst = ring + slot * 2 * NI * NF * 32;
+        if (jl < n1) {                                       // (positions without a cached key are zeroed)
 #pragma unroll
-        for (int i = 0; i < NI; i++) {
-            const int j = j0 + KPI * i + kg;
-            const float *p = nullptr;
-            if (j < cached) p = (j < n1s ? s1 + (int64_t)(k00 + j) * ld1 : s2 + (int64_t)(k20 + j - n1s) * ld2) + kvh * HD + 4 * dp;
+            for (int i = 0; i < NI; i++) {
+                const int j = jl + KPI * i + kg;
+                const bool on = j < cached, seg1 = j < n1s;
+                const int64_t at = on ? (seg1 ? (int64_t)(k00 + j) * a.ldk : (int64_t)(k20 + j - n1s) * a.ldk2) + kvh * HD + 4 * dp : 0;
+                const float *kp = seg1 || !on ? a.k : a.k2, *vp = seg1 || !on ? a.v : a.v2;
 #pragma unroll
-            for (int h = 0; h < NF; h++) r[i][h] = p ? *(const float4 *)(p + 32 * h) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int h = 0; h < NF; h++) {
+                    cp_async16(smem_addr(dst + (i * NF + h) * 32), kp + at + 32 * h, on);
+                    cp_async16(smem_addr(dst + ((NI + i) * NF + h) * 32), vp + at + 32 * h, on);
+                }
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        jl += step;
     };
-    if (first < cached) {
-        load(kf, a.k, a.ldk, a.k2, a.ldk2, first);
-        load(vf, a.v, a.ldk, a.v2, a.ldk2, first);
-    } else {
 #pragma unroll
-        for (int i = 0; i < NI; i++)
-#pragma unroll
-            for (int h = 0; h < NF; h++) kf[i][h] = vf[i][h] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    for (int r = 0; r < DEPTH - 1; r++) request(r);
     if constexpr (FUSED) {
-        pdl_wait();
         const int Wq = (a.H + 2 * a.Hkv) * HD;
-        for (int it = tid; it < (Gh + 2) * (HD / 2); it += blockDim.x) {
-            const int hh = it / (HD / 2), d = it % (HD / 2);
+        const int64_t rot = f.cos_t ? (int64_t)f.pos[st * f.pos_step + row] * HD : 0;
+        pdl_wait();
+        for (int it = tid; it < (Gh + 2) * 8; it += blockDim.x) {            // four rotation pairs (d, d + 32) each
+            const int hh = it >> 3, d = (it & 7) * 4;
             const int h = hh < Gh ? kvh * Gh + hh : (hh == Gh ? a.H + kvh : a.H + a.Hkv + kvh);
             const float *p = f.part + (int64_t)row * Wq + h * HD + d;
             const int64_t ps = (int64_t)a.rows * Wq;
-            float v0 = 0.f, v1 = 0.f;
+            float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
             for (int s = 0; s < f.S; s += 8) {
-                float t0[8], t1[8];
+                float4 t0[8], t1[8];
 #pragma unroll
                 for (int u = 0; u < 8; u++)
-                    if (s + u < f.S) { t0[u] = __ldcg(p + (s + u) * ps); t1[u] = __ldcg(p + (s + u) * ps + HD / 2); }
+                    if (s + u < f.S) { t0[u] = __ldcg((const float4 *)(p + (s + u) * ps)); t1[u] = __ldcg((const float4 *)(p + (s + u) * ps + HD / 2)); }
 #pragma unroll
                 for (int u = 0; u < 8; u++)
-                    if (s + u < f.S) { v0 += t0[u]; v1 += t1[u]; }
+                    if (s + u < f.S) {
+                        v0.x += t0[u].x; v0.y += t0[u].y; v0.z += t0[u].z; v0.w += t0[u].w;
+                        v1.x += t1[u].x; v1.y += t1[u].y; v1.z += t1[u].z; v1.w += t1[u].w;
+                    }
             }
-            if (f.bias) { v0 += __ldg(f.bias + h * HD + d); v1 += __ldg(f.bias + h * HD + d + HD / 2); }
+            if (f.bias) {
+                const float4 b0 = __ldg((const float4 *)(f.bias + h * HD + d)), b1 = __ldg((const float4 *)(f.bias + h * HD + d + HD / 2));
+                v0.x += b0.x; v0.y += b0.y; v0.z += b0.z; v0.w += b0.w;
+                v1.x += b1.x; v1.y += b1.y; v1.z += b1.z; v1.w += b1.w;
+            }
             if (f.cos_t && hh <= Gh) {
-                const int64_t at = (int64_t)f.pos[st * f.pos_step + row] * HD + d;
-                const float y0 = __fadd_rn(__fmul_rn(v0, f.cos_t[at]), __fmul_rn(-v1, f.sin_t[at]));
-                const float y1 = __fadd_rn(__fmul_rn(v1, f.cos_t[at + HD / 2]), __fmul_rn(v0, f.sin_t[at + HD / 2]));
-                v0 = y0; v1 = y1;
+                const float4 c0 = *(const float4 *)(f.cos_t + rot + d), c1 = *(const float4 *)(f.cos_t + rot + d + HD / 2);
+                const float4 s0 = *(const float4 *)(f.sin_t + rot + d), s1 = *(const float4 *)(f.sin_t + rot + d + HD / 2);
+                auto turn = [](float &x, float &y, float ca, float sa, float cb, float sb) {
+                    const float y0 = __fadd_rn(__fmul_rn(x, ca), __fmul_rn(-y, sa)), y1 = __fadd_rn(__fmul_rn(y, cb), __fmul_rn(x, sb));
+                    x = y0; y = y1;
+                };
+                turn(v0.x, v1.x, c0.x, s0.x, c1.x, s1.x); turn(v0.y, v1.y, c0.y, s0.y, c1.y, s1.y);
+                turn(v0.z, v1.z, c0.z, s0.z, c1.z, s1.z); turn(v0.w, v1.w, c0.w, s0.w, c1.w, s1.w);
             }
             const int slot = hh < Gh ? hh : GM + hh - Gh;
-            qn[slot][d] = v0; qn[slot][d + HD / 2] = v1;
+            *(float4 *)&qn[slot][d] = v0; *(float4 *)&qn[slot][d + HD / 2] = v1;
             if (hh >= Gh && rank == 0) {
                 float *kv = f.kv + (int64_t)row * f.seq_pitch + st * f.step + (h - a.H) * HD + d;
-                kv[0] = v0; kv[HD / 2] = v1;
+                *(float4 *)kv = v0; *(float4 *)(kv + HD / 2) = v1;
             }
         }
         __syncthreads();
@@ -399,13 +425,21 @@ __global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a, AttnFus
     for (int g = 0; g < GM; g++)
 #pragma unroll
         for (int d = 0; d < DPL; d++) acc[g][d] = 0.f;
+    int slot = 0;
     for (int j0 = first; j0 < n1; j0 += step) {
+        request((slot + DEPTH - 1) % DEPTH);
+        asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH - 1) : "memory");
+        float4 kf[NI][NF], vf[NI][NF];
+#pragma unroll
+        for (int i = 0; i < NI; i++)
+#pragma unroll
+            for (int h = 0; h < NF; h++) kf[i][h] = ring[(slot * 2 * NI * NF + i * NF + h) * 32];
         if constexpr (FUSED) {                                // the new token's key and value
 #pragma unroll
             for (int i = 0; i < NI; i++)
                 if (j0 + KPI * i + kg == cached) {
 #pragma unroll
-                    for (int h = 0; h < NF; h++) { kf[i][h] = *(const float4 *)&qn[GM][4 * dp + 32 * h]; vf[i][h] = *(const float4 *)&qn[GM + 1][4 * dp + 32 * h]; }
+                    for (int h = 0; h < NF; h++) kf[i][h] = *(const float4 *)&qn[GM][4 * dp + 32 * h];
                 }
         }
         float s[NI];
@@ -436,8 +470,13 @@ __global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a, AttnFus
             for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
             s[i] = (j0 + KPI * i + kg < n1) ? v[0] : -INFINITY;
         }
-        const bool more = j0 + step < n1;
-        if (more) load(kf, a.k, a.ldk, a.k2, a.ldk2, j0 + step);
+#pragma unroll
+        for (int i = 0; i < NI; i++)
+#pragma unroll
+            for (int h = 0; h < NF; h++) {
+                vf[i][h] = ring[(slot * 2 * NI * NF + (NI + i) * NF + h) * 32];
+                if (FUSED && j0 + KPI * i + kg == cached) vf[i][h] = *(const float4 *)&qn[FUSED ? GM + 1 : 0][4 * dp + 32 * h];
+            }
         float mx = m;
 #pragma unroll
         for (int i = 0; i < NI; i++) mx = fmaxf(mx, s[i]);
@@ -468,8 +507,9 @@ __global__ void __launch_bounds__(256) k_attention_dec_gqa(AttnDecDev a, AttnFus
                 }
             }
         }
-        if (more) load(vf, a.v, a.ldk, a.v2, a.ldk2, j0 + step);
+        slot = (slot + 1) % DEPTH;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     // the key groups of the warp, then the warps, then the CTAs of the cluster
 #pragma unroll
     for (int o = LPK; o < 32; o <<= 1) {
@@ -848,15 +888,15 @@ static bool gqa_shape(const AttnArgs &a) {
     return a.hd == 64 && (a.H / a.Hkv) * a.max_q <= 8 && (a.ldk1 & 3) == 0 && (!a.k2 || (a.ldk2 & 3) == 0) && al16(a.k1) && al16(a.v1) && (!a.k2 || (al16(a.k2) && al16(a.v2)));
 }
 
-// CTAs of a (row, kv head) pair: with enough pairs to fill the SMs one of four warps; with fewer, eight warps each and a cluster
-// that gives every SM about a CTA, at least a run of keys per warp.
+// CTAs of a (row, kv head) pair: a cluster of as many (up to eight) as keep all CTAs resident at once, three of four warps per
+// SM, each warp with at least a run of keys.
 static void attention_gqa(const AttnArgs &a, const AttnFused &f, bool fused) {
     const int64_t pairs = (int64_t)a.rows * a.Hkv;
     const int gq = (a.H / a.Hkv) * a.max_q, gm = gq <= 1 ? 1 : gq <= 2 ? 2 : gq <= 4 ? 4 : 8, sms = ctx().sm_count;
     const int runs = (int)cdiv(a.max_k1 + a.max_k2, ADG_NI * (gm == 8 ? 2 : 4));
-    const int nw = std::min(pairs >= 2 * (int64_t)sms ? 4 : ADG_MAXW, runs);
+    const int nw = std::min(ADG_MAXW, runs);
     int nc = 1;
-    while (nc < ADG_MAXC && pairs * nc * 2 <= 2 * (int64_t)sms && nw * nc < runs) nc *= 2;
+    while (nc < ADG_MAXC && pairs * nc * 2 <= 3 * (int64_t)sms && nw * nc < runs) nc *= 2;
     AttnDecDev d{};
     d.q = a.q; d.ldq = a.ldq; d.k = a.k1; d.v = a.v1; d.ldk = a.ldk1;
     d.k2 = a.k2; d.v2 = a.v2; d.ldk2 = a.ldk2; d.k2_start = a.k2 ? a.k2_start : nullptr; d.out = a.out; d.out_lo = a.out_lo; d.out_fmt = a.out_fmt; d.ldo = a.ldo;
@@ -865,8 +905,14 @@ static void attention_gqa(const AttnArgs &a, const AttnFused &f, bool fused) {
     d.H = a.H; d.Hkv = a.Hkv; d.rows = a.rows; d.scale = 1.0f / sqrtf((float)a.hd);
     const dim3 grid((unsigned)nc, (unsigned)a.Hkv, (unsigned)a.rows);
     ProfScope ps(NCMB_K_ATTN, 4.0 * (double)a.total_q * a.avg_keys * a.H * a.hd, 0);
-#define GQA_LAUNCH(GM_) do { if (fused) launch_pdl_cluster(k_attention_dec_gqa<GM_, true>, grid, dim3(nw * 32), nc, d, f); \
-                             else launch_pdl_cluster(k_attention_dec_gqa<GM_, false>, grid, dim3(nw * 32), nc, d, f); } while (0)
+#define GQA_LAUNCH(GM_) do { \
+        static bool set = false; \
+        if (!set) { \
+            CUDA_CHECK(cudaFuncSetAttribute((k_attention_dec_gqa<GM_, true>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adg_smem(GM_, ADG_MAXW))); \
+            CUDA_CHECK(cudaFuncSetAttribute((k_attention_dec_gqa<GM_, false>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adg_smem(GM_, ADG_MAXW))); \
+            set = true; } \
+        if (fused) launch_pdl_cluster(k_attention_dec_gqa<GM_, true>, grid, dim3(nw * 32), adg_smem(GM_, nw), nc, d, f); \
+                             else launch_pdl_cluster(k_attention_dec_gqa<GM_, false>, grid, dim3(nw * 32), adg_smem(GM_, nw), nc, d, f); } while (0)
     if (gm == 1) GQA_LAUNCH(1);
     else if (gm == 2) GQA_LAUNCH(2);
     else if (gm == 4) GQA_LAUNCH(4);

@@ -195,6 +195,16 @@ __global__ void __launch_bounds__(FR_T) k_few_reduce_norm(float *__restrict__ x,
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c4n = C >> 2;
     // the successor may start only once everything before this kernel is complete: attention reads the cache and the step
     // counter before it waits for the product that follows here
+    // (the norm's gains and the bias are weights: requested before the wait)
+    float4 w4[FR_V], b4[FR_V], bias4[FR_V];
+#pragma unroll
+    for (int i = 0; i < FR_V; i++) {
+        const int c = (tid + i * FR_T) * 4;
+        const bool on = tid + i * FR_T < c4n;
+        w4[i] = on && ln_w ? __ldg((const float4 *)(ln_w + c)) : make_float4(1.f, 1.f, 1.f, 1.f);
+        b4[i] = on && ln_b ? __ldg((const float4 *)(ln_b + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        bias4[i] = on && bias ? __ldg((const float4 *)(bias + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     pdl_wait();
     pdl_launch_dependents();
     float4 v[FR_V];
@@ -218,7 +228,7 @@ __global__ void __launch_bounds__(FR_T) k_few_reduce_norm(float *__restrict__ x,
                 for (int u = 0; u < FR_IN; u++)
                     if (s + u < S) { a.x += t[u].x; a.y += t[u].y; a.z += t[u].z; a.w += t[u].w; }
             }
-            if (bias) { const float4 b = __ldg((const float4 *)(bias + c * 4)); a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+            a.x += bias4[i].x; a.y += bias4[i].y; a.z += bias4[i].z; a.w += bias4[i].w;
             v[i] = make_float4(a.x + r.x, a.y + r.y, a.z + r.z, a.w + r.w);
             *(float4 *)(x + (int64_t)row * C + c * 4) = v[i];
         } else v[i] = r;
@@ -253,8 +263,7 @@ __global__ void __launch_bounds__(FR_T) k_few_reduce_norm(float *__restrict__ x,
     for (int i = 0; i < FR_V; i++) {
         const int c = (tid + i * FR_T) * 4;
         if (tid + i * FR_T >= c4n) continue;
-        const float4 w = ln_w ? __ldg((const float4 *)(ln_w + c)) : make_float4(1.f, 1.f, 1.f, 1.f);
-        const float4 b = ln_b ? __ldg((const float4 *)(ln_b + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 w = w4[i], b = b4[i];
         const float4 o = make_float4(__fadd_rn(__fmul_rn(__fmul_rn(v[i].x - mean, inv), w.x), b.x), __fadd_rn(__fmul_rn(__fmul_rn(v[i].y - mean, inv), w.y), b.y),
                                      __fadd_rn(__fmul_rn(__fmul_rn(v[i].z - mean, inv), w.z), b.z), __fadd_rn(__fmul_rn(__fmul_rn(v[i].w - mean, inv), w.w), b.w));
         store_split4((float *)y1, (float *)y2, (int64_t)row * C + c, o, SPLIT_H16);
@@ -338,6 +347,17 @@ void gemm_few(const FewGemm &g) {
 #undef FEW_CASE
 }
 
+void few_head(const void *x1, const void *x2, int rows, const float *W, const float *bias, int N, int K, float *y) {
+    if (rows <= 64) {
+        FewGemm g{x1, x2, K, W, rows, N, K};
+        g.bias = bias; g.y = y; g.ldy = N;
+        gemm_few(g);
+        return;
+    }
+    GemmArgs g;
+    g.x = (const float *)x1; g.x_lo = (const float *)x2; g.x_fmt = SPLIT_H16; g.ldx = K; g.W = W; g.bias = bias; g.y = y; g.ldy = N; g.M = rows; g.N = N; g.K = K;
+    gemm(g);
+}
 void few_reduce_norm(float *x, const float *part, int S, const float *bias, int rows, int C, int ln_kind, const float *ln_w, const float *ln_b,
                      float eps, void *y1, void *y2) {
     if (C % 4 || C > FR_T * FR_V * 4) fatal("few_reduce_norm: width %d", C);

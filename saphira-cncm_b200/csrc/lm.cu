@@ -266,9 +266,7 @@ NormSpec lm_last_norm(const NcmbLM *m) { return NormSpec{m->is_qwen ? 2 : 1, m->
 void lm_head(LMRun &r, const float *h, int64_t rows, float *logits, const FewChain *few = nullptr) {
     NcmbLM *m = r.m;
     if (few && few->on && few->ready) {
-        FewGemm g{few->y1, few->y2, m->C, m->wte, (int)rows, m->V, m->C};
-        g.y = logits; g.ldy = m->V;
-        gemm_few(g);
+        few_head(few->y1, few->y2, (int)rows, m->wte, nullptr, m->V, m->C, logits);
         return;
     }
     GemmArgs g;

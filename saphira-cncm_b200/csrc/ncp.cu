@@ -272,9 +272,7 @@ extern "C" VQState *ncp_vq(NCPState *m) { return m->vq; }
 static void final_logits(NCPState *m, int k, const float *x, int64_t rows, const BlockBufs &bufs, float *lg, const FewChain &few) {
     const HeadW &h = m->heads[k];
     if (few.on && few.ready && !h.proj && gemm_few_supported(rows, h.V, m->C)) {
-        FewGemm g{few.y1, few.y2, m->C, h.W, (int)rows, h.V, m->C};
-        g.bias = h.b; g.y = lg; g.ldy = h.V;
-        gemm_few(g);
+        few_head(few.y1, few.y2, (int)rows, h.W, h.b, h.V, m->C, lg);
         return;
     }
     layernorm(x, m->lnfw, m->lnfb, bufs.ln, rows, m->C, 1e-6f);
