@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(AD_THREADS) k_attention_decode(AttnDecDev a) {
 //
 // Bound: the K|V cache read once; for few rows the chain product -> sums -> scores -> merge.
 constexpr int ADG_NI = 4;              // loads of a run per lane
-constexpr int adg_depth(int GM) { return GM > 4 ? 4 : 2; }   // runs in flight per warp, the current one included (16 KB per warp either way)
+constexpr int adg_depth(int GM) { return GM > 4 ? 3 : 2; }   // runs in flight per warp, the current one included (12 or 16 KB per warp)
 constexpr int ADG_MAXW = 4;            // warps of a CTA at most
 constexpr int ADG_MAXC = 8;            // CTAs of a cluster at most
 
@@ -888,15 +888,16 @@ static bool gqa_shape(const AttnArgs &a) {
     return a.hd == 64 && (a.H / a.Hkv) * a.max_q <= 8 && (a.ldk1 & 3) == 0 && (!a.k2 || (a.ldk2 & 3) == 0) && al16(a.k1) && al16(a.v1) && (!a.k2 || (al16(a.k2) && al16(a.v2)));
 }
 
-// CTAs of a (row, kv head) pair: a cluster of as many (up to eight) as keep all CTAs resident at once, three of four warps per
-// SM, each warp with at least a run of keys.
+// Warps and CTAs of a (row, kv head) pair. An SM holds about twelve of these warps; all pairs should be resident at once (a
+// second wave of a few CTAs costs as much as the first), so many pairs get CTAs of two or three warps; few pairs get a cluster
+// of up to eight CTAs, two per SM, each warp with at least a run of keys.
 static void attention_gqa(const AttnArgs &a, const AttnFused &f, bool fused) {
     const int64_t pairs = (int64_t)a.rows * a.Hkv;
     const int gq = (a.H / a.Hkv) * a.max_q, gm = gq <= 1 ? 1 : gq <= 2 ? 2 : gq <= 4 ? 4 : 8, sms = ctx().sm_count;
     const int runs = (int)cdiv(a.max_k1 + a.max_k2, ADG_NI * (gm == 8 ? 2 : 4));
-    const int nw = std::min(ADG_MAXW, runs);
-    int nc = 1;
-    while (nc < ADG_MAXC && pairs * nc * 2 <= 3 * (int64_t)sms && nw * nc < runs) nc *= 2;
+    int nw = std::min(ADG_MAXW, runs), nc = 1;
+    while (nw > 2 && pairs > sms * (int64_t)(12 / nw)) nw--;
+    while (nc < ADG_MAXC && pairs * nc * 2 <= 2 * (int64_t)sms && nw * nc < runs) nc *= 2;
     AttnDecDev d{};
     d.q = a.q; d.ldq = a.ldq; d.k = a.k1; d.v = a.v1; d.ldk = a.ldk1;
     d.k2 = a.k2; d.v2 = a.v2; d.ldk2 = a.ldk2; d.k2_start = a.k2 ? a.k2_start : nullptr; d.out = a.out; d.out_lo = a.out_lo; d.out_fmt = a.out_fmt; d.ldo = a.ldo;

@@ -270,6 +270,39 @@ __global__ void __launch_bounds__(FR_T) k_few_reduce_norm(float *__restrict__ x,
     }
 }
 
+// The sums of an up-projection that was cut into slices, through bias and activation to an fp16 pair; glu: columns are
+// interleaved gate / up pairs and the result has N / 2 of them. Four columns per thread.
+__global__ void __launch_bounds__(256) k_few_reduce_act(const float *__restrict__ part, int S, int64_t rows, int N, const float *__restrict__ bias, int act, int glu,
+                                                       unsigned short *__restrict__ y1, unsigned short *__restrict__ y2) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int n4 = N >> 2;
+    if (i >= rows * n4) return;
+    const int64_t row = i / n4; const int c = (int)(i - row * n4) * 4;
+    const float *p = part + row * N + c;
+    const int64_t step = rows * N;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < S; s += 8) {
+        float4 t[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (s + u < S) t[u] = __ldcg((const float4 *)(p + (s + u) * step));
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (s + u < S) { a.x += t[u].x; a.y += t[u].y; a.z += t[u].z; a.w += t[u].w; }
+    }
+    if (bias) { const float4 b = __ldg((const float4 *)(bias + c)); a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+    if (glu) {
+        uint32_t hi, lo;
+        h16_pair2(__fmul_rn(fw_act(a.x, act), a.y), __fmul_rn(fw_act(a.z, act), a.w), hi, lo);
+        *(uint32_t *)(y1 + row * (N / 2) + c / 2) = hi;
+        *(uint32_t *)(y2 + row * (N / 2) + c / 2) = lo;
+    } else {
+        store_split4((float *)y1, (float *)y2, row * N + c, make_float4(fw_act(a.x, act), fw_act(a.y, act), fw_act(a.z, act), fw_act(a.w, act)), SPLIT_H16);
+    }
+}
+
 // One thread per pair (d, d + hd / 2) of a head of a row: slice sums and bias, rotation of query / key heads, q to its buffer,
 // k | v to the buffer and / or the cache.
 __global__ void __launch_bounds__(256) k_few_reduce_qkv(FewQkv a) {
@@ -363,6 +396,15 @@ void few_reduce_norm(float *x, const float *part, int S, const float *bias, int 
     if (C % 4 || C > FR_T * FR_V * 4) fatal("few_reduce_norm: width %d", C);
     ProfScope ps(NCMB_K_NORM, 0, (double)rows * C * 4 * (S + 3));
     LAUNCH_PDL(k_few_reduce_norm, (unsigned)rows, FR_T, 0, x, part, S, bias, rows, C, ln_kind, ln_w, ln_b, eps, (unsigned short *)y1, (unsigned short *)y2);
+}
+int few_up_slices(int M, int N, int K, int max_slices) {
+    const int64_t tiles = cdiv(N, 128) * cdiv(M, 128);
+    return tiles * 3 > ctx().sm_count || N % 8 ? 1 : gemm_few_slices(M, N, K, max_slices);
+}
+void few_reduce_act(const float *part, int S, int rows, int N, const float *bias, int act, int glu, void *y1, void *y2) {
+    const int64_t n = (int64_t)rows * (N / 4);
+    ProfScope ps(NCMB_K_ELEM, 0, (double)rows * N * 4 * (S + 1));
+    LAUNCH_PDL(k_few_reduce_act, grid1d(n, 256), 256, 0, part, S, (int64_t)rows, N, bias, act, glu, (unsigned short *)y1, (unsigned short *)y2);
 }
 void few_reduce_qkv(const FewQkv &a) {
     const int items = (a.H + 2 * a.Hkv) * a.hd / 2;

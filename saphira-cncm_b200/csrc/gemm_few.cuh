@@ -28,6 +28,11 @@ void few_head(const void *x1, const void *x2, int rows, const float *W, const fl
 void few_reduce_norm(float *x, const float *part, int S, const float *bias, int rows, int C, int ln_kind, const float *ln_w, const float *ln_b,
                      float eps, void *y1, void *y2);
 
+// An up-projection with so few 128-row tiles that most SMs would idle is cut into slices too (GPT-2's 3072 rows are 24 tiles:
+// 15.5 us at 64 tokens against 8 with the kernel that adds the slices); 1 = store the result directly.
+int few_up_slices(int M, int N, int K, int max_slices);
+void few_reduce_act(const float *part, int S, int rows, int N, const float *bias, int act, int glu, void *y1, void *y2);
+
 // q | k | v = bias + sum_s part[s][row], rotated (tables may be null), q to q[row * ldq], k | v to q as well (kv_self) and / or
 // to the cache row kv + (row / rps) * seq_pitch + (row % rps) * pitch + *step_d * step
 struct FewQkv {

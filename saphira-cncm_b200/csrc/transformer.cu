@@ -116,7 +116,8 @@ static void run_block_few(float *x, int64_t ntok, int C, int H, int nkv, const B
     const int hd = C / H, kvd = nkv * hd, Wq = C + 2 * kvd, M = (int)ntok, ms = few_max_slices(ntok);
     static Workspace ws;
     const int Sq = gemm_few_slices(M, Wq, C, ms), So = gemm_few_slices(M, C, C, ms), Sd = gemm_few_slices(M, C, w.Hh, ms);
-    const size_t part_fl = (size_t)M * std::max((size_t)Sq * Wq, (size_t)std::max(So, Sd) * C);
+    const int Nu = w.gated ? 2 * w.Hh : w.Hh, Su = few_up_slices(M, Nu, C, ms);
+    const size_t part_fl = (size_t)M * std::max(std::max((size_t)Sq * Wq, (size_t)std::max(So, Sd) * C), Su > 1 ? (size_t)Su * Nu : (size_t)0);
     const size_t need = part_fl * 4 + (size_t)M * (2 * C + w.Hh) * 4 + 4096;
     if (need > ws.cap) { ws.reserve(need + need / 4); fc.ready = false; }
     ws.reset();
@@ -145,9 +146,15 @@ static void run_block_few(float *x, int64_t ntok, int C, int H, int nkv, const B
     g.part = part; g.max_slices = ms;
     gemm_few(g);
     few_reduce_norm(x, part, So, w.ob, M, C, ln2.kind, ln2.w, ln2.b, ln2.eps, n1, n2);
-    g = FewGemm{n1, n2, C, w.gated ? w.fcw_il : w.fcw, M, w.gated ? 2 * w.Hh : w.Hh, C};
-    g.bias = w.gated ? w.fcb_il : w.fcb; g.act = w.act; g.glu = w.gated; g.y = b.h; g.y_lo = h_lo; g.ldy = w.Hh;
-    gemm_few(g);
+    g = FewGemm{n1, n2, C, w.gated ? w.fcw_il : w.fcw, M, Nu, C};
+    if (Su > 1) {
+        g.part = part; g.max_slices = ms;
+        gemm_few(g);
+        few_reduce_act(part, Su, M, Nu, w.gated ? w.fcb_il : w.fcb, w.act, w.gated, b.h, h_lo);
+    } else {
+        g.bias = w.gated ? w.fcb_il : w.fcb; g.act = w.act; g.glu = w.gated; g.y = b.h; g.y_lo = h_lo; g.ldy = w.Hh;
+        gemm_few(g);
+    }
     g = FewGemm{b.h, h_lo, w.Hh, w.pw, M, C, w.Hh};
     g.part = part; g.max_slices = ms;
     gemm_few(g);
