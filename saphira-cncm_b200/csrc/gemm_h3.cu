@@ -28,16 +28,20 @@
 namespace ncmb {
 
 constexpr int H3_BM = 128, H3_BK = 64;                   // BK halfs = 128 bytes = one swizzle row
-// Tile widths: 128 columns for large problems; 64 or 32 columns for small ones (batched decode steps, the first
-// NCP levels), chosen per call so that the busiest CTA moves the fewest bytes.
-// (256-column tiles: two stages of 96 KB. Four stages of 48 KB -- k-blocks of 32 halfs in 64-byte-swizzled rows --
-// were measured 8% slower: the MMAs fetch 64-byte rows less efficiently)
-constexpr int h3_stages(int BN) { return BN >= 256 ? 2 : BN >= 128 ? 3 : 4; }
+// Tile widths: 192 to 256 columns for large problems, 128, or 64 and 32 columns for small ones (the
+// NCP levels), chosen per call (h3_tile_width). A stage holds x1 | x2 | W1 (| W2 unless it is all zero); as many stages as fit.
 constexpr int H3_EPI_WARPS = 8;                         // two per TMEM lane quadrant, 64 columns each
 constexpr int H3_THREADS = 64 + 32 * H3_EPI_WARPS;
 constexpr int H3_TILE = 128 * H3_BK * 2;                 // one 128-row operand tile: 16 KB
 constexpr int h3_wtile(int BN) { return BN * H3_BK * 2; }  // one BN-row weight tile
-constexpr int h3_stage(int BN) { return 2 * H3_TILE + 2 * h3_wtile(BN); }   // x1 | x2 | W1 | W2
+constexpr int h3_stage(int BN, bool skip) { return 2 * H3_TILE + (skip ? 1 : 2) * h3_wtile(BN); }
+constexpr int H3_MAX_STAGES = 6;
+constexpr int H3_FIXED = 1024 + H3_EPI_WARPS * 4096 + (2 * H3_MAX_STAGES + 4) * 8 + 16;      // alignment, store staging, barriers
+constexpr int h3_stages(int BN, bool skip) {
+    int n = (227 * 1024 - H3_FIXED) / h3_stage(BN, skip);
+    return n > 4 ? 4 : n;
+}
+constexpr int h3_acc_pitch(int BN) { return BN <= 128 ? BN : 256; }                          // TMEM columns between the two accumulators
 
 
 // QKP: the epilogue applies the per-head RMSNorm / rotary embedding of a fused QKV projection (128-column tiles)
@@ -48,22 +52,22 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
                                                        const __grid_constant__ CUtensorMap tmW2,
                                                        const __grid_constant__ CUtensorMap tmY,
                                                        TcEpi ep, int num_kb, int tiles_n, int num_tiles, int ksplit, int kb_per,
-                                                       int m_pad, int skip_w2) {
+                                                       int m_pad, int skip_w2, int H3_STAGES, int H3_STAGE) {
     // skip_w2: every element of the W2 half is zero (a matrix whose scaled elements are all fp16 values, which is the
     // case for bf16 weights): the x1 W2 product is not issued -- two MMAs per k-step instead of three, same result
     // ksplit > 1: a work item is (output tile, slice of K); the item's raw sums go to slice s of a partial buffer whose
     // slices are m_pad rows apart (the tensor map of the stores covers all slices), and a second kernel adds the slices
     pdl_launch_dependents();          // programmatic dependent launch: see launch_pdl()
     pdl_wait();
-    constexpr int H3_STAGES = h3_stages(H3_BN), H3_STAGE = h3_stage(H3_BN), H3_WTILE = h3_wtile(H3_BN);
+    constexpr int H3_WTILE = h3_wtile(H3_BN), PITCH = h3_acc_pitch(H3_BN);
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     // barriers: full[STAGES], empty[STAGES], acc_full[2], acc_empty[2]
     unsigned char *stage0 = smem + H3_STAGES * H3_STAGE;         // one 4 KB store staging buffer per epilogue warp
     uint64_t *bars = (uint64_t *)(stage0 + H3_EPI_WARPS * 4096);
-    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * H3_STAGES + 4);
-    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + H3_STAGES);
-    const uint32_t afull0 = smem_u32(bars + 2 * H3_STAGES), aempty0 = smem_u32(bars + 2 * H3_STAGES + 2);
+    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * H3_MAX_STAGES + 4);
+    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + H3_MAX_STAGES);
+    const uint32_t afull0 = smem_u32(bars + 2 * H3_MAX_STAGES), aempty0 = smem_u32(bars + 2 * H3_MAX_STAGES + 2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -76,7 +80,7 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmW2) : "memory");
     }
     if (warp == 1) {   // two accumulators of BN columns: a tile's epilogue runs under the next tile's MMAs
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * H3_BN) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * PITCH) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -86,23 +90,24 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
 
     if (warp == 0) {
         if (lane == 0) {
-            int kbg = 0, armed = 0;                       // k-block counter over all of this CTA's tiles
+            int s = 0, armed = 0;                         // ring slot; slots filled and not yet known to be consumed are waited for on an error
+            uint32_t ph = 0;
             bool ok = true;
             for (int w = blockIdx.x; w < num_tiles * ksplit && ok; w += gridDim.x) {
                 const int t = w / ksplit, ks = w - t * ksplit;
                 const int n0 = (t % tiles_n) * H3_BN, m0 = (t / tiles_n) * H3_BM;
                 const int kb1 = min(num_kb, (ks + 1) * kb_per);
-                for (int kb = ks * kb_per; kb < kb1; kb++, kbg++) {
-                    int s = kbg % H3_STAGES; uint32_t ph = (uint32_t)(kbg / H3_STAGES) & 1u;
+                for (int kb = ks * kb_per; kb < kb1; kb++) {
                     ok = mbar_wait(empty0 + 8 * s, ph ^ 1u, ep.err, 21);
                     if (!ok) break;
                     const uint32_t dst = smem_u32(smem + s * H3_STAGE), bar = full0 + 8 * s;
-                    mbar_expect_tx(bar, skip_w2 ? H3_STAGE - H3_WTILE : H3_STAGE);       // an all-zero second half is neither fetched nor multiplied
+                    mbar_expect_tx(bar, H3_STAGE);                 // an all-zero second half is neither fetched nor multiplied
                     tma_load_2d(dst, &tmX1, kb * H3_BK, m0, bar);
                     tma_load_2d(dst + H3_TILE, &tmX2, kb * H3_BK, m0, bar);
                     tma_load_2d(dst + 2 * H3_TILE, &tmW1, kb * H3_BK, n0, bar);
                     if (!skip_w2) tma_load_2d(dst + 2 * H3_TILE + H3_WTILE, &tmW2, kb * H3_BK, n0, bar);
-                    armed = kbg + 1;
+                    armed++;
+                    if (++s == H3_STAGES) { s = 0; ph ^= 1u; }
                 }
             }
             if (!ok) {   // drain: wait (bounded) for the copies already in flight before leaving
@@ -113,17 +118,17 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
     } else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc = umma_idesc_f16(H3_BM, H3_BN);
-            int kbg = 0, it = 0;
+            int s = 0, it = 0;
+            uint32_t ph = 0;
             bool ok = true;
             for (int w = blockIdx.x; w < num_tiles * ksplit && ok; w += gridDim.x, it++) {
                 const int acc = it & 1; const uint32_t use = (uint32_t)(it >> 1);
                 ok = mbar_wait(aempty0 + 8 * acc, (use & 1u) ^ 1u, ep.err, 25);    // epilogue has drained this accumulator pair
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t tacc = tmem_base + (uint32_t)(acc * H3_BN);
+                const uint32_t tacc = tmem_base + (uint32_t)(acc * PITCH);
                 const int nkb = min(num_kb, (w % ksplit + 1) * kb_per) - (w % ksplit) * kb_per;
-                for (int kb = 0; kb < nkb; kb++, kbg++) {
-                    int s = kbg % H3_STAGES; uint32_t ph = (uint32_t)(kbg / H3_STAGES) & 1u;
+                for (int kb = 0; kb < nkb; kb++) {
                     ok = mbar_wait(full0 + 8 * s, ph, ep.err, 22);
                     if (!ok) break;
                     tc_fence_after();
@@ -138,6 +143,7 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
                         umma_f16(tacc, x1 + o, w1 + o, idesc, 1u);
                     }
                     umma_commit(empty0 + 8 * s);             // stage reusable once these MMAs have read it
+                    if (++s == H3_STAGES) { s = 0; ph ^= 1u; }
                 }
                 umma_commit(afull0 + 8 * acc);               // accumulators complete (also reached on the error path)
             }
@@ -145,9 +151,10 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
     } else {
         const int q = warp & 3;                              // TMEM lane quadrant this warp may read
         const int ch = (warp - 2) >> 2;                      // which half of the tile's 32-column chunks this warp drains
-        constexpr int NCH = H3_BN / 64;                      // chunks per warp (BN = 32: the first four warps take the one chunk)
-        constexpr int NCH1 = NCH > 0 ? NCH : 1;
-        const bool has_cols = NCH > 0 || ch == 0;
+        // 32-column chunks: the first four warps take the first CH0 of them, the others the rest
+        constexpr int NCH = H3_BN / 32, CH0 = (NCH + 1) / 2, NCH1 = CH0;
+        const int nch = ch == 0 ? CH0 : NCH - CH0;
+        const bool has_cols = nch > 0;
         int it = 0;
         bool ok = true;
         const bool glu_fast = tc_glu_silu_h16(ep);
@@ -156,7 +163,7 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
             const int t = w / ksplit;
             const int64_t slice_row0 = (int64_t)(w - t * ksplit) * m_pad;          // row offset of this K slice's partial sums
             const int acc = it & 1; const uint32_t use = (uint32_t)(it >> 1);
-            const int n0 = (t % tiles_n) * H3_BN + ch * (H3_BN / 2);
+            const int n0 = (t % tiles_n) * H3_BN + ch * CH0 * 32;
             const int64_t m = (int64_t)(t / tiles_n) * H3_BM + q * 32 + lane;
             // the residual of this thread's 64 outputs is requested before the accumulators are waited for,
             // so its latency runs under the tile's MMAs
@@ -187,11 +194,11 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
                 }
             };
 #pragma unroll
-            for (int c = 0; c < NPRE; c++) fetch_res(c);
+            for (int c = 0; c < NPRE; c++) if (c < nch) fetch_res(c);
             ok = mbar_wait(afull0 + 8 * acc, use & 1u, ep.err, 23);
             tc_fence_after();
             if (!ok) break;
-            const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * H3_BN + ch * (H3_BN / 2));
+            const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * PITCH + ch * CH0 * 32);
             if constexpr (QKP) {
                 // both halves of the thread's head (64 columns) before anything is stored
                 uint32_t r0[32], r1[32];
@@ -207,7 +214,7 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
             } else
 #pragma unroll
             for (int c = 0; c < NCH1; c++) {
-                if (!has_cols) break;
+                if (c >= nch) break;
                 uint32_t r[32];
                 tmem_ld32(trow + (uint32_t)(c * 32), r);
 #pragma unroll
@@ -219,7 +226,7 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
                 else if (ep.tma_store && n0 + c * 32 + 32 <= ep.N)
                     tc_epilogue_chunk_tma(ep, r, m, m - lane + slice_row0, n0, c * 32, pre[c] ? rv : nullptr, stage, &tmY, lane);
                 else tc_epilogue_chunk(ep, r, m, n0, c * 32, pre[c] ? rv : nullptr);
-                if (c + NPRE < NCH1) fetch_res(c + NPRE);
+                if (c + NPRE < NCH1 && c + NPRE < nch) fetch_res(c + NPRE);
             }
             tc_fence_before();
             __syncwarp();
@@ -232,7 +239,7 @@ __global__ void __launch_bounds__(H3_THREADS, 1) k_gemm_h3(const __grid_constant
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * H3_BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * PITCH) : "memory");
     }
 }
 
@@ -390,6 +397,31 @@ static bool qk_epilogue_on() {
     return e && e[0] == '1';
 }
 
+// Tile width: the one with which the busiest CTA is done first. Its time is waves x 64-wide steps x the time of a step, plus the
+// last tile's epilogue, which nothing hides (about 85 ns per column). The step times are measured (M = 6144 to 41120, K = 512 to
+// 4864): 128-column tiles run into the operands' way from L2 (64 KB per step and SM, 12.5 TB/s for all SMs), wider tiles read
+// the activation pair once for more columns but have two or three stages only (columns beyond N are counted by the rounding). With three products 256 columns took the 24-layer
+// model's up-projection from 1711 to 1497 us, with two (bf16 weights) the Qwen2 shape's from 226 to 177 us at 6144 rows.
+static int h3_tile_width(const GemmArgs &a, bool skip) {
+    const char *bn_s = getenv("NCM_B200_H3_BN");                   // read per call: the tests force each tile width
+    const int bn_env = bn_s ? atoi(bn_s) : 0;
+    for (int v : {32, 64, 128, 192, 224, 256}) if (bn_env == v) return v;
+    int bn = 128;
+    double best = -1, t128 = 0;
+    for (int cand : {256, 224, 192, 128, 64, 32}) {
+        if (cand > 128 && a.N < cand) continue;
+        const double waves = (double)cdiv(cdiv(a.N, cand) * cdiv(a.M, H3_BM), ctx().sm_count);
+        const double step = skip ? (cand == 256 ? 0.95 : cand == 224 ? 0.83 : cand == 192 ? 0.74 : cand == 128 ? 0.62 : cand == 64 ? 0.50 : 0.44)
+                                 : (cand == 256 ? 1.32 : cand == 224 ? 1.20 : cand == 192 ? 1.05 : cand == 128 ? 0.72 : cand == 64 ? 0.52 : 0.45);
+        const double t = waves * (double)cdiv(a.K, H3_BK) * step + 0.085 * cand;
+        if (cand == 128) t128 = t;
+        if (best < 0 || t < best) { best = t; bn = cand; }
+    }
+    // a fused QKV projection needs 128-column tiles (two heads each) and saves a whole pass over q and k
+    if (qk_epilogue_on() && a.qk_heads > 0 && a.qk_applied && a.N % 128 == 0 && t128 <= 2 * best) bn = 128;
+    return bn;
+}
+
 void gemm_h3(const GemmArgs &a) {
     if (a.M <= 0 || a.N <= 0) return;
     TcEpi ep{};
@@ -425,33 +457,7 @@ void gemm_h3(const GemmArgs &a) {
         split_h16(a.W, a.K, p1, p2, a.N, a.K);
         w1 = p1; w2 = p2;
     }
-    // Tile width. Small problems (decode steps, the first NCP levels) leave most SMs idle with 128-wide tiles and
-    // are paced by what ONE CTA pulls through its shared memory: tiles per CTA x bytes per k-step (the 128-row
-    // activation pair plus the bn-row weight pair). The width with the least of that wins; ties go to the wider.
-    static const bool narrow_ok = !getenv("NCM_B200_NO_BN32");
-    const char *bn_s = getenv("NCM_B200_H3_BN");                   // read per call: the tests force each tile width
-    const int bn_env = bn_s ? atoi(bn_s) : 0;
-    int bn = 128;
-    static const bool wide_ok = !getenv("NCM_B200_NO_BN256");
-    static const int wide_min_n = getenv("NCM_B200_BN256_MIN_N") ? atoi(getenv("NCM_B200_BN256_MIN_N")) : 1024;
-    static const int wide_max_kb = getenv("NCM_B200_BN256_MAX_KB") ? atoi(getenv("NCM_B200_BN256_MAX_KB")) : 8;   // longest K, in 64s
-    if (bn_env == 32 || bn_env == 64 || bn_env == 128 || bn_env == 256) bn = bn_env;
-    else if (narrow_ok) {
-        int64_t best = -1;
-        int64_t cost128 = 0;
-        for (int cand : {256, 128, 64, 32}) {
-            // 256-column tiles run on two stages of 96 KB: enough for a short K, not for a long one, where three
-            // stages of 128-column tiles measured faster (the down-projection, K = 2048); at 512 output columns the
-            // 128-column tiles were no slower either
-            if (cand == 256 && (!wide_ok || a.N % 256 != 0 || a.N < wide_min_n || cdiv(a.K, H3_BK) > wide_max_kb)) continue;
-            const int64_t waves = cdiv(cdiv(a.N, cand) * cdiv(a.M, H3_BM), ctx().sm_count);
-            const int64_t cost = waves * (2 * 128 + 2 * cand) * 128;     // bytes per 64 halfs of K
-            if (cand == 128) cost128 = cost;
-            if (best < 0 || cost < best) { best = cost; bn = cand; }
-        }
-        // a fused QKV projection needs 128-column tiles (two heads each) and saves a whole pass over q and k
-        if (qk_epilogue_on() && a.qk_heads > 0 && a.qk_applied && a.N % 128 == 0 && cost128 <= 2 * best) bn = 128;
-    }
+    const int bn = h3_tile_width(a, skip_w2 != 0);
     const CUtensorMap mx1 = tc_get_map_h16(x1, a.M, a.K, ldh, H3_BM), mx2 = tc_get_map_h16(x2, a.M, a.K, ldh, H3_BM);
     const CUtensorMap mw1 = tc_get_map_h16(w1, a.N, a.K, a.K, bn), mw2 = tc_get_map_h16(w2, a.N, a.K, a.K, bn);
     // fp32 results leave through TMA stores when the rows keep 16-byte strides
@@ -495,27 +501,29 @@ void gemm_h3(const GemmArgs &a) {
     int grid = (int)(items < ctx().sm_count ? items : ctx().sm_count);     // persistent: one CTA per SM
     ProfScope ps(NCMB_K_GEMM, 2.0 * (double)a.M * a.N * a.K,
                  4.0 * ((double)a.M * a.K + (double)a.N * a.K + (double)a.M * a.N));
-#define H3_LAUNCH(BN_)                                                                                                      \
+    const bool skip = skip_w2 != 0;
+#define H3_LAUNCH(BN_, QKP_)                                                                                                \
     do {                                                                                                                    \
-        constexpr size_t smem = 1024 + (size_t)h3_stages(BN_) * h3_stage(BN_) + H3_EPI_WARPS * 4096 + (2 * h3_stages(BN_) + 4) * 8 + 16; \
-        static_assert(smem <= 227 * 1024, "stage ring + store staging exceed shared memory");                               \
+        static_assert(h3_stages(BN_, false) >= 2, "two stages have to fit");                                                \
         static bool set = false;                                                                                            \
-        if (!set) { CUDA_CHECK(cudaFuncSetAttribute(k_gemm_h3<BN_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; } \
-        LAUNCH_PDL_IF(pdl_small(tiles * 4), k_gemm_h3<BN_>, grid, H3_THREADS, smem, mx1, mx2, mw1, mw2, my, ep, num_kb, tiles_n, (int)tiles, ksplit, kb_per, m_pad, skip_w2);        \
+        if (!set) { CUDA_CHECK(cudaFuncSetAttribute((k_gemm_h3<BN_, QKP_>), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)); set = true; } \
+        const size_t smem = H3_FIXED + (size_t)h3_stages(BN_, skip) * h3_stage(BN_, skip);                                  \
+        LAUNCH_PDL_IF(pdl_small(tiles * 4), (k_gemm_h3<BN_, QKP_>), grid, H3_THREADS, smem, mx1, mx2, mw1, mw2, my, ep, num_kb, tiles_n, (int)tiles, ksplit, kb_per, m_pad, skip_w2, \
+                      h3_stages(BN_, skip), h3_stage(BN_, skip));                                                           \
     } while (0)
     // fused QKV projection: heads are 64 columns, a 128-column tile holds two, results leave as fp32 tiles
     const bool qkp = qk_epilogue_on() && a.qk_heads > 0 && a.qk_applied && bn == 128 && ep.tma_store && a.N % 128 == 0 && !a.res &&
                      a.act == ACT_NONE && (a.qk_qw || a.qk_kw || a.qk_cos) && (!a.qk_cos || a.qk_pos);
     if (a.qk_applied) *a.qk_applied = qkp;
-    if (qkp) {
-        constexpr size_t smem = 1024 + (size_t)h3_stages(128) * h3_stage(128) + H3_EPI_WARPS * 4096 + (2 * h3_stages(128) + 4) * 8 + 16;
-        static bool set = false;
-        if (!set) { CUDA_CHECK(cudaFuncSetAttribute((k_gemm_h3<128, true>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
-        LAUNCH_PDL_IF(pdl_small(tiles * 4), (k_gemm_h3<128, true>), grid, H3_THREADS, smem, mx1, mx2, mw1, mw2, my, ep, num_kb, tiles_n, (int)tiles, ksplit, kb_per, m_pad, skip_w2);
-    } else if (bn == 32) H3_LAUNCH(32);
-    else if (bn == 64) H3_LAUNCH(64);
-    else if (bn == 256) H3_LAUNCH(256);
-    else H3_LAUNCH(128);
+    if (qkp) H3_LAUNCH(128, true);
+    else switch (bn) {
+        case 32: H3_LAUNCH(32, false); break;
+        case 64: H3_LAUNCH(64, false); break;
+        case 192: H3_LAUNCH(192, false); break;
+        case 224: H3_LAUNCH(224, false); break;
+        case 256: H3_LAUNCH(256, false); break;
+        default: H3_LAUNCH(128, false);
+    }
 #undef H3_LAUNCH
     if (ksplit > 1) {
         const int64_t n4 = a.M * (int64_t)(a.N / 4), g = cdiv(n4, 256), cap = (int64_t)ctx().sm_count * 8;

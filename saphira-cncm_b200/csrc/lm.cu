@@ -589,32 +589,79 @@ extern "C" void ncmb_lm_logits(NcmbLM *m, const int *ids, int T, int last_only, 
 // in fp64. Here the logits stay on the device: one CTA per token row takes the row maximum and the fp64 sum of
 // exponentials, and one double per position goes back to the host, which adds them in position order as the
 // reference does.
-__global__ void __launch_bounds__(256) k_nll_rows(const float *__restrict__ logits, const int *__restrict__ target, int V,
-                                                  double *__restrict__ out) {
-    __shared__ double red[256];
+//
+// exp() in fp64 of a difference x <= 0, by table and polynomial (Tang, "Table-driven implementation of the exponential function",
+// ACM TOMS 15, 1989): x = (64 k + j) ln2 / 64 + r with |r| <= ln2 / 128, e^x = 2^k 2^(j/64) (1 + r + r^2/2 + ... + r^5/120). The
+// truncation is below 2^-54; eleven fp64 operations a term instead of the library call's thirty-odd, which were the kernel.
+constexpr int NLL_T = 512;
+__device__ __forceinline__ double nll_exp(double x, const double *tab) {
+    if (x < -700.0) return 0.0;                                    // below any sum this is added to
+    const double magic = 6755399441055744.0;                       // 1.5 * 2^52: adding it rounds to an integer
+    const double t = fma(x, 92.332482616893656877, magic);         // 64 / ln 2
+    const int n = __double2loint(t);
+    const double kd = t - magic;
+    double r = fma(kd, -0x1.62e42fefa0000p-7, x);                  // ln2 / 64 in two parts, the first short enough for an exact product
+    r = fma(kd, -0x1.cf79abc9e3b39p-46, r);
+    double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+    q = fma(r, q, 1.0 / 6.0);
+    q = fma(r, q, 0.5);
+    q = fma(r * r, q, r);
+    const double b = tab[n & 63], e = fma(b, q, b);
+    return __hiloint2double(__double2hiint(e) + ((n >> 6) << 20), __double2loint(e));
+}
+// One pass over a row: every thread keeps its own maximum and the sum against it (rescaled when the maximum grows, which
+// becomes rare after a few elements). Memory bound: 4 bytes per logit, read once.
+__global__ void __launch_bounds__(NLL_T) k_nll_rows(const float *__restrict__ logits, const int *__restrict__ target, int V,
+                                                    double *__restrict__ out) {
+    __shared__ double tab[64], red[NLL_T / 32];
+    __shared__ float mred[NLL_T / 32];
     const int64_t r = blockIdx.x;
-    const int tg = target[r];
-    if (tg < 0) { if (threadIdx.x == 0) out[r] = 0.0; return; }      // block-uniform: position without a successor
+    const int tg = target[r], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tg < 0) { if (tid == 0) out[r] = 0.0; return; }      // block-uniform: position without a successor
+    if (tid < 64) tab[tid] = exp2((double)tid / 64.0);
+    __syncthreads();
     const float *row = logits + r * V;
-    float mxf = -INFINITY;
-    for (int v = threadIdx.x; v < V; v += 256) mxf = fmaxf(mxf, row[v]);
-    red[threadIdx.x] = (double)mxf;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-        __syncthreads();
+    float m = -INFINITY;
+    double s = 0.0;
+    auto add = [&](float4 v) {
+        const float mx = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
+        if (mx > m) { s = m == -INFINITY ? 0.0 : s * nll_exp((double)m - (double)mx, tab); m = mx; }
+        const double md = (double)m;
+        s += (nll_exp((double)v.x - md, tab) + nll_exp((double)v.y - md, tab)) + (nll_exp((double)v.z - md, tab) + nll_exp((double)v.w - md, tab));
+    };
+    // rows of an odd vocabulary start anywhere: single elements up to the first 16-byte boundary and behind the last
+    const int head = min(V, (int)((16u - (unsigned)((uintptr_t)row & 15)) & 15u) / 4), n4 = (V - head) >> 2, tail = head + n4 * 4;
+    const float4 *body = (const float4 *)(row + head);
+    int i = tid;
+    for (; i + 3 * NLL_T < n4; i += 4 * NLL_T) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = __ldcs(body + i + u * NLL_T);
+#pragma unroll
+        for (int u = 0; u < 4; u++) add(v[u]);
     }
-    const double mx = red[0];
+    for (; i < n4; i += NLL_T) add(__ldcs(body + i));
+    if (tid < head) add(make_float4(row[tid], -INFINITY, -INFINITY, -INFINITY));
+    if (tid < V - tail) add(make_float4(row[tail + tid], -INFINITY, -INFINITY, -INFINITY));
+    float mx = m;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) mred[warp] = mx;
     __syncthreads();
-    double den = 0.0;
-    for (int v = threadIdx.x; v < V; v += 256) den += exp((double)row[v] - mx);
-    red[threadIdx.x] = den;
+    mx = mred[0];
+#pragma unroll
+    for (int w = 1; w < NLL_T / 32; w++) mx = fmaxf(mx, mred[w]);
+    s = m == -INFINITY ? 0.0 : s * nll_exp((double)m - (double)mx, tab);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) red[warp] = s;
     __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
+    if (tid == 0) {
+        double den = 0.0;
+#pragma unroll
+        for (int w = 0; w < NLL_T / 32; w++) den += red[w];
+        out[r] = -log(exp((double)row[tg] - (double)mx) / den + 1e-30);
     }
-    if (threadIdx.x == 0) out[r] = -log(exp((double)row[tg] - mx) / red[0] + 1e-30);
 }
 
 // B windows of up to T ids each (row pitch T, lens[b] ids used; lens == NULL means T everywhere); nll_out[b] = mean
@@ -650,7 +697,7 @@ extern "C" void ncmb_lm_nll(NcmbLM *m, const int *ids, int B, int T, const int *
         const int64_t rows = n - r0 < chunk ? n - r0 : chunk;
         lm_head(r, r.x + r0 * m->C, rows, r.logits);
         ProfScope ps(NCMB_K_SAMPLE, 0, (double)rows * m->V * 4);
-        k_nll_rows<<<(unsigned)rows, 256, 0, stream()>>>(r.logits, tgt_d + r0, m->V, nll_d + r0);
+        k_nll_rows<<<(unsigned)rows, NLL_T, 0, stream()>>>(r.logits, tgt_d + r0, m->V, nll_d + r0);
         CUDA_CHECK(cudaGetLastError());
     }
     std::vector<double> h((size_t)n);
