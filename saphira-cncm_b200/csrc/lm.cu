@@ -36,6 +36,7 @@ struct NcmbLM {
     std::vector<BlockWeights> blocks;
     std::vector<void *> owned;
     Workspace work;
+    MegaModel mega;                             // weights as the persistent decode step streams them (laid out at first use)
 };
 
 static const float *need(WeightStore *ws, const char *who, const char *fmt, int li, const char *leaf) {
@@ -183,6 +184,7 @@ extern "C" NcmbLM *ncmb_lm_open(const NCMConfig *c, const char *weights, int is_
 extern "C" void ncmb_lm_close(NcmbLM *m) {
     if (!m) return;
     for (void *p : m->owned) dev_free(p);
+    lm_mega_free(m->mega);
     m->work.release();
     weights_free(&m->ws);
     delete m;
@@ -204,14 +206,15 @@ struct LMRun {
     // decode loop state on the device: absolute position of the step, this step's picks / packed argmax / uniforms
     int *step_d = nullptr, *pick_d = nullptr;
     long long graph_launches = 0;
-    // persistent decode kernel (up to four rows, head dim 64)
-    float *mg_part = nullptr; unsigned *mg_count = nullptr, *mg_bar = nullptr; MegaLayer *mg_layers = nullptr;                      // kernel launches one replay of the captured step stands for
+    uint2 *mg_ll = nullptr; MegaLayer *mg_layers = nullptr;      // persistent decode step: exchange words, per-layer pointers
     unsigned long long *amax_d = nullptr;
     double *uni_cur = nullptr;
     FewChain few;                 // the decode step's few-row chain
     // likelihood runs: next-token target and result per token row
     int64_t nll_rows = 0; int *tgt_d = nullptr; double *nll_d = nullptr;
 };
+
+MegaShape mega_shape(const NcmbLM *m, int B) { return MegaShape{B, m->C, m->H, m->nkv, m->I, m->NL, m->V, m->blocks.empty() ? 0 : m->blocks[0].gated}; }
 
 void lm_layout(LMRun &r, Workspace &w, int n_new, int64_t logit_rows) {
     NcmbLM *m = r.m;
@@ -243,11 +246,10 @@ void lm_layout(LMRun &r, Workspace &w, int n_new, int64_t logit_rows) {
     r.amax_d = w.get<unsigned long long>(r.B);
     r.pick_d = w.get<int>(r.B);
     r.step_d = w.get<int>(4);
-    const int max_split = (r.cap + 31) / 32;
-    r.mg_part = w.get<float>((size_t)r.B * m->H * max_split * 66);
-    r.mg_count = w.get<unsigned>((size_t)r.B * m->nkv + 4);
-    r.mg_bar = w.get<unsigned>(4);
-    r.mg_layers = (MegaLayer *)w.get<unsigned char>(sizeof(MegaLayer) * (size_t)m->NL);
+    if (r.B <= MG_MAXB) {
+        r.mg_ll = w.get<uint2>(lm_mega_exchange_words(mega_shape(m, r.B)));
+        r.mg_layers = w.get<MegaLayer>((size_t)m->NL);
+    }
     if (r.nll_rows > 0) { r.tgt_d = w.get<int>((size_t)r.nll_rows); r.nll_d = w.get<double>((size_t)r.nll_rows); }
 }
 
@@ -474,37 +476,31 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
     // runs eagerly (it sizes every workspace), the second is captured, the rest are graph launches. The work
     // moves to a stream of its own for that, because the caller's stream may be the legacy default stream,
     // which cannot be captured.
-    // Up to four rows (head dim 64): the whole decode step is one persistent cooperative kernel; nothing to replay.
+    // Up to four rows (head dim 64): the whole decode step is one persistent cooperative kernel (lm_mega.cu).
     bool qk_norm = false;
     for (auto &bw : m->blocks) qk_norm = qk_norm || bw.qnw || bw.knw;
-    const bool mega = lm_mega_eligible(B, m->hd, m->C, m->I, qk_norm) && r.cap <= 2048 && n_new >= 2;
+    const MegaShape ms = mega_shape(m, B);
+    const bool mega = lm_mega_enabled() && B <= MG_MAXB && n_new >= 2 && lm_mega_supported(ms, m->hd, qk_norm);
     MegaArgs mg{};
     if (mega) {
+        lm_mega_pack(m->mega, ms, m->blocks, m->wte, m->wte16);
         std::vector<MegaLayer> hl(m->NL);
         for (int li = 0; li < m->NL; li++) {
             const BlockWeights &bw = m->blocks[li];
-            hl[li] = MegaLayer{bw.ln1w, bw.ln1b, bw.qkvw, bw.qkvb, bw.ow, bw.ob, bw.ln2w, bw.ln2b, bw.fcw, bw.fcb, bw.pw, bw.pb, r.kv[li]};
+            hl[li] = MegaLayer{bw.ln1w, bw.ln1b, bw.qkvb, bw.ob, bw.ln2w, bw.ln2b, bw.fcb, bw.pb, r.kv[li]};
         }
         upload(r.mg_layers, hl.data(), sizeof(MegaLayer) * hl.size());
-        CUDA_CHECK(cudaMemsetAsync(r.mg_count, 0, ((size_t)B * m->nkv + 4) * 4, stream()));
-        CUDA_CHECK(cudaMemsetAsync(r.mg_bar, 0, 16, stream()));
-        CUDA_CHECK(cudaStreamSynchronize(stream()));             // hl goes out of scope
-        const BlockWeights &b0 = m->blocks[0];
-        mg.B = B; mg.C = m->C; mg.H = m->H; mg.nkv = m->nkv; mg.I = m->I; mg.NL = m->NL; mg.V = m->V;
-        mg.norm = b0.norm == NORM_RMS ? 2 : 1; mg.gated = b0.gated; mg.act = b0.act; mg.rope = m->is_qwen ? 1 : 0;
-        mg.eps = b0.norm == NORM_RMS ? 1e-6f : b0.eps; mg.eps_f = m->is_qwen ? 1e-6f : 1e-5f;
-        mg.layers = r.mg_layers; mg.wte = m->wte; mg.wpe = m->is_qwen ? nullptr : m->wpe; mg.lnfw = m->lnfw; mg.lnfb = m->lnfb;
-        mg.cosb = m->cosb; mg.sinb = m->sinb;
-        mg.x = r.x; mg.qkv = r.bufs.qkv; mg.ctx = r.bufs.ctx; mg.h = r.bufs.h; mg.logits = r.logits;
-        mg.part = r.mg_part; mg.count = r.mg_count;
-        mg.ids = r.ids_d; mg.posmat = r.posmat; mg.lenmat = r.lenmat; mg.step_d = r.step_d;
-        mg.np = np; mg.cap = r.cap; mg.n_new = n_new; mg.max_split = (r.cap + 31) / 32;
+        CUDA_CHECK(cudaMemsetAsync(r.mg_ll, 0, lm_mega_exchange_words(ms) * sizeof(uint2), stream()));
+        const NormSpec n1 = ln1_of(m->blocks[0]), nf = lm_last_norm(m);
+        mg.s = ms; mg.norm = n1.kind; mg.eps = n1.eps; mg.eps_f = nf.eps; mg.act = m->blocks[0].act;
+        mg.layers = r.mg_layers; mg.wte = m->wte; mg.wpe = m->is_qwen ? nullptr : m->wpe; mg.lnfw = nf.w; mg.lnfb = nf.b;
+        mg.cosb = m->cosb; mg.sinb = m->sinb; mg.logits = r.logits;
+        mg.ids = r.ids_d; mg.posmat = r.posmat; mg.step_d = r.step_d; mg.pos_base = np - 1;
         mg.kv_seq_pitch = (int64_t)r.cap * 2 * m->nkv * m->hd;
-        mg.bar = r.mg_bar; mg.bar_base = r.mg_bar + 1; mg.err = tc_err_flag();
-        mg.greedy = !(temp > 0.f); mg.amax = r.amax_d; mg.out = r.out_d; mg.ids_out = r.ids_d;
+        mg.ll = r.mg_ll; mg.err = tc_err_flag();
     }
     static const bool graphs_ok = !getenv("NCM_B200_NO_GRAPH");
-    const bool use_graph = !mega && graphs_ok && eos < 0 && n_new >= 4 && !prof_enabled();
+    const bool use_graph = graphs_ok && eos < 0 && n_new >= 4 && !prof_enabled();
     cudaStream_t user = stream(), gs = nullptr;
     cudaEvent_t ev = nullptr;
     cudaGraph_t graph = nullptr; cudaGraphExec_t gexec = nullptr;
@@ -516,8 +512,8 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
         ctx().stream = gs;
     }
     for (int s = 0; s < n_new; s++) {
-        // (the sample + finish of a step is inside the graph for replayed steps, inside the kernel for greedy persistent steps)
-        if (s == 0 || (!gexec && !(mega && mg.greedy))) lm_sample(r, temp, top_k, top_p, n_new);
+        // (the sample + finish of a step is inside the graph for replayed steps)
+        if (s == 0 || !gexec) lm_sample(r, temp, top_k, top_p, n_new);
         produced = s + 1;
         if (eos >= 0) {
             mem_d2h(col.data(), r.ids_d, (size_t)B * 4);
@@ -526,13 +522,12 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
             if (all) break;
         }
         if (s + 1 == n_new) break;
-        if (mega) { lm_mega_launch(mg); continue; }
         if (gexec) { CUDA_CHECK(cudaGraphLaunch(gexec, gs)); ctx().launches += r.graph_launches; continue; }
         const bool capture = use_graph && s == 1;
         long long l0 = ctx().launches;
         if (capture) CUDA_CHECK(cudaStreamBeginCapture(gs, cudaStreamCaptureModeThreadLocal));
-        lm_decode_step(r, r.ids_d);
-        lm_head(r, r.x, B, r.logits, &r.few);
+        if (mega) lm_mega_launch(m->mega, mg);
+        else { lm_decode_step(r, r.ids_d); lm_head(r, r.x, B, r.logits, &r.few); }
         if (capture) {
             lm_sample(r, temp, top_k, top_p, n_new);
             CUDA_CHECK(cudaStreamEndCapture(gs, &graph));

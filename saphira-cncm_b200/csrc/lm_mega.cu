@@ -1,500 +1,674 @@
-// One decode step of a decoder LM (up to four sequences, head dim 64) as ONE persistent cooperative kernel.
+// One decode step of one to four sequences (head dim 64) as ONE persistent kernel: every layer and the vocabulary projection.
 //
-// A decode step is a chain of small dependent matrix-vector products: launched one by one, each costs a
-// launch, a first DRAM round trip and a reduction (~6 us) for ~1.5 us of weight streaming. Here one CTA per SM
-// walks the whole step -- embed, then per layer [norm + QKV (+RoPE, K|V to the cache)] [split-key attention]
-// [output projection + residual] [norm + MLP up (+ gated product)] [MLP down + residual], then the final norm,
-// the vocabulary projection and the greedy pick -- with a grid-wide barrier between phases. Before it arrives
-// at a barrier a CTA issues L2 prefetches for the weight rows it will read in the next phase, so the DRAM
-// latency of the weight stream runs under the barrier instead of after it.
+// A step streams all weights once (4.6 us of HBM time a layer for the Qwen2 shape in bf16) through five products that depend on
+// one another; as separate kernels each boundary and each cold start of the weight stream costs several times that (28 us a
+// layer). Here one CTA per SM stays for the whole step:
 //
-// Work split inside a GEMV phase: one warp per output column (or per pair of columns that belong together: a
-// rotary pair (d, d+32) of a head, so RoPE is applied by the warp that produced both halves; a gate column and
-// its up column of a gated MLP). The lanes stride over K with 128-bit loads; normalised input rows sit in
-// shared memory (once per CTA), un-normalised ones are read from L2. No block-level synchronisation happens
-// inside a phase.
+//   * Weights. A model's rows are dealt to the CTAs once, and each CTA's rows of all layers lie in one buffer in the order it
+//     uses them. A producer warp copies that stream through a 128 KB ring in shared memory (bulk copies of 8 KB), as far ahead
+//     as the ring allows, whatever the other warps wait for: the stream only pauses when the ring is full.
+//   * Exchange. A product's results are needed by all CTAs (the hidden state) or many (attention). They travel as 8-byte words
+//     {value, tag}, written with one store and polled by whoever needs them; the tag is the layer's number in the generate, so
+//     a word says itself whether it has arrived. That is one trip through L2 per hop instead of fence, barrier and read.
+//     A buffer is written again one layer later, which cannot happen before every CTA has read it: the new value depends, by
+//     way of the MLP that all CTAs take part in, on results each of them produced after its read.
+//   * Products. Sixteen warps: four quarters of K x four groups of rows. A lane keeps its eight elements of the input in
+//     registers; eight rows at a time meet in a reduce-scatter.
 //
-// Every barrier wait is bounded (2 s): on a timeout the CTA records a code and keeps going, so the kernel always
-// ends; the host reads the code and discards the step. The launch is cooperative (all CTAs co-resident).
-#include "common.cuh"
+// Hops of a layer: hidden -> q k v -> attention partials -> hidden -> MLP -> hidden. Every wait is bounded (2 s): a wait that
+// runs out records a code, the other CTAs see it and stop waiting, and the kernel ends.
 #include "lm_mega.cuh"
+#include "tc_common.cuh"
+#include "tc_epilogue.cuh"
+
+#include <algorithm>
 
 namespace ncmb {
 
-constexpr int MG_THREADS = 512;
-constexpr int MG_KEYS = 32, MG_TEAMS = 4, MG_TEAM = MG_THREADS / MG_TEAMS, MG_MAXG = 8, MG_MAXSPLIT = 64;
+constexpr int MS_WARPS = 16, MS_T = MS_WARPS * 32;       // consumer threads; one more warp feeds the ring
+constexpr int MS_CH = 8192, MS_SLOTS = 16, MS_RING = MS_CH * MS_SLOTS;
+constexpr int MS_MAXC = 1024, MS_MAXI = 8192, MS_MAXSPLIT = 4, MS_PW = 66;       // words of an attention partial: max, sum, context
+constexpr int MS_UPROWS = 128, MS_HROWS = 64;            // rows a CTA may have of an up-projection; vocabulary rows per round
 
-__device__ __forceinline__ float mg_act(float v, int act) {
-    switch (act) {
-        case ACT_GELU: return 0.5f * v * (1.0f + erff(v * 0.7071067811865475f));
-        case ACT_GELU_TANH: return 0.5f * v * (1.0f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
-        case ACT_SILU: return v / (1.0f + expf(-v));
-        case ACT_RELU2: { float r = v > 0.f ? v : 0.f; return r * r; }
-        default: return v;
+// contiguous share of n items for CTA c of g
+__host__ __device__ __forceinline__ int ms_begin(int n, int c, int g) { return (int)((long long)n * c / g); }
+
+struct MsLL {                                            // offsets of the exchange buffers, in words
+    size_t x, x1, q, p, h, total;
+    __host__ __device__ explicit MsLL(const MegaShape &s) {
+        const size_t B = s.B;
+        x = 0; x1 = x + B * s.C; q = x1 + B * s.C; p = q + B * (s.C + 128 * (size_t)s.nkv); h = p + B * s.H * MS_MAXSPLIT * MS_PW; total = h + B * s.I;
     }
-}
-__device__ __forceinline__ unsigned long long mg_time() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// grid-wide barrier on a counter that only grows: the k-th barrier of this launch is passed when the counter
-// reaches base + k * gridDim.x
-__device__ __forceinline__ void mg_barrier(const MegaArgs &a, unsigned base, unsigned &k) {
-    k++;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned target = base + k * gridDim.x;
-        atomicAdd(a.bar, 1u);
-        unsigned long long t0 = 0;
-        for (unsigned it = 0;; it++) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-            if ((int)(v - target) >= 0) break;
-            if ((it & 1023u) == 1023u) {
-                if (*(volatile int *)a.err) break;               // some CTA already gave up: do not wait out every barrier
-                unsigned long long now = mg_time();
-                if (t0 == 0) t0 = now;
-                else if (now - t0 > 2000000000ull) { atomicExch(a.err, 31); break; }
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-}
-
-// block-wide sum of one value per thread (16 warps); red needs 16 floats; every thread gets the result
-__device__ __forceinline__ float mg_block_sum(float v, float *red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float s = 0.f;
-#pragma unroll
-    for (int w = 0; w < MG_THREADS / 32; w++) s += red[w];
-    return s;
-}
-
-// input rows -> shared memory, optionally normalised (1 LayerNorm, 2 RMSNorm) exactly like the stand-alone kernels
-__device__ void mg_stage(const MegaArgs &a, const float *src, int64_t ld, int K, int norm, const float *w, const float *b,
-                         float eps, float *xs, float *red) {
-    for (int r = 0; r < a.B; r++) {
-        const float *xr = src + r * ld;
-        float mean = 0.f, rstd = 1.f;
-        if (norm) {
-            if (norm == 1) {
-                float p = 0.f;
-                for (int k = threadIdx.x * 4; k < K; k += MG_THREADS * 4) { float4 v = *(const float4 *)(xr + k); p += (v.x + v.y) + (v.z + v.w); }
-                mean = mg_block_sum(p, red) / (float)K;
-            }
-            float q = 0.f;
-            for (int k = threadIdx.x * 4; k < K; k += MG_THREADS * 4) {
-                float4 v = *(const float4 *)(xr + k);
-                float d0 = v.x - mean, d1 = v.y - mean, d2 = v.z - mean, d3 = v.w - mean;
-                q += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
-            }
-            rstd = 1.0f / sqrtf(mg_block_sum(q, red) / (float)K + eps);
-        }
-        for (int k = threadIdx.x * 4; k < K; k += MG_THREADS * 4) {
-            float4 v = *(const float4 *)(xr + k);
-            if (norm) {
-                float4 lw = w ? *(const float4 *)(w + k) : make_float4(1.f, 1.f, 1.f, 1.f);
-                float4 lb = b ? *(const float4 *)(b + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-                v.x = __fadd_rn(__fmul_rn(__fmul_rn(v.x - mean, rstd), lw.x), lb.x);
-                v.y = __fadd_rn(__fmul_rn(__fmul_rn(v.y - mean, rstd), lw.y), lb.y);
-                v.z = __fadd_rn(__fmul_rn(__fmul_rn(v.z - mean, rstd), lw.z), lb.z);
-                v.w = __fadd_rn(__fmul_rn(__fmul_rn(v.w - mean, rstd), lw.w), lb.w);
-            }
-            *(float4 *)(xs + (size_t)r * K + k) = v;
-        }
-    }
-    __syncthreads();
-}
-
-// ---- GEMV phases: one warp per item, no block-level synchronisation inside a phase ----
-// An item is one output column, or the two columns that belong together: a rotary pair (c, c + 32) of a q / k
-// head, or a gate column j and its up column half + j. The lanes stride over K with 128-bit loads (all of a
-// column's loads in flight), the B input rows come from shared memory (normalised) or straight from L2, and a
-// shuffle reduction leaves the dot products in every lane.
-//   layout 0: item = column        1: rotary pair p -> (p/32)*64 + p%32, +32        2: gated j -> j, half + j
-__device__ __forceinline__ void mg_item_cols(int layout, int it, int half, int &c0, int &c1) {
-    if (layout == 1) { c0 = (it >> 5) * 64 + (it & 31); c1 = c0 + 32; }
-    else if (layout == 2) { c0 = it; c1 = half + it; }
-    else { c0 = it; c1 = -1; }
-}
-
-// L2 prefetch of the weight rows of this warp's first item of the next phase
-__device__ __forceinline__ void mg_prefetch(const float *W, int K, int layout, int half, int nitems) {
-    const int wg = blockIdx.x * (MG_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (wg >= nitems) return;
-    int c0, c1;
-    mg_item_cols(layout, wg, half, c0, c1);
-    const int lines = (K * 4 + 127) / 128;
-    for (int l = lane; l < lines; l += 32) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (size_t)c0 * K + l * 32));
-        if (c1 >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (size_t)c1 * K + l * 32));
-    }
-}
-
-// d0[r], d1[r] = W[c0] . x[r], W[c1] . x[r] (c1 < 0: one column); x rows are K floats apart at xrow (shared or global)
-template <bool TWO>
-__device__ __forceinline__ void mg_item_dot(const MegaArgs &a, const float *W, int K, int c0, int c1, const float *xrow, int64_t ldx,
-                                            float *d0, float *d1) {
-    const int lane = threadIdx.x & 31, K4 = K >> 2;
-    const float4 *w0 = (const float4 *)(W + (size_t)c0 * K), *w1 = (const float4 *)(W + (size_t)(TWO ? c1 : c0) * K);
-#pragma unroll
-    for (int r = 0; r < MG_MAXB; r++) { d0[r] = 0.f; d1[r] = 0.f; }
-#pragma unroll 4
-    for (int k4 = lane; k4 < K4; k4 += 32) {
-        const float4 p = __ldg(w0 + k4);
-        float4 q = p;
-        if (TWO) q = __ldg(w1 + k4);
-#pragma unroll
-        for (int r = 0; r < MG_MAXB; r++) {
-            if (r < a.B) {
-                const float4 xv = *((const float4 *)(xrow + (size_t)r * ldx) + k4);
-                d0[r] = fmaf(xv.x, p.x, d0[r]); d0[r] = fmaf(xv.y, p.y, d0[r]); d0[r] = fmaf(xv.z, p.z, d0[r]); d0[r] = fmaf(xv.w, p.w, d0[r]);
-                if (TWO) { d1[r] = fmaf(xv.x, q.x, d1[r]); d1[r] = fmaf(xv.y, q.y, d1[r]); d1[r] = fmaf(xv.z, q.z, d1[r]); d1[r] = fmaf(xv.w, q.w, d1[r]); }
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < MG_MAXB; r++) {
-        if (r < a.B) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                d0[r] += __shfl_xor_sync(0xffffffffu, d0[r], o);
-                if (TWO) d1[r] += __shfl_xor_sync(0xffffffffu, d1[r], o);
-            }
-        }
-    }
-}
-
-// ---- split-key attention of one (row, kv head, 32-key chunk) by a team of 128 threads; the last chunk of a
-// (row, kv head) to finish merges the partials (same scheme as attention_decode.cu) ----
-struct MgAttnSmem {
-    float qs[MG_MAXG][64];
-    float sc[MG_MAXG][MG_KEYS];
-    float red[2][MG_MAXG][64];
-    float mg[MG_MAXG], lg[MG_MAXG];
-    float wsm[MG_MAXSPLIT][MG_MAXG], lsm[MG_MAXSPLIT][MG_MAXG], Lg[MG_MAXG];
-    int last;
 };
-__device__ __forceinline__ void mg_team_sync(int team) { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(MG_TEAM) : "memory"); }
-
-__device__ void mg_attn_unit(const MegaArgs &a, const MegaLayer &L, int row, int kvh, int sp, int n1, MgAttnSmem &sm, int team, int t) {
-    constexpr int HD = 64, DP = 16, GROUPS = 2, KPG = 16;
-    const int G = a.H / a.nkv, kvd = a.nkv * HD, Wq = a.C + 2 * kvd;
-    const int warp = t >> 5, lane = t & 31;
-    const int nsplit = (n1 + MG_KEYS - 1) / MG_KEYS, k0 = sp * MG_KEYS;
-    const float *kbase = L.kv + (size_t)row * a.kv_seq_pitch;
-    const int64_t ldk = 2 * kvd;
-    const float scale = 0.125f;
-    for (int i = t; i < G * HD; i += MG_TEAM) { int g = i / HD, d = i % HD; sm.qs[g][d] = a.qkv[(size_t)row * Wq + (kvh * G + g) * HD + d]; }
-    mg_team_sync(team);
-    {
-        const int j = t >> 2, part = t & 3;
-        const bool valid = k0 + j < n1;
-        float kr[DP];
-        if (valid) {
-            const float4 *kp = (const float4 *)(kbase + (int64_t)(k0 + j) * ldk + kvh * HD + part * DP);
-#pragma unroll
-            for (int i = 0; i < DP / 4; i++) { float4 v = kp[i]; kr[4 * i] = v.x; kr[4 * i + 1] = v.y; kr[4 * i + 2] = v.z; kr[4 * i + 3] = v.w; }
-        } else {
-#pragma unroll
-            for (int i = 0; i < DP; i++) kr[i] = 0.f;
-        }
-        for (int g = 0; g < G; g++) {
-            float dot = 0.f;
-#pragma unroll
-            for (int i = 0; i < DP; i++) dot = fmaf(kr[i], sm.qs[g][part * DP + i], dot);
-            dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-            dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-            if (part == 0) sm.sc[g][j] = valid ? dot * scale : -INFINITY;
-        }
-    }
-    mg_team_sync(team);
-    for (int g = warp; g < G; g += MG_TEAM / 32) {
-        float s = sm.sc[g][lane], m = s;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        float p = (s == -INFINITY) ? 0.f : expf(s - m), l = p;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-        sm.sc[g][lane] = p;
-        if (lane == 0) { sm.mg[g] = m; sm.lg[g] = l; }
-    }
-    mg_team_sync(team);
-    {
-        const int grp = t / HD, d = t % HD;
-        float acc[MG_MAXG], vr[KPG];
-#pragma unroll
-        for (int g = 0; g < MG_MAXG; g++) acc[g] = 0.f;
-#pragma unroll
-        for (int jj = 0; jj < KPG; jj++) {
-            const int j = grp * KPG + jj;
-            vr[jj] = (k0 + j < n1) ? kbase[(int64_t)(k0 + j) * ldk + kvd + kvh * HD + d] : 0.f;
-        }
-#pragma unroll
-        for (int jj = 0; jj < KPG; jj++) {
-            const int j = grp * KPG + jj;
-#pragma unroll
-            for (int g = 0; g < MG_MAXG; g++) if (g < G) acc[g] = fmaf(sm.sc[g][j], vr[jj], acc[g]);
-        }
-#pragma unroll
-        for (int g = 0; g < MG_MAXG; g++) if (g < G) sm.red[grp][g][d] = acc[g];
-    }
-    mg_team_sync(team);
-    float *mine = a.part + ((int64_t)(row * a.nkv + kvh) * a.max_split + sp) * G * (HD + 2);
-    for (int i = t; i < G * HD; i += MG_TEAM) {
-        int g = i / HD, d = i % HD;
-        mine[g * (HD + 2) + 2 + d] = sm.red[0][g][d] + sm.red[1][g][d];
-        if (d == 0) { mine[g * (HD + 2)] = sm.mg[g]; mine[g * (HD + 2) + 1] = sm.lg[g]; }
-    }
-    __threadfence();
-    mg_team_sync(team);
-    if (t == 0) {
-        unsigned old = atomicAdd(a.count + row * a.nkv + kvh, 1u);
-        sm.last = (old == (unsigned)(nsplit - 1));
-    }
-    mg_team_sync(team);
-    if (!sm.last) return;
-    __threadfence();
-    const float *base = a.part + (int64_t)(row * a.nkv + kvh) * a.max_split * G * (HD + 2);
-    for (int i = t; i < nsplit * G; i += MG_TEAM) {
-        int s = i / G, g = i % G;
-        const float *ps = base + ((int64_t)s * G + g) * (HD + 2);
-        sm.wsm[s][g] = __ldcg(ps); sm.lsm[s][g] = __ldcg(ps + 1);
-    }
-    mg_team_sync(team);
-    if (t < G) {
-        float M = -INFINITY, Ls = 0.f;
-        for (int s = 0; s < nsplit; s++) M = fmaxf(M, sm.wsm[s][t]);
-        for (int s = 0; s < nsplit; s++) { float w = expf(sm.wsm[s][t] - M); sm.wsm[s][t] = w; Ls = fmaf(sm.lsm[s][t], w, Ls); }
-        sm.Lg[t] = Ls;
-    }
-    mg_team_sync(team);
-    for (int i = t; i < G * HD; i += MG_TEAM) {
-        int g = i / HD, d = i % HD;
-        float O = 0.f;
-        int s = 0;
-        for (; s + 4 <= nsplit; s += 4) {
-            float o0 = __ldcg(base + ((int64_t)(s + 0) * G + g) * (HD + 2) + 2 + d);
-            float o1 = __ldcg(base + ((int64_t)(s + 1) * G + g) * (HD + 2) + 2 + d);
-            float o2 = __ldcg(base + ((int64_t)(s + 2) * G + g) * (HD + 2) + 2 + d);
-            float o3 = __ldcg(base + ((int64_t)(s + 3) * G + g) * (HD + 2) + 2 + d);
-            O = fmaf(o0, sm.wsm[s][g], O); O = fmaf(o1, sm.wsm[s + 1][g], O); O = fmaf(o2, sm.wsm[s + 2][g], O); O = fmaf(o3, sm.wsm[s + 3][g], O);
-        }
-        for (; s < nsplit; s++) O = fmaf(__ldcg(base + ((int64_t)s * G + g) * (HD + 2) + 2 + d), sm.wsm[s][g], O);
-        const float Ls = sm.Lg[g];
-        a.ctx[(size_t)row * a.C + (kvh * G + g) * HD + d] = Ls > 0.f ? O / Ls : 0.f;
-    }
-    if (t == 0) a.count[row * a.nkv + kvh] = 0;
+__host__ __device__ __forceinline__ int ms_splits(const MegaShape &s, int grid) {
+    const int n = grid / (s.B * s.H);
+    return n < 1 ? 1 : (n > MS_MAXSPLIT ? MS_MAXSPLIT : n);
 }
 
-// ---- the step ----
-__global__ void __launch_bounds__(MG_THREADS, 1) k_lm_decode_mega(MegaArgs a) {
-    extern __shared__ __align__(16) unsigned char mg_smem[];
-    float *xs = (float *)mg_smem;                               // staged input rows [B][K] (GEMV phases)
-    MgAttnSmem *asmem = (MgAttnSmem *)mg_smem;                  // four team scratch areas (attention phase)
-    __shared__ float bred[MG_THREADS / 32];
-    __shared__ unsigned long long s_best[MG_MAXB];
-    const int tid = threadIdx.x;
-    if (*(volatile int *)a.err) return;                         // an earlier launch timed out: the host will discard the run
-    const unsigned base = *a.bar_base;
-    unsigned nb = 0;
-    const int v = *a.step_d;                                    // tokens finalised so far
-    const int pos = a.np - 1 + v;                               // absolute position of this step's token
-    const int C = a.C, HD = 64, kvd = a.nkv * HD, Wq = C + 2 * kvd, I = a.I;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int wg = blockIdx.x * (MG_THREADS / 32) + warp, TW = gridDim.x * (MG_THREADS / 32);
-    const int n_qkv = a.rope ? Wq / 2 : Wq, l_qkv = a.rope ? 1 : 0;      // items of the QKV phase
-    // gated MLP: item j = (gate j, up j); plain MLP: item j = columns (j, I/2 + j), two per warp so one round covers it
-    const int n_fc = a.gated ? I : I / 2, l_fc = 2, h_fc = a.gated ? I : I / 2;
+struct MsSm {                                            // fixed part of shared memory, behind the ring
+    unsigned long long full[MS_SLOTS], empty[MS_SLOTS];
+    int dead;
+    float red[2][MS_WARPS];
+    float att[MS_WARPS][MS_PW + 2];
+    float qn[3][64];                                     // this CTA's query head; the new key and value
+    float xres[8][MG_MAXB];                              // hidden state of the rows this CTA owns
+};
 
-    // embed: x[r] = wte[id] (+ wpe[pos])
-    for (int i = blockIdx.x * MG_THREADS + tid; i < a.B * C; i += gridDim.x * MG_THREADS) {
-        int r = i / C, c = i % C;
-        float e = a.wte[(size_t)a.ids[r] * C + c];
-        if (a.wpe) e = __fadd_rn(e, a.wpe[(size_t)a.posmat[(size_t)pos * a.B + r] * C + c]);
-        a.x[i] = e;
+__device__ __forceinline__ void ms_bar() { asm volatile("bar.sync 1, %0;" ::"n"(MS_T) : "memory"); }
+__device__ __forceinline__ void ll_store(uint2 *p, float v, unsigned tag) {
+    asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(__float_as_uint(v)), "r"(tag) : "memory");
+}
+__device__ __forceinline__ uint4 ll_load2(const uint2 *p) {
+    uint4 v;
+    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+struct MsCtx {
+    MsSm *sm; int *err;
+    // one slow step of a spin: false when the wait is over (limit, or another CTA gave up)
+    __device__ __forceinline__ bool still(unsigned &it, unsigned long long &t0) const {
+        if ((++it & 255u) != 0) return true;
+        if (*(volatile int *)&sm->dead) return false;
+        const unsigned long long now = gtime_ns();
+        if (t0 == 0) t0 = now;
+        if (*(volatile int *)err != 0) { *(volatile int *)&sm->dead = 1; return false; }
+        if (now - t0 > TC_WAIT_NS) { atomicExch(err, 61); *(volatile int *)&sm->dead = 1; return false; }
+        return true;
     }
-    mg_prefetch(a.layers[0].qkvw, C, l_qkv, 0, n_qkv);
-    mg_barrier(a, base, nb);
-
-    for (int li = 0; li < a.NL; li++) {
-        const MegaLayer L = a.layers[li];
-        // ---- norm + QKV, rotary pairs, K|V into the cache ----
-        mg_stage(a, a.x, C, C, a.norm, L.ln1w, L.ln1b, a.eps, xs, bred);
-        for (int it = wg; it < n_qkv; it += TW) {
-            int c0, c1;
-            mg_item_cols(l_qkv, it, 0, c0, c1);
-            float d0[MG_MAXB], d1[MG_MAXB];
-            if (a.rope) mg_item_dot<true>(a, L.qkvw, C, c0, c1, xs, C, d0, d1);
-            else mg_item_dot<false>(a, L.qkvw, C, c0, c1, xs, C, d0, d1);
-            if (lane < a.B) {
-                const int r = lane;
-                float y0 = 0.f, y1 = 0.f;
+    // N pairs of words at p[i] (16-byte aligned); absent ones (null) are zero
+    template <int N>
+    __device__ __forceinline__ void poll(const uint2 *const (&p)[N], unsigned tag, float2 (&v)[N]) const {
+        unsigned it = 0;
+        unsigned long long t0 = 0;
+        for (;;) {
+            uint4 w[N];
+            bool ok = true;
 #pragma unroll
-                for (int q = 0; q < MG_MAXB; q++) if (q == r) { y0 = d0[q]; y1 = d1[q]; }
-                if (L.qkvb) { y0 += L.qkvb[c0]; if (a.rope) y1 += L.qkvb[c1]; }
-                if (a.rope && c0 < C + kvd) {                    // q and k heads rotate, v does not
-                    const int d = c0 & 63;
-                    const size_t tp = (size_t)a.posmat[(size_t)pos * a.B + r] * HD;
-                    const float z0 = __fadd_rn(__fmul_rn(y0, a.cosb[tp + d]), __fmul_rn(-y1, a.sinb[tp + d]));
-                    const float z1 = __fadd_rn(__fmul_rn(y1, a.cosb[tp + d + 32]), __fmul_rn(y0, a.sinb[tp + d + 32]));
-                    y0 = z0; y1 = z1;
-                }
-                float *dst = L.kv + (size_t)r * a.kv_seq_pitch + (size_t)pos * 2 * kvd;
-                a.qkv[(size_t)r * Wq + c0] = y0;
-                if (c0 >= C) dst[c0 - C] = y0;
-                if (a.rope) { a.qkv[(size_t)r * Wq + c1] = y1; if (c1 >= C) dst[c1 - C] = y1; }
+            for (int i = 0; i < N; i++) w[i] = p[i] ? ll_load2(p[i]) : make_uint4(0u, tag, 0u, tag);
+#pragma unroll
+            for (int i = 0; i < N; i++) { ok = ok && w[i].y == tag && w[i].w == tag; v[i] = make_float2(__uint_as_float(w[i].x), __uint_as_float(w[i].z)); }
+            if (ok || !still(it, t0)) return;
+        }
+    }
+    __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) const {
+        unsigned it = 0;
+        unsigned long long t0 = 0;
+        for (;;) {
+            uint32_t ok;
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+            if (ok || !still(it, t0)) return;
+        }
+    }
+};
+
+// A warp's view of the weight stream: chunks known to have arrived, chunks it has given back.
+struct MsStream {
+    const unsigned char *ring; uint32_t full, empty;
+    int have = 0, rel = 0;
+    __device__ __forceinline__ void ensure(const MsCtx &c, long long end) {
+        while ((long long)have * MS_CH < end) { c.wait(full + 8 * (have % MS_SLOTS), (uint32_t)(have / MS_SLOTS) & 1u); have++; }
+    }
+    __device__ __forceinline__ void release(long long upto, int lane) {       // every byte below has been read by this warp
+        __syncwarp();
+        while ((long long)(rel + 1) * MS_CH <= upto) { if (lane == 0) mbar_arrive(empty + 8 * (rel % MS_SLOTS)); rel++; }
+    }
+};
+
+// eight weights at byte offset `off` of the stream
+template <bool W16>
+__device__ __forceinline__ void ms_w8(const unsigned char *ring, long long off, float *w) {
+    if (W16) {
+        const uint4 u = *(const uint4 *)(ring + (off & (MS_RING - 1)));
+        w[0] = __uint_as_float(u.x << 16); w[1] = __uint_as_float(u.x & 0xffff0000u);
+        w[2] = __uint_as_float(u.y << 16); w[3] = __uint_as_float(u.y & 0xffff0000u);
+        w[4] = __uint_as_float(u.z << 16); w[5] = __uint_as_float(u.z & 0xffff0000u);
+        w[6] = __uint_as_float(u.w << 16); w[7] = __uint_as_float(u.w & 0xffff0000u);
+    } else {
+        const float4 a = *(const float4 *)(ring + (off & (MS_RING - 1))), b = *(const float4 *)(ring + ((off + 16) & (MS_RING - 1)));
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    }
+}
+// eight sums of 32 lanes: afterwards lane l holds sum number l >> 2 (all four lanes of a group the same)
+__device__ __forceinline__ float ms_reduce8(float (&v)[8], int lane) {
+#pragma unroll
+    for (int w = 4, o = 16; w > 0; w >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < w; i++) {
+            const float give = up ? v[i] : v[i + w], keep = up ? v[i + w] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    return v[0];
+}
+
+// Rows [r0, r0 + n) of a [..][C] product whose stream begins at `base` (row r0's first byte): a warp takes quarter `warp & 3` of K
+// and every fourth row; part[row][quarter][m].
+template <int MT, bool W16>
+__device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long base, int n, int C, const float *xs, float *part, int warp, int lane) {
+    const int seg = warp & 3, rg = warp >> 2, L = C >> 5, esz = W16 ? 2 : 4;      // lanes of a quarter
+    const bool on = lane < L;
+    const long long rowb = (long long)C * esz, lo = (long long)(seg * (C >> 2) + lane * 8) * esz;
+    float xr[MT][8];
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int e = 0; e < 8; e += 4) {
+            const float4 v = on ? *(const float4 *)(xs + m * C + seg * (C >> 2) + lane * 8 + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xr[m][e] = v.x; xr[m][e + 1] = v.y; xr[m][e + 2] = v.z; xr[m][e + 3] = v.w;
+        }
+    for (int i0 = rg; i0 < n; i0 += 32) {
+        const int last = min(n - 1, i0 + 28);
+        st.ensure(c, base + (long long)(last + 1) * rowb);
+        float acc[MT][8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int r = i0 + 4 * j;
+            float w[8];
+            if (r < n && on) ms_w8<W16>(st.ring, base + r * rowb + lo, w);
+            else {
+#pragma unroll
+                for (int e = 0; e < 8; e++) w[e] = 0.f;
+            }
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                float t = w[0] * xr[m][0];
+#pragma unroll
+                for (int e = 1; e < 8; e++) t = fmaf(w[e], xr[m][e], t);
+                acc[m][j] = t;
             }
         }
-        mg_prefetch(L.ow, C, 0, 0, C);
-        {   // the cached K|V rows of this CTA's attention units: one 128-byte line per thread of the team
-            const int team = tid / MG_TEAM, t = tid % MG_TEAM, u = blockIdx.x * MG_TEAMS + team;
-            if (u < a.B * a.nkv * a.max_split) {
-                const int sp = u % a.max_split, kvh = (u / a.max_split) % a.nkv, row = u / (a.max_split * a.nkv);
-                const int key = sp * MG_KEYS + (t >> 2);
-                if (key < pos)                                      // rows of earlier steps only: this step's row is being written
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(L.kv + (size_t)row * a.kv_seq_pitch + (size_t)key * 2 * kvd +
-                                                                      ((t >> 1) & 1) * kvd + kvh * HD + (t & 1) * 32));
+        st.release(base + (long long)(i0 - rg + 32 <= n ? i0 - rg + 32 : n) * rowb, lane);
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+            const float s = ms_reduce8(acc[m], lane);
+            const int r = i0 + 4 * (lane >> 2);
+            if ((lane & 3) == 0 && r < n) part[(r * 4 + seg) * MT + m] = s;
+        }
+    }
+    st.release(base + (long long)n * rowb, lane);
+}
+
+// Down-projection rows [r0, r0 + n), n <= 8: the warp takes 256-wide pieces `warp`, `warp + 16` of K, whose inputs its lanes poll
+// straight into registers; part[row][warp][m].
+template <int MT, bool W16>
+__device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long base, int n, int I, const uint2 *hw, unsigned tag, float *part, int warp, int lane) {
+    const int esz = W16 ? 2 : 4;
+    const long long rowb = (long long)I * esz;
+    float acc[MT][8];
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[m][j] = 0.f;
+    float xr[2][MT][8];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int k = (warp + MS_WARPS * u) * 256 + lane * 8;
+        const uint2 *p[4 * MT];
+        float2 v[4 * MT];
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) p[4 * m + e] = k < I ? hw + (size_t)m * I + k + 2 * e : nullptr;
+        c.poll<4 * MT>(p, tag, v);
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) { xr[u][m][2 * e] = v[4 * m + e].x; xr[u][m][2 * e + 1] = v[4 * m + e].y; }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        if (r >= n) break;
+        st.ensure(c, base + (r + 1) * rowb);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int k = (warp + MS_WARPS * u) * 256 + lane * 8;
+            if (k < I) {
+                float w[8];
+                ms_w8<W16>(st.ring, base + r * rowb + (long long)k * esz, w);
+#pragma unroll
+                for (int m = 0; m < MT; m++)
+#pragma unroll
+                    for (int e = 0; e < 8; e++) acc[m][r] = fmaf(w[e], xr[u][m][e], acc[m][r]);
             }
         }
-        mg_barrier(a, base, nb);
-        // ---- attention over the cache (this step's key included) ----
+        st.release(base + (r + 1) * rowb, lane);
+    }
+#pragma unroll
+    for (int m = 0; m < MT; m++) {
+        const float s = ms_reduce8(acc[m], lane);
+        if ((lane & 3) == 0 && (lane >> 2) < n) part[((lane >> 2) * MS_WARPS + warp) * MT + m] = s;
+    }
+}
+
+// norm of MT rows of C values held as pairs by threads t < C / 2, into xs
+template <int MT>
+__device__ __forceinline__ void ms_norm(MsSm *sm, float2 (&v)[MT], int C, int kind, float2 w, float2 b, float eps, float *xs, int tid) {
+    const int lane = tid & 31, warp = tid >> 5;
+    const bool on = tid < (C >> 1);
+#pragma unroll
+    for (int m = 0; m < MT; m++) {
+        float mean = 0.f;
+        auto sum = [&](float s, int k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) sm->red[k][warp] = s;
+            ms_bar();
+            float t = 0.f;
+#pragma unroll
+            for (int q = 0; q < MS_WARPS; q++) t += sm->red[k][q];
+            return t;
+        };
+        if (kind == 1) mean = sum(on ? v[m].x + v[m].y : 0.f, 0) / (float)C;
+        const float d0 = v[m].x - mean, d1 = v[m].y - mean;
+        const float inv = 1.0f / sqrtf(sum(on ? d0 * d0 + d1 * d1 : 0.f, 1) / (float)C + eps);
+        if (on) *(float2 *)(xs + m * C + 2 * tid) = make_float2(__fadd_rn(__fmul_rn(__fmul_rn(d0, inv), w.x), b.x), __fadd_rn(__fmul_rn(__fmul_rn(d1, inv), w.y), b.y));
+        if (MT > 1) ms_bar();                                // red is reused by the next row
+    }
+    if (MT == 1) ms_bar();
+}
+
+// attention of query head h of row b over keys [k0, k1): `cached` keys in kv, key `cached` (the new token's) in sm->qn; the
+// first four groups of 32 keys were requested by the caller (kf, vf). Partial to p.
+struct MsKV { float4 k[4], v[4]; };
+__device__ __forceinline__ void ms_kv_load(MsKV &f, const float *kv, int64_t pitch, int kvd, int j0, int k1, int cached, int warp, int lane) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int j = j0 + 32 * i + warp * 2 + (lane >> 4);
+        if (j < k1 && j < cached) {
+            const float *p = kv + (int64_t)j * pitch + 4 * (lane & 15);
+            f.k[i] = *(const float4 *)p; f.v[i] = *(const float4 *)(p + kvd);
+        } else f.k[i] = f.v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+__device__ __forceinline__ void ms_attend(MsSm *sm, MsKV &f, const float *kv, int64_t pitch, int kvd, int k0, int k1, int cached, uint2 *out, unsigned tag, int tid) {
+    const int lane = tid & 31, warp = tid >> 5, dp = lane & 15, kg = lane >> 4;
+    const float4 q = *(const float4 *)&sm->qn[0][4 * dp];
+    float m = -INFINITY, l = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j0 = k0; j0 < k1; j0 += 128) {
+        if (j0 > k0) ms_kv_load(f, kv, pitch, kvd, j0, k1, cached, warp, lane);
+        float s[4], mx = m;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int j = j0 + 32 * i + warp * 2 + kg;
+            if (j == cached) { f.k[i] = *(const float4 *)&sm->qn[1][4 * dp]; f.v[i] = *(const float4 *)&sm->qn[2][4 * dp]; }
+            float t = q.x * f.k[i].x;
+            t = fmaf(q.y, f.k[i].y, t); t = fmaf(q.z, f.k[i].z, t); t = fmaf(q.w, f.k[i].w, t);
+#pragma unroll
+            for (int x = 8; x > 0; x >>= 1) t += __shfl_xor_sync(0xffffffffu, t, x);
+            s[i] = j < k1 ? t * 0.125f : -INFINITY;          // 1 / sqrt(64)
+            mx = fmaxf(mx, s[i]);
+        }
+        if (mx > -INFINITY) {
+            const float al = m == -INFINITY ? 0.f : expf(m - mx);
+            l *= al; o.x *= al; o.y *= al; o.z *= al; o.w *= al;
+            m = mx;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float p = expf(s[i] - m);
+                l += p;
+                o.x = fmaf(p, f.v[i].x, o.x); o.y = fmaf(p, f.v[i].y, o.y); o.z = fmaf(p, f.v[i].z, o.z); o.w = fmaf(p, f.v[i].w, o.w);
+            }
+        }
+    }
+    // the two halves of the warp, then the warps
+    const float m2 = __shfl_xor_sync(0xffffffffu, m, 16), M = fmaxf(m, m2), e = m == -INFINITY ? 0.f : expf(m - M);
+    l *= e; o.x *= e; o.y *= e; o.z *= e; o.w *= e;
+    l += __shfl_xor_sync(0xffffffffu, l, 16);
+    o.x += __shfl_xor_sync(0xffffffffu, o.x, 16); o.y += __shfl_xor_sync(0xffffffffu, o.y, 16);
+    o.z += __shfl_xor_sync(0xffffffffu, o.z, 16); o.w += __shfl_xor_sync(0xffffffffu, o.w, 16);
+    if (kg == 0) {
+        float *a = sm->att[warp];
+        if (dp == 0) { a[0] = M; a[1] = l; }
+        a[2 + 4 * dp] = o.x; a[3 + 4 * dp] = o.y; a[4 + 4 * dp] = o.z; a[5 + 4 * dp] = o.w;
+    }
+    ms_bar();
+    if (tid < MS_PW) {
+        float X = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < MS_WARPS; w++) X = fmaxf(X, sm->att[w][0]);
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < MS_WARPS; w++) {
+            const float mw = sm->att[w][0];
+            if (mw != -INFINITY) t = fmaf(sm->att[w][tid == 0 ? 1 : tid], expf(mw - X), t);
+        }
+        ll_store(out + tid, tid == 0 ? X : t, tag);
+    }
+}
+
+template <int MT, bool W16>
+__global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ MegaArgs a, const unsigned char *stream_w, const long long *stream_off, const unsigned char *head_w) {
+    extern __shared__ __align__(1024) unsigned char ms_raw[];
+    const MegaShape &S = a.s;
+    unsigned char *ring = ms_raw;
+    MsSm *sm = (MsSm *)(ring + MS_RING);
+    float *xs = (float *)(((uintptr_t)(sm + 1) + 15) & ~(uintptr_t)15);          // [MT][C] normed input of a product
+    float *part = xs + MT * S.C;                                                 // sums by quarter of K (or by warp)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x, g = gridDim.x;
+    const int C = S.C, I = S.I, kvd = S.nkv * 64, Wq = C + 2 * kvd, esz = W16 ? 2 : 4;
+    // this CTA's share of every product
+    const int q0 = ms_begin(Wq >> 1, cta, g), nq = ms_begin(Wq >> 1, cta + 1, g) - q0;        // pairs (d, d + 32) of a head
+    const int c0 = ms_begin(C, cta, g), ncr = ms_begin(C, cta + 1, g) - c0;                   // rows of the o- and down-projections
+    const int u0 = ms_begin(I, cta, g), nu = ms_begin(I, cta + 1, g) - u0, ur = S.gated ? 2 * nu : nu;
+    const int v0 = ms_begin(S.V, cta, g), nv = ms_begin(S.V, cta + 1, g) - v0;
+    const long long b_qkv = 2LL * nq * C * esz, b_o = (long long)ncr * C * esz, b_up = (long long)ur * C * esz, b_dn = (long long)ncr * I * esz;
+    const long long b_layer = b_qkv + b_o + b_up + b_dn, b_all = b_layer * S.NL, b_head = (long long)nv * C * esz;
+    const long long head_at = ((b_all + MS_CH - 1) / MS_CH) * MS_CH;                          // the head starts on a chunk of its own
+    const uint32_t full = smem_u32(sm->full), empty = smem_u32(sm->empty);
+    if (tid == 0) {
+        for (int s = 0; s < MS_SLOTS; s++) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, MS_WARPS); }
+        sm->dead = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    MsCtx c{sm, a.err};
+
+    if (warp == MS_WARPS) {                                  // ---- the weight stream ----
+        if (lane == 0) {
+            const unsigned char *src = stream_w + stream_off[cta], *hsrc = head_w + (long long)v0 * C * esz;
+            const int n_body = (int)(head_at / MS_CH), n_all = n_body + (int)((b_head + MS_CH - 1) / MS_CH);
+            int k = 0;
+            for (; k < n_all; k++) {
+                const int s = k % MS_SLOTS;
+                if (k >= MS_SLOTS) c.wait(empty + 8 * s, (uint32_t)(k / MS_SLOTS - 1) & 1u);
+                if (*(volatile int *)&sm->dead) break;
+                const bool body = k < n_body;
+                const long long off = (long long)(body ? k : k - n_body) * MS_CH, left = (body ? b_all : b_head) - off;
+                const uint32_t bytes = left < MS_CH ? (uint32_t)left : MS_CH;
+                mbar_expect_tx(full + 8 * s, bytes);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             ::"r"(smem_u32(ring + s * MS_CH)), "l"((body ? src : hsrc) + off), "r"(bytes), "r"(full + 8 * s) : "memory");
+            }
+            for (int j = k - MS_SLOTS < 0 ? 0 : k - MS_SLOTS; j < k; j++)       // every copy has landed before the CTA may end
+                mbar_wait(full + 8 * (j % MS_SLOTS), (uint32_t)(j / MS_SLOTS) & 1u, a.err, 62);
+        }
+        return;
+    }
+
+    // ---- consumers ----
+    MsStream st{ring, full, empty};
+    const MsLL ll(S);
+    uint2 *Lx = a.ll + ll.x, *Lx1 = a.ll + ll.x1, *Lq = a.ll + ll.q, *Lp = a.ll + ll.p, *Lh = a.ll + ll.h;
+    const int step = *a.step_d, nsp = ms_splits(S, g);
+    const unsigned tag0 = (unsigned)step * (unsigned)S.NL + 1u;
+    const int *pos = a.posmat + (int64_t)(step + a.pos_base) * S.B;
+    const bool on2 = tid < (C >> 1);                          // this thread holds elements 2 tid, 2 tid + 1 of a hidden row
+    auto pair_of = [&](const float *p, float none) { return p && on2 ? __ldg((const float2 *)p + tid) : make_float2(none, none); };
+    // attention share: query head ah of row ab, part asp of its keys
+    const bool att = cta < S.B * S.H * nsp;
+    const int ab = att ? cta / (S.H * nsp) : 0, ah = att ? (cta / nsp) % S.H : 0, asp = cta % nsp, akv = ah / (S.H / S.nkv);
+    const int cached = att ? pos[ab] : 0, n_keys = cached + 1, per = (n_keys + nsp - 1) / nsp;
+    const int k0 = min(n_keys, asp * per), k1 = min(n_keys, k0 + per);
+    long long at = 0;                                         // stream offset
+    float2 xv[MT];
+    for (int li = 0; li < S.NL; li++) {
+        const MegaLayer &L = a.layers[li];
+        const unsigned tag = tag0 + (unsigned)li;
+        const float *kvb = att ? L.kv + (int64_t)ab * a.kv_seq_pitch + akv * 64 : nullptr;
+        // ---- hidden state, norm, q k v ----
         {
-            const int team = tid / MG_TEAM, t = tid % MG_TEAM;
-            const int nunits = a.B * a.nkv * a.max_split;
-            for (int u = blockIdx.x * MG_TEAMS + team; u < nunits; u += gridDim.x * MG_TEAMS) {
-                const int sp = u % a.max_split, kvh = (u / a.max_split) % a.nkv, row = u / (a.max_split * a.nkv);
-                const int n1 = a.lenmat[(size_t)pos * a.B + row];
-                if (sp * MG_KEYS < n1) mg_attn_unit(a, L, row, kvh, sp, n1, asmem[team], team, t);
-            }
-        }
-        mg_barrier(a, base, nb);
-        // ---- output projection + residual (input rows straight from L2) ----
-        for (int it = wg; it < C; it += TW) {
-            float d0[MG_MAXB], d1[MG_MAXB];
-            mg_item_dot<false>(a, L.ow, C, it, -1, a.ctx, C, d0, d1);
-            if (lane < a.B) {
-                float y = 0.f;
+            const float2 w = pair_of(L.ln1w, 1.f), b = pair_of(L.ln1b, 0.f);
+            if (li == 0) {
 #pragma unroll
-                for (int q = 0; q < MG_MAXB; q++) if (q == lane) y = d0[q];
-                if (L.ob) y += L.ob[it];
-                a.x[(size_t)lane * C + it] = y + a.x[(size_t)lane * C + it];
-            }
-        }
-        mg_prefetch(L.fcw, C, l_fc, h_fc, n_fc);
-        mg_barrier(a, base, nb);
-        // ---- norm + MLP up (+ gated product) ----
-        mg_stage(a, a.x, C, C, a.norm, L.ln2w, L.ln2b, a.eps, xs, bred);
-        for (int it = wg; it < n_fc; it += TW) {
-            float d0[MG_MAXB], d1[MG_MAXB];
-            mg_item_dot<true>(a, L.fcw, C, it, h_fc + it, xs, C, d0, d1);
-            if (lane < a.B) {
-                float g = 0.f, up = 0.f;
+                for (int m = 0; m < MT; m++) {
+                    xv[m] = make_float2(0.f, 0.f);
+                    if (m < S.B && on2) {
+                        xv[m] = *((const float2 *)(a.wte + (int64_t)a.ids[m] * C) + tid);
+                        if (a.wpe) { const float2 p = *((const float2 *)(a.wpe + (int64_t)pos[m] * C) + tid); xv[m].x = __fadd_rn(xv[m].x, p.x); xv[m].y = __fadd_rn(xv[m].y, p.y); }
+                    }
+                }
+            } else {
+                const uint2 *p[MT];
 #pragma unroll
-                for (int q = 0; q < MG_MAXB; q++) if (q == lane) { g = d0[q]; up = d1[q]; }
-                if (L.fcb) { g += L.fcb[it]; up += L.fcb[h_fc + it]; }
-                if (a.gated) a.h[(size_t)lane * I + it] = __fmul_rn(mg_act(g, a.act), up);
-                else { a.h[(size_t)lane * I + it] = mg_act(g, a.act); a.h[(size_t)lane * I + h_fc + it] = mg_act(up, a.act); }
+                for (int m = 0; m < MT; m++) p[m] = m < S.B && on2 ? Lx + (size_t)m * C + 2 * tid : nullptr;
+                c.poll<MT>(p, tag - 1u, xv);
             }
-        }
-        mg_prefetch(L.pw, I, 0, 0, C);
-        mg_barrier(a, base, nb);
-        // ---- MLP down + residual ----
-        for (int it = wg; it < C; it += TW) {
-            float d0[MG_MAXB], d1[MG_MAXB];
-            mg_item_dot<false>(a, L.pw, I, it, -1, a.h, I, d0, d1);
-            if (lane < a.B) {
-                float y = 0.f;
 #pragma unroll
-                for (int q = 0; q < MG_MAXB; q++) if (q == lane) y = d0[q];
-                if (L.pb) y += L.pb[it];
-                a.x[(size_t)lane * C + it] = y + a.x[(size_t)lane * C + it];
+            for (int m = 0; m < MT; m++) {
+                const int r = 2 * tid - c0;
+                if (on2 && r >= 0 && r < ncr) sm->xres[r][m] = xv[m].x;
+                if (on2 && r + 1 >= 0 && r + 1 < ncr) sm->xres[r + 1][m] = xv[m].y;
+            }
+            ms_norm<MT>(sm, xv, C, a.norm, w, b, a.eps, xs, tid);
+        }
+        ms_rows<MT, W16>(c, st, at, 2 * nq, C, xs, part, warp, lane);
+        at += b_qkv;
+        ms_bar();
+        for (int t = tid; t < nq * S.B; t += MS_T) {
+            const int i = t / S.B, m = t - i * S.B, pr = q0 + i, h = pr >> 5, d = pr & 31;
+            const float *p0 = part + (size_t)(2 * i) * 4 * MT + m, *p1 = p0 + 4 * MT;
+            float y0 = (p0[0] + p0[MT]) + (p0[2 * MT] + p0[3 * MT]), y1 = (p1[0] + p1[MT]) + (p1[2 * MT] + p1[3 * MT]);
+            if (L.qkvb) { y0 += __ldg(L.qkvb + h * 64 + d); y1 += __ldg(L.qkvb + h * 64 + d + 32); }
+            if (a.cosb && h < S.H + S.nkv) {
+                const float *co = a.cosb + (int64_t)pos[m] * 64 + d, *si = a.sinb + (int64_t)pos[m] * 64 + d;
+                const float z0 = __fadd_rn(__fmul_rn(y0, co[0]), __fmul_rn(-y1, si[0])), z1 = __fadd_rn(__fmul_rn(y1, co[32]), __fmul_rn(y0, si[32]));
+                y0 = z0; y1 = z1;
+            }
+            uint2 *o = Lq + (size_t)m * Wq + h * 64 + d;
+            ll_store(o, y0, tag); ll_store(o + 32, y1, tag);
+            if (h >= S.H) {
+                float *kv = L.kv + (int64_t)m * a.kv_seq_pitch + (int64_t)pos[m] * 2 * kvd + (h - S.H) * 64 + d;
+                kv[0] = y0; kv[32] = y1;
             }
         }
-        if (li + 1 < a.NL) mg_prefetch(a.layers[li + 1].qkvw, C, l_qkv, 0, n_qkv);
-        else mg_prefetch(a.wte, C, 0, 0, a.V);
-        mg_barrier(a, base, nb);
+        // ---- attention partials ----
+        if (att) {
+            MsKV f;
+            ms_kv_load(f, kvb, 2 * kvd, kvd, k0, k1, cached, warp, lane);
+            if (warp < 3) {
+                const int h = warp == 0 ? ah : (warp == 1 ? S.H + akv : S.H + S.nkv + akv);
+                const uint2 *p[1] = {warp == 0 || k1 == n_keys ? Lq + (size_t)ab * Wq + h * 64 + 2 * lane : nullptr};
+                float2 v[1];
+                c.poll<1>(p, tag, v);
+                *(float2 *)&sm->qn[warp][2 * lane] = v[0];
+            }
+            ms_bar();
+            ms_attend(sm, f, kvb, 2 * kvd, kvd, k0, k1, cached, Lp + ((size_t)(ab * S.H + ah) * MS_MAXSPLIT + asp) * MS_PW, tag, tid);
+        }
+        // ---- context, o-projection, residual ----
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+            if (m >= S.B) { if (on2) *(float2 *)(xs + m * C + 2 * tid) = make_float2(0.f, 0.f); continue; }
+            const uint2 *p[2 * MS_MAXSPLIT];
+            float2 v[2 * MS_MAXSPLIT];
+#pragma unroll
+            for (int s = 0; s < MS_MAXSPLIT; s++) {
+                const uint2 *b = on2 && s < nsp ? Lp + ((size_t)(m * S.H + (tid >> 5)) * MS_MAXSPLIT + s) * MS_PW : nullptr;
+                p[2 * s] = b; p[2 * s + 1] = b ? b + 2 + 2 * (tid & 31) : nullptr;
+            }
+            c.poll<2 * MS_MAXSPLIT>(p, tag, v);
+            float M = -INFINITY;
+#pragma unroll
+            for (int s = 0; s < MS_MAXSPLIT; s++) if (s < nsp) M = fmaxf(M, v[2 * s].x);
+            float l = 0.f, o0 = 0.f, o1 = 0.f;
+#pragma unroll
+            for (int s = 0; s < MS_MAXSPLIT; s++)
+                if (s < nsp && v[2 * s].x != -INFINITY) {
+                    const float e = expf(v[2 * s].x - M);
+                    l = fmaf(v[2 * s].y, e, l); o0 = fmaf(v[2 * s + 1].x, e, o0); o1 = fmaf(v[2 * s + 1].y, e, o1);
+                }
+            const float inv = l > 0.f ? 1.0f / l : 0.f;
+            if (on2) *(float2 *)(xs + m * C + 2 * tid) = make_float2(o0 * inv, o1 * inv);
+        }
+        ms_bar();
+        ms_rows<MT, W16>(c, st, at, ncr, C, xs, part, warp, lane);
+        at += b_o;
+        ms_bar();
+        if (tid < ncr * S.B) {
+            const int r = tid / S.B, m = tid - r * S.B;
+            const float *p = part + (size_t)r * 4 * MT + m;
+            float y = (p[0] + p[MT]) + (p[2 * MT] + p[3 * MT]);
+            if (L.ob) y += __ldg(L.ob + c0 + r);
+            y += sm->xres[r][m];
+            sm->xres[r][m] = y;
+            ll_store(Lx1 + (size_t)m * C + c0 + r, y, tag);
+        }
+        // ---- second norm, up-projection, activation ----
+        {
+            const float2 w = pair_of(L.ln2w, 1.f), b = pair_of(L.ln2b, 0.f);
+            const uint2 *p[MT];
+#pragma unroll
+            for (int m = 0; m < MT; m++) p[m] = m < S.B && on2 ? Lx1 + (size_t)m * C + 2 * tid : nullptr;
+            c.poll<MT>(p, tag, xv);
+            ms_norm<MT>(sm, xv, C, a.norm, w, b, a.eps, xs, tid);
+        }
+        ms_rows<MT, W16>(c, st, at, ur, C, xs, part, warp, lane);
+        at += b_up;
+        ms_bar();
+        for (int t = tid; t < nu * S.B; t += MS_T) {
+            const int i = t / S.B, m = t - i * S.B;
+            float y;
+            if (S.gated) {
+                const float *p0 = part + (size_t)(2 * i) * 4 * MT + m, *p1 = p0 + 4 * MT;
+                float gt = (p0[0] + p0[MT]) + (p0[2 * MT] + p0[3 * MT]), up = (p1[0] + p1[MT]) + (p1[2 * MT] + p1[3 * MT]);
+                if (L.fcb) { gt += __ldg(L.fcb + u0 + i); up += __ldg(L.fcb + I + u0 + i); }
+                y = __fmul_rn(tc_act(gt, a.act), up);
+            } else {
+                const float *p = part + (size_t)i * 4 * MT + m;
+                y = (p[0] + p[MT]) + (p[2 * MT] + p[3 * MT]);
+                if (L.fcb) y += __ldg(L.fcb + u0 + i);
+                y = tc_act(y, a.act);
+            }
+            ll_store(Lh + (size_t)m * I + u0 + i, y, tag);
+        }
+        ms_bar();                                             // part is rewritten by the down-projection
+        // ---- down-projection, residual ----
+        ms_down<MT, W16>(c, st, at, ncr, I, Lh, tag, part, warp, lane);
+        at += b_dn;
+        ms_bar();
+        if (tid < ncr * S.B) {
+            const int r = tid / S.B, m = tid - r * S.B;
+            float y = 0.f;
+#pragma unroll
+            for (int q = 0; q < MS_WARPS; q++) y += part[((size_t)r * MS_WARPS + q) * MT + m];
+            if (L.pb) y += __ldg(L.pb + c0 + r);
+            y += sm->xres[r][m];
+            ll_store(Lx + (size_t)m * C + c0 + r, y, tag);
+        }
     }
-    // ---- final norm, vocabulary projection, greedy pick ----
-    mg_stage(a, a.x, C, C, a.norm, a.lnfw, a.lnfb, a.eps_f, xs, bred);
-    if (tid < MG_MAXB) s_best[tid] = 0;
-    __syncthreads();
+    // ---- final norm, vocabulary projection ----
     {
-        unsigned long long best = 0;
-        for (int it = wg; it < a.V; it += TW) {
-            float d0[MG_MAXB], d1[MG_MAXB];
-            mg_item_dot<false>(a, a.wte, C, it, -1, xs, C, d0, d1);
-            if (lane < a.B) {
-                float y = 0.f;
+        const float2 w = pair_of(a.lnfw, 1.f), b = pair_of(a.lnfb, 0.f);
+        const uint2 *p[MT];
 #pragma unroll
-                for (int q = 0; q < MG_MAXB; q++) if (q == lane) y = d0[q];
-                a.logits[(size_t)lane * a.V + it] = y;
-                unsigned ub = __float_as_uint(y);
-                ub = (ub & 0x80000000u) ? ~ub : (ub | 0x80000000u);
-                const unsigned long long pk = ((unsigned long long)ub << 32) | (0xffffffffu - (unsigned)it);
-                if (pk > best) best = pk;
-            }
-        }
-        if (a.greedy && lane < a.B && best) atomicMax(&s_best[lane], best);
+        for (int m = 0; m < MT; m++) p[m] = m < S.B && on2 ? Lx + (size_t)m * C + 2 * tid : nullptr;
+        c.poll<MT>(p, tag0 + (unsigned)S.NL - 1u, xv);
+        ms_norm<MT>(sm, xv, C, a.norm, w, b, a.eps_f, xs, tid);
     }
-    __syncthreads();
-    if (a.greedy && tid < a.B && s_best[tid]) atomicMax(a.amax + tid, s_best[tid]);
-    mg_barrier(a, base, nb);
-    if (blockIdx.x == 0) {
-        if (a.greedy && tid < a.B) {                             // close the step: token v of every row
-            const int tkn = (int)(0xffffffffu - (unsigned)(a.amax[tid] & 0xffffffffull));
-            a.out[(size_t)tid * a.n_new + v] = tkn;
-            a.ids_out[tid] = tkn;
-            a.amax[tid] = 0;
+    st.release(head_at, lane);
+    at = head_at;
+    int buf = 0;
+    for (int r0 = 0; r0 < nv; r0 += MS_HROWS, buf ^= 1) {
+        const int n = min(MS_HROWS, nv - r0);
+        float *pb = part + buf * MS_HROWS * 4 * MT;
+        ms_rows<MT, W16>(c, st, at, n, C, xs, pb, warp, lane);
+        at += (long long)n * C * esz;
+        ms_bar();                                             // (the other half of `part` is free by the next barrier)
+        for (int t = tid; t < n * S.B; t += MS_T) {
+            const int m = t / n, r = t - m * n;
+            const float *p = pb + (size_t)r * 4 * MT + m;
+            a.logits[(size_t)m * S.V + v0 + r0 + r] = (p[0] + p[MT]) + (p[2 * MT] + p[3 * MT]);
         }
-        __syncthreads();
-        if (tid == 0) {
-            if (a.greedy) *a.step_d = v + 1;
-            *a.bar_base = base + nb * gridDim.x;                 // where the counter stands for the next launch
-        }
+    }
+    st.release(head_at + ((b_head + MS_CH - 1) / MS_CH) * MS_CH, lane);
+}
+
+// one layer's rows into the CTAs' streams: block (cta, matrix)
+__global__ void __launch_bounds__(256) k_mega_pack(MegaShape S, int li, int esz, const unsigned char *qkv, const unsigned char *o, const unsigned char *up, const unsigned char *dn,
+                                                   const long long *off, unsigned char *dst) {
+    const int cta = blockIdx.x, g = gridDim.x, mat = blockIdx.y, C = S.C, I = S.I, Wq = C + 128 * S.nkv;
+    const int q0 = ms_begin(Wq >> 1, cta, g), nq = ms_begin(Wq >> 1, cta + 1, g) - q0;
+    const int c0 = ms_begin(C, cta, g), ncr = ms_begin(C, cta + 1, g) - c0;
+    const int u0 = ms_begin(I, cta, g), nu = ms_begin(I, cta + 1, g) - u0, ur = S.gated ? 2 * nu : nu;
+    const long long rc = (long long)C * esz, rI = (long long)I * esz;
+    const long long layer = 2LL * nq * rc + ncr * rc + ur * rc + ncr * rI;
+    unsigned char *d = dst + off[cta] + li * layer + (mat > 0 ? 2LL * nq * rc : 0) + (mat > 1 ? ncr * rc : 0) + (mat > 2 ? ur * rc : 0);
+    const int n = mat == 0 ? 2 * nq : mat == 1 ? ncr : mat == 2 ? ur : ncr;
+    const long long row = mat == 3 ? rI : rc;
+    const unsigned char *src = mat == 0 ? qkv : mat == 1 ? o : mat == 2 ? up : dn;
+    for (int i = 0; i < n; i++) {
+        int r;
+        if (mat == 0) { const int pr = q0 + (i >> 1); r = (pr >> 5) * 64 + (pr & 31) + (i & 1) * 32; }
+        else if (mat == 2) r = S.gated ? u0 + (i >> 1) + (i & 1) * I : u0 + i;
+        else r = c0 + i;
+        for (long long b = threadIdx.x * 16; b < row; b += 256 * 16) *(uint4 *)(d + i * row + b) = *(const uint4 *)(src + r * row + b);
     }
 }
 
-// Off unless asked for (ncmb_set_lm_persistent(1) or NCM_B200_LM_PERSISTENT=1): measured on GPT-2 124M, batch 1,
-// the persistent kernel takes 0.51 ms per token against 0.47 ms for the graph-replayed kernel chain -- its 62
-// grid barriers cost 2-4 us each, as much as the launches they replace.
 static int g_lm_persistent = -1;
 void lm_mega_enable(int on) { g_lm_persistent = on ? 1 : 0; }
-bool lm_mega_eligible(int B, int hd, int C, int I, bool qk_norm) {
-    if (g_lm_persistent < 0) g_lm_persistent = getenv("NCM_B200_LM_PERSISTENT") ? 1 : 0;
-    return g_lm_persistent == 1 && B >= 1 && B <= MG_MAXB && hd == 64 && (C % 64) == 0 && (I % 8) == 0 && !qk_norm;
+bool lm_mega_enabled() {
+    if (g_lm_persistent < 0) { const char *e = getenv("NCM_B200_LM_PERSISTENT"); g_lm_persistent = e ? atoi(e) != 0 : 1; }
+    return g_lm_persistent == 1;
+}
+bool lm_mega_supported(const MegaShape &s, int hd, bool qk_norm) {
+    const int g = ctx().sm_count;
+    return s.B >= 1 && s.B <= MG_MAXB && hd == 64 && s.C == s.H * 64 && s.C % 32 == 0 && s.C <= MS_MAXC && s.I % 8 == 0 && s.I <= MS_MAXI && !qk_norm &&
+           s.H % s.nkv == 0 && s.B * s.H <= g && cdiv(s.C, g) <= 8 && 2 * cdiv(s.I, g) <= MS_UPROWS && cdiv(s.C + 128 * s.nkv, g) + 2 <= MS_UPROWS &&
+           (int64_t)s.C * 4 * 32 + 2 * MS_CH <= MS_RING && (int64_t)s.I * 4 + 2 * MS_CH <= MS_RING;
 }
 
-size_t lm_mega_smem(const MegaArgs &a) {
-    size_t rows = (size_t)a.B * (a.C > a.I ? a.C : a.I) * 4;
-    size_t attn = sizeof(MgAttnSmem) * MG_TEAMS;
-    return (rows > attn ? rows : attn) + 16;
+void lm_mega_free(MegaModel &m) {
+    if (m.stream_w) dev_free(m.stream_w);
+    if (m.stream_off) dev_free(m.stream_off);
+    m = MegaModel();
 }
 
-void lm_mega_launch(const MegaArgs &a) {
-    const size_t smem = lm_mega_smem(a);
-    static size_t attr = 0;
-    if (smem > attr) {
-        CUDA_CHECK(cudaFuncSetAttribute(k_lm_decode_mega, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr = smem;
+void lm_mega_pack(MegaModel &m, const MegaShape &s, const std::vector<BlockWeights> &blocks, const float *wte, const unsigned short *wte16) {
+    if (m.ready) return;
+    const int g = ctx().sm_count;
+    m.grid = g;
+    m.w16 = wte16 != nullptr;
+    for (auto &b : blocks) m.w16 = m.w16 && b.qkvw16 && b.ow16 && b.fcw16 && b.pw16;
+    const int esz = m.w16 ? 2 : 4, Wq = s.C + 128 * s.nkv;
+    std::vector<long long> off(g + 1, 0);
+    for (int c = 0; c < g; c++) {
+        const long long nq = ms_begin(Wq / 2, c + 1, g) - ms_begin(Wq / 2, c, g), nc = ms_begin(s.C, c + 1, g) - ms_begin(s.C, c, g);
+        const long long nu = ms_begin(s.I, c + 1, g) - ms_begin(s.I, c, g);
+        off[c + 1] = off[c] + s.NL * esz * ((2 * nq + nc + (s.gated ? 2 : 1) * nu) * s.C + nc * s.I);
     }
-    int per_sm = 0;
-    CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lm_decode_mega, MG_THREADS, smem));
-    if (per_sm < 1) fatal("lm_mega: the persistent decode kernel does not fit an SM (%zu bytes of shared memory)", smem);
+    m.stream_w = dev_alloc((size_t)off[g]);
+    m.stream_off = (long long *)dev_alloc(sizeof(long long) * (g + 1));
+    upload(m.stream_off, off.data(), sizeof(long long) * (g + 1));
+    for (int li = 0; li < s.NL; li++) {
+        const BlockWeights &b = blocks[li];
+        auto pick = [&](const float *w, const unsigned short *w16) { return m.w16 ? (const unsigned char *)w16 : (const unsigned char *)w; };
+        LAUNCH(k_mega_pack, dim3((unsigned)g, 4), 256, 0, s, li, esz, pick(b.qkvw, b.qkvw16), pick(b.ow, b.ow16), pick(b.fcw, b.fcw16), pick(b.pw, b.pw16),
+               (const long long *)m.stream_off, (unsigned char *)m.stream_w);
+    }
+    m.head_w = m.w16 ? (const void *)wte16 : (const void *)wte;
+    m.ready = true;
+}
+
+size_t lm_mega_exchange_words(const MegaShape &s) { return MsLL(s).total; }
+
+template <int MT, bool W16>
+static void launch_step(const MegaModel &m, const MegaArgs &a) {
+    const MegaShape &s = a.s;
+    const size_t part = (size_t)std::max<int64_t>(2 * MS_HROWS, 2 * cdiv(s.I, m.grid) + 2) * 4;
+    const size_t smem = MS_RING + sizeof(MsSm) + 16 + ((size_t)MT * s.C + part * MT) * 4;
+    static size_t set = 0;
+    if (smem > set) { CUDA_CHECK(cudaFuncSetAttribute((k_lm_step<MT, W16>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = smem; }
     MegaArgs arg = a;
-    void *params[] = {&arg};
-    ProfScope ps(NCMB_K_GEMM, 0, 0);
-    cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_lm_decode_mega, dim3(ctx().sm_count), dim3(MG_THREADS), params, smem, stream());
+    const unsigned char *w = (const unsigned char *)m.stream_w, *h = (const unsigned char *)m.head_w;
+    const long long *off = m.stream_off;
+    void *params[] = {&arg, &w, &off, &h};
+    cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_lm_step<MT, W16>, dim3((unsigned)m.grid), dim3(MS_T + 32), params, smem, stream());
     if (e != cudaSuccess) fatal("lm_mega: cooperative launch failed: %s", cudaGetErrorString(e));
     ctx().launches++;
+}
+void lm_mega_launch(const MegaModel &m, const MegaArgs &a) {
+    ProfScope ps(NCMB_K_GEMM, 0, 0);
+    const int mt = a.s.B <= 1 ? 1 : a.s.B <= 2 ? 2 : 4;
+    if (mt == 1) { if (m.w16) launch_step<1, true>(m, a); else launch_step<1, false>(m, a); }
+    else if (mt == 2) { if (m.w16) launch_step<2, true>(m, a); else launch_step<2, false>(m, a); }
+    else { if (m.w16) launch_step<4, true>(m, a); else launch_step<4, false>(m, a); }
 }
 
 } // namespace ncmb

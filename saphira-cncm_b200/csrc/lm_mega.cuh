@@ -1,4 +1,4 @@
-// Persistent decode-step kernel of the decoder LMs (lm_mega.cu): argument block shared with lm.cu.
+// Persistent decode-step kernel of the decoder LMs (lm_mega.cu).
 #pragma once
 #include "common.cuh"
 
@@ -6,34 +6,40 @@ namespace ncmb {
 
 constexpr int MG_MAXB = 4;            // sequences per step the persistent kernel takes
 
-struct MegaLayer {
-    const float *ln1w, *ln1b, *qkvw, *qkvb, *ow, *ob, *ln2w, *ln2b, *fcw, *fcb, *pw, *pb;
-    float *kv;                        // this layer's cache [B][cap][2*nkv*hd]
+struct MegaLayer { const float *ln1w, *ln1b, *qkvb, *ob, *ln2w, *ln2b, *fcb, *pb; float *kv; };
+
+// What the kernel needs of a model, laid out once: every CTA's weight rows of all layers, in the order it uses them, as one
+// stream (bf16 where every matrix holds bf16 values, else fp32).
+struct MegaModel {
+    bool ready = false, w16 = false;
+    int grid = 0;
+    void *stream_w = nullptr;             // [CTA][layer][qkv pairs | o rows | up pairs or rows | down rows]
+    long long *stream_off = nullptr;      // device: byte offset of each CTA's stream
+    const void *head_w = nullptr;         // vocabulary projection [V][C], fp32 or bf16
 };
+struct MegaShape { int B, C, H, nkv, I, NL, V; int gated; };
+bool lm_mega_supported(const MegaShape &s, int hd, bool qk_norm);
+void lm_mega_pack(MegaModel &m, const MegaShape &s, const std::vector<BlockWeights> &blocks, const float *wte, const unsigned short *wte16);
+void lm_mega_free(MegaModel &m);
 
 struct MegaArgs {
-    int B, C, H, nkv, I, NL, V;
-    int norm;                         // 1 LayerNorm, 2 RMSNorm
-    int gated, act, rope;
-    float eps, eps_f;                 // block norms / final norm
-    const MegaLayer *layers;          // device array [NL]
+    MegaShape s;
+    int norm;                             // 1 LayerNorm, 2 RMSNorm
+    int act;
+    float eps, eps_f;                     // block norms / final norm
+    const MegaLayer *layers;              // device array [NL]
     const float *wte, *wpe, *lnfw, *lnfb, *cosb, *sinb;
-    float *x, *qkv, *ctx, *h, *logits, *part;
-    unsigned *count;
-    const int *ids, *posmat, *lenmat;
-    int *step_d;                      // tokens finalised so far (v); this step's position is np - 1 + v
-    int np, cap, n_new, max_split;
+    float *logits;
+    const int *ids, *posmat;
+    const int *step_d;                    // tokens finalised so far (v); this step's position is posmat[(v + pos_base) * B + b]
+    int pos_base;
     int64_t kv_seq_pitch;
-    unsigned *bar, *bar_base;         // barrier counter (only grows) and its value at the start of this launch
+    uint2 *ll;                            // exchange buffers, zeroed before the first step of a generate: lm_mega_exchange_words() words
     int *err;
-    int greedy;                       // 1: pick the arg max and close the step in the kernel
-    unsigned long long *amax;
-    int *out, *ids_out;
 };
-
+size_t lm_mega_exchange_words(const MegaShape &s);
 void lm_mega_enable(int on);
-bool lm_mega_eligible(int B, int hd, int C, int I, bool qk_norm);
-size_t lm_mega_smem(const MegaArgs &a);
-void lm_mega_launch(const MegaArgs &a);     // on stream(); fatal when the cooperative launch is refused
+bool lm_mega_enabled();
+void lm_mega_launch(const MegaModel &m, const MegaArgs &a);     // on stream(); fatal when the cooperative launch is refused
 
 } // namespace ncmb
