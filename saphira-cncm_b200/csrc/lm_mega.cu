@@ -50,7 +50,7 @@ struct MsSm {                                            // fixed part of shared
     int dead;
     float red[2][MS_WARPS];
     float att[MS_WARPS][MS_PW + 2];
-    float qn[3][64];                                     // this CTA's query head; the new key and value
+    alignas(16) float qn[3][64];                         // this CTA's query head; the new key and value (read as float4)
     float xres[8][MG_MAXB];                              // hidden state of the rows this CTA owns
 };
 
@@ -196,7 +196,7 @@ __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long 
 // Down-projection rows [r0, r0 + n), n <= 8: the warp takes 256-wide pieces `warp`, `warp + 16` of K, whose inputs its lanes poll
 // straight into registers; part[row][warp][m].
 template <int MT, bool W16>
-__device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long base, int n, int I, const uint2 *hw, unsigned tag, float *part, int warp, int lane) {
+__device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long base, int n, int I, int B, const uint2 *hw, unsigned tag, float *part, int warp, int lane) {
     const int esz = W16 ? 2 : 4;
     const long long rowb = (long long)I * esz;
     float acc[MT][8];
@@ -213,7 +213,7 @@ __device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long 
 #pragma unroll
         for (int m = 0; m < MT; m++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) p[4 * m + e] = k < I ? hw + (size_t)m * I + k + 2 * e : nullptr;
+            for (int e = 0; e < 4; e++) p[4 * m + e] = k < I && m < B ? hw + (size_t)m * I + k + 2 * e : nullptr;
         c.poll<4 * MT>(p, tag, v);
 #pragma unroll
         for (int m = 0; m < MT; m++)
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         }
         ms_bar();                                             // part is rewritten by the down-projection
         // ---- down-projection, residual ----
-        ms_down<MT, W16>(c, st, at, ncr, I, Lh, tag, part, warp, lane);
+        ms_down<MT, W16>(c, st, at, ncr, I, S.B, Lh, tag, part, warp, lane);
         at += b_dn;
         ms_bar();
         if (tid < ncr * S.B) {
