@@ -103,22 +103,31 @@ struct MsCtx {
     }
 };
 
-// A warp's view of the weight stream: chunks known to have arrived, chunks it has given back.
+// A warp's view of the weight stream: chunks known to have arrived, chunks given back. Lanes wait for (and give back) different
+// chunks at once: one chunk after the other, by all lanes and returned by all warps, these took more of a layer than its products.
 struct MsStream {
     const unsigned char *ring; uint32_t full, empty;
     int have = 0, rel = 0;
-    __device__ __forceinline__ void ensure(const MsCtx &c, long long end) {
-        while ((long long)have * MS_CH < end) { c.wait(full + 8 * (have % MS_SLOTS), (uint32_t)(have / MS_SLOTS) & 1u); have++; }
+    __device__ __forceinline__ void ensure(const MsCtx &c, long long end, int lane) {
+        const int need = (int)((end + MS_CH - 1) / MS_CH);
+        if (need > have) {
+            const int k = max(have, rel) + lane;             // (what was given back had arrived)
+            if (k < need) c.wait(full + 8 * (k % MS_SLOTS), (uint32_t)(k / MS_SLOTS) & 1u);
+            __syncwarp();
+            have = need;
+        }
     }
-    __device__ __forceinline__ void release(long long upto, int lane) {       // every byte below has been read by this warp
-        __syncwarp();
-        while ((long long)(rel + 1) * MS_CH <= upto) { if (lane == 0) mbar_arrive(empty + 8 * (rel % MS_SLOTS)); rel++; }
+    // every byte below `upto` has been read by every warp (a barrier lies between); warp 0 tells the producer
+    __device__ __forceinline__ void release(long long upto, int warp, int lane) {
+        const int r = (int)(upto / MS_CH);
+        if (warp == 0 && rel + lane < r) mbar_arrive(empty + 8 * ((rel + lane) % MS_SLOTS));
+        rel = r;
     }
 };
 
 // eight weights at byte offset `off` of the stream
 template <bool W16>
-__device__ __forceinline__ void ms_w8(const unsigned char *ring, long long off, float *w) {
+__device__ __forceinline__ void ms_w8(const unsigned char *ring, uint32_t off, float *w) {
     if (W16) {
         const uint4 u = *(const uint4 *)(ring + (off & (MS_RING - 1)));
         w[0] = __uint_as_float(u.x << 16); w[1] = __uint_as_float(u.x & 0xffff0000u);
@@ -161,15 +170,16 @@ __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long 
             const float4 v = on ? *(const float4 *)(xs + m * C + seg * (C >> 2) + lane * 8 + e) : make_float4(0.f, 0.f, 0.f, 0.f);
             xr[m][e] = v.x; xr[m][e + 1] = v.y; xr[m][e + 2] = v.z; xr[m][e + 3] = v.w;
         }
-    for (int i0 = rg; i0 < n; i0 += 32) {
-        const int last = min(n - 1, i0 + 28);
-        st.ensure(c, base + (long long)(last + 1) * rowb);
+    const uint32_t rb = (uint32_t)rowb, at = (uint32_t)(base & (MS_RING - 1)) + (uint32_t)lo + rg * rb;
+    for (int b0 = 0; b0 < n; b0 += 32) {
+        if (b0 > 0) { ms_bar(); st.release(base + (long long)b0 * rowb, warp, lane); }
+        st.ensure(c, base + (long long)min(n, b0 + 32) * rowb, lane);
+        const int i0 = b0 + rg;
         float acc[MT][8];
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            const int r = i0 + 4 * j;
             float w[8];
-            if (r < n && on) ms_w8<W16>(st.ring, base + r * rowb + lo, w);
+            if (i0 + 4 * j < n && on) ms_w8<W16>(st.ring, at + (b0 + 4 * j) * rb, w);
             else {
 #pragma unroll
                 for (int e = 0; e < 8; e++) w[e] = 0.f;
@@ -182,7 +192,6 @@ __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long 
                 acc[m][j] = t;
             }
         }
-        st.release(base + (long long)(i0 - rg + 32 <= n ? i0 - rg + 32 : n) * rowb, lane);
 #pragma unroll
         for (int m = 0; m < MT; m++) {
             const float s = ms_reduce8(acc[m], lane);
@@ -190,7 +199,6 @@ __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long 
             if ((lane & 3) == 0 && r < n) part[(r * 4 + seg) * MT + m] = s;
         }
     }
-    st.release(base + (long long)n * rowb, lane);
 }
 
 // Down-projection rows [r0, r0 + n), n <= 8: the warp takes 256-wide pieces `warp`, `warp + 16` of K, whose inputs its lanes poll
@@ -204,39 +212,49 @@ __device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long 
     for (int m = 0; m < MT; m++)
 #pragma unroll
         for (int j = 0; j < 8; j++) acc[m][j] = 0.f;
-    float xr[2][MT][8];
+    constexpr int NU = MT == 1 ? 2 : 1;                       // pieces polled at once (one row: both, for one trip to L2)
+    const uint32_t at = (uint32_t)(base & (MS_RING - 1)), rb = (uint32_t)rowb;
+#pragma unroll 1
+    for (int u0 = 0; u0 < 2; u0 += NU) {
+        if ((warp + MS_WARPS * u0) * 256 >= I) break;
+        float xr[NU][MT][8];
+        {
+            const uint2 *p[4 * MT * NU];
+            float2 v[4 * MT * NU];
 #pragma unroll
-    for (int u = 0; u < 2; u++) {
-        const int k = (warp + MS_WARPS * u) * 256 + lane * 8;
-        const uint2 *p[4 * MT];
-        float2 v[4 * MT];
-#pragma unroll
-        for (int m = 0; m < MT; m++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) p[4 * m + e] = k < I && m < B ? hw + (size_t)m * I + k + 2 * e : nullptr;
-        c.poll<4 * MT>(p, tag, v);
-#pragma unroll
-        for (int m = 0; m < MT; m++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) { xr[u][m][2 * e] = v[4 * m + e].x; xr[u][m][2 * e + 1] = v[4 * m + e].y; }
-    }
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-        if (r >= n) break;
-        st.ensure(c, base + (r + 1) * rowb);
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int k = (warp + MS_WARPS * u) * 256 + lane * 8;
-            if (k < I) {
-                float w[8];
-                ms_w8<W16>(st.ring, base + r * rowb + (long long)k * esz, w);
+            for (int u = 0; u < NU; u++)
 #pragma unroll
                 for (int m = 0; m < MT; m++)
 #pragma unroll
-                    for (int e = 0; e < 8; e++) acc[m][r] = fmaf(w[e], xr[u][m][e], acc[m][r]);
+                    for (int e = 0; e < 4; e++) {
+                        const int k = (warp + MS_WARPS * (u0 + u)) * 256 + lane * 8;
+                        p[4 * (u * MT + m) + e] = k < I && m < B ? hw + (size_t)m * I + k + 2 * e : nullptr;
+                    }
+            c.poll<4 * MT * NU>(p, tag, v);
+#pragma unroll
+            for (int u = 0; u < NU; u++)
+#pragma unroll
+                for (int m = 0; m < MT; m++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) { xr[u][m][2 * e] = v[4 * (u * MT + m) + e].x; xr[u][m][2 * e + 1] = v[4 * (u * MT + m) + e].y; }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            if (r >= n) break;
+            if ((r & 3) == 0) st.ensure(c, base + min(r + 4, n) * rowb, lane);
+#pragma unroll
+            for (int u = 0; u < NU; u++) {
+                const int k = (warp + MS_WARPS * (u0 + u)) * 256 + lane * 8;
+                if (k < I) {
+                    float w[8];
+                    ms_w8<W16>(st.ring, at + r * rb + (uint32_t)(k * esz), w);
+#pragma unroll
+                    for (int m = 0; m < MT; m++)
+#pragma unroll
+                        for (int e = 0; e < 8; e++) acc[m][r] = fmaf(w[e], xr[u][m][e], acc[m][r]);
+                }
             }
         }
-        st.release(base + (r + 1) * rowb, lane);
     }
 #pragma unroll
     for (int m = 0; m < MT; m++) {
@@ -328,17 +346,20 @@ __device__ __forceinline__ void ms_attend(MsSm *sm, MsKV &f, const float *kv, in
         a[2 + 4 * dp] = o.x; a[3 + 4 * dp] = o.y; a[4 + 4 * dp] = o.z; a[5 + 4 * dp] = o.w;
     }
     ms_bar();
-    if (tid < MS_PW) {
-        float X = -INFINITY;
+    if (warp < (MS_PW + 31) / 32) {
+        const float mw = lane < MS_WARPS ? sm->att[lane][0] : -INFINITY;
+        float X = mw;
 #pragma unroll
-        for (int w = 0; w < MS_WARPS; w++) X = fmaxf(X, sm->att[w][0]);
+        for (int x = 16; x > 0; x >>= 1) X = fmaxf(X, __shfl_xor_sync(0xffffffffu, X, x));
+        const float ew = mw == -INFINITY ? 0.f : expf(mw - X);
+        const int d = min(max(tid, 1), MS_PW - 1);
         float t = 0.f;
 #pragma unroll
         for (int w = 0; w < MS_WARPS; w++) {
-            const float mw = sm->att[w][0];
-            if (mw != -INFINITY) t = fmaf(sm->att[w][tid == 0 ? 1 : tid], expf(mw - X), t);
+            const float e1 = __shfl_sync(0xffffffffu, ew, w);
+            if (e1 != 0.f) t = fmaf(sm->att[w][d], e1, t);
         }
-        ll_store(out + tid, tid == 0 ? X : t, tag);
+        if (tid < MS_PW) ll_store(out + tid, tid == 0 ? X : t, tag);
     }
 }
 
@@ -362,7 +383,7 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
     const long long head_at = ((b_all + MS_CH - 1) / MS_CH) * MS_CH;                          // the head starts on a chunk of its own
     const uint32_t full = smem_u32(sm->full), empty = smem_u32(sm->empty);
     if (tid == 0) {
-        for (int s = 0; s < MS_SLOTS; s++) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, MS_WARPS); }
+        for (int s = 0; s < MS_SLOTS; s++) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, 1); }
         sm->dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -411,6 +432,9 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         const MegaLayer &L = a.layers[li];
         const unsigned tag = tag0 + (unsigned)li;
         const float *kvb = att ? L.kv + (int64_t)ab * a.kv_seq_pitch + akv * 64 : nullptr;
+        if (att)                                              // this layer's keys and values: on their way from HBM during the product
+            for (int i = tid; i < (k1 - k0) * 4; i += MS_T)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(kvb + (int64_t)(k0 + (i >> 2)) * 2 * kvd + (i & 2 ? kvd : 0) + (i & 1) * 32));
         // ---- hidden state, norm, q k v ----
         {
             const float2 w = pair_of(L.ln1w, 1.f), b = pair_of(L.ln1b, 0.f);
@@ -440,6 +464,7 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         ms_rows<MT, W16>(c, st, at, 2 * nq, C, xs, part, warp, lane);
         at += b_qkv;
         ms_bar();
+        st.release(at, warp, lane);
         for (int t = tid; t < nq * S.B; t += MS_T) {
             const int i = t / S.B, m = t - i * S.B, pr = q0 + i, h = pr >> 5, d = pr & 31;
             const float *p0 = part + (size_t)(2 * i) * 4 * MT + m, *p1 = p0 + 4 * MT;
@@ -500,6 +525,7 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         ms_rows<MT, W16>(c, st, at, ncr, C, xs, part, warp, lane);
         at += b_o;
         ms_bar();
+        st.release(at, warp, lane);
         if (tid < ncr * S.B) {
             const int r = tid / S.B, m = tid - r * S.B;
             const float *p = part + (size_t)r * 4 * MT + m;
@@ -521,6 +547,7 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         ms_rows<MT, W16>(c, st, at, ur, C, xs, part, warp, lane);
         at += b_up;
         ms_bar();
+        st.release(at, warp, lane);
         for (int t = tid; t < nu * S.B; t += MS_T) {
             const int i = t / S.B, m = t - i * S.B;
             float y;
@@ -542,6 +569,7 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         ms_down<MT, W16>(c, st, at, ncr, I, S.B, Lh, tag, part, warp, lane);
         at += b_dn;
         ms_bar();
+        st.release(at, warp, lane);
         if (tid < ncr * S.B) {
             const int r = tid / S.B, m = tid - r * S.B;
             float y = 0.f;
@@ -561,7 +589,7 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         c.poll<MT>(p, tag0 + (unsigned)S.NL - 1u, xv);
         ms_norm<MT>(sm, xv, C, a.norm, w, b, a.eps_f, xs, tid);
     }
-    st.release(head_at, lane);
+    st.release(head_at, warp, lane);
     at = head_at;
     int buf = 0;
     for (int r0 = 0; r0 < nv; r0 += MS_HROWS, buf ^= 1) {
@@ -570,13 +598,13 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         ms_rows<MT, W16>(c, st, at, n, C, xs, pb, warp, lane);
         at += (long long)n * C * esz;
         ms_bar();                                             // (the other half of `part` is free by the next barrier)
+        st.release(at, warp, lane);
         for (int t = tid; t < n * S.B; t += MS_T) {
             const int m = t / n, r = t - m * n;
             const float *p = pb + (size_t)r * 4 * MT + m;
             a.logits[(size_t)m * S.V + v0 + r0 + r] = (p[0] + p[MT]) + (p[2 * MT] + p[3 * MT]);
         }
     }
-    st.release(head_at + ((b_head + MS_CH - 1) / MS_CH) * MS_CH, lane);
 }
 
 // one layer's rows into the CTAs' streams: block (cta, matrix)
