@@ -383,9 +383,8 @@ typedef struct NcmbLM NcmbLM;
 NcmbLM *ncmb_lm_open(const NCMConfig *c, const char *weights, int is_qwen, int bf16_weights);   /* weights: .ncm, .nckpt or .safetensors */
 void   ncmb_lm_close(NcmbLM *m);
 int    ncmb_lm_vocab(const NcmbLM *m);
-/* Decode steps of up to four sequences (head dim 64) can run as ONE persistent cooperative kernel with grid
- * barriers between the phases of a layer instead of a replayed chain of kernels. Off by default (it is the
- * slower of the two today); results are the same either way. No counterpart in the reference. */
+/* Decode steps of one sequence (head dim 64) run as ONE persistent cooperative kernel instead of a replayed chain
+ * of kernels; 0 turns that off. Results agree within fp32 rounding either way. No counterpart in the reference. */
 void  ncmb_set_lm_persistent(int on);
 /* prompts: host int[B][np]; out: host int[B][n_new]; eos < 0 disables stopping.
  * Returns the number of ids generated per row (n_new unless every row hit eos). */

@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(256) k_few_reduce_qkv(FewQkv a) {
 
 // ---- host side ----
 bool gemm_few_supported(int64_t M, int N, int K) {
-    return ctx().gemm_mode >= 3 && M >= 5 && M <= FEW_MAX_ROWS && N >= 32 && K >= 32 && (K & 7) == 0;
+    return ctx().gemm_mode >= 3 && M >= 2 && M <= FEW_MAX_ROWS && N >= 32 && K >= 32 && (K & 7) == 0;
 }
 // Slices of K: as many as give every SM one CTA, each at least two 64-wide steps; a slice more costs another read of the rows in
 // the kernel that adds them, so a long row count takes fewer.

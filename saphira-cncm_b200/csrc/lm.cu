@@ -246,7 +246,7 @@ void lm_layout(LMRun &r, Workspace &w, int n_new, int64_t logit_rows) {
     r.amax_d = w.get<unsigned long long>(r.B);
     r.pick_d = w.get<int>(r.B);
     r.step_d = w.get<int>(4);
-    if (r.B <= MG_MAXB) {
+    if (r.B == 1) {
         r.mg_ll = w.get<uint2>(lm_mega_exchange_words(mega_shape(m, r.B)));
         r.mg_layers = w.get<MegaLayer>((size_t)m->NL);
     }
@@ -476,11 +476,11 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
     // runs eagerly (it sizes every workspace), the second is captured, the rest are graph launches. The work
     // moves to a stream of its own for that, because the caller's stream may be the legacy default stream,
     // which cannot be captured.
-    // Up to four rows (head dim 64): the whole decode step is one persistent cooperative kernel (lm_mega.cu).
+    // One row (head dim 64): the whole decode step is one persistent cooperative kernel (lm_mega.cu).
     bool qk_norm = false;
     for (auto &bw : m->blocks) qk_norm = qk_norm || bw.qnw || bw.knw;
     const MegaShape ms = mega_shape(m, B);
-    const bool mega = lm_mega_enabled() && B <= MG_MAXB && n_new >= 2 && lm_mega_supported(ms, m->hd, qk_norm);
+    const bool mega = lm_mega_enabled() && n_new >= 2 && lm_mega_supported(ms, m->hd, qk_norm);
     MegaArgs mg{};
     if (mega) {
         lm_mega_pack(m->mega, ms, m->blocks, m->wte, m->wte16);
@@ -496,7 +496,6 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
         mg.layers = r.mg_layers; mg.wte = m->wte; mg.wpe = m->is_qwen ? nullptr : m->wpe; mg.lnfw = nf.w; mg.lnfb = nf.b;
         mg.cosb = m->cosb; mg.sinb = m->sinb; mg.logits = r.logits;
         mg.ids = r.ids_d; mg.posmat = r.posmat; mg.step_d = r.step_d; mg.pos_base = np - 1;
-        mg.kv_seq_pitch = (int64_t)r.cap * 2 * m->nkv * m->hd;
         mg.ll = r.mg_ll; mg.err = tc_err_flag();
     }
     static const bool graphs_ok = !getenv("NCM_B200_NO_GRAPH");

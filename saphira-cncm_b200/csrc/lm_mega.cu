@@ -1,4 +1,4 @@
-// One decode step of one to four sequences (head dim 64) as ONE persistent kernel: every layer and the vocabulary projection.
+// One decode step of one sequence (head dim 64) as ONE persistent kernel: every layer and the vocabulary projection.
 //
 // A step streams all weights once (4.6 us of HBM time a layer for the Qwen2 shape in bf16) through five products that depend on
 // one another; as separate kernels each boundary and each cold start of the weight stream costs several times that (28 us a
@@ -15,6 +15,10 @@
 //   * Products. Sixteen warps: four quarters of K x four groups of rows. A lane keeps its eight elements of the input in
 //     registers; eight rows at a time meet in a reduce-scatter.
 //
+// One row only: 681 us a step for the Qwen2 shape (the kernel chain: 757) and 307 for GPT-2 in fp32 (308). What is left is the
+// six exchanges of a layer, about 1 us each, and the reductions between them; from two rows on the few-row kernel chain is faster
+// (two rows 783 us against 837 here, four 806 against 1187), since its tensor-core products do not grow with the rows.
+//
 // Hops of a layer: hidden -> q k v -> attention partials -> hidden -> MLP -> hidden. Every wait is bounded (2 s): a wait that
 // runs out records a code, the other CTAs see it and stop waiting, and the kernel ends.
 #include "lm_mega.cuh"
@@ -27,7 +31,7 @@ namespace ncmb {
 
 constexpr int MS_WARPS = 16, MS_T = MS_WARPS * 32;       // consumer threads; one more warp feeds the ring
 constexpr int MS_CH = 8192, MS_SLOTS = 16, MS_RING = MS_CH * MS_SLOTS;
-constexpr int MS_MAXC = 1024, MS_MAXI = 8192, MS_MAXSPLIT = 4, MS_PW = 66;       // words of an attention partial: max, sum, context
+constexpr int MS_MAXC = 1024, MS_MAXI = 8192, MS_MAXNL = 256, MS_MAXSPLIT = 4, MS_PW = 66;       // words of an attention partial: max, sum, context
 constexpr int MS_UPROWS = 128, MS_HROWS = 64;            // rows a CTA may have of an up-projection; vocabulary rows per round
 
 // contiguous share of n items for CTA c of g
@@ -36,12 +40,11 @@ __host__ __device__ __forceinline__ int ms_begin(int n, int c, int g) { return (
 struct MsLL {                                            // offsets of the exchange buffers, in words
     size_t x, x1, q, p, h, total;
     __host__ __device__ explicit MsLL(const MegaShape &s) {
-        const size_t B = s.B;
-        x = 0; x1 = x + B * s.C; q = x1 + B * s.C; p = q + B * (s.C + 128 * (size_t)s.nkv); h = p + B * s.H * MS_MAXSPLIT * MS_PW; total = h + B * s.I;
+        x = 0; x1 = x + s.C; q = x1 + s.C; p = q + s.C + 128 * (size_t)s.nkv; h = p + (size_t)s.H * MS_MAXSPLIT * MS_PW; total = h + s.I;
     }
 };
 __host__ __device__ __forceinline__ int ms_splits(const MegaShape &s, int grid) {
-    const int n = grid / (s.B * s.H);
+    const int n = grid / s.H;
     return n < 1 ? 1 : (n > MS_MAXSPLIT ? MS_MAXSPLIT : n);
 }
 
@@ -51,7 +54,7 @@ struct MsSm {                                            // fixed part of shared
     float red[2][MS_WARPS];
     float att[MS_WARPS][MS_PW + 2];
     alignas(16) float qn[3][64];                         // this CTA's query head; the new key and value (read as float4)
-    float xres[8][MG_MAXB];                              // hidden state of the rows this CTA owns
+    float xres[8];                                       // hidden state of the rows this CTA owns
 };
 
 __device__ __forceinline__ void ms_bar() { asm volatile("bar.sync 1, %0;" ::"n"(MS_T) : "memory"); }
@@ -156,26 +159,24 @@ __device__ __forceinline__ float ms_reduce8(float (&v)[8], int lane) {
 }
 
 // Rows [r0, r0 + n) of a [..][C] product whose stream begins at `base` (row r0's first byte): a warp takes quarter `warp & 3` of K
-// and every fourth row; part[row][quarter][m].
-template <int MT, bool W16>
+// and every fourth row; part[row][quarter].
+template <bool W16>
 __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long base, int n, int C, const float *xs, float *part, int warp, int lane) {
     const int seg = warp & 3, rg = warp >> 2, L = C >> 5, esz = W16 ? 2 : 4;      // lanes of a quarter
     const bool on = lane < L;
     const long long rowb = (long long)C * esz, lo = (long long)(seg * (C >> 2) + lane * 8) * esz;
-    float xr[MT][8];
+    float xr[8];
 #pragma unroll
-    for (int m = 0; m < MT; m++)
-#pragma unroll
-        for (int e = 0; e < 8; e += 4) {
-            const float4 v = on ? *(const float4 *)(xs + m * C + seg * (C >> 2) + lane * 8 + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-            xr[m][e] = v.x; xr[m][e + 1] = v.y; xr[m][e + 2] = v.z; xr[m][e + 3] = v.w;
-        }
+    for (int e = 0; e < 8; e += 4) {
+        const float4 v = on ? *(const float4 *)(xs + seg * (C >> 2) + lane * 8 + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+        xr[e] = v.x; xr[e + 1] = v.y; xr[e + 2] = v.z; xr[e + 3] = v.w;
+    }
     const uint32_t rb = (uint32_t)rowb, at = (uint32_t)(base & (MS_RING - 1)) + (uint32_t)lo + rg * rb;
     for (int b0 = 0; b0 < n; b0 += 32) {
         if (b0 > 0) { ms_bar(); st.release(base + (long long)b0 * rowb, warp, lane); }
         st.ensure(c, base + (long long)min(n, b0 + 32) * rowb, lane);
         const int i0 = b0 + rg;
-        float acc[MT][8];
+        float acc[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             float w[8];
@@ -184,110 +185,77 @@ __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long 
 #pragma unroll
                 for (int e = 0; e < 8; e++) w[e] = 0.f;
             }
+            acc[j] = w[0] * xr[0];
 #pragma unroll
-            for (int m = 0; m < MT; m++) {
-                float t = w[0] * xr[m][0];
-#pragma unroll
-                for (int e = 1; e < 8; e++) t = fmaf(w[e], xr[m][e], t);
-                acc[m][j] = t;
-            }
+            for (int e = 1; e < 8; e++) acc[j] = fmaf(w[e], xr[e], acc[j]);
         }
-#pragma unroll
-        for (int m = 0; m < MT; m++) {
-            const float s = ms_reduce8(acc[m], lane);
-            const int r = i0 + 4 * (lane >> 2);
-            if ((lane & 3) == 0 && r < n) part[(r * 4 + seg) * MT + m] = s;
-        }
+        const float s = ms_reduce8(acc, lane);
+        const int r = i0 + 4 * (lane >> 2);
+        if ((lane & 3) == 0 && r < n) part[r * 4 + seg] = s;
     }
 }
 
 // Down-projection rows [r0, r0 + n), n <= 8: the warp takes 256-wide pieces `warp`, `warp + 16` of K, whose inputs its lanes poll
-// straight into registers; part[row][warp][m].
-template <int MT, bool W16>
-__device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long base, int n, int I, int B, const uint2 *hw, unsigned tag, float *part, int warp, int lane) {
+// straight into registers; part[row][warp].
+template <bool W16>
+__device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long base, int n, int I, const uint2 *hw, unsigned tag, float *part, int warp, int lane) {
     const int esz = W16 ? 2 : 4;
     const long long rowb = (long long)I * esz;
-    float acc[MT][8];
-#pragma unroll
-    for (int m = 0; m < MT; m++)
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[m][j] = 0.f;
-    constexpr int NU = MT == 1 ? 2 : 1;                       // pieces polled at once (one row: both, for one trip to L2)
     const uint32_t at = (uint32_t)(base & (MS_RING - 1)), rb = (uint32_t)rowb;
-#pragma unroll 1
-    for (int u0 = 0; u0 < 2; u0 += NU) {
-        if ((warp + MS_WARPS * u0) * 256 >= I) break;
-        float xr[NU][MT][8];
-        {
-            const uint2 *p[4 * MT * NU];
-            float2 v[4 * MT * NU];
+    float acc[8], xr[2][8];
 #pragma unroll
-            for (int u = 0; u < NU; u++)
+    for (int j = 0; j < 8; j++) acc[j] = 0.f;
+    {
+        const uint2 *p[8];
+        float2 v[8];
 #pragma unroll
-                for (int m = 0; m < MT; m++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const int k = (warp + MS_WARPS * (u0 + u)) * 256 + lane * 8;
-                        p[4 * (u * MT + m) + e] = k < I && m < B ? hw + (size_t)m * I + k + 2 * e : nullptr;
-                    }
-            c.poll<4 * MT * NU>(p, tag, v);
-#pragma unroll
-            for (int u = 0; u < NU; u++)
-#pragma unroll
-                for (int m = 0; m < MT; m++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) { xr[u][m][2 * e] = v[4 * (u * MT + m) + e].x; xr[u][m][2 * e + 1] = v[4 * (u * MT + m) + e].y; }
+        for (int i = 0; i < 8; i++) {
+            const int k = (warp + MS_WARPS * (i >> 2)) * 256 + lane * 8;
+            p[i] = k < I ? hw + k + 2 * (i & 3) : nullptr;
         }
+        c.poll<8>(p, tag, v);
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
-            if (r >= n) break;
-            if ((r & 3) == 0) st.ensure(c, base + min(r + 4, n) * rowb, lane);
+        for (int i = 0; i < 8; i++) { xr[i >> 2][2 * (i & 3)] = v[i].x; xr[i >> 2][2 * (i & 3) + 1] = v[i].y; }
+    }
 #pragma unroll
-            for (int u = 0; u < NU; u++) {
-                const int k = (warp + MS_WARPS * (u0 + u)) * 256 + lane * 8;
-                if (k < I) {
-                    float w[8];
-                    ms_w8<W16>(st.ring, at + r * rb + (uint32_t)(k * esz), w);
+    for (int r = 0; r < 8; r++) {
+        if (r >= n) break;
+        if ((r & 3) == 0) st.ensure(c, base + min(r + 4, n) * rowb, lane);
 #pragma unroll
-                    for (int m = 0; m < MT; m++)
+        for (int u = 0; u < 2; u++) {
+            const int k = (warp + MS_WARPS * u) * 256 + lane * 8;
+            if (k < I) {
+                float w[8];
+                ms_w8<W16>(st.ring, at + r * rb + (uint32_t)(k * esz), w);
 #pragma unroll
-                        for (int e = 0; e < 8; e++) acc[m][r] = fmaf(w[e], xr[u][m][e], acc[m][r]);
-                }
+                for (int e = 0; e < 8; e++) acc[r] = fmaf(w[e], xr[u][e], acc[r]);
             }
         }
     }
-#pragma unroll
-    for (int m = 0; m < MT; m++) {
-        const float s = ms_reduce8(acc[m], lane);
-        if ((lane & 3) == 0 && (lane >> 2) < n) part[((lane >> 2) * MS_WARPS + warp) * MT + m] = s;
-    }
+    const float s = ms_reduce8(acc, lane);
+    if ((lane & 3) == 0 && (lane >> 2) < n) part[(lane >> 2) * MS_WARPS + warp] = s;
 }
 
-// norm of MT rows of C values held as pairs by threads t < C / 2, into xs
-template <int MT>
-__device__ __forceinline__ void ms_norm(MsSm *sm, float2 (&v)[MT], int C, int kind, float2 w, float2 b, float eps, float *xs, int tid) {
+// norm of the row of C values held as pairs by threads t < C / 2, into xs
+__device__ __forceinline__ void ms_norm(MsSm *sm, float2 v, int C, int kind, float2 w, float2 b, float eps, float *xs, int tid) {
     const int lane = tid & 31, warp = tid >> 5;
     const bool on = tid < (C >> 1);
+    float mean = 0.f;
+    auto sum = [&](float s, int k) {
 #pragma unroll
-    for (int m = 0; m < MT; m++) {
-        float mean = 0.f;
-        auto sum = [&](float s, int k) {
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) sm->red[k][warp] = s;
+        ms_bar();
+        float t = 0.f;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) sm->red[k][warp] = s;
-            ms_bar();
-            float t = 0.f;
-#pragma unroll
-            for (int q = 0; q < MS_WARPS; q++) t += sm->red[k][q];
-            return t;
-        };
-        if (kind == 1) mean = sum(on ? v[m].x + v[m].y : 0.f, 0) / (float)C;
-        const float d0 = v[m].x - mean, d1 = v[m].y - mean;
-        const float inv = 1.0f / sqrtf(sum(on ? d0 * d0 + d1 * d1 : 0.f, 1) / (float)C + eps);
-        if (on) *(float2 *)(xs + m * C + 2 * tid) = make_float2(__fadd_rn(__fmul_rn(__fmul_rn(d0, inv), w.x), b.x), __fadd_rn(__fmul_rn(__fmul_rn(d1, inv), w.y), b.y));
-        if (MT > 1) ms_bar();                                // red is reused by the next row
-    }
-    if (MT == 1) ms_bar();
+        for (int q = 0; q < MS_WARPS; q++) t += sm->red[k][q];
+        return t;
+    };
+    if (kind == 1) mean = sum(on ? v.x + v.y : 0.f, 0) / (float)C;
+    const float d0 = v.x - mean, d1 = v.y - mean;
+    const float inv = 1.0f / sqrtf(sum(on ? d0 * d0 + d1 * d1 : 0.f, 1) / (float)C + eps);
+    if (on) *(float2 *)(xs + 2 * tid) = make_float2(__fadd_rn(__fmul_rn(__fmul_rn(d0, inv), w.x), b.x), __fadd_rn(__fmul_rn(__fmul_rn(d1, inv), w.y), b.y));
+    ms_bar();
 }
 
 // attention of query head h of row b over keys [k0, k1): `cached` keys in kv, key `cached` (the new token's) in sm->qn; the
@@ -363,14 +331,15 @@ __device__ __forceinline__ void ms_attend(MsSm *sm, MsKV &f, const float *kv, in
     }
 }
 
-template <int MT, bool W16>
+template <bool W16>
 __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ MegaArgs a, const unsigned char *stream_w, const long long *stream_off, const unsigned char *head_w) {
     extern __shared__ __align__(1024) unsigned char ms_raw[];
     const MegaShape &S = a.s;
     unsigned char *ring = ms_raw;
     MsSm *sm = (MsSm *)(ring + MS_RING);
-    float *xs = (float *)(((uintptr_t)(sm + 1) + 15) & ~(uintptr_t)15);          // [MT][C] normed input of a product
-    float *part = xs + MT * S.C;                                                 // sums by quarter of K (or by warp)
+    float *xs = (float *)(((uintptr_t)(sm + 1) + 15) & ~(uintptr_t)15);          // [C] input of a product
+    MegaLayer *layers = (MegaLayer *)(xs + S.C);                                 // [NL]
+    float *part = (float *)(((uintptr_t)(layers + S.NL) + 15) & ~(uintptr_t)15);            // sums by quarter of K (or by warp)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x, g = gridDim.x;
     const int C = S.C, I = S.I, kvd = S.nkv * 64, Wq = C + 2 * kvd, esz = W16 ? 2 : 4;
     // this CTA's share of every product
@@ -387,6 +356,7 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         sm->dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    for (int i = tid; i < S.NL * (int)(sizeof(MegaLayer) / 8); i += MS_T + 32) ((unsigned long long *)layers)[i] = ((const unsigned long long *)a.layers)[i];
     __syncthreads();
     MsCtx c{sm, a.err};
 
@@ -418,20 +388,21 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
     uint2 *Lx = a.ll + ll.x, *Lx1 = a.ll + ll.x1, *Lq = a.ll + ll.q, *Lp = a.ll + ll.p, *Lh = a.ll + ll.h;
     const int step = *a.step_d, nsp = ms_splits(S, g);
     const unsigned tag0 = (unsigned)step * (unsigned)S.NL + 1u;
-    const int *pos = a.posmat + (int64_t)(step + a.pos_base) * S.B;
+    const int pos = a.posmat[step + a.pos_base];
     const bool on2 = tid < (C >> 1);                          // this thread holds elements 2 tid, 2 tid + 1 of a hidden row
     auto pair_of = [&](const float *p, float none) { return p && on2 ? __ldg((const float2 *)p + tid) : make_float2(none, none); };
-    // attention share: query head ah of row ab, part asp of its keys
-    const bool att = cta < S.B * S.H * nsp;
-    const int ab = att ? cta / (S.H * nsp) : 0, ah = att ? (cta / nsp) % S.H : 0, asp = cta % nsp, akv = ah / (S.H / S.nkv);
-    const int cached = att ? pos[ab] : 0, n_keys = cached + 1, per = (n_keys + nsp - 1) / nsp;
+    // attention share: query head ah, part asp of its keys
+    const bool att = cta < S.H * nsp;
+    const int ah = att ? cta / nsp : 0, asp = cta % nsp, akv = ah / (S.H / S.nkv);
+    const int n_keys = pos + 1, per = (n_keys + nsp - 1) / nsp;
     const int k0 = min(n_keys, asp * per), k1 = min(n_keys, k0 + per);
+    auto one = [&](const float *p, bool on, int i) { return p && on ? __ldg(p + i) : 0.f; };
     long long at = 0;                                         // stream offset
-    float2 xv[MT];
+    float2 xv[1];
     for (int li = 0; li < S.NL; li++) {
-        const MegaLayer &L = a.layers[li];
+        const MegaLayer &L = layers[li];
         const unsigned tag = tag0 + (unsigned)li;
-        const float *kvb = att ? L.kv + (int64_t)ab * a.kv_seq_pitch + akv * 64 : nullptr;
+        const float *kvb = L.kv + akv * 64;
         if (att)                                              // this layer's keys and values: on their way from HBM during the product
             for (int i = tid; i < (k1 - k0) * 4; i += MS_T)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(kvb + (int64_t)(k0 + (i >> 2)) * 2 * kvd + (i & 2 ? kvd : 0) + (i & 1) * 32));
@@ -439,72 +410,62 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         {
             const float2 w = pair_of(L.ln1w, 1.f), b = pair_of(L.ln1b, 0.f);
             if (li == 0) {
-#pragma unroll
-                for (int m = 0; m < MT; m++) {
-                    xv[m] = make_float2(0.f, 0.f);
-                    if (m < S.B && on2) {
-                        xv[m] = *((const float2 *)(a.wte + (int64_t)a.ids[m] * C) + tid);
-                        if (a.wpe) { const float2 p = *((const float2 *)(a.wpe + (int64_t)pos[m] * C) + tid); xv[m].x = __fadd_rn(xv[m].x, p.x); xv[m].y = __fadd_rn(xv[m].y, p.y); }
-                    }
+                xv[0] = make_float2(0.f, 0.f);
+                if (on2) {
+                    xv[0] = *((const float2 *)(a.wte + (int64_t)a.ids[0] * C) + tid);
+                    if (a.wpe) { const float2 p = *((const float2 *)(a.wpe + (int64_t)pos * C) + tid); xv[0].x = __fadd_rn(xv[0].x, p.x); xv[0].y = __fadd_rn(xv[0].y, p.y); }
                 }
             } else {
-                const uint2 *p[MT];
-#pragma unroll
-                for (int m = 0; m < MT; m++) p[m] = m < S.B && on2 ? Lx + (size_t)m * C + 2 * tid : nullptr;
-                c.poll<MT>(p, tag - 1u, xv);
+                const uint2 *p[1] = {on2 ? Lx + 2 * tid : nullptr};
+                c.poll<1>(p, tag - 1u, xv);
             }
-#pragma unroll
-            for (int m = 0; m < MT; m++) {
-                const int r = 2 * tid - c0;
-                if (on2 && r >= 0 && r < ncr) sm->xres[r][m] = xv[m].x;
-                if (on2 && r + 1 >= 0 && r + 1 < ncr) sm->xres[r + 1][m] = xv[m].y;
-            }
-            ms_norm<MT>(sm, xv, C, a.norm, w, b, a.eps, xs, tid);
+            const int r = 2 * tid - c0;
+            if (on2 && r >= 0 && r < ncr) sm->xres[r] = xv[0].x;
+            if (on2 && r + 1 >= 0 && r + 1 < ncr) sm->xres[r + 1] = xv[0].y;
+            ms_norm(sm, xv[0], C, a.norm, w, b, a.eps, xs, tid);
         }
-        ms_rows<MT, W16>(c, st, at, 2 * nq, C, xs, part, warp, lane);
+        ms_rows<W16>(c, st, at, 2 * nq, C, xs, part, warp, lane);
         at += b_qkv;
         ms_bar();
-        st.release(at, warp, lane);
-        for (int t = tid; t < nq * S.B; t += MS_T) {
-            const int i = t / S.B, m = t - i * S.B, pr = q0 + i, h = pr >> 5, d = pr & 31;
-            const float *p0 = part + (size_t)(2 * i) * 4 * MT + m, *p1 = p0 + 4 * MT;
-            float y0 = (p0[0] + p0[MT]) + (p0[2 * MT] + p0[3 * MT]), y1 = (p1[0] + p1[MT]) + (p1[2 * MT] + p1[3 * MT]);
-            if (L.qkvb) { y0 += __ldg(L.qkvb + h * 64 + d); y1 += __ldg(L.qkvb + h * 64 + d + 32); }
+        if (tid < nq) {
+            const int h = (q0 + tid) >> 5, d = (q0 + tid) & 31;
+            const float4 p0 = *(const float4 *)(part + 8 * tid), p1 = *(const float4 *)(part + 8 * tid + 4);
+            float y0 = (p0.x + p0.y) + (p0.z + p0.w), y1 = (p1.x + p1.y) + (p1.z + p1.w);
+            y0 += one(L.qkvb, true, h * 64 + d); y1 += one(L.qkvb, true, h * 64 + d + 32);
             if (a.cosb && h < S.H + S.nkv) {
-                const float *co = a.cosb + (int64_t)pos[m] * 64 + d, *si = a.sinb + (int64_t)pos[m] * 64 + d;
+                const float *co = a.cosb + (int64_t)pos * 64 + d, *si = a.sinb + (int64_t)pos * 64 + d;
                 const float z0 = __fadd_rn(__fmul_rn(y0, co[0]), __fmul_rn(-y1, si[0])), z1 = __fadd_rn(__fmul_rn(y1, co[32]), __fmul_rn(y0, si[32]));
                 y0 = z0; y1 = z1;
             }
-            uint2 *o = Lq + (size_t)m * Wq + h * 64 + d;
+            uint2 *o = Lq + h * 64 + d;
             ll_store(o, y0, tag); ll_store(o + 32, y1, tag);
             if (h >= S.H) {
-                float *kv = L.kv + (int64_t)m * a.kv_seq_pitch + (int64_t)pos[m] * 2 * kvd + (h - S.H) * 64 + d;
+                float *kv = L.kv + (int64_t)pos * 2 * kvd + (h - S.H) * 64 + d;
                 kv[0] = y0; kv[32] = y1;
             }
         }
+        st.release(at, warp, lane);
         // ---- attention partials ----
         if (att) {
             MsKV f;
-            ms_kv_load(f, kvb, 2 * kvd, kvd, k0, k1, cached, warp, lane);
+            ms_kv_load(f, kvb, 2 * kvd, kvd, k0, k1, pos, warp, lane);
             if (warp < 3) {
                 const int h = warp == 0 ? ah : (warp == 1 ? S.H + akv : S.H + S.nkv + akv);
-                const uint2 *p[1] = {warp == 0 || k1 == n_keys ? Lq + (size_t)ab * Wq + h * 64 + 2 * lane : nullptr};
+                const uint2 *p[1] = {warp == 0 || k1 == n_keys ? Lq + h * 64 + 2 * lane : nullptr};
                 float2 v[1];
                 c.poll<1>(p, tag, v);
                 *(float2 *)&sm->qn[warp][2 * lane] = v[0];
             }
             ms_bar();
-            ms_attend(sm, f, kvb, 2 * kvd, kvd, k0, k1, cached, Lp + ((size_t)(ab * S.H + ah) * MS_MAXSPLIT + asp) * MS_PW, tag, tid);
+            ms_attend(sm, f, kvb, 2 * kvd, kvd, k0, k1, pos, Lp + ((size_t)ah * MS_MAXSPLIT + asp) * MS_PW, tag, tid);
         }
         // ---- context, o-projection, residual ----
-#pragma unroll
-        for (int m = 0; m < MT; m++) {
-            if (m >= S.B) { if (on2) *(float2 *)(xs + m * C + 2 * tid) = make_float2(0.f, 0.f); continue; }
+        {
             const uint2 *p[2 * MS_MAXSPLIT];
             float2 v[2 * MS_MAXSPLIT];
 #pragma unroll
             for (int s = 0; s < MS_MAXSPLIT; s++) {
-                const uint2 *b = on2 && s < nsp ? Lp + ((size_t)(m * S.H + (tid >> 5)) * MS_MAXSPLIT + s) * MS_PW : nullptr;
+                const uint2 *b = on2 && s < nsp ? Lp + ((size_t)(tid >> 5) * MS_MAXSPLIT + s) * MS_PW : nullptr;
                 p[2 * s] = b; p[2 * s + 1] = b ? b + 2 + 2 * (tid & 31) : nullptr;
             }
             c.poll<2 * MS_MAXSPLIT>(p, tag, v);
@@ -519,90 +480,75 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
                     l = fmaf(v[2 * s].y, e, l); o0 = fmaf(v[2 * s + 1].x, e, o0); o1 = fmaf(v[2 * s + 1].y, e, o1);
                 }
             const float inv = l > 0.f ? 1.0f / l : 0.f;
-            if (on2) *(float2 *)(xs + m * C + 2 * tid) = make_float2(o0 * inv, o1 * inv);
+            if (on2) *(float2 *)(xs + 2 * tid) = make_float2(o0 * inv, o1 * inv);
         }
         ms_bar();
-        ms_rows<MT, W16>(c, st, at, ncr, C, xs, part, warp, lane);
+        ms_rows<W16>(c, st, at, ncr, C, xs, part, warp, lane);
         at += b_o;
         ms_bar();
-        st.release(at, warp, lane);
-        if (tid < ncr * S.B) {
-            const int r = tid / S.B, m = tid - r * S.B;
-            const float *p = part + (size_t)r * 4 * MT + m;
-            float y = (p[0] + p[MT]) + (p[2 * MT] + p[3 * MT]);
-            if (L.ob) y += __ldg(L.ob + c0 + r);
-            y += sm->xres[r][m];
-            sm->xres[r][m] = y;
-            ll_store(Lx1 + (size_t)m * C + c0 + r, y, tag);
+        if (tid < ncr) {
+            const float4 p = *(const float4 *)(part + 4 * tid);
+            const float y = (p.x + p.y) + (p.z + p.w) + one(L.ob, true, c0 + tid) + sm->xres[tid];
+            sm->xres[tid] = y;
+            ll_store(Lx1 + c0 + tid, y, tag);
         }
+        st.release(at, warp, lane);
         // ---- second norm, up-projection, activation ----
         {
             const float2 w = pair_of(L.ln2w, 1.f), b = pair_of(L.ln2b, 0.f);
-            const uint2 *p[MT];
-#pragma unroll
-            for (int m = 0; m < MT; m++) p[m] = m < S.B && on2 ? Lx1 + (size_t)m * C + 2 * tid : nullptr;
-            c.poll<MT>(p, tag, xv);
-            ms_norm<MT>(sm, xv, C, a.norm, w, b, a.eps, xs, tid);
+            const uint2 *p[1] = {on2 ? Lx1 + 2 * tid : nullptr};
+            c.poll<1>(p, tag, xv);
+            ms_norm(sm, xv[0], C, a.norm, w, b, a.eps, xs, tid);
         }
-        ms_rows<MT, W16>(c, st, at, ur, C, xs, part, warp, lane);
+        ms_rows<W16>(c, st, at, ur, C, xs, part, warp, lane);
         at += b_up;
         ms_bar();
-        st.release(at, warp, lane);
-        for (int t = tid; t < nu * S.B; t += MS_T) {
-            const int i = t / S.B, m = t - i * S.B;
+        if (tid < nu) {
             float y;
             if (S.gated) {
-                const float *p0 = part + (size_t)(2 * i) * 4 * MT + m, *p1 = p0 + 4 * MT;
-                float gt = (p0[0] + p0[MT]) + (p0[2 * MT] + p0[3 * MT]), up = (p1[0] + p1[MT]) + (p1[2 * MT] + p1[3 * MT]);
-                if (L.fcb) { gt += __ldg(L.fcb + u0 + i); up += __ldg(L.fcb + I + u0 + i); }
+                const float4 p0 = *(const float4 *)(part + 8 * tid), p1 = *(const float4 *)(part + 8 * tid + 4);
+                const float gt = (p0.x + p0.y) + (p0.z + p0.w) + one(L.fcb, true, u0 + tid), up = (p1.x + p1.y) + (p1.z + p1.w) + one(L.fcb, true, I + u0 + tid);
                 y = __fmul_rn(tc_act(gt, a.act), up);
             } else {
-                const float *p = part + (size_t)i * 4 * MT + m;
-                y = (p[0] + p[MT]) + (p[2 * MT] + p[3 * MT]);
-                if (L.fcb) y += __ldg(L.fcb + u0 + i);
-                y = tc_act(y, a.act);
+                const float4 p = *(const float4 *)(part + 4 * tid);
+                y = tc_act((p.x + p.y) + (p.z + p.w) + one(L.fcb, true, u0 + tid), a.act);
             }
-            ll_store(Lh + (size_t)m * I + u0 + i, y, tag);
+            ll_store(Lh + u0 + tid, y, tag);
         }
+        st.release(at, warp, lane);
         ms_bar();                                             // part is rewritten by the down-projection
         // ---- down-projection, residual ----
-        ms_down<MT, W16>(c, st, at, ncr, I, S.B, Lh, tag, part, warp, lane);
+        ms_down<W16>(c, st, at, ncr, I, Lh, tag, part, warp, lane);
         at += b_dn;
         ms_bar();
-        st.release(at, warp, lane);
-        if (tid < ncr * S.B) {
-            const int r = tid / S.B, m = tid - r * S.B;
-            float y = 0.f;
+        if (tid < ncr) {
+            float y = one(L.pb, true, c0 + tid) + sm->xres[tid];
 #pragma unroll
-            for (int q = 0; q < MS_WARPS; q++) y += part[((size_t)r * MS_WARPS + q) * MT + m];
-            if (L.pb) y += __ldg(L.pb + c0 + r);
-            y += sm->xres[r][m];
-            ll_store(Lx + (size_t)m * C + c0 + r, y, tag);
+            for (int q = 0; q < MS_WARPS; q++) y += part[tid * MS_WARPS + q];
+            ll_store(Lx + c0 + tid, y, tag);
         }
+        st.release(at, warp, lane);
     }
     // ---- final norm, vocabulary projection ----
     {
         const float2 w = pair_of(a.lnfw, 1.f), b = pair_of(a.lnfb, 0.f);
-        const uint2 *p[MT];
-#pragma unroll
-        for (int m = 0; m < MT; m++) p[m] = m < S.B && on2 ? Lx + (size_t)m * C + 2 * tid : nullptr;
-        c.poll<MT>(p, tag0 + (unsigned)S.NL - 1u, xv);
-        ms_norm<MT>(sm, xv, C, a.norm, w, b, a.eps_f, xs, tid);
+        const uint2 *p[1] = {on2 ? Lx + 2 * tid : nullptr};
+        c.poll<1>(p, tag0 + (unsigned)S.NL - 1u, xv);
+        ms_norm(sm, xv[0], C, a.norm, w, b, a.eps_f, xs, tid);
     }
     st.release(head_at, warp, lane);
     at = head_at;
     int buf = 0;
     for (int r0 = 0; r0 < nv; r0 += MS_HROWS, buf ^= 1) {
         const int n = min(MS_HROWS, nv - r0);
-        float *pb = part + buf * MS_HROWS * 4 * MT;
-        ms_rows<MT, W16>(c, st, at, n, C, xs, pb, warp, lane);
+        float *pb = part + buf * MS_HROWS * 4;
+        ms_rows<W16>(c, st, at, n, C, xs, pb, warp, lane);
         at += (long long)n * C * esz;
         ms_bar();                                             // (the other half of `part` is free by the next barrier)
         st.release(at, warp, lane);
-        for (int t = tid; t < n * S.B; t += MS_T) {
-            const int m = t / n, r = t - m * n;
-            const float *p = pb + (size_t)r * 4 * MT + m;
-            a.logits[(size_t)m * S.V + v0 + r0 + r] = (p[0] + p[MT]) + (p[2 * MT] + p[3 * MT]);
+        if (tid < n) {
+            const float4 p = *(const float4 *)(pb + 4 * tid);
+            a.logits[v0 + r0 + tid] = (p.x + p.y) + (p.z + p.w);
         }
     }
 }
@@ -637,9 +583,9 @@ bool lm_mega_enabled() {
 }
 bool lm_mega_supported(const MegaShape &s, int hd, bool qk_norm) {
     const int g = ctx().sm_count;
-    return s.B >= 1 && s.B <= MG_MAXB && hd == 64 && s.C == s.H * 64 && s.C % 32 == 0 && s.C <= MS_MAXC && s.I % 8 == 0 && s.I <= MS_MAXI && !qk_norm &&
-           s.H % s.nkv == 0 && s.B * s.H <= g && cdiv(s.C, g) <= 8 && 2 * cdiv(s.I, g) <= MS_UPROWS && cdiv(s.C + 128 * s.nkv, g) + 2 <= MS_UPROWS &&
-           (int64_t)s.C * 4 * 32 + 2 * MS_CH <= MS_RING && (int64_t)s.I * 4 + 2 * MS_CH <= MS_RING;
+    return s.B == 1 && hd == 64 && s.C == s.H * 64 && s.C % 32 == 0 && s.C <= MS_MAXC && s.I % 8 == 0 && s.I <= MS_MAXI && !qk_norm &&
+           s.H % s.nkv == 0 && s.H <= g && cdiv(s.C, g) <= 8 && 2 * cdiv(s.I, g) <= MS_UPROWS && cdiv(s.C + 128 * s.nkv, g) + 2 <= MS_UPROWS &&
+           (int64_t)s.C * 4 * 32 + 2 * MS_CH <= MS_RING && s.NL <= MS_MAXNL && (int64_t)s.I * 4 + 2 * MS_CH <= MS_RING;
 }
 
 void lm_mega_free(MegaModel &m) {
@@ -676,27 +622,24 @@ void lm_mega_pack(MegaModel &m, const MegaShape &s, const std::vector<BlockWeigh
 
 size_t lm_mega_exchange_words(const MegaShape &s) { return MsLL(s).total; }
 
-template <int MT, bool W16>
+template <bool W16>
 static void launch_step(const MegaModel &m, const MegaArgs &a) {
     const MegaShape &s = a.s;
     const size_t part = (size_t)std::max<int64_t>(2 * MS_HROWS, 2 * cdiv(s.I, m.grid) + 2) * 4;
-    const size_t smem = MS_RING + sizeof(MsSm) + 16 + ((size_t)MT * s.C + part * MT) * 4;
+    const size_t smem = MS_RING + sizeof(MsSm) + 32 + ((size_t)s.C + part) * 4 + s.NL * sizeof(MegaLayer);
     static size_t set = 0;
-    if (smem > set) { CUDA_CHECK(cudaFuncSetAttribute((k_lm_step<MT, W16>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = smem; }
+    if (smem > set) { CUDA_CHECK(cudaFuncSetAttribute(k_lm_step<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = smem; }
     MegaArgs arg = a;
     const unsigned char *w = (const unsigned char *)m.stream_w, *h = (const unsigned char *)m.head_w;
     const long long *off = m.stream_off;
     void *params[] = {&arg, &w, &off, &h};
-    cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_lm_step<MT, W16>, dim3((unsigned)m.grid), dim3(MS_T + 32), params, smem, stream());
+    cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_lm_step<W16>, dim3((unsigned)m.grid), dim3(MS_T + 32), params, smem, stream());
     if (e != cudaSuccess) fatal("lm_mega: cooperative launch failed: %s", cudaGetErrorString(e));
     ctx().launches++;
 }
 void lm_mega_launch(const MegaModel &m, const MegaArgs &a) {
     ProfScope ps(NCMB_K_GEMM, 0, 0);
-    const int mt = a.s.B <= 1 ? 1 : a.s.B <= 2 ? 2 : 4;
-    if (mt == 1) { if (m.w16) launch_step<1, true>(m, a); else launch_step<1, false>(m, a); }
-    else if (mt == 2) { if (m.w16) launch_step<2, true>(m, a); else launch_step<2, false>(m, a); }
-    else { if (m.w16) launch_step<4, true>(m, a); else launch_step<4, false>(m, a); }
+    if (m.w16) launch_step<true>(m, a); else launch_step<false>(m, a);
 }
 
 } // namespace ncmb

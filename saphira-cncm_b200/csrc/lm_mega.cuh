@@ -4,8 +4,6 @@
 
 namespace ncmb {
 
-constexpr int MG_MAXB = 4;            // sequences per step the persistent kernel takes
-
 struct MegaLayer { const float *ln1w, *ln1b, *qkvb, *ob, *ln2w, *ln2b, *fcb, *pb; float *kv; };
 
 // What the kernel needs of a model, laid out once: every CTA's weight rows of all layers, in the order it uses them, as one
@@ -31,9 +29,8 @@ struct MegaArgs {
     const float *wte, *wpe, *lnfw, *lnfb, *cosb, *sinb;
     float *logits;
     const int *ids, *posmat;
-    const int *step_d;                    // tokens finalised so far (v); this step's position is posmat[(v + pos_base) * B + b]
+    const int *step_d;                    // tokens finalised so far (v); this step's position is posmat[v + pos_base]
     int pos_base;
-    int64_t kv_seq_pitch;
     uint2 *ll;                            // exchange buffers, zeroed before the first step of a generate: lm_mega_exchange_words() words
     int *err;
 };
