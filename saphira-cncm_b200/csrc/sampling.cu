@@ -300,100 +300,106 @@ struct SampleCand {
     unsigned long long *cand;       // [Bn][Lc][Kc]: ordered key << 32 | ~index of the raw (blended) logit
 };
 
-__global__ void __launch_bounds__(SM_THREADS) k_sample_topc(SampleCand sc) {
+// The Kc best of the entries a CTA's threads hold, best first, to out[0, Kc). get(i) is a thread's i-th entry (0: none), Kc <= TC_T
+// (entries are distinct: a key and an index).
+//
+// The Kc-th best of the threads' own maxima bounds the Kc-th best entry from below, so only entries from there on -- some Kc to
+// 2 Kc of them, by the spread of entries over threads -- have to be ranked, by counting, in shared memory. Nothing is sorted and no
+// entry touches a histogram; the bound comes out of 32 barriers that count. Where ties or an odd order of the entries put more
+// than TC_LIST above the bound (a constant row), the cut is searched bit by bit over all entries instead.
+constexpr int TC_T = 512, TC_LIST = 1024, TC_MAXPARTS = 32;
+template <int N, class F>
+__device__ __forceinline__ void topc_select(F get, int Kc, unsigned long long *out) {
+    __shared__ unsigned long long list[TC_LIST];
+    __shared__ int s_n;
+    const int tid = threadIdx.x;
+    unsigned top = 0;
+#pragma unroll
+    for (int i = 0; i < N; i++) top = max(top, (unsigned)(get(i) >> 32));
+    unsigned cut = 0;
+#pragma unroll 1
+    for (unsigned bit = 0x80000000u; bit; bit >>= 1)
+        if (__syncthreads_count(top >= (cut | bit)) >= Kc) cut |= bit;
+    if (tid == 0) s_n = 0;
+    __syncthreads();
+    unsigned long long least = (unsigned long long)cut << 32;
+    auto collect = [&]() {
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const unsigned long long k = get(i);
+            if (k != 0 && k >= least) { const int at = atomicAdd(&s_n, 1); if (at < TC_LIST) list[at] = k; }
+        }
+        __syncthreads();
+    };
+    collect();
+    if (s_n > TC_LIST) {
+        unsigned long long c64 = 0;
+#pragma unroll 1
+        for (int bit = 63; bit >= 0; bit--) {
+            const unsigned long long t = c64 | 1ull << bit;
+            __syncthreads();
+            if (tid == 0) s_n = 0;
+            __syncthreads();
+            int n = 0;
+#pragma unroll
+            for (int i = 0; i < N; i++) n += get(i) >= t;
+            n = __reduce_add_sync(0xffffffffu, n);
+            if ((tid & 31) == 0) atomicAdd(&s_n, n);
+            __syncthreads();
+            if (s_n >= Kc) c64 = t;
+        }
+        __syncthreads();
+        if (tid == 0) s_n = 0;
+        __syncthreads();
+        least = c64;
+        collect();
+    }
+    const int n = s_n;
+    for (int e = tid; e < n; e += TC_T) {
+        const unsigned long long k = list[e];
+        int r = 0;
+        for (int f = 0; f < n; f++) r += list[f] > k;
+        if (r < Kc) out[r] = k;
+    }
+}
+
+// CTA (part, row x position): the Kc best of one of gridDim.x equal parts (a part may hold fewer entries than Kc: zeros follow).
+// Entries stay in registers, N per thread. Bound by latency: one trip to the logits, 32 barriers, one short list.
+template <int N>
+__global__ void __launch_bounds__(TC_T) k_sample_topc(SampleCand sc, unsigned long long *parts) {
     const SampleArgs &a = sc.a;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    float *vals = (float *)smraw;
-    __shared__ int hist[256];
-    __shared__ unsigned s_prefix, s_mask;
-    __shared__ int s_remaining, s_ncand, s_eqbase[SM_THREADS + 1];
-    const int tid = threadIdx.x, V = a.V, Lc = a.Lc, keep = sc.Kc;
-    const int b = blockIdx.x / Lc, t = blockIdx.x % Lc;
-    const float *lc = a.logits + ((size_t)b * Lc + t) * V;
-    const float *lu = a.uncond_off ? a.logits + (((size_t)b + a.uncond_off) * Lc + t) * V : nullptr;
-    float *bo = a.blend_out ? a.blend_out + ((size_t)b * Lc + t) * V : nullptr;
-    unsigned long long *out = sc.cand + ((size_t)b * Lc + t) * keep;
-    for (int v = tid; v < V; v += SM_THREADS) {
-        float x = lc[v];
-        if (lu) x = (float)((1.0 + a.cfg_w) * (double)x - a.cfg_w * (double)lu[v]);
-        if (bo) bo[v] = x;
-        vals[v] = x;
-    }
-    if (tid == 0) { s_prefix = 0; s_mask = 0; s_remaining = keep; }
-    __syncthreads();
-    for (int pass = 3; pass >= 0; pass--) {
-        hist[tid] = 0;
-        __syncthreads();
-        unsigned prefix = s_prefix, mask = s_mask;
-        for (int v = tid; v < V; v += SM_THREADS) {
-            unsigned k = okey(vals[v]);
-            if ((k & mask) == prefix) atomicAdd(&hist[(k >> (8 * pass)) & 0xff], 1);
-        }
-        __syncthreads();
-        if (tid < 32) {
-            const int rem = s_remaining, top = 255 - 8 * tid;
-            int h8[8], tot = 0;
+    const int tid = threadIdx.x, V = a.V, Lc = a.Lc, G = gridDim.x;
+    const int b = blockIdx.y / Lc, t = blockIdx.y % Lc;
+    const int v0 = (int)((long long)V * blockIdx.x / G), n = (int)((long long)V * (blockIdx.x + 1) / G) - v0;
+    const float *lc = a.logits + ((size_t)b * Lc + t) * V + v0;
+    const float *lu = a.uncond_off ? a.logits + (((size_t)b + a.uncond_off) * Lc + t) * V + v0 : nullptr;
+    float *bo = a.blend_out ? a.blend_out + ((size_t)b * Lc + t) * V + v0 : nullptr;
+    unsigned long long *out = (G > 1 ? parts : sc.cand) + ((size_t)blockIdx.y * G + blockIdx.x) * sc.Kc;
+    float x[N];
 #pragma unroll
-            for (int i = 0; i < 8; i++) { h8[i] = hist[top - i]; tot += h8[i]; }
-            int incl = tot;
+    for (int i = 0; i < N; i++) { const int v = i * TC_T + tid; x[i] = v < n ? lc[v] : 0.f; }
+    if (lu) {
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { int t2 = __shfl_up_sync(0xffffffffu, incl, o); if (tid >= o) incl += t2; }
-            int cum = incl - tot;
-            const bool here = cum < rem && incl >= rem;
-            const unsigned who = __ballot_sync(0xffffffffu, here);
-            if (who == 0) {
-                if (tid == 31) { s_remaining = rem - (incl - h8[7]); s_prefix = prefix; s_mask = mask | (0xffu << (8 * pass)); }
-            } else if (tid == __ffs(who) - 1) {
-                int bin = top;
-                for (int i = 0; i < 8; i++) {
-                    bin = top - i;
-                    if (bin == 0 || cum + h8[i] >= rem) break;
-                    cum += h8[i];
-                }
-                s_remaining = rem - cum;
-                s_prefix = prefix | ((unsigned)bin << (8 * pass));
-                s_mask = mask | (0xffu << (8 * pass));
-            }
-        }
-        __syncthreads();
+        for (int i = 0; i < N; i++) { const int v = i * TC_T + tid; if (v < n) x[i] = (float)((1.0 + a.cfg_w) * (double)x[i] - a.cfg_w * (double)lu[v]); }
     }
-    const unsigned thr = s_prefix;
-    const int need_eq = s_remaining;
-    if (tid == 0) s_ncand = 0;
-    __syncthreads();
-    for (int v = tid; v < V; v += SM_THREADS) {
-        unsigned k = okey(vals[v]);
-        if (k > thr) {
-            int p = atomicAdd(&s_ncand, 1);
-            out[p] = ((unsigned long long)k << 32) | (unsigned)(0xffffffffu - (unsigned)v);
-        }
-    }
-    const int chunk = (V + SM_THREADS - 1) / SM_THREADS;
-    const int v0 = tid * chunk, v1 = (v0 + chunk < V) ? v0 + chunk : V;
-    int eq = 0;
-    for (int v = v0; v < v1; v++) if (okey(vals[v]) == thr) eq++;
-    {
-        const int lane = tid & 31, wp = tid >> 5;
-        int v = eq;
+    if (bo) {
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { int t2 = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += t2; }
-        __syncthreads();                       // hist is reused for the warp totals
-        if (lane == 31) hist[wp] = v;
-        __syncthreads();
-        int base = 0;
-        for (int i = 0; i < wp; i++) base += hist[i];
-        s_eqbase[tid + 1] = base + v;
-        if (tid == 0) s_eqbase[0] = 0;
+        for (int i = 0; i < N; i++) { const int v = i * TC_T + tid; if (v < n) bo[v] = x[i]; }
     }
-    __syncthreads();
-    {
-        int rank = s_eqbase[tid], gt = s_ncand;
-        for (int v = v0; v < v1 && rank < need_eq; v++)
-            if (okey(vals[v]) == thr) {
-                out[gt + rank] = ((unsigned long long)thr << 32) | (unsigned)(0xffffffffu - (unsigned)v);
-                rank++;
-            }
-    }
+    auto get = [&](int i) -> unsigned long long {
+        const int v = i * TC_T + tid;
+        return v < n ? ((unsigned long long)okey(x[i]) << 32) | (unsigned)(0xffffffffu - (unsigned)(v0 + v)) : 0ull;
+    };
+    if (n < sc.Kc) for (int e = n + tid; e < sc.Kc; e += TC_T) out[e] = 0;
+    topc_select<N>(get, sc.Kc < n ? sc.Kc : n, out);
+}
+template <int N>
+__global__ void __launch_bounds__(TC_T) k_sample_merge(SampleCand sc, const unsigned long long *parts, int G) {
+    const int tid = threadIdx.x, n = G * sc.Kc;
+    unsigned long long k[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) k[i] = i * TC_T + tid < n ? parts[(size_t)blockIdx.x * n + i * TC_T + tid] : 0;
+    topc_select<N>([&](int i) { return k[i]; }, sc.Kc, sc.cand + (size_t)blockIdx.x * sc.Kc);
 }
 
 __global__ void __launch_bounds__(SC_MAXC) k_sample_seq(SampleCand sc) {
@@ -509,7 +515,7 @@ __global__ void __launch_bounds__(SC_MAXC) k_sample_seq(SampleCand sc) {
 
 // Kc for the two-phase path, or 0 when it does not apply
 static int two_phase_width(const SampleArgs &a) {
-    if (!(a.temp > 0.f) || a.top_k <= 0 || a.V > SM_SMEM_V) return 0;
+    if (!(a.temp > 0.f) || a.top_k <= 0 || a.V > TC_MAXPARTS * TC_T * 32) return 0;
     const char *e = getenv("NCM_B200_SAMPLE_PHASES");          // 1 = one kernel always, 2 = two phases whenever valid
     const int mode = e ? atoi(e) : 0;
     if (mode == 1) return 0;
@@ -521,7 +527,7 @@ static int two_phase_width(const SampleArgs &a) {
     int need = keep + (penal ? a.picks_bound : 0), Kc = 32;
     while (Kc < need) Kc <<= 1;
     if (Kc > SC_MAXC || Kc > a.V) return 0;
-    if (mode != 2 && (a.V < 8 * Kc || a.Lc < 2)) return 0;      // nothing to gain on short rows or a single position
+    if (mode != 2 && a.V < 8 * Kc) return 0;                    // nothing to gain on short rows
     return Kc;
 }
 
@@ -1086,18 +1092,41 @@ void sample_rows(const SampleArgs &a) {
         if (keep > SM_MAXKEEP) { sample_rows_large(a, keep); return; }
     }
     if (const int Kc = two_phase_width(a)) {
+        // parts of a row: one where the entries of a row fit a CTA's registers; long rows so that few of them still occupy the GPU
+        const int rows = a.Bn * a.Lc;
+        int G = 1;
+        if (a.V > TC_T * 32) {
+            const int want = (2 * ctx().sm_count + rows - 1) / rows, cap = std::min(std::min(TC_MAXPARTS, (int)cdiv(a.V, TC_T * 8)), TC_T * 16 / Kc);
+            G = std::max((int)cdiv(a.V, TC_T * 32), std::min(want, cap));
+        }
         static unsigned long long *cand = nullptr; static size_t cand_cap = 0;
-        const size_t need = (size_t)a.Bn * a.Lc * Kc;
+        const size_t need = (size_t)rows * Kc * (G > 1 ? G + 1 : 1);
         if (need > cand_cap) {
             if (cand) { CUDA_CHECK(cudaStreamSynchronize(stream())); dev_free(cand); }
             cand = (unsigned long long *)dev_alloc(need * 8); cand_cap = need;
         }
         SampleCand sc;
         sc.a = a; sc.Kc = Kc; sc.cand = cand;
-        static bool set = false;
-        if (!set) { CUDA_CHECK(cudaFuncSetAttribute(k_sample_topc, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * SM_SMEM_V)); set = true; }
-        ProfScope ps(NCMB_K_SAMPLE, 0, (double)a.Bn * a.Lc * a.V * (a.uncond_off ? 8 : 4));
-        LAUNCH(k_sample_topc, (unsigned)(a.Bn * a.Lc), SM_THREADS, sizeof(float) * (size_t)a.V, sc);
+        unsigned long long *parts = cand + (size_t)rows * Kc;
+        ProfScope ps(NCMB_K_SAMPLE, 0, (double)rows * a.V * (a.uncond_off ? 8 : 4));
+        for (int r0 = 0; r0 < a.Bn; r0 += 65535 / a.Lc) {
+            // (grid.y holds 65535 rows x positions)
+            const int nb = std::min(a.Bn - r0, 65535 / a.Lc);
+            SampleCand c = sc;
+            const size_t at = (size_t)r0 * a.Lc;
+            c.a.logits += at * a.V; if (c.a.blend_out) c.a.blend_out += at * a.V;
+            c.cand += at * Kc;
+            const dim3 grid((unsigned)G, (unsigned)(nb * a.Lc));
+            const int64_t n = cdiv(a.V, G);
+            if (n <= TC_T * 4) LAUNCH(k_sample_topc<4>, grid, TC_T, 0, c, parts + at * G * Kc);
+            else if (n <= TC_T * 8) LAUNCH(k_sample_topc<8>, grid, TC_T, 0, c, parts + at * G * Kc);
+            else if (n <= TC_T * 16) LAUNCH(k_sample_topc<16>, grid, TC_T, 0, c, parts + at * G * Kc);
+            else LAUNCH(k_sample_topc<32>, grid, TC_T, 0, c, parts + at * G * Kc);
+        }
+        if (G > 1) {
+            if (G * Kc <= TC_T * 4) LAUNCH(k_sample_merge<4>, (unsigned)rows, TC_T, 0, sc, (const unsigned long long *)parts, G);
+            else LAUNCH(k_sample_merge<16>, (unsigned)rows, TC_T, 0, sc, (const unsigned long long *)parts, G);
+        }
         LAUNCH(k_sample_seq, (unsigned)a.Bn, Kc, 0, sc);           // one thread per candidate
         return;
     }
