@@ -645,58 +645,36 @@ __global__ void __launch_bounds__(SL_THREADS) k_pick_sorted(const void *__restri
 // sums, so runs are reproducible whatever order the atomics land in); the absolute error of a cumulative sum is
 // below 1e-11 of the row's mass, which moves a draw only when it falls that close to a boundary. Ties of equal
 // logits are ranked by ascending index, like the stable sort.
-constexpr int NS_THREADS = 1024;
+constexpr int NS_THREADS = 1024, ND_THREADS = 512;
 constexpr int NS_BINS = 2048;
 constexpr double NS_FIX = 17592186044416.0;                       // 2^44
 
 struct NsHist {
     unsigned long long sum[NS_BINS];
     unsigned cnt[NS_BINS];
-    unsigned kmin_inv[NS_BINS];       // ~(smallest key of the bin): zero-initialised storage, atomicMax
+    unsigned kmin_inv[NS_BINS];       // ~(smallest key of the bin)
+    __device__ __forceinline__ bool any(int i) const { return cnt[i] != 0; }
 };
-// A CTA's shared-memory copy. The 45-bit masses are added as three 15-bit limbs with native 32-bit atomics (a 64-bit
-// shared-memory add is a compare-and-swap loop, and the rows' keys cluster in a few bins: it was 0.6 of the 0.7 ms
-// the first sweep took at 256 rows). A limb sum stays below 2^32 for up to 2^17 elements per CTA.
-constexpr int NS_MAX_PER_CTA = 1 << 17;
-struct NsShHist {
-    unsigned s0[NS_BINS], s1[NS_BINS], s2[NS_BINS];
-    unsigned cnt[NS_BINS];
-    unsigned kmin_inv[NS_BINS];
-    __device__ __forceinline__ void clear(int nbins) {
-        for (int i = threadIdx.x; i < nbins; i += NS_THREADS) { s0[i] = 0; s1[i] = 0; s2[i] = 0; cnt[i] = 0; kmin_inv[i] = 0; }
-    }
-    __device__ __forceinline__ void add(int bin, unsigned k, unsigned long long qv) {
-        atomicAdd(&s0[bin], (unsigned)(qv & 0x7fffull));
-        atomicAdd(&s1[bin], (unsigned)((qv >> 15) & 0x7fffull));
-        atomicAdd(&s2[bin], (unsigned)(qv >> 30));
-        atomicAdd(&cnt[bin], 1u);
-        atomicMax(&kmin_inv[bin], ~k);
-    }
-    __device__ __forceinline__ void flush(int nbins, NsHist *gh) {
-        for (int i = threadIdx.x; i < nbins; i += NS_THREADS)
-            if (cnt[i]) {
-                atomicAdd(&gh->sum[i], (unsigned long long)s0[i] + ((unsigned long long)s1[i] << 15) + ((unsigned long long)s2[i] << 30));
-                atomicAdd(&gh->cnt[i], cnt[i]);
-                atomicMax(&gh->kmin_inv[i], kmin_inv[i]);
-            }
-    }
+// Mass by distance below the row's largest value: bin NS_BINS - 1 holds [0, 1/64) and so on down to 32, where exp() is below half a
+// unit of mass. Distances spread logits over most of the bins (top key bits put a whole octave of values into four).
+struct NsDist {
+    unsigned long long sum[NS_BINS];
+    unsigned kmin_inv[NS_BINS];       // ~(smallest key of the bin); 0: empty
+    __device__ __forceinline__ bool any(int i) const { return kmin_inv[i] != 0; }
 };
-// Per-row state handed from one kernel of the sequence to the next. A field is written by the first CTA of a row
-// in one kernel and read only by LATER kernels (the CTAs of a kernel each repeat its decision for themselves), hence
-// one slot per stage for the fields that change from stage to stage.
+// Per-row state; zeroed before the first kernel.
 struct NsRow {
     unsigned maxkey;
-    int n_done[2];                     // nucleus cut resolved by the first / second level (den2 valid)
-    unsigned n_prefix[2];              // key bits fixed by the nucleus descent after its first / second level
-    unsigned long long n_above[2];     // mass strictly above the nucleus descent's range after those levels
-    unsigned long long total, den2;    // mass of the row / of the kept prefix
-    unsigned p_prefix[2];
-    unsigned long long p_above[2];
-    double U;                          // the draw, in fixed-point units of mass
-    unsigned n_cand;                   // entries the last histogram pass put on the row's candidate list
+    int n_nuc, n_pick;                 // entries on the row's two lists
+    int nuc;                           // bin the nucleus cut lies in; -1: everything is kept
+    unsigned long long total, nuc_above, pick_above;     // mass of the row; above the cut's bin; above the draw's first bin
 };
-constexpr int NS_CAND = 2048;          // (key, index) pairs per row kept for the final index search
+constexpr int NS_LIST = 2048;          // (key, index) entries a list holds
 
+__device__ __forceinline__ int ns_bin(float mx, float x) {        // monotone in x; -1: no mass
+    const float d = mx - x;
+    return d < 32.f ? NS_BINS - 1 - (int)(d * 64.f) : -1;
+}
 __device__ __forceinline__ unsigned long long ns_q_of_key(unsigned key, double mx) {
     return __double2ull_rn(exp((double)okey_inv(key) - mx) * NS_FIX);
 }
@@ -721,10 +699,10 @@ __device__ __forceinline__ unsigned long long ns_block_excl_scan(unsigned long l
 // One level of a descent over a histogram of `nbins` bins, highest bin first. NUCLEUS: the first bin whose LAST
 // element satisfies cum_before - p > T (the cut then lies inside that bin or exactly in front of it; the descent
 // into the bin settles which). Otherwise: the first bin with cum_incl >= T. Results through shared memory:
-// *sel = bin (-1: no bin satisfies), *sel_above = mass above that bin; *first_hit is always 0.
-template <bool NUCLEUS>
-__device__ void ns_decide(const NsHist *h, int nbins, unsigned long long above, double T, double mx, unsigned key_hi, int shift,
-                          unsigned long long *wsum, int *sel, unsigned long long *sel_above, int *first_hit) {
+// *sel = bin (-1: no bin satisfies), *sel_above = mass above that bin.
+template <bool NUCLEUS, class H>
+__device__ void ns_decide(const H *h, int nbins, unsigned long long above, double T, double mx, unsigned long long *wsum, int *sel,
+                          unsigned long long *sel_above) {
     const int tid = threadIdx.x;
     unsigned long long s[2]; int bin[2];
 #pragma unroll
@@ -733,13 +711,13 @@ __device__ void ns_decide(const NsHist *h, int nbins, unsigned long long above, 
         bin[e] = nbins - 1 - d;
         s[e] = (d < nbins) ? h->sum[bin[e]] : 0ull;
     }
-    if (tid == 0) { *sel = 0x7fffffff; *first_hit = 0; }
+    if (tid == 0) *sel = 0x7fffffff;
     const unsigned long long ex = ns_block_excl_scan(s[0] + s[1], wsum);    // contains a __syncthreads after the init above
     unsigned long long ab = above + ex;
 #pragma unroll
     for (int e = 0; e < 2; e++) {
         const int d = 2 * tid + e;
-        if (d < nbins && h->cnt[bin[e]] > 0) {
+        if (d < nbins && h->any(bin[e])) {
             bool hit;
             if (NUCLEUS) {
                 const unsigned kmin = ~h->kmin_inv[bin[e]];
@@ -774,224 +752,245 @@ __global__ void __launch_bounds__(NS_THREADS) k_ns_max(const float *__restrict__
     if ((threadIdx.x & 31) == 0) atomicMax(&rows[b].maxkey, m);
 }
 
-// accumulates the elements of this CTA's slice whose key, shifted right by `fshift`, equals `want` (fshift = 32:
-// every element) into the histogram of the next `bits` key bits below that; shared histogram, then one atomic
-// per touched bin into the row's global one
-__device__ void ns_histogram(const unsigned *__restrict__ keys, const unsigned long long *__restrict__ q, int V, int fshift, unsigned want,
-                             int shift, int nbins, NsShHist *sh, NsHist *gh, unsigned *n_cand = nullptr, unsigned long long *cand = nullptr) {
-    sh->clear(nbins);
+// mass by distance: one sweep over the logits, the masses as 16-bit limbs (mass below 2^32 or 2^16 -- most of a row -- takes fewer
+// atomics); at most 2^16 elements per CTA
+__global__ void __launch_bounds__(ND_THREADS) k_ns_dist(const float *__restrict__ logits, float temp, int V, const NsRow *rows, NsDist *dist) {
+    __shared__ unsigned s0[NS_BINS], s1[NS_BINS], s2[NS_BINS], km[NS_BINS];
+    const int b = blockIdx.y, tid = threadIdx.x;
+    const float *lg = logits + (size_t)b * V;
+    const unsigned mk = rows[b].maxkey;
+    const float mxf = okey_inv(mk);
+    const double mx = (double)mxf;
+    for (int i = tid; i < NS_BINS; i += ND_THREADS) { s0[i] = 0; s1[i] = 0; s2[i] = 0; km[i] = 0; }
     __syncthreads();
-    // (Combining the lanes of a warp that fall into the same bin first -- match + warp reductions, one lane per
-    // distinct bin touching shared memory -- measured slower than these plain shared-memory atomics: 2.6 against
-    // 1.5 ms per step at 256 rows of 151 936 entries.)
-    for (int i = blockIdx.x * NS_THREADS + threadIdx.x; i < V; i += gridDim.x * NS_THREADS) {
-        const unsigned k = keys[i];
-        if (fshift < 32 && (k >> fshift) != want) continue;
-        const int bin = (int)((k >> shift) & (unsigned)(nbins - 1));
-        sh->add(bin, k, q[i]);
-        if (n_cand) {      // last level of the pick descent: the handful of entries left are kept with their indices
-            const unsigned at = atomicAdd(n_cand, 1u);
-            if (at < (unsigned)NS_CAND) cand[at] = ((unsigned long long)k << 32) | (unsigned)i;
+    const int v0 = (int)((long long)V * blockIdx.x / gridDim.x), v1 = (int)((long long)V * (blockIdx.x + 1) / gridDim.x);
+    for (int i0 = v0 + tid; i0 < v1; i0 += 4 * ND_THREADS) {
+        float x[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) x[u] = i0 + u * ND_THREADS < v1 ? lg[i0 + u * ND_THREADS] / temp : -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int bin = ns_bin(mxf, x[u]);
+            if (bin < 0) continue;
+            const unsigned k = okey(x[u]);
+            const unsigned long long q = ns_q_of_key(k, mx);
+            const unsigned mid = (unsigned)(q >> 16) & 0xffffu, hi = (unsigned)(q >> 32);
+            atomicAdd(&s0[bin], (unsigned)q & 0xffffu);
+            if (mid) atomicAdd(&s1[bin], mid);
+            if (hi) atomicAdd(&s2[bin], hi);
+            atomicMax(&km[bin], ~k);
         }
     }
     __syncthreads();
-    sh->flush(nbins, gh);
+    NsDist *D = dist + b;
+    for (int i = tid; i < NS_BINS; i += ND_THREADS)
+        if (km[i]) {
+            atomicAdd(&D->sum[i], (unsigned long long)s0[i] + ((unsigned long long)s1[i] << 16) + ((unsigned long long)s2[i] << 32));
+            atomicMax(&D->kmin_inv[i], km[i]);
+        }
 }
 
-// keys, fixed-point probabilities and the histogram of the top 11 key bits
-__global__ void __launch_bounds__(NS_THREADS) k_ns_prob(const float *__restrict__ logits, float temp, int V, NsRow *rows, unsigned *keys,
-                                                        unsigned long long *q, NsHist *hist) {
-    __shared__ NsShHist sh;
-    const int b = blockIdx.y;
-    const float *lg = logits + (size_t)b * V;
-    unsigned *kr = keys + (size_t)b * V;
-    unsigned long long *qr = q + (size_t)b * V;
-    const double mx = (double)okey_inv(rows[b].maxkey);
-    NsHist *gh = hist + (size_t)b * 5;
-    sh.clear(NS_BINS);
-    __syncthreads();
-    // keys and masses are stored for the later passes and enter the top-level histogram in the same sweep
-    for (int i = blockIdx.x * NS_THREADS + threadIdx.x; i < V; i += gridDim.x * NS_THREADS) {
-        const unsigned k = okey(lg[i] / temp);
-        const unsigned long long qv = ns_q_of_key(k, mx);
-        kr[i] = k;
-        qr[i] = qv;
-        sh.add((int)(k >> 21), k, qv);
-    }
-    __syncthreads();
-    sh.flush(NS_BINS, gh);
-}
-
-// STAGE 2, 3: nucleus descent (decide on the previous histogram, build the next); 4: end of the nucleus descent,
-// the draw, first level of the pick descent; 5: second level of the pick descent
-template <int STAGE>
-__global__ void __launch_bounds__(NS_THREADS) k_ns_refine(int V, float top_p, const double *__restrict__ uniforms, unsigned long long seed,
-                                                          long long row0, int level, NsRow *rows, const unsigned *keys,
-                                                          const unsigned long long *q, NsHist *hist, unsigned long long *cand) {
-    __shared__ NsShHist sh;
-    __shared__ unsigned long long wsum[32];
-    __shared__ int s_sel, s_first;
-    __shared__ unsigned long long s_above;
+// The bin of the nucleus cut and the bins the draw can fall into (the kept mass lies between the masses above and through the
+// cut's bin); their elements go on the row's lists. Every CTA of a row repeats the decision.
+__global__ void __launch_bounds__(NS_THREADS) k_ns_collect(const float *__restrict__ logits, float temp, int V, float top_p, const double *__restrict__ uniforms,
+                                                           unsigned long long seed, long long row0, int level, NsRow *rows, const NsDist *dist,
+                                                           unsigned long long *lists) {
+    __shared__ unsigned long long wsum[32], s_above, s_total;
+    __shared__ int s_sel;
     const int b = blockIdx.y, tid = threadIdx.x;
     NsRow *row = rows + b;
-    NsHist *H = hist + (size_t)b * 5;                              // 0: top bits | 1, 2: nucleus levels | 3, 4: pick levels
-    const unsigned *kr = keys + (size_t)b * V;
-    const unsigned long long *qr = q + (size_t)b * V;
-    const double mx = (double)okey_inv(row->maxkey);
-    const bool lead = blockIdx.x == 0 && tid == 0;
-    const unsigned long long total = (STAGE == 2) ? 0ull : row->total;
-    if (STAGE == 2) {
-        // total mass = sum over the top-level bins (every CTA computes it; the leader records it)
-        unsigned long long t = H[0].sum[2 * tid] + H[0].sum[2 * tid + 1];
-        const unsigned long long ex = ns_block_excl_scan(t, wsum);
-        __shared__ unsigned long long s_total;
-        if (tid == NS_THREADS - 1) s_total = ex + t;
+    const NsDist *D = dist + b;
+    const float mxf = okey_inv(row->maxkey);
+    const double mx = (double)mxf;
+    const unsigned long long two = D->sum[2 * tid] + D->sum[2 * tid + 1], ex = ns_block_excl_scan(two, wsum);
+    if (tid == NS_THREADS - 1) s_total = ex + two;
+    __syncthreads();
+    const unsigned long long total = s_total;
+    int nuc = -1;
+    unsigned long long lo = total, hi = total, na = 0, pa = 0;       // bounds of the kept mass
+    if (top_p < 1.0f) {
+        ns_decide<true>(D, NS_BINS, 0ull, (double)top_p * (double)total, mx, wsum, &s_sel, &s_above);
+        nuc = s_sel;
+        if (nuc >= 0) { na = s_above; lo = na; hi = na + D->sum[nuc]; }
         __syncthreads();
-        const unsigned long long tot = s_total;
-        if (lead) row->total = tot;
-        if (!(top_p < 1.0f)) { if (lead) { row->n_done[0] = 1; row->den2 = tot; } return; }
-        const double T = (double)top_p * (double)tot;
-        ns_decide<true>(&H[0], NS_BINS, 0ull, T, mx, 0u, 21, wsum, &s_sel, &s_above, &s_first);
-        if (s_sel < 0) { if (lead) { row->n_done[0] = 1; row->den2 = tot; } return; }       // the cut is never reached
-        if (s_first) { if (lead) { row->n_done[0] = 1; row->den2 = s_above; } return; }
-        if (lead) { row->n_prefix[0] = (unsigned)s_sel; row->n_above[0] = s_above; }
-        ns_histogram(kr, qr, V, 21, (unsigned)s_sel, 10, NS_BINS, &sh, &H[1]);
-        return;
     }
-    if (STAGE == 3) {
-        if (row->n_done[0]) return;
-        const double T = (double)top_p * (double)total;
-        ns_decide<true>(&H[1], NS_BINS, row->n_above[0], T, mx, 0u, 10, wsum, &s_sel, &s_above, &s_first);
-        // the parent bin's last element satisfies the predicate, so a bin is always found
-        const unsigned pre = (row->n_prefix[0] << 11) | (unsigned)(s_sel < 0 ? 0 : s_sel);
-        if (s_first || s_sel < 0) { __syncthreads(); if (lead) { row->n_done[1] = 1; row->den2 = s_sel < 0 ? total : s_above; } return; }
-        __syncthreads();
-        if (lead) { row->n_prefix[1] = pre; row->n_above[1] = s_above; }
-        ns_histogram(kr, qr, V, 10, pre, 0, 1024, &sh, &H[2]);
-        return;
-    }
-    if (STAGE == 4) {
-        unsigned long long den2 = row->den2;
-        if (!row->n_done[0] && !row->n_done[1]) {
-            const double T = (double)top_p * (double)total;
-            ns_decide<true>(&H[2], 1024, row->n_above[1], T, mx, 0u, 0, wsum, &s_sel, &s_above, &s_first);
-            // the bin is one exact key held by cnt tied elements of mass qk each: the j-th of them (ascending index)
-            // has cum_before - p = above + (j - 1) qk; the cut is the first j for which that exceeds T
-            den2 = total;
-            if (s_sel >= 0) {
-                const unsigned long long qk = ns_q_of_key((row->n_prefix[1] << 10) | (unsigned)s_sel, mx);
-                const long long cnt = (long long)H[2].cnt[s_sel];
-                long long j = 0;
-                if (qk > 0) {
-                    j = (long long)floor((T - (double)s_above) / (double)qk) + 1;
-                    if (j < 0) j = 0;
-                    if (j > cnt) j = cnt;
-                    while (j > 0 && (double)((long long)s_above + (j - 2) * (long long)qk) > T) j--;       // smallest j with the predicate true
-                    while (j < cnt && !((double)((long long)s_above + (j - 1) * (long long)qk) > T)) j++;
-                }
-                den2 = s_above + (unsigned long long)j * qk;
-            }
-            __syncthreads();
+    const double u01 = uniforms ? uniforms[b] : counter_uniform(seed, row0 + b, level, 0);
+    ns_decide<false>(D, NS_BINS, 0ull, u01 * (double)lo, mx, wsum, &s_sel, &s_above);
+    const int p0 = s_sel < 0 ? NS_BINS - 1 : s_sel;
+    if (s_sel >= 0) pa = s_above;
+    __syncthreads();
+    ns_decide<false>(D, NS_BINS, 0ull, u01 * (double)hi, mx, wsum, &s_sel, &s_above);
+    const int p1 = s_sel < 0 ? 0 : s_sel;                            // p1 <= p0: bins count downwards
+    if (blockIdx.x == 0 && tid == 0) { row->nuc = nuc; row->total = total; row->nuc_above = na; row->pick_above = pa; }
+    const float *lg = logits + (size_t)b * V;
+    unsigned long long *Ln = lists + (size_t)b * 2 * NS_LIST, *Lp = Ln + NS_LIST;
+    const int v0 = (int)((long long)V * blockIdx.x / gridDim.x), v1 = (int)((long long)V * (blockIdx.x + 1) / gridDim.x);
+    for (int i0 = v0 + tid; i0 < v1; i0 += 4 * NS_THREADS) {
+        float x[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) x[u] = i0 + u * NS_THREADS < v1 ? lg[i0 + u * NS_THREADS] / temp : -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int bin = ns_bin(mxf, x[u]);
+            if (bin < 0 || (bin != nuc && (bin > p0 || bin < p1))) continue;
+            const unsigned long long e = ((unsigned long long)okey(x[u]) << 32) | (unsigned)(0xffffffffu - (unsigned)(i0 + u * NS_THREADS));
+            if (bin == nuc) { const int at = atomicAdd(&row->n_nuc, 1); if (at < NS_LIST) Ln[at] = e; }
+            if (bin <= p0 && bin >= p1) { const int at = atomicAdd(&row->n_pick, 1); if (at < NS_LIST) Lp[at] = e; }
         }
-        const double u01 = uniforms ? uniforms[b] : counter_uniform(seed, row0 + b, level, 0);
-        const double U = u01 * (double)den2;
-        if (lead) { row->den2 = den2; row->U = U; }
-        ns_decide<false>(&H[0], NS_BINS, 0ull, U, mx, 0u, 21, wsum, &s_sel, &s_above, &s_first);
-        int sel = s_sel;
-        unsigned long long ab = s_above;
-        if (sel < 0) {                                              // rounding put the draw past the last mass: take the lowest occupied bin
-            sel = 0; ab = 0;
-            __syncthreads();
-            if (tid == 0) { int bsel = -1; unsigned long long acc = 0, accb = 0; for (int i = NS_BINS - 1; i >= 0; i--) if (H[0].cnt[i]) { bsel = i; accb = acc; acc += H[0].sum[i]; } s_sel = bsel; s_above = accb; }
-            __syncthreads();
-            sel = s_sel; ab = s_above;
-        }
-        __syncthreads();
-        if (lead) { row->p_prefix[0] = (unsigned)sel; row->p_above[0] = ab; }
-        ns_histogram(kr, qr, V, 21, (unsigned)sel, 10, NS_BINS, &sh, &H[3]);
-        return;
-    }
-    if (STAGE == 5) {
-        ns_decide<false>(&H[3], NS_BINS, row->p_above[0], row->U, mx, 0u, 10, wsum, &s_sel, &s_above, &s_first);
-        int sel = s_sel;
-        unsigned long long ab = s_above;
-        if (sel < 0) {
-            __syncthreads();
-            if (tid == 0) { int bsel = 0; unsigned long long acc = row->p_above[0], accb = acc; for (int i = NS_BINS - 1; i >= 0; i--) if (H[3].cnt[i]) { bsel = i; accb = acc; acc += H[3].sum[i]; } s_sel = bsel; s_above = accb; }
-            __syncthreads();
-            sel = s_sel; ab = s_above;
-        }
-        const unsigned pre = (row->p_prefix[0] << 11) | (unsigned)sel;
-        __syncthreads();
-        if (lead) { row->p_prefix[1] = pre; row->p_above[1] = ab; }
-        ns_histogram(kr, qr, V, 10, pre, 0, 1024, &sh, &H[4], &row->n_cand, cand + (size_t)b * NS_CAND);
-        return;
     }
 }
 
-// last level of the pick descent, then the index: the pick_tie-th (ascending index) element holding the chosen key
-__global__ void __launch_bounds__(NS_THREADS) k_ns_pick(int V, NsRow *rows, const unsigned *keys, NsHist *hist, const unsigned long long *cand,
-                                                        int *__restrict__ out, int out_stride, int out_off) {
-    __shared__ unsigned long long wsum[32];
-    __shared__ int s_sel, s_first, s_n, s_list[2048];
-    __shared__ unsigned long long s_above;
-    const int b = blockIdx.x, tid = threadIdx.x;
-    NsRow *row = rows + b;
-    NsHist *H = hist + (size_t)b * 5;
-    const unsigned *kr = keys + (size_t)b * V;
-    const double mx = (double)okey_inv(row->maxkey);
-    ns_decide<false>(&H[4], 1024, row->p_above[1], row->U, mx, 0u, 0, wsum, &s_sel, &s_above, &s_first);
-    if (s_sel < 0) {
-        __syncthreads();
-        if (tid == 0) { int bsel = 0; unsigned long long acc = row->p_above[1], accb = acc; for (int i = 1023; i >= 0; i--) if (H[4].cnt[i]) { bsel = i; accb = acc; acc += H[4].sum[i]; } s_sel = bsel; s_above = accb; }
+// Shared memory of the last kernel: a histogram over key bits with the limbs it is summed from, or a list and its masses.
+struct NsWork { NsHist h; unsigned s0[NS_BINS], s1[NS_BINS], s2[NS_BINS]; };
+struct NsListWork { unsigned long long e[NS_LIST], q[NS_LIST]; };
+static_assert(sizeof(NsListWork) <= sizeof(NsWork), "the list fits the histogram's place");
+
+// A list too long for NS_LIST (ties, or logits all but equal): one CTA finds the element by descending over the key's bits, 11, 11
+// and 10 at a time, each level a sweep over the row. The 45-bit masses are summed as 15-bit limbs, 2^17 elements at a time.
+// Returns the key; *above = mass above it, *cnt = elements that hold it; false: no element satisfies.
+template <bool NUCLEUS>
+__device__ bool ns_descend(const float *lg, float temp, int V, double mx, double T, NsWork *w, unsigned long long *wsum, int *s_sel,
+                           unsigned long long *s_above, unsigned *key, unsigned long long *above, long long *cnt) {
+    const int tid = threadIdx.x;
+    unsigned prefix = 0;
+    unsigned long long ab = 0;
+    for (int level = 0; level < 3; level++) {
+        const int nbins = level < 2 ? NS_BINS : 1024, shift = level == 0 ? 21 : level == 1 ? 10 : 0, fshift = level == 0 ? 32 : level == 1 ? 21 : 10;
+        for (int i = tid; i < NS_BINS; i += NS_THREADS) { w->h.sum[i] = 0; w->h.cnt[i] = 0; w->h.kmin_inv[i] = 0; }
+        for (int c0 = 0; c0 < V; c0 += 1 << 17) {
+            for (int i = tid; i < NS_BINS; i += NS_THREADS) { w->s0[i] = 0; w->s1[i] = 0; w->s2[i] = 0; }
+            __syncthreads();
+            for (int i = c0 + tid; i < min(V, c0 + (1 << 17)); i += NS_THREADS) {
+                const unsigned k = okey(lg[i] / temp);
+                if (level > 0 && (k >> fshift) != prefix) continue;
+                const int bin = (int)((k >> shift) & (unsigned)(nbins - 1));
+                const unsigned long long q = ns_q_of_key(k, mx);
+                atomicAdd(&w->s0[bin], (unsigned)(q & 0x7fffull));
+                atomicAdd(&w->s1[bin], (unsigned)((q >> 15) & 0x7fffull));
+                atomicAdd(&w->s2[bin], (unsigned)(q >> 30));
+                atomicAdd(&w->h.cnt[bin], 1u);
+                atomicMax(&w->h.kmin_inv[bin], ~k);
+            }
+            __syncthreads();
+            for (int i = tid; i < NS_BINS; i += NS_THREADS)
+                w->h.sum[i] += (unsigned long long)w->s0[i] + ((unsigned long long)w->s1[i] << 15) + ((unsigned long long)w->s2[i] << 30);
+            __syncthreads();
+        }
+        ns_decide<NUCLEUS>(&w->h, nbins, ab, T, mx, wsum, s_sel, s_above);
+        if (*s_sel < 0) {
+            if (NUCLEUS) return false;
+            __syncthreads();                                        // rounding put the draw past the last mass: the lowest occupied bin
+            if (tid == 0) {
+                int bin = 0;
+                unsigned long long acc = ab, before = ab;
+                for (int i = nbins - 1; i >= 0; i--) if (w->h.cnt[i]) { bin = i; before = acc; acc += w->h.sum[i]; }
+                *s_sel = bin; *s_above = before;
+            }
+            __syncthreads();
+        }
+        prefix = level == 0 ? (unsigned)*s_sel : (prefix << (level == 1 ? 11 : 10)) | (unsigned)*s_sel;
+        ab = *s_above;
+        *cnt = (long long)w->h.cnt[*s_sel];
         __syncthreads();
     }
-    const unsigned key = (row->p_prefix[1] << 10) | (unsigned)s_sel;
-    const long long cnt = (long long)H[4].cnt[s_sel];
-    const unsigned long long qk = ns_q_of_key(key, mx);
+    *key = prefix; *above = ab;
+    return true;
+}
+
+// The cut and the draw, one CTA per row. On a list, an element's cumulative mass is the mass above the list's bins plus that of the
+// list's entries before and with it (key descending, index ascending), summed by every entry for itself.
+__global__ void __launch_bounds__(NS_THREADS) k_ns_pick(const float *__restrict__ logits, float temp, int V, float top_p, const double *__restrict__ uniforms,
+                                                        unsigned long long seed, long long row0, int level, const NsRow *rows,
+                                                        const unsigned long long *lists, int *__restrict__ out, int out_stride, int out_off) {
+    extern __shared__ __align__(16) unsigned char nsraw[];
+    NsWork *W = (NsWork *)nsraw;
+    NsListWork *L = (NsListWork *)nsraw;
+    __shared__ unsigned long long wsum[32], s_above, s_hit;
+    __shared__ int s_sel;
+    const int b = blockIdx.x, tid = threadIdx.x;
+    const NsRow *row = rows + b;
+    const float *lg = logits + (size_t)b * V;
+    const double mx = (double)okey_inv(row->maxkey);
+    const unsigned long long total = row->total;
+    const double u01 = uniforms ? uniforms[b] : counter_uniform(seed, row0 + b, level, 0);
+    // largest entry e of a list for which pred(cumulative mass with e, mass of e) holds -> s_hit (0: none); returns its cumulative mass
+    auto first = [&](const unsigned long long *list, int n, unsigned long long above, auto pred) -> unsigned long long {
+        if (tid == 0) s_hit = 0;
+        for (int i = tid; i < n; i += NS_THREADS) { L->e[i] = list[i]; L->q[i] = ns_q_of_key((unsigned)(list[i] >> 32), mx); }
+        __syncthreads();
+        unsigned long long best = 0, bc = 0;
+        for (int i = tid; i < n; i += NS_THREADS) {
+            const unsigned long long e = L->e[i];
+            unsigned long long cum = above;
+            for (int f = 0; f < n; f++) if (L->e[f] >= e) cum += L->q[f];
+            if (e > best && pred(cum, L->q[i])) { best = e; bc = cum; }
+        }
+        if (best) atomicMax(&s_hit, best);
+        __syncthreads();
+        if (best && best == s_hit) s_above = bc - ns_q_of_key((unsigned)(best >> 32), mx);   // mass before it
+        __syncthreads();
+        return s_above;
+    };
+    // ---- the mass that is kept ----
+    unsigned long long den = total;
+    if (row->nuc >= 0) {
+        const double T = (double)top_p * (double)total;
+        if (row->n_nuc <= NS_LIST) {
+            const unsigned long long before = first(lists + (size_t)b * 2 * NS_LIST, row->n_nuc, row->nuc_above,
+                                                    [&](unsigned long long cum, unsigned long long q) { return (double)((long long)cum - 2ll * (long long)q) > T; });
+            if (s_hit) den = before;
+        } else {
+            unsigned key; unsigned long long above; long long cnt;
+            if (ns_descend<true>(lg, temp, V, mx, T, W, wsum, &s_sel, &s_above, &key, &above, &cnt)) {
+                // the j-th of the key's cnt elements (mass qk each, ascending index) has cum_before - p = above + (j - 1) qk; the
+                // cut is the first j for which that exceeds T
+                const unsigned long long qk = ns_q_of_key(key, mx);
+                long long j = 0;
+                if (qk > 0) {
+                    j = (long long)floor((T - (double)above) / (double)qk) + 1;
+                    if (j < 0) j = 0;
+                    if (j > cnt) j = cnt;
+                    while (j > 0 && (double)((long long)above + (j - 2) * (long long)qk) > T) j--;
+                    while (j < cnt && !((double)((long long)above + (j - 1) * (long long)qk) > T)) j++;
+                }
+                den = above + (unsigned long long)j * qk;
+            }
+        }
+        __syncthreads();
+    }
+    // ---- the draw ----
+    const double U = u01 * (double)den;
+    int *o = out + (size_t)b * out_stride + out_off;
+    if (row->n_pick <= NS_LIST) {
+        first(lists + (size_t)b * 2 * NS_LIST + NS_LIST, row->n_pick, row->pick_above, [&](unsigned long long cum, unsigned long long) { return (double)cum >= U; });
+        unsigned long long hit = s_hit;
+        if (!hit) {                                                 // rounding put the draw past the last mass: the last entry
+            if (tid == 0) { hit = ~0ull; for (int i = 0; i < row->n_pick; i++) hit = min(hit, L->e[i]); }
+        }
+        if (tid == 0) *o = (int)(0xffffffffu - (unsigned)(hit & 0xffffffffull));
+        return;
+    }
+    unsigned key; unsigned long long above; long long cnt;
+    ns_descend<false>(lg, temp, V, mx, U, W, wsum, &s_sel, &s_above, &key, &above, &cnt);
     // the j-th tied element has cum_incl = above + (j + 1) qk: the first j for which that reaches U
+    const unsigned long long qk = ns_q_of_key(key, mx);
     long long j = 0;
     if (qk > 0 && cnt > 1) {
-        j = (long long)ceil((row->U - (double)s_above) / (double)qk) - 1;
+        j = (long long)ceil((U - (double)above) / (double)qk) - 1;
         if (j < 0) j = 0;
         if (j > cnt - 1) j = cnt - 1;
-        while (j > 0 && (double)(s_above + (unsigned long long)j * qk) >= row->U) j--;
-        while (j < cnt - 1 && !((double)(s_above + (unsigned long long)(j + 1) * qk) >= row->U)) j++;
+        while (j > 0 && (double)(above + (unsigned long long)j * qk) >= U) j--;
+        while (j < cnt - 1 && !((double)(above + (unsigned long long)(j + 1) * qk) >= U)) j++;
     }
-    if (tid == 0) s_n = 0;
-    __syncthreads();
-    // indices holding the key (a handful at most for real logits; a constant row makes it the whole vocabulary)
-    if (cnt <= 2048) {
-        const unsigned nc = row->n_cand;
-        if (nc <= (unsigned)NS_CAND) {
-            // the entries sharing the key's upper 22 bits were listed by the last histogram pass: no sweep over the row
-            const unsigned long long *cl = cand + (size_t)b * NS_CAND;
-            for (unsigned i = tid; i < nc; i += NS_THREADS) {
-                const unsigned long long e = cl[i];
-                if ((unsigned)(e >> 32) == key) { int at = atomicAdd(&s_n, 1); if (at < 2048) s_list[at] = (int)(unsigned)(e & 0xffffffffull); }
-            }
-        } else {
-            for (int i = tid; i < V; i += NS_THREADS)
-                if (kr[i] == key) { int at = atomicAdd(&s_n, 1); if (at < 2048) s_list[at] = i; }
-        }
-        __syncthreads();
-        const int n = s_n < 2048 ? s_n : 2048;
-        for (int e = tid; e < n; e += NS_THREADS) {
-            int r = 0;
-            for (int f = 0; f < n; f++) r += s_list[f] < s_list[e];
-            if (r == (int)j) out[(size_t)b * out_stride + out_off] = s_list[e];
-        }
-    } else {
-        // many ties: the j-th match in index order, by counting matches per thread slice and scanning
-        const int per = (V + NS_THREADS - 1) / NS_THREADS, i0 = tid * per, i1 = min(V, i0 + per);
-        unsigned long long c = 0;
-        for (int i = i0; i < i1; i++) c += kr[i] == key;
-        const unsigned long long ex = ns_block_excl_scan(c, wsum);
-        if ((unsigned long long)j >= ex && (unsigned long long)j < ex + c) {
-            long long need = j - (long long)ex;
-            for (int i = i0; i < i1; i++)
-                if (kr[i] == key && need-- == 0) { out[(size_t)b * out_stride + out_off] = i; break; }
-        }
+    // its index: matches per thread slice, scanned
+    const int per = (V + NS_THREADS - 1) / NS_THREADS, i0 = min(V, tid * per), i1 = min(V, i0 + per);
+    unsigned long long c = 0;
+    for (int i = i0; i < i1; i++) c += okey(lg[i] / temp) == key;
+    const unsigned long long ex = ns_block_excl_scan(c, wsum);
+    if ((unsigned long long)j >= ex && (unsigned long long)j < ex + c) {
+        long long need = j - (long long)ex;
+        for (int i = i0; i < i1; i++)
+            if (okey(lg[i] / temp) == key && need-- == 0) { *o = i; break; }
     }
 }
 
@@ -1002,34 +1001,28 @@ static bool sample_rows_select(const SampleArgs &a) {
     if ((e && atoi(e)) || a.V < (mv ? atoi(mv) : 4096)) return false;
     static Workspace ws;
     const size_t n = (size_t)a.Bn * a.V;
-    const size_t head = ((size_t)a.Bn * sizeof(NsRow) + (size_t)a.Bn * 5 * sizeof(NsHist) + 255) & ~(size_t)255;
-    const size_t need = head + n * 12 + (size_t)a.Bn * NS_CAND * 8 + 8192;
+    const size_t head = (size_t)a.Bn * (sizeof(NsDist) + sizeof(NsRow));
+    const size_t need = head + (size_t)a.Bn * 2 * NS_LIST * 8 + 8192;
     if (need > ws.cap) ws.reserve(need + need / 8);
     ws.reset();
-    char *base = (char *)ws.alloc(head);
-    NsRow *rows = (NsRow *)base;
-    NsHist *hist = (NsHist *)(base + (((size_t)a.Bn * sizeof(NsRow) + 15) & ~(size_t)15));
-    unsigned long long *q = ws.get<unsigned long long>(n);
-    unsigned *keys = ws.get<unsigned>(n);
-    unsigned long long *cand = ws.get<unsigned long long>((size_t)a.Bn * NS_CAND);
-    ProfScope ps(NCMB_K_SAMPLE, 0, (double)n * 40);
-    CUDA_CHECK(cudaMemsetAsync(base, 0, head, stream()));
-    // CTAs per row: enough to occupy the GPU when there are few rows
-    int G = (2 * ctx().sm_count + a.Bn - 1) / a.Bn;
-    const int gmax = (a.V + 4 * NS_THREADS - 1) / (4 * NS_THREADS);
-    if (G > gmax) G = gmax;
-    if (G > 32) G = 32;
-    const int gmin = (a.V + NS_MAX_PER_CTA - 1) / NS_MAX_PER_CTA;          // the limb sums of a CTA's histogram must not wrap
-    if (G < gmin) G = gmin;
-    if (G < 1) G = 1;
-    const dim3 grid((unsigned)G, (unsigned)a.Bn);
-    LAUNCH(k_ns_max, grid, NS_THREADS, 0, a.logits, a.temp, a.V, rows);
-    LAUNCH(k_ns_prob, grid, NS_THREADS, 0, a.logits, a.temp, a.V, rows, keys, q, hist);
-    LAUNCH(k_ns_refine<2>, grid, NS_THREADS, 0, a.V, a.top_p, a.uniforms, a.rng_seed, a.rng_row0, a.rng_level, rows, (const unsigned *)keys, (const unsigned long long *)q, hist, cand);
-    LAUNCH(k_ns_refine<3>, grid, NS_THREADS, 0, a.V, a.top_p, a.uniforms, a.rng_seed, a.rng_row0, a.rng_level, rows, (const unsigned *)keys, (const unsigned long long *)q, hist, cand);
-    LAUNCH(k_ns_refine<4>, grid, NS_THREADS, 0, a.V, a.top_p, a.uniforms, a.rng_seed, a.rng_row0, a.rng_level, rows, (const unsigned *)keys, (const unsigned long long *)q, hist, cand);
-    LAUNCH(k_ns_refine<5>, grid, NS_THREADS, 0, a.V, a.top_p, a.uniforms, a.rng_seed, a.rng_row0, a.rng_level, rows, (const unsigned *)keys, (const unsigned long long *)q, hist, cand);
-    LAUNCH(k_ns_pick, (unsigned)a.Bn, NS_THREADS, 0, a.V, rows, (const unsigned *)keys, hist, (const unsigned long long *)cand, a.out, a.out_stride, a.out_off);
+    NsDist *dist = (NsDist *)ws.alloc(head);
+    NsRow *rows = (NsRow *)(dist + a.Bn);
+    unsigned long long *lists = ws.get<unsigned long long>((size_t)a.Bn * 2 * NS_LIST);
+    ProfScope ps(NCMB_K_SAMPLE, 0, (double)n * 12);
+    CUDA_CHECK(cudaMemsetAsync(dist, 0, head, stream()));
+    // CTAs per row: enough to occupy the GPU when there are few rows, some elements per thread, and no limb of a sum may wrap
+    auto parts = [&](int threads, int per_sm) {
+        const int want = (per_sm * ctx().sm_count + a.Bn - 1) / a.Bn, most = std::min(32, (int)cdiv(a.V, 4 * threads));
+        return (unsigned)std::max(std::max(std::min(want, most), (int)cdiv(a.V, 1 << 16)), 1);
+    };
+    static bool set = false;
+    if (!set) { CUDA_CHECK(cudaFuncSetAttribute(k_ns_pick, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NsWork))); set = true; }
+    LAUNCH(k_ns_max, dim3(parts(NS_THREADS, 2), (unsigned)a.Bn), NS_THREADS, 0, a.logits, a.temp, a.V, rows);
+    LAUNCH(k_ns_dist, dim3(parts(ND_THREADS, 4), (unsigned)a.Bn), ND_THREADS, 0, a.logits, a.temp, a.V, (const NsRow *)rows, dist);
+    LAUNCH(k_ns_collect, dim3(parts(NS_THREADS, 2), (unsigned)a.Bn), NS_THREADS, 0, a.logits, a.temp, a.V, a.top_p, a.uniforms, a.rng_seed, a.rng_row0, a.rng_level,
+           rows, (const NsDist *)dist, lists);
+    LAUNCH(k_ns_pick, (unsigned)a.Bn, NS_THREADS, sizeof(NsWork), a.logits, a.temp, a.V, a.top_p, a.uniforms, a.rng_seed, a.rng_row0, a.rng_level,
+           (const NsRow *)rows, (const unsigned long long *)lists, a.out, a.out_stride, a.out_off);
     return true;
 }
 
