@@ -5,6 +5,7 @@
 // reference run. Layers reuse the transformer block of the NCP stack.
 #include "common.cuh"
 #include "lm_mega.cuh"
+#include "exp_tab.cuh"
 #include "tc_common.cuh"
 #include "gemm_few.cuh"
 
@@ -583,45 +584,26 @@ extern "C" void ncmb_lm_logits(NcmbLM *m, const int *ids, int T, int last_only, 
 // in fp64. Here the logits stay on the device: one CTA per token row takes the row maximum and the fp64 sum of
 // exponentials, and one double per position goes back to the host, which adds them in position order as the
 // reference does.
-//
-// exp() in fp64 of a difference x <= 0, by table and polynomial (Tang, "Table-driven implementation of the exponential function",
-// ACM TOMS 15, 1989): x = (64 k + j) ln2 / 64 + r with |r| <= ln2 / 128, e^x = 2^k 2^(j/64) (1 + r + r^2/2 + ... + r^5/120). The
-// truncation is below 2^-54; eleven fp64 operations a term instead of the library call's thirty-odd, which were the kernel.
 constexpr int NLL_T = 512;
-__device__ __forceinline__ double nll_exp(double x, const double *tab) {
-    if (x < -700.0) return 0.0;                                    // below any sum this is added to
-    const double magic = 6755399441055744.0;                       // 1.5 * 2^52: adding it rounds to an integer
-    const double t = fma(x, 92.332482616893656877, magic);         // 64 / ln 2
-    const int n = __double2loint(t);
-    const double kd = t - magic;
-    double r = fma(kd, -0x1.62e42fefa0000p-7, x);                  // ln2 / 64 in two parts, the first short enough for an exact product
-    r = fma(kd, -0x1.cf79abc9e3b39p-46, r);
-    double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
-    q = fma(r, q, 1.0 / 6.0);
-    q = fma(r, q, 0.5);
-    q = fma(r * r, q, r);
-    const double b = tab[n & 63], e = fma(b, q, b);
-    return __hiloint2double(__double2hiint(e) + ((n >> 6) << 20), __double2loint(e));
-}
 // One pass over a row: every thread keeps its own maximum and the sum against it (rescaled when the maximum grows, which
 // becomes rare after a few elements). Memory bound: 4 bytes per logit, read once.
 __global__ void __launch_bounds__(NLL_T) k_nll_rows(const float *__restrict__ logits, const int *__restrict__ target, int V,
                                                     double *__restrict__ out) {
-    __shared__ double tab[64], red[NLL_T / 32];
+    __shared__ double tab[EXP_TAB], red[NLL_T / 32];
     __shared__ float mred[NLL_T / 32];
     const int64_t r = blockIdx.x;
     const int tg = target[r], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tg < 0) { if (tid == 0) out[r] = 0.0; return; }      // block-uniform: position without a successor
-    if (tid < 64) tab[tid] = exp2((double)tid / 64.0);
+    exp_tab_fill(tab);
     __syncthreads();
     const float *row = logits + r * V;
     float m = -INFINITY;
     double s = 0.0;
     auto add = [&](float4 v) {
         const float mx = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
-        if (mx > m) { s = m == -INFINITY ? 0.0 : s * nll_exp((double)m - (double)mx, tab); m = mx; }
+        if (mx > m) { s = m == -INFINITY ? 0.0 : s * exp_tab((double)m - (double)mx, tab); m = mx; }
         const double md = (double)m;
-        s += (nll_exp((double)v.x - md, tab) + nll_exp((double)v.y - md, tab)) + (nll_exp((double)v.z - md, tab) + nll_exp((double)v.w - md, tab));
+        s += (exp_tab((double)v.x - md, tab) + exp_tab((double)v.y - md, tab)) + (exp_tab((double)v.z - md, tab) + exp_tab((double)v.w - md, tab));
     };
     // rows of an odd vocabulary start anywhere: single elements up to the first 16-byte boundary and behind the last
     const int head = min(V, (int)((16u - (unsigned)((uintptr_t)row & 15)) & 15u) / 4), n4 = (V - head) >> 2, tail = head + n4 * 4;
@@ -645,7 +627,7 @@ __global__ void __launch_bounds__(NLL_T) k_nll_rows(const float *__restrict__ lo
     mx = mred[0];
 #pragma unroll
     for (int w = 1; w < NLL_T / 32; w++) mx = fmaxf(mx, mred[w]);
-    s = m == -INFINITY ? 0.0 : s * nll_exp((double)m - (double)mx, tab);
+    s = m == -INFINITY ? 0.0 : s * exp_tab((double)m - (double)mx, tab);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) red[warp] = s;

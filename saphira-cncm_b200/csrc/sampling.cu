@@ -13,6 +13,7 @@
 // host in the reference's (level, row, position) order) or from a counter-based
 // generator keyed by (seed, global row, level, position).
 #include "common.cuh"
+#include "exp_tab.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
 #include <vector>
@@ -675,8 +676,8 @@ __device__ __forceinline__ int ns_bin(float mx, float x) {        // monotone in
     const float d = mx - x;
     return d < 32.f ? NS_BINS - 1 - (int)(d * 64.f) : -1;
 }
-__device__ __forceinline__ unsigned long long ns_q_of_key(unsigned key, double mx) {
-    return __double2ull_rn(exp((double)okey_inv(key) - mx) * NS_FIX);
+__device__ __forceinline__ unsigned long long ns_q_of_key(unsigned key, double mx, const double *tab) {
+    return __double2ull_rn(exp_tab((double)okey_inv(key) - mx, tab) * NS_FIX);
 }
 
 // exclusive block scan of one u64 per thread (NS_THREADS threads); every thread gets its prefix
@@ -701,7 +702,7 @@ __device__ __forceinline__ unsigned long long ns_block_excl_scan(unsigned long l
 // into the bin settles which). Otherwise: the first bin with cum_incl >= T. Results through shared memory:
 // *sel = bin (-1: no bin satisfies), *sel_above = mass above that bin.
 template <bool NUCLEUS, class H>
-__device__ void ns_decide(const H *h, int nbins, unsigned long long above, double T, double mx, unsigned long long *wsum, int *sel,
+__device__ void ns_decide(const H *h, int nbins, unsigned long long above, double T, double mx, const double *tab, unsigned long long *wsum, int *sel,
                           unsigned long long *sel_above) {
     const int tid = threadIdx.x;
     unsigned long long s[2]; int bin[2];
@@ -721,7 +722,7 @@ __device__ void ns_decide(const H *h, int nbins, unsigned long long above, doubl
             bool hit;
             if (NUCLEUS) {
                 const unsigned kmin = ~h->kmin_inv[bin[e]];
-                const long long g = (long long)(ab + s[e]) - 2ll * (long long)ns_q_of_key(kmin, mx);
+                const long long g = (long long)(ab + s[e]) - 2ll * (long long)ns_q_of_key(kmin, mx, tab);
                 hit = (double)g > T;
             } else {
                 hit = (double)(ab + s[e]) >= T;
@@ -743,19 +744,29 @@ __device__ void ns_decide(const H *h, int nbins, unsigned long long above, doubl
     __syncthreads();
 }
 
+// (the largest quotient is the quotient of the largest: one division a thread, not one an element)
 __global__ void __launch_bounds__(NS_THREADS) k_ns_max(const float *__restrict__ logits, float temp, int V, NsRow *rows) {
-    const int b = blockIdx.y;
+    const int b = blockIdx.y, stride = gridDim.x * NS_THREADS;
     const float *lg = logits + (size_t)b * V;
-    unsigned m = 0;
-    for (int i = blockIdx.x * NS_THREADS + threadIdx.x; i < V; i += gridDim.x * NS_THREADS) m = max(m, okey(lg[i] / temp));
-    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(&rows[b].maxkey, m);
+    float m = -INFINITY;
+    for (int i0 = blockIdx.x * NS_THREADS + threadIdx.x; i0 < V; i0 += 8 * stride) {
+        float x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = i0 + u * stride < V ? lg[i0 + u * stride] : -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 8; u++) m = fmaxf(m, x[u]);
+    }
+    unsigned k = okey(m / temp);
+    for (int o = 16; o; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(&rows[b].maxkey, k);
 }
 
 // mass by distance: one sweep over the logits, the masses as 16-bit limbs (mass below 2^32 or 2^16 -- most of a row -- takes fewer
 // atomics); at most 2^16 elements per CTA
 __global__ void __launch_bounds__(ND_THREADS) k_ns_dist(const float *__restrict__ logits, float temp, int V, const NsRow *rows, NsDist *dist) {
     __shared__ unsigned s0[NS_BINS], s1[NS_BINS], s2[NS_BINS], km[NS_BINS];
+    __shared__ double tab[EXP_TAB];
+    exp_tab_fill(tab);
     const int b = blockIdx.y, tid = threadIdx.x;
     const float *lg = logits + (size_t)b * V;
     const unsigned mk = rows[b].maxkey;
@@ -773,7 +784,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_ns_dist(const float *__restrict_
             const int bin = ns_bin(mxf, x[u]);
             if (bin < 0) continue;
             const unsigned k = okey(x[u]);
-            const unsigned long long q = ns_q_of_key(k, mx);
+            const unsigned long long q = ns_q_of_key(k, mx, tab);
             const unsigned mid = (unsigned)(q >> 16) & 0xffffu, hi = (unsigned)(q >> 32);
             atomicAdd(&s0[bin], (unsigned)q & 0xffffu);
             if (mid) atomicAdd(&s1[bin], mid);
@@ -796,7 +807,9 @@ __global__ void __launch_bounds__(NS_THREADS) k_ns_collect(const float *__restri
                                                            unsigned long long seed, long long row0, int level, NsRow *rows, const NsDist *dist,
                                                            unsigned long long *lists) {
     __shared__ unsigned long long wsum[32], s_above, s_total;
+    __shared__ double tab[EXP_TAB];
     __shared__ int s_sel;
+    exp_tab_fill(tab);
     const int b = blockIdx.y, tid = threadIdx.x;
     NsRow *row = rows + b;
     const NsDist *D = dist + b;
@@ -809,31 +822,35 @@ __global__ void __launch_bounds__(NS_THREADS) k_ns_collect(const float *__restri
     int nuc = -1;
     unsigned long long lo = total, hi = total, na = 0, pa = 0;       // bounds of the kept mass
     if (top_p < 1.0f) {
-        ns_decide<true>(D, NS_BINS, 0ull, (double)top_p * (double)total, mx, wsum, &s_sel, &s_above);
+        ns_decide<true>(D, NS_BINS, 0ull, (double)top_p * (double)total, mx, tab, wsum, &s_sel, &s_above);
         nuc = s_sel;
         if (nuc >= 0) { na = s_above; lo = na; hi = na + D->sum[nuc]; }
         __syncthreads();
     }
     const double u01 = uniforms ? uniforms[b] : counter_uniform(seed, row0 + b, level, 0);
-    ns_decide<false>(D, NS_BINS, 0ull, u01 * (double)lo, mx, wsum, &s_sel, &s_above);
+    ns_decide<false>(D, NS_BINS, 0ull, u01 * (double)lo, mx, tab, wsum, &s_sel, &s_above);
     const int p0 = s_sel < 0 ? NS_BINS - 1 : s_sel;
     if (s_sel >= 0) pa = s_above;
     __syncthreads();
-    ns_decide<false>(D, NS_BINS, 0ull, u01 * (double)hi, mx, wsum, &s_sel, &s_above);
+    ns_decide<false>(D, NS_BINS, 0ull, u01 * (double)hi, mx, tab, wsum, &s_sel, &s_above);
     const int p1 = s_sel < 0 ? 0 : s_sel;                            // p1 <= p0: bins count downwards
     if (blockIdx.x == 0 && tid == 0) { row->nuc = nuc; row->total = total; row->nuc_above = na; row->pick_above = pa; }
     const float *lg = logits + (size_t)b * V;
     unsigned long long *Ln = lists + (size_t)b * 2 * NS_LIST, *Lp = Ln + NS_LIST;
     const int v0 = (int)((long long)V * blockIdx.x / gridDim.x), v1 = (int)((long long)V * (blockIdx.x + 1) / gridDim.x);
-    for (int i0 = v0 + tid; i0 < v1; i0 += 4 * NS_THREADS) {
-        float x[4];
+    // almost every element lies below all of these bins: told by one comparison, with room for the rounding of both sides
+    const float far = (float)(NS_BINS - (nuc >= 0 ? min(nuc, p1) : p1)) / 64.f, least = (mxf - far) * temp - 1e-5f * (fabsf(mxf) + far + 1.f) * temp;
+    for (int i0 = v0 + tid; i0 < v1; i0 += 8 * NS_THREADS) {
+        float x[8];
 #pragma unroll
-        for (int u = 0; u < 4; u++) x[u] = i0 + u * NS_THREADS < v1 ? lg[i0 + u * NS_THREADS] / temp : -INFINITY;
+        for (int u = 0; u < 8; u++) x[u] = i0 + u * NS_THREADS < v1 ? lg[i0 + u * NS_THREADS] : -INFINITY;
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int bin = ns_bin(mxf, x[u]);
+        for (int u = 0; u < 8; u++) {
+            if (x[u] < least) continue;
+            const float y = x[u] / temp;
+            const int bin = ns_bin(mxf, y);
             if (bin < 0 || (bin != nuc && (bin > p0 || bin < p1))) continue;
-            const unsigned long long e = ((unsigned long long)okey(x[u]) << 32) | (unsigned)(0xffffffffu - (unsigned)(i0 + u * NS_THREADS));
+            const unsigned long long e = ((unsigned long long)okey(y) << 32) | (unsigned)(0xffffffffu - (unsigned)(i0 + u * NS_THREADS));
             if (bin == nuc) { const int at = atomicAdd(&row->n_nuc, 1); if (at < NS_LIST) Ln[at] = e; }
             if (bin <= p0 && bin >= p1) { const int at = atomicAdd(&row->n_pick, 1); if (at < NS_LIST) Lp[at] = e; }
         }
@@ -849,7 +866,7 @@ static_assert(sizeof(NsListWork) <= sizeof(NsWork), "the list fits the histogram
 // and 10 at a time, each level a sweep over the row. The 45-bit masses are summed as 15-bit limbs, 2^17 elements at a time.
 // Returns the key; *above = mass above it, *cnt = elements that hold it; false: no element satisfies.
 template <bool NUCLEUS>
-__device__ bool ns_descend(const float *lg, float temp, int V, double mx, double T, NsWork *w, unsigned long long *wsum, int *s_sel,
+__device__ bool ns_descend(const float *lg, float temp, int V, double mx, const double *tab, double T, NsWork *w, unsigned long long *wsum, int *s_sel,
                            unsigned long long *s_above, unsigned *key, unsigned long long *above, long long *cnt) {
     const int tid = threadIdx.x;
     unsigned prefix = 0;
@@ -864,7 +881,7 @@ __device__ bool ns_descend(const float *lg, float temp, int V, double mx, double
                 const unsigned k = okey(lg[i] / temp);
                 if (level > 0 && (k >> fshift) != prefix) continue;
                 const int bin = (int)((k >> shift) & (unsigned)(nbins - 1));
-                const unsigned long long q = ns_q_of_key(k, mx);
+                const unsigned long long q = ns_q_of_key(k, mx, tab);
                 atomicAdd(&w->s0[bin], (unsigned)(q & 0x7fffull));
                 atomicAdd(&w->s1[bin], (unsigned)((q >> 15) & 0x7fffull));
                 atomicAdd(&w->s2[bin], (unsigned)(q >> 30));
@@ -876,7 +893,7 @@ __device__ bool ns_descend(const float *lg, float temp, int V, double mx, double
                 w->h.sum[i] += (unsigned long long)w->s0[i] + ((unsigned long long)w->s1[i] << 15) + ((unsigned long long)w->s2[i] << 30);
             __syncthreads();
         }
-        ns_decide<NUCLEUS>(&w->h, nbins, ab, T, mx, wsum, s_sel, s_above);
+        ns_decide<NUCLEUS>(&w->h, nbins, ab, T, mx, tab, wsum, s_sel, s_above);
         if (*s_sel < 0) {
             if (NUCLEUS) return false;
             __syncthreads();                                        // rounding put the draw past the last mass: the lowest occupied bin
@@ -906,7 +923,10 @@ __global__ void __launch_bounds__(NS_THREADS) k_ns_pick(const float *__restrict_
     NsWork *W = (NsWork *)nsraw;
     NsListWork *L = (NsListWork *)nsraw;
     __shared__ unsigned long long wsum[32], s_above, s_hit;
+    __shared__ double tab[EXP_TAB];
     __shared__ int s_sel;
+    exp_tab_fill(tab);
+    __syncthreads();
     const int b = blockIdx.x, tid = threadIdx.x;
     const NsRow *row = rows + b;
     const float *lg = logits + (size_t)b * V;
@@ -916,7 +936,7 @@ __global__ void __launch_bounds__(NS_THREADS) k_ns_pick(const float *__restrict_
     // largest entry e of a list for which pred(cumulative mass with e, mass of e) holds -> s_hit (0: none); returns its cumulative mass
     auto first = [&](const unsigned long long *list, int n, unsigned long long above, auto pred) -> unsigned long long {
         if (tid == 0) s_hit = 0;
-        for (int i = tid; i < n; i += NS_THREADS) { L->e[i] = list[i]; L->q[i] = ns_q_of_key((unsigned)(list[i] >> 32), mx); }
+        for (int i = tid; i < n; i += NS_THREADS) { L->e[i] = list[i]; L->q[i] = ns_q_of_key((unsigned)(list[i] >> 32), mx, tab); }
         __syncthreads();
         unsigned long long best = 0, bc = 0;
         for (int i = tid; i < n; i += NS_THREADS) {
@@ -927,7 +947,7 @@ __global__ void __launch_bounds__(NS_THREADS) k_ns_pick(const float *__restrict_
         }
         if (best) atomicMax(&s_hit, best);
         __syncthreads();
-        if (best && best == s_hit) s_above = bc - ns_q_of_key((unsigned)(best >> 32), mx);   // mass before it
+        if (best && best == s_hit) s_above = bc - ns_q_of_key((unsigned)(best >> 32), mx, tab);   // mass before it
         __syncthreads();
         return s_above;
     };
@@ -941,10 +961,10 @@ __global__ void __launch_bounds__(NS_THREADS) k_ns_pick(const float *__restrict_
             if (s_hit) den = before;
         } else {
             unsigned key; unsigned long long above; long long cnt;
-            if (ns_descend<true>(lg, temp, V, mx, T, W, wsum, &s_sel, &s_above, &key, &above, &cnt)) {
+            if (ns_descend<true>(lg, temp, V, mx, tab, T, W, wsum, &s_sel, &s_above, &key, &above, &cnt)) {
                 // the j-th of the key's cnt elements (mass qk each, ascending index) has cum_before - p = above + (j - 1) qk; the
                 // cut is the first j for which that exceeds T
-                const unsigned long long qk = ns_q_of_key(key, mx);
+                const unsigned long long qk = ns_q_of_key(key, mx, tab);
                 long long j = 0;
                 if (qk > 0) {
                     j = (long long)floor((T - (double)above) / (double)qk) + 1;
@@ -971,9 +991,9 @@ __global__ void __launch_bounds__(NS_THREADS) k_ns_pick(const float *__restrict_
         return;
     }
     unsigned key; unsigned long long above; long long cnt;
-    ns_descend<false>(lg, temp, V, mx, U, W, wsum, &s_sel, &s_above, &key, &above, &cnt);
+    ns_descend<false>(lg, temp, V, mx, tab, U, W, wsum, &s_sel, &s_above, &key, &above, &cnt);
     // the j-th tied element has cum_incl = above + (j + 1) qk: the first j for which that reaches U
-    const unsigned long long qk = ns_q_of_key(key, mx);
+    const unsigned long long qk = ns_q_of_key(key, mx, tab);
     long long j = 0;
     if (qk > 0 && cnt > 1) {
         j = (long long)ceil((U - (double)above) / (double)qk) - 1;
