@@ -677,7 +677,8 @@ __device__ __forceinline__ int ns_bin(float mx, float x) {        // monotone in
     return d < 32.f ? NS_BINS - 1 - (int)(d * 64.f) : -1;
 }
 __device__ __forceinline__ unsigned long long ns_q_of_key(unsigned key, double mx, const double *tab) {
-    return __double2ull_rn(exp_tab((double)okey_inv(key) - mx, tab) * NS_FIX);
+    // (adding 2^52 rounds to an integer, in the low bits of the sum)
+    return (unsigned long long)__double_as_longlong(fma(exp_tab((double)okey_inv(key) - mx, tab), NS_FIX, 4503599627370496.0)) & 0xfffffffffffffull;
 }
 
 // exclusive block scan of one u64 per thread (NS_THREADS threads); every thread gets its prefix
@@ -789,7 +790,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_ns_dist(const float *__restrict_
             atomicAdd(&s0[bin], (unsigned)q & 0xffffu);
             if (mid) atomicAdd(&s1[bin], mid);
             if (hi) atomicAdd(&s2[bin], hi);
-            atomicMax(&km[bin], ~k);
+            if (~k > *(volatile unsigned *)&km[bin]) atomicMax(&km[bin], ~k);      // (rarely: a bin's minimum settles early)
         }
     }
     __syncthreads();
@@ -1030,16 +1031,17 @@ static bool sample_rows_select(const SampleArgs &a) {
     unsigned long long *lists = ws.get<unsigned long long>((size_t)a.Bn * 2 * NS_LIST);
     ProfScope ps(NCMB_K_SAMPLE, 0, (double)n * 12);
     CUDA_CHECK(cudaMemsetAsync(dist, 0, head, stream()));
-    // CTAs per row: enough to occupy the GPU when there are few rows, some elements per thread, and no limb of a sum may wrap
-    auto parts = [&](int threads, int per_sm) {
-        const int want = (per_sm * ctx().sm_count + a.Bn - 1) / a.Bn, most = std::min(32, (int)cdiv(a.V, 4 * threads));
-        return (unsigned)std::max(std::max(std::min(want, most), (int)cdiv(a.V, 1 << 16)), 1);
+    // CTAs per row: one wave of what is resident at once, where that gives every row one and no limb of a sum can wrap (2^16
+    // elements a CTA); else about four waves, so that the last one's idle part is small
+    auto parts = [&](int threads, int per_sm, int least) {
+        const int res = per_sm * ctx().sm_count, one = res / a.Bn, most = std::min(32, (int)cdiv(a.V, 4 * threads));
+        return (unsigned)std::max(std::max(std::min(one >= least ? one : 4 * res / a.Bn, most), least), 1);
     };
     static bool set = false;
     if (!set) { CUDA_CHECK(cudaFuncSetAttribute(k_ns_pick, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NsWork))); set = true; }
-    LAUNCH(k_ns_max, dim3(parts(NS_THREADS, 2), (unsigned)a.Bn), NS_THREADS, 0, a.logits, a.temp, a.V, rows);
-    LAUNCH(k_ns_dist, dim3(parts(ND_THREADS, 4), (unsigned)a.Bn), ND_THREADS, 0, a.logits, a.temp, a.V, (const NsRow *)rows, dist);
-    LAUNCH(k_ns_collect, dim3(parts(NS_THREADS, 2), (unsigned)a.Bn), NS_THREADS, 0, a.logits, a.temp, a.V, a.top_p, a.uniforms, a.rng_seed, a.rng_row0, a.rng_level,
+    LAUNCH(k_ns_max, dim3(parts(NS_THREADS, 2, 1), (unsigned)a.Bn), NS_THREADS, 0, a.logits, a.temp, a.V, rows);
+    LAUNCH(k_ns_dist, dim3(parts(ND_THREADS, 4, (int)cdiv(a.V, 1 << 16)), (unsigned)a.Bn), ND_THREADS, 0, a.logits, a.temp, a.V, (const NsRow *)rows, dist);
+    LAUNCH(k_ns_collect, dim3(parts(NS_THREADS, 2, 1), (unsigned)a.Bn), NS_THREADS, 0, a.logits, a.temp, a.V, a.top_p, a.uniforms, a.rng_seed, a.rng_row0, a.rng_level,
            rows, (const NsDist *)dist, lists);
     LAUNCH(k_ns_pick, (unsigned)a.Bn, NS_THREADS, sizeof(NsWork), a.logits, a.temp, a.V, a.top_p, a.uniforms, a.rng_seed, a.rng_row0, a.rng_level,
            (const NsRow *)rows, (const unsigned long long *)lists, a.out, a.out_stride, a.out_off);
