@@ -1,0 +1,51 @@
+"""Decode steps of 1 to 257 rows (the loop of reference src/gpt2.c:179, src/qwen.c:209): the persistent kernel at one row, the
+few-row products and their folded reductions up to 256, the general path above -- at the edges of their row tiles (16, 32, 64,
+128), with widths that fill no tile. Greedy ids of a few rows against the oracle's independent runs."""
+import numpy as np
+import pytest
+
+import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cuda():
+    import capi
+    return capi.NcmLib(helpers.CUDA_LIB)
+
+
+@pytest.fixture(scope="module")
+def models(cuda, tmp_path_factory):
+    import orc
+    import synth
+    made = {}
+    for kind in ("gpt2", "qwen", "qwen_bf16"):
+        d = str(tmp_path_factory.mktemp(kind))
+        if kind == "gpt2":
+            spec = synth.LMSpec(kind, "gpt2", 3, 192, 3, 3, 200, 301, 48, rand_affine=1)
+        else:
+            spec = synth.LMSpec(kind, "qwen", 3, 192, 3, 1, 200, 301, 48, rope_theta=1e6, rand_affine=1, bf16_round=int(kind == "qwen_bf16"))
+        conf, w = synth.write_lm(spec, d)
+        made[kind] = (spec, cuda.ncmb_lm_open(cuda.load_config(conf), w.encode(), int(kind != "gpt2"), spec.bf16_round),
+                      orc.LM(conf, w, kind != "gpt2"))
+    yield made
+    for _, m, _ in made.values():
+        cuda.ncmb_lm_close(m)
+    cuda.ncmb_set_lm_persistent(0)
+
+
+@pytest.mark.parametrize("B", [1, 2, 4, 5, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257])
+@pytest.mark.parametrize("kind", ["gpt2", "qwen", "qwen_bf16"])
+def test_greedy_ids(cuda, models, kind, B):
+    import synth
+    spec, m, om = models[kind]
+    cuda.ncmb_set_lm_persistent(1)
+    n_new = 6
+    P = np.ascontiguousarray(synth.lm_prompts(spec, B, 35, B))
+    out = np.zeros((B, n_new), np.int32)
+    cuda.ncmb_lm_generate(m, P.ctypes.data, B, P.shape[1], n_new, 0.0, 0, 1.0, 0, -1, out.ctypes.data)
+    for b in sorted({0, B // 2, B - 1}):
+        want = om.generate(P[b], n_new, temp=0.0)
+        assert (out[b] == want).all(), (kind, B, b, out[b], want)
+    assert cuda.ncmb_gemm_tc_check() == 0
