@@ -1,4 +1,4 @@
-// Products of a weight matrix with 5 to 256 rows, and what stands between them in a block.
+// Products of a weight matrix with 2 to 640 rows, and what stands between them in a block.
 //
 // A decode step of a batch (and the first levels of a generate) multiplies every weight matrix with few rows, so it is bound
 // by streaming the weights. The fp16-pair engine (gemm_h3.cu) makes the rows of x the 128-row side of its tiles: with 27 rows

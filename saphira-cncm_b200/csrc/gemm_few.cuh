@@ -15,7 +15,10 @@ struct FewGemm {
     float *y = nullptr, *y_lo = nullptr; int64_t ldy = 0;
     float *part = nullptr; int max_slices = 1;
 };
-constexpr int FEW_MAX_ROWS = 256;
+// Five 128-row tiles: up to there the K slices and the folded reductions win over 128 x N tiles that leave SMs idle (config 2, 38 rows
+// x 16 tokens: 4% of a generate; a Qwen2 decode step of 300 rows 3.81 -> 2.31 ms, of 600 rows 5.10 -> 3.60); at 1216 rows they are even,
+// at 3000 they lose 10%.
+constexpr int FEW_MAX_ROWS = 640;
 bool gemm_few_supported(int64_t M, int N, int K);
 int gemm_few_slices(int M, int N, int K, int max_slices);      // slices gemm_few() will use for a call with `part`
 void gemm_few(const FewGemm &g);
