@@ -345,7 +345,8 @@ void make_gated_interleaved(BlockWeights &w, int C, std::vector<void *> &owned);
 Tensor *wget(WeightStore *ws, const char *fmt, ...);      // null when missing
 Tensor *wneed(WeightStore *ws, const char *fmt, ...);     // fatal when missing
 float *dev_concat_rows(const float *a, int64_t na, const float *b, int64_t nb);   // new buffer [na+nb]; null parts -> zeros
-void upload(void *dev, const void *host, size_t bytes);
+void upload(void *dev, const void *host, size_t bytes);          // done on return
+void upload_queued(void *dev, const void *host, size_t bytes);   // in order on stream(); host may be reused on return
 void *dev_alloc(size_t bytes);
 void dev_free(void *p);
 

@@ -367,14 +367,14 @@ void lm_setup(LMRun &r, const int *prompts, int n_new, int64_t logit_rows) {
     for (int b = 0; b <= B; b++) { st[b] = b * np; s1[b] = b; ks[b] = b * cap; }
     for (int s = 0; s < cap; s++) for (int b = 0; b < B; b++) { pm[(size_t)s * B + b] = s; lm[(size_t)s * B + b] = s + 1; }
     for (int b = 0; b < B; b++) lr[b] = b * np + np - 1;
-    upload(r.ids_d, prompts, (size_t)B * np * 4);
-    upload(r.pos_d, pos.data(), pos.size() * 4);
-    upload(r.start_np, st.data(), st.size() * 4);
-    upload(r.start_1, s1.data(), s1.size() * 4);
-    upload(r.kstart, ks.data(), ks.size() * 4);
-    upload(r.posmat, pm.data(), pm.size() * 4);
-    upload(r.lenmat, lm.data(), lm.size() * 4);
-    upload(r.last_rows, lr.data(), lr.size() * 4);
+    upload_queued(r.ids_d, prompts, (size_t)B * np * 4);
+    upload_queued(r.pos_d, pos.data(), pos.size() * 4);
+    upload_queued(r.start_np, st.data(), st.size() * 4);
+    upload_queued(r.start_1, s1.data(), s1.size() * 4);
+    upload_queued(r.kstart, ks.data(), ks.size() * 4);
+    upload_queued(r.posmat, pm.data(), pm.size() * 4);
+    upload_queued(r.lenmat, lm.data(), lm.size() * 4);
+    upload_queued(r.last_rows, lr.data(), lr.size() * 4);
 }
 
 // greedy pick over a long vocabulary row on many CTAs: block-local first-index argmax, then one atomicMax per
@@ -462,7 +462,7 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
             double v = (double)(rng_next(&st) >> 11) * (1.0 / 9007199254740992.0);
             for (int b = 0; b < B; b++) u[(size_t)s * B + b] = v;
         }
-        upload(r.uni_d, u.data(), u.size() * 8);
+        upload_queued(r.uni_d, u.data(), u.size() * 8);
     }
     CUDA_CHECK(cudaMemsetAsync(r.step_d, 0, 4 * sizeof(int), stream()));
     CUDA_CHECK(cudaMemsetAsync(r.amax_d, 0, (size_t)B * 8, stream()));
@@ -490,7 +490,7 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
             const BlockWeights &bw = m->blocks[li];
             hl[li] = MegaLayer{bw.ln1w, bw.ln1b, bw.qkvb, bw.ob, bw.ln2w, bw.ln2b, bw.fcb, bw.pb, r.kv[li]};
         }
-        upload(r.mg_layers, hl.data(), sizeof(MegaLayer) * hl.size());
+        upload_queued(r.mg_layers, hl.data(), sizeof(MegaLayer) * hl.size());
         CUDA_CHECK(cudaMemsetAsync(r.mg_ll, 0, lm_mega_exchange_words(ms) * sizeof(uint2), stream()));
         const NormSpec n1 = ln1_of(m->blocks[0]), nf = lm_last_norm(m);
         mg.s = ms; mg.norm = n1.kind; mg.eps = n1.eps; mg.eps_f = nf.eps; mg.act = m->blocks[0].act;
@@ -667,7 +667,7 @@ extern "C" void ncmb_lm_nll(NcmbLM *m, const int *ids, int B, int T, const int *
     lm_setup(r, clean.data(), 0, chunk);
     int *tgt_d = r.tgt_d;
     double *nll_d = r.nll_d;
-    upload(tgt_d, tgt.data(), (size_t)n * 4);
+    upload_queued(tgt_d, tgt.data(), (size_t)n * 4);
     lm_prefill(r);
     for (int64_t r0 = 0; r0 < n; r0 += chunk) {
         const int64_t rows = n - r0 < chunk ? n - r0 : chunk;

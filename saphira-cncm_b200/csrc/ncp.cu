@@ -487,20 +487,20 @@ static void gen_plan(NCPGen *g, const int *l0, const int *prefix_ids, const doub
         m->work.reset();
         layout(m->work);
     }
-    upload(g->row_start_d, row_start.data(), (size_t)(Bm + 1) * 4);
-    upload(g->tok_pos_d, tok_pos.data(), (size_t)g->ntok * 4);
-    upload(g->tok_src_d, tok_id.data(), (size_t)g->ntok * 4);
+    upload_queued(g->row_start_d, row_start.data(), (size_t)(Bm + 1) * 4);
+    upload_queued(g->tok_pos_d, tok_pos.data(), (size_t)g->ntok * 4);
+    upload_queued(g->tok_src_d, tok_id.data(), (size_t)g->ntok * 4);
     // per-level uniform row starts and rotary positions (P + t)
     for (int k = 0; k < nlev; k++) {
         int Lk = c->levels[k];
         std::vector<int> st(Bm + 1), ps((size_t)Bm * Lk);
         for (int b = 0; b <= Bm; b++) st[b] = b * Lk;
         for (int b = 0; b < Bm; b++) for (int t = 0; t < Lk; t++) ps[(size_t)b * Lk + t] = P + t;
-        upload((void *)g->lev_start_d[k], st.data(), st.size() * 4);
-        upload(g->lev_pos_d[k], ps.data(), ps.size() * 4);
+        upload_queued((void *)g->lev_start_d[k], st.data(), st.size() * 4);
+        upload_queued(g->lev_pos_d[k], ps.data(), ps.size() * 4);
     }
-    if (g->uni_d) upload(g->uni_d, uni.data(), ndraw * 8);
-    if (g->allow_d) upload(g->allow_d, allow, (size_t)g->Vmax * 8);
+    if (g->uni_d) upload_queued(g->uni_d, uni.data(), ndraw * 8);
+    if (g->allow_d) upload_queued(g->allow_d, allow, (size_t)g->Vmax * 8);
     CUDA_CHECK(cudaMemsetAsync(g->z_hat, 0, nzl * 4, stream()));
     CUDA_CHECK(cudaMemsetAsync(g->cnt_d, 0, (size_t)Bm * g->Vmax * 8, stream()));
     CUDA_CHECK(cudaMemsetAsync(g->hist_len_d, 0, 2 * (size_t)Bm * 4, stream()));
@@ -509,7 +509,7 @@ static void gen_plan(NCPGen *g, const int *l0, const int *prefix_ids, const doub
         g->have_l0 = 1;
         std::vector<int> tmp((size_t)B * g->total, 0);
         for (int b = 0; b < B; b++) memcpy(&tmp[(size_t)b * g->total], l0 + (size_t)b * l0len, (size_t)l0len * 4);
-        upload(g->codes_d, tmp.data(), tmp.size() * 4);
+        upload_queued(g->codes_d, tmp.data(), tmp.size() * 4);
     }
     if (g->cap_host) {
         g->cap_row = 0;
@@ -839,7 +839,7 @@ void ncp_forward(NCPState *m, const float *x, const int *prefix_ids, float *logi
         mem_d2h(rs.data(), g->row_start_d, rs.size() * 4);
         mem_d2h(pos.data(), g->tok_pos_d, pos.size() * 4);
         for (int b = 0; b < B; b++) for (int i = rs[b]; i < rs[b + 1]; i++) src[i] = b * S + pos[i];
-        upload(g->tok_src_d, src.data(), src.size() * 4);
+        upload_queued(g->tok_src_d, src.data(), src.size() * 4);
         float *zpre = g->bufs.h;
         embed_rows(x, g->tok_src_d, zpre, g->ntok, D);
         GemmArgs a;

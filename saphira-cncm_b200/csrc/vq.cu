@@ -265,7 +265,7 @@ int *vq_codes_to_dev(VQState *v, const int *host, size_t n) {
     v->codes_ws.reserve(n * sizeof(int) + 256);
     v->codes_ws.reset();
     int *d = v->codes_ws.get<int>(n);
-    upload(d, host, n * sizeof(int));
+    upload_queued(d, host, n * sizeof(int));
     return d;
 }
 

@@ -184,7 +184,7 @@ void vqvae_encode_z(VQVAEState *v, const int *ids, float *z, int B) {
     float *x = v->work.get<float>(n * D);
     float *t1 = v->work.get<float>(n * D), *t2 = v->work.get<float>(n * D);
     BlockBufs bufs = vae_bufs(v->work, n, D, Hh);
-    upload(ids_dev, ids, (size_t)n * sizeof(int));
+    upload_queued(ids_dev, ids, (size_t)n * sizeof(int));
     if (c->enc_conv_layers == 0 && c->vq_compression <= 1 && c->pre_quant_groupnorm <= 0 && vae_stack_supported(v->enc, D, c->vq_n_layers, T, c->enc_attn_window)) {
         VaeStackIO io;
         io.ids = ids_dev; io.wte = v->enc_wte; io.wpe = c->enc_positional ? v->enc_wpe : nullptr; io.y = z;
