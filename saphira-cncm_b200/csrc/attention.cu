@@ -18,8 +18,6 @@ namespace ncmb {
 
 constexpr int AT_KT = 64;      // keys per shared-memory tile
 constexpr int AT_WARPS = 4;
-constexpr int AT_QW = 8;       // queries per warp
-constexpr int AT_QT = AT_WARPS * AT_QW;
 
 struct AttnDev {
     const float *q; int64_t ldq;
@@ -32,19 +30,20 @@ struct AttnDev {
     float scale;
 };
 
-template <int HD>
+template <int HD, int QW>
 __global__ void __launch_bounds__(AT_WARPS * 32) k_attention(AttnDev a) {
-    constexpr int LDK = HD + 4;
+    constexpr int LDK = HD + 4, QT = AT_WARPS * QW;
     constexpr int DPL = (HD + 31) / 32;          // output dims per lane
     extern __shared__ __align__(16) float smem[];
     float *Ks = smem;                             // [AT_KT][LDK]
     float *Vs = Ks + AT_KT * LDK;                 // [AT_KT][HD]
-    float *Qs = Vs + AT_KT * HD;                  // [AT_QT][HD]
-    float *Ps = Qs + AT_QT * HD;                  // [AT_WARPS][AT_QW][AT_KT]
+    float *Qs = Vs + AT_KT * HD;                  // [QT][HD]
+    float *Ps = Qs + QT * HD;                  // [AT_WARPS][QW][AT_KT]
 
+    pdl_wait();
     const int row = blockIdx.z, h = blockIdx.y, qt = blockIdx.x;
     const int q0 = a.q_start[row], nq = a.q_start[row + 1] - q0;
-    if (qt * AT_QT >= nq) return;
+    if (qt * QT >= nq) return;
     const int k10 = a.k1_start[row], n1 = a.k1_len ? a.k1_len[row] : a.k1_start[row + 1] - k10;
     const int k20 = a.k2_start ? a.k2_start[row] : 0;
     const int n2 = a.k2_start ? a.k2_start[row + 1] - k20 : 0;
@@ -53,50 +52,71 @@ __global__ void __launch_bounds__(AT_WARPS * 32) k_attention(AttnDev a) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     // stage this block's queries (pre-scaled by nothing; the scale is applied to the score)
-    for (int i = tid; i < AT_QT * (HD / 4); i += AT_WARPS * 32) {
+    for (int i = tid; i < QT * (HD / 4); i += AT_WARPS * 32) {
         int t = i / (HD / 4), d4 = i % (HD / 4);
-        int qi = qt * AT_QT + t;
+        int qi = qt * QT + t;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (qi < nq) v = *(const float4 *)(a.q + (int64_t)(q0 + qi) * a.ldq + h * HD + d4 * 4);
         *(float4 *)(Qs + t * HD + d4 * 4) = v;
     }
-    float m[AT_QW], l[AT_QW], o[AT_QW][DPL];
+    float m[QW], l[QW], o[QW][DPL];
 #pragma unroll
-    for (int t = 0; t < AT_QW; t++) {
+    for (int t = 0; t < QW; t++) {
         m[t] = -INFINITY; l[t] = 0.f;
 #pragma unroll
         for (int i = 0; i < DPL; i++) o[t][i] = 0.f;
     }
-    float *Pw = Ps + warp * AT_QW * AT_KT;
+    float *Pw = Ps + warp * QW * AT_KT;
 
+    // A tile's keys and values are requested a tile ahead, into registers, where these suffice: with one short row the loads' way
+    // from L2 was most of a tile's time (config 1, one sequence, 290 keys: 13.1 -> 6.4 us a launch with two queries a warp).
+    constexpr int NT = AT_WARPS * 32, NPF = AT_KT * (HD / 4) / NT;
+    constexpr bool AHEAD = NPF <= 4 && AT_KT * (HD / 4) % NT == 0;
+    float4 kpf[AHEAD ? NPF : 1], vpf[AHEAD ? NPF : 1];
+    auto load = [&](int j, int d4, float4 &kv, float4 &vv) {
+        kv = vv = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j >= nk) return;
+        const float *kp, *vp;
+        if (j < n1) { int64_t tok = k10 + j; kp = a.k1 + tok * a.ldk1; vp = a.v1 + tok * a.ldk1; }
+        else { int64_t tok = k20 + (j - n1); kp = a.k2 + tok * a.ldk2; vp = a.v2 + tok * a.ldk2; }
+        kv = *(const float4 *)(kp + kvh * HD + d4 * 4);
+        vv = *(const float4 *)(vp + kvh * HD + d4 * 4);
+    };
+    auto ahead = [&](int kt0) {
+#pragma unroll
+        for (int u = 0; u < (AHEAD ? NPF : 0); u++) { const int i = tid + u * NT; load(kt0 + i / (HD / 4), i % (HD / 4), kpf[u], vpf[u]); }
+    };
+    if (AHEAD) ahead(0);
     for (int kt0 = 0; kt0 < nk; kt0 += AT_KT) {
         __syncthreads();                           // previous tile fully consumed (and Qs visible)
-        for (int i = tid; i < AT_KT * (HD / 4); i += AT_WARPS * 32) {
-            int r = i / (HD / 4), d4 = i % (HD / 4);
-            int j = kt0 + r;
-            float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-            if (j < nk) {
-                const float *kp, *vp;
-                if (j < n1) { int64_t tok = k10 + j; kp = a.k1 + tok * a.ldk1; vp = a.v1 + tok * a.ldk1; }
-                else { int64_t tok = k20 + (j - n1); kp = a.k2 + tok * a.ldk2; vp = a.v2 + tok * a.ldk2; }
-                kv = *(const float4 *)(kp + kvh * HD + d4 * 4);
-                vv = *(const float4 *)(vp + kvh * HD + d4 * 4);
-            }
-            *(float4 *)(Ks + r * LDK + d4 * 4) = kv;
-            *(float4 *)(Vs + r * HD + d4 * 4) = vv;
-        }
-        __syncthreads();
-        // scores: lane owns keys (lane, lane + 32) of the tile, for the warp's AT_QW queries
-        float s0[AT_QW], s1[AT_QW];
+        if (AHEAD) {
 #pragma unroll
-        for (int t = 0; t < AT_QW; t++) { s0[t] = 0.f; s1[t] = 0.f; }
+            for (int u = 0; u < (AHEAD ? NPF : 0); u++) {
+                const int i = tid + u * NT, r = i / (HD / 4), d4 = i % (HD / 4);
+                *(float4 *)(Ks + r * LDK + d4 * 4) = kpf[u];
+                *(float4 *)(Vs + r * HD + d4 * 4) = vpf[u];
+            }
+            ahead(kt0 + AT_KT);
+        } else
+            for (int i = tid; i < AT_KT * (HD / 4); i += NT) {
+                const int r = i / (HD / 4), d4 = i % (HD / 4);
+                float4 kv, vv;
+                load(kt0 + r, d4, kv, vv);
+                *(float4 *)(Ks + r * LDK + d4 * 4) = kv;
+                *(float4 *)(Vs + r * HD + d4 * 4) = vv;
+            }
+        __syncthreads();
+        // scores: lane owns keys (lane, lane + 32) of the tile, for the warp's QW queries
+        float s0[QW], s1[QW];
+#pragma unroll
+        for (int t = 0; t < QW; t++) { s0[t] = 0.f; s1[t] = 0.f; }
 #pragma unroll 4
         for (int d4 = 0; d4 < HD / 4; d4++) {
             float4 ka = *(const float4 *)(Ks + lane * LDK + d4 * 4);
             float4 kb = *(const float4 *)(Ks + (lane + 32) * LDK + d4 * 4);
 #pragma unroll
-            for (int t = 0; t < AT_QW; t++) {
-                float4 qv = *(const float4 *)(Qs + (warp * AT_QW + t) * HD + d4 * 4);
+            for (int t = 0; t < QW; t++) {
+                float4 qv = *(const float4 *)(Qs + (warp * QW + t) * HD + d4 * 4);
                 s0[t] = fmaf(qv.x, ka.x, s0[t]); s0[t] = fmaf(qv.y, ka.y, s0[t]);
                 s0[t] = fmaf(qv.z, ka.z, s0[t]); s0[t] = fmaf(qv.w, ka.w, s0[t]);
                 s1[t] = fmaf(qv.x, kb.x, s1[t]); s1[t] = fmaf(qv.y, kb.y, s1[t]);
@@ -105,8 +125,8 @@ __global__ void __launch_bounds__(AT_WARPS * 32) k_attention(AttnDev a) {
         }
         const int ja = kt0 + lane, jb = kt0 + lane + 32;
 #pragma unroll
-        for (int t = 0; t < AT_QW; t++) {
-            int qi = qt * AT_QT + warp * AT_QW + t;
+        for (int t = 0; t < QW; t++) {
+            int qi = qt * QT + warp * QW + t;
             bool va = ja < nk, vb = jb < nk;
             if (a.causal) {                        // applies to segment-1 keys only
                 if (ja < n1 && ja > qi + a.causal_off) va = false;
@@ -154,7 +174,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32) k_attention(AttnDev a) {
                     vv[jj][i] = (d < HD) ? Vs[(j4 + jj) * HD + d] : 0.f;   // rows beyond nk hold zeros
                 }
 #pragma unroll
-            for (int t = 0; t < AT_QW; t++) {
+            for (int t = 0; t < QW; t++) {
                 float4 p = *(const float4 *)(Pw + t * AT_KT + j4);
 #pragma unroll
                 for (int i = 0; i < DPL; i++) {
@@ -166,8 +186,8 @@ __global__ void __launch_bounds__(AT_WARPS * 32) k_attention(AttnDev a) {
         __syncwarp();
     }
 #pragma unroll
-    for (int t = 0; t < AT_QW; t++) {
-        int qi = qt * AT_QT + warp * AT_QW + t;
+    for (int t = 0; t < QW; t++) {
+        int qi = qt * QT + warp * QW + t;
         if (qi >= nq) continue;
         float inv = l[t] > 0.f ? 1.0f / l[t] : 0.f;
 #pragma unroll
@@ -183,16 +203,24 @@ __global__ void __launch_bounds__(AT_WARPS * 32) k_attention(AttnDev a) {
     }
 }
 
-template <int HD>
-static void launch_attention(const AttnDev &d, dim3 grid) {
-    size_t smem = sizeof(float) * ((size_t)AT_KT * (HD + 4) + (size_t)AT_KT * HD + (size_t)AT_QT * HD +
-                                   (size_t)AT_WARPS * AT_QW * AT_KT);
+template <int HD, int QW>
+static void launch_attention_q(const AttnDev &d, dim3 grid) {
+    size_t smem = sizeof(float) * ((size_t)AT_KT * (HD + 4) + (size_t)AT_KT * HD + (size_t)AT_WARPS * QW * HD +
+                                   (size_t)AT_WARPS * QW * AT_KT);
     static bool set = false;
     if (!set) {
-        CUDA_CHECK(cudaFuncSetAttribute(k_attention<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CUDA_CHECK(cudaFuncSetAttribute((k_attention<HD, QW>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         set = true;
     }
-    LAUNCH(k_attention<HD>, grid, AT_WARPS * 32, smem, d);
+    LAUNCH_PDL((k_attention<HD, QW>), grid, AT_WARPS * 32, smem, d);
+}
+// Eight queries a warp share every key they read; two where eight would leave most SMs idle (one sequence's level: the warps' serial
+// work, not the reads, is then the launch).
+template <int HD>
+static void launch_attention(const AttnDev &d, int rows, int max_q) {
+    const dim3 grid((unsigned)cdiv(max_q, AT_WARPS * 8), (unsigned)d.H, (unsigned)rows);
+    if ((int64_t)grid.x * grid.y * grid.z * 2 <= ctx().sm_count) launch_attention_q<HD, 2>(d, dim3((unsigned)cdiv(max_q, AT_WARPS * 2), grid.y, grid.z));
+    else launch_attention_q<HD, 8>(d, grid);
 }
 
 void attention(const AttnArgs &a) {
@@ -209,14 +237,13 @@ void attention(const AttnArgs &a) {
     d.causal = a.causal; d.causal_off = a.causal_off; d.window = a.window;
     d.scale = 1.0f / sqrtf((float)a.hd);
     if ((a.ldq | a.ldk1 | a.ldk2 | a.ldo) % 4) fatal("attention: row strides must be multiples of 4 floats");
-    dim3 grid((unsigned)cdiv(a.max_q, AT_QT), (unsigned)a.H, (unsigned)a.rows);
     ProfScope ps(NCMB_K_ATTN, 4.0 * (double)a.total_q * a.avg_keys * a.H * a.hd, 0);
     switch (a.hd) {
-        case 8: launch_attention<8>(d, grid); break;
-        case 16: launch_attention<16>(d, grid); break;
-        case 32: launch_attention<32>(d, grid); break;
-        case 64: launch_attention<64>(d, grid); break;
-        case 128: launch_attention<128>(d, grid); break;
+        case 8: launch_attention<8>(d, a.rows, a.max_q); break;
+        case 16: launch_attention<16>(d, a.rows, a.max_q); break;
+        case 32: launch_attention<32>(d, a.rows, a.max_q); break;
+        case 64: launch_attention<64>(d, a.rows, a.max_q); break;
+        case 128: launch_attention<128>(d, a.rows, a.max_q); break;
         default: fatal("attention: head dim %d not supported (8, 16, 32, 64, 128)", a.hd);
     }
 }
