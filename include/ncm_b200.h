@@ -386,6 +386,9 @@ int    ncmb_lm_vocab(const NcmbLM *m);
 /* Decode steps of one sequence (head dim 64) run as ONE persistent cooperative kernel instead of a replayed chain
  * of kernels; 0 turns that off. Results agree within fp32 rounding either way. No counterpart in the reference. */
 void  ncmb_set_lm_persistent(int on);
+/* The most 8 KB chunks of its weights that such a step holds in shared memory at once on `sms` SMs (it has 16), or 0
+ * for a shape it does not take. Host arithmetic: needs no GPU. */
+int   ncmb_lm_persistent_ring(int C, int n_kv, int I, int n_layer, int V, int gated, int elem_bytes, int sms);
 /* prompts: host int[B][np]; out: host int[B][n_new]; eos < 0 disables stopping.
  * Returns the number of ids generated per row (n_new unless every row hit eos). */
 int    ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, int n_new,

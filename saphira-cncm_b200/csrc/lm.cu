@@ -192,6 +192,9 @@ extern "C" void ncmb_lm_close(NcmbLM *m) {
 }
 extern "C" int ncmb_lm_vocab(const NcmbLM *m) { return m->V; }
 extern "C" void ncmb_set_lm_persistent(int on) { lm_mega_enable(on); }
+extern "C" int ncmb_lm_persistent_ring(int C, int n_kv, int I, int n_layer, int V, int gated, int elem_bytes, int sms) {
+    return lm_mega_ring_need(MegaShape{1, C, C / 64, n_kv, I, n_layer, V, gated}, elem_bytes, sms);
+}
 
 namespace {
 

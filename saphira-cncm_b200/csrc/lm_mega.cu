@@ -34,6 +34,12 @@ constexpr int MS_CH = 8192, MS_SLOTS = 16, MS_RING = MS_CH * MS_SLOTS;
 constexpr int MS_MAXC = 1024, MS_MAXI = 8192, MS_MAXNL = 256, MS_MAXSPLIT = 4, MS_PW = 66;       // words of an attention partial: max, sum, context
 constexpr int MS_UPROWS = 128, MS_HROWS = 64;            // rows a CTA may have of an up-projection; vocabulary rows per round
 
+// Rows of `rowb` bytes that may be in use at once: wherever in a chunk the first of them starts, they and what shares their chunks fit
+// the ring. What needs more rows than that gives the first ones back in between, or the stream would wait for itself.
+__host__ __device__ constexpr int ms_hold(long long rowb) { return (int)((MS_RING - MS_CH) / rowb); }
+constexpr int MS_RGRP = 32;                              // rows of a [..][C] product in use at once: four groups of warps x eight rows
+static_assert(ms_hold((long long)MS_MAXI * 4) >= 1, "a down-projection row has to fit the ring");
+
 // contiguous share of n items for CTA c of g
 __host__ __device__ __forceinline__ int ms_begin(int n, int c, int g) { return (int)((long long)n * c / g); }
 
@@ -172,9 +178,9 @@ __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long 
         xr[e] = v.x; xr[e + 1] = v.y; xr[e + 2] = v.z; xr[e + 3] = v.w;
     }
     const uint32_t rb = (uint32_t)rowb, at = (uint32_t)(base & (MS_RING - 1)) + (uint32_t)lo + rg * rb;
-    for (int b0 = 0; b0 < n; b0 += 32) {
+    for (int b0 = 0; b0 < n; b0 += MS_RGRP) {
         if (b0 > 0) { ms_bar(); st.release(base + (long long)b0 * rowb, warp, lane); }
-        st.ensure(c, base + (long long)min(n, b0 + 32) * rowb, lane);
+        st.ensure(c, base + (long long)min(n, b0 + MS_RGRP) * rowb, lane);
         const int i0 = b0 + rg;
         float acc[8];
 #pragma unroll
@@ -196,12 +202,14 @@ __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long 
 }
 
 // Down-projection rows [r0, r0 + n), n <= 8: the warp takes 256-wide pieces `warp`, `warp + 16` of K, whose inputs its lanes poll
-// straight into registers; part[row][warp].
+// straight into registers; part[row][warp]. Rows that do not fit the ring together (seven of the Qwen2-0.5B shape in fp32 are 136 KB) are
+// given back in groups.
 template <bool W16>
 __device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long base, int n, int I, const uint2 *hw, unsigned tag, float *part, int warp, int lane) {
     const int esz = W16 ? 2 : 4;
     const long long rowb = (long long)I * esz;
     const uint32_t at = (uint32_t)(base & (MS_RING - 1)), rb = (uint32_t)rowb;
+    const int hold = ms_hold(rowb);
     float acc[8], xr[2][8];
 #pragma unroll
     for (int j = 0; j < 8; j++) acc[j] = 0.f;
@@ -217,10 +225,12 @@ __device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long 
 #pragma unroll
         for (int i = 0; i < 8; i++) { xr[i >> 2][2 * (i & 3)] = v[i].x; xr[i >> 2][2 * (i & 3) + 1] = v[i].y; }
     }
+    int g0 = 0;                                              // first row of the group in use
 #pragma unroll
     for (int r = 0; r < 8; r++) {
         if (r >= n) break;
-        if ((r & 3) == 0) st.ensure(c, base + min(r + 4, n) * rowb, lane);
+        if (r == g0 + hold) { ms_bar(); st.release(base + r * rowb, warp, lane); g0 = r; }
+        if (r == g0 || (r & 3) == 0) st.ensure(c, base + min(min(r + 4, n), g0 + hold) * rowb, lane);
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int k = (warp + MS_WARPS * u) * 256 + lane * 8;
@@ -581,11 +591,41 @@ bool lm_mega_enabled() {
     if (g_lm_persistent < 0) { const char *e = getenv("NCM_B200_LM_PERSISTENT"); g_lm_persistent = e ? atoi(e) != 0 : 1; }
     return g_lm_persistent == 1;
 }
-bool lm_mega_supported(const MegaShape &s, int hd, bool qk_norm) {
-    const int g = ctx().sm_count;
+static bool shape_fits(const MegaShape &s, int hd, bool qk_norm, int g) {
     return s.B == 1 && hd == 64 && s.C == s.H * 64 && s.C % 32 == 0 && s.C <= MS_MAXC && s.I % 8 == 0 && s.I <= MS_MAXI && !qk_norm &&
            s.H % s.nkv == 0 && s.H <= g && cdiv(s.C, g) <= 8 && 2 * cdiv(s.I, g) <= MS_UPROWS && cdiv(s.C + 128 * s.nkv, g) + 2 <= MS_UPROWS &&
-           (int64_t)s.C * 4 * 32 + 2 * MS_CH <= MS_RING && s.NL <= MS_MAXNL && (int64_t)s.I * 4 + 2 * MS_CH <= MS_RING;
+           (int64_t)s.C * 4 * MS_RGRP + 2 * MS_CH <= MS_RING && s.NL <= MS_MAXNL;
+}
+bool lm_mega_supported(const MegaShape &s, int hd, bool qk_norm) { return shape_fits(s, hd, qk_norm, ctx().sm_count); }
+
+// The most chunks between what a CTA of g has given back and what it waits for, over the products of a step in the kernel's order (layers
+// repeat at other offsets within a chunk); with more than MS_SLOTS the stream waits for a release that comes later. 0: not a shape of
+// the kernel.
+int lm_mega_ring_need(const MegaShape &s, int esz, int g) {
+    if (!shape_fits(s, 64, false, g)) return 0;
+    long long need = 0;
+    for (int c = 0; c < g; c++) {
+        auto share = [&](int n) { return ms_begin(n, c + 1, g) - ms_begin(n, c, g); };
+        long long at = 0, rel = 0;
+        auto product = [&](int n, int K, int group) {
+            const long long rowb = (long long)K * esz;
+            for (int r = 0; r < n; r += group) {
+                rel = (at + r * rowb) / MS_CH;
+                need = std::max(need, (at + std::min(n, r + group) * rowb + MS_CH - 1) / MS_CH - rel);
+            }
+            at += n * rowb;
+        };
+        const int ncr = share(s.C);
+        for (int li = 0; li < s.NL; li++) {
+            product(2 * share((s.C + 128 * s.nkv) >> 1), s.C, MS_RGRP);
+            product(ncr, s.C, MS_RGRP);
+            product((s.gated ? 2 : 1) * share(s.I), s.C, MS_RGRP);
+            product(ncr, s.I, ms_hold((long long)s.I * esz));
+        }
+        at = (at + MS_CH - 1) / MS_CH * MS_CH;
+        product(share(s.V), s.C, MS_RGRP);
+    }
+    return (int)need;
 }
 
 void lm_mega_free(MegaModel &m) {

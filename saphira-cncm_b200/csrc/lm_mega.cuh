@@ -17,6 +17,7 @@ struct MegaModel {
 };
 struct MegaShape { int B, C, H, nkv, I, NL, V; int gated; };
 bool lm_mega_supported(const MegaShape &s, int hd, bool qk_norm);
+int lm_mega_ring_need(const MegaShape &s, int esz, int g);       // host arithmetic only
 void lm_mega_pack(MegaModel &m, const MegaShape &s, const std::vector<BlockWeights> &blocks, const float *wte, const unsigned short *wte16);
 void lm_mega_free(MegaModel &m);
 
