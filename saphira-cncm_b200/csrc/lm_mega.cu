@@ -11,7 +11,8 @@
 //     {value, tag}, written with one store and polled by whoever needs them; the tag is the layer's number in the generate, so
 //     a word says itself whether it has arrived. That is one trip through L2 per hop instead of fence, barrier and read.
 //     A buffer is written again one layer later, which cannot happen before every CTA has read it: the new value depends, by
-//     way of the MLP that all CTAs take part in, on results each of them produced after its read.
+//     way of the MLP that all CTAs take part in (I >= the number of CTAs), on results each of them produced after its read. The
+//     MLP's own results are read by the CTAs that own hidden rows only, and the next ones depend on those rows.
 //   * Products. Sixteen warps: four quarters of K x four groups of rows. A lane keeps its eight elements of the input in
 //     registers; eight rows at a time meet in a reduce-scatter.
 //
@@ -203,9 +204,10 @@ __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long 
 
 // Down-projection rows [r0, r0 + n), n <= 8: the warp takes 256-wide pieces `warp`, `warp + 16` of K, whose inputs its lanes poll
 // straight into registers; part[row][warp]. Rows that do not fit the ring together (seven of the Qwen2-0.5B shape in fp32 are 136 KB) are
-// given back in groups.
+// given back in groups. A CTA without rows does not wait for the inputs: nothing that it writes would keep them from being overwritten.
 template <bool W16>
 __device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long base, int n, int I, const uint2 *hw, unsigned tag, float *part, int warp, int lane) {
+    if (n == 0) return;
     const int esz = W16 ? 2 : 4;
     const long long rowb = (long long)I * esz;
     const uint32_t at = (uint32_t)(base & (MS_RING - 1)), rb = (uint32_t)rowb;
@@ -592,7 +594,7 @@ bool lm_mega_enabled() {
     return g_lm_persistent == 1;
 }
 static bool shape_fits(const MegaShape &s, int hd, bool qk_norm, int g) {
-    return s.B == 1 && hd == 64 && s.C == s.H * 64 && s.C % 32 == 0 && s.C <= MS_MAXC && s.I % 8 == 0 && s.I <= MS_MAXI && !qk_norm &&
+    return s.B == 1 && hd == 64 && s.C == s.H * 64 && s.C % 32 == 0 && s.C <= MS_MAXC && s.I % 8 == 0 && s.I >= g && s.I <= MS_MAXI && !qk_norm &&
            s.H % s.nkv == 0 && s.H <= g && cdiv(s.C, g) <= 8 && 2 * cdiv(s.I, g) <= MS_UPROWS && cdiv(s.C + 128 * s.nkv, g) + 2 <= MS_UPROWS &&
            (int64_t)s.C * 4 * MS_RGRP + 2 * MS_CH <= MS_RING && s.NL <= MS_MAXNL;
 }

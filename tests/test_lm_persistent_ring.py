@@ -22,3 +22,14 @@ def test_no_accepted_shape_needs_more_than_the_ring():
                     assert need <= RING_CHUNKS, (C, inner, kv, gated, esz, sms, need)
                     taken += need > 0
     assert taken > 400
+
+
+def test_every_block_of_the_step_owns_mlp_rows():
+    """An exchange buffer is free to be written again because each block has since given the MLP something it computed after its
+    read; a block without MLP rows could still be waiting for what is overwritten."""
+    import capi
+    lib = capi.NcmLib(helpers.CUDA_LIB)
+    for sms in (132, 148, 160):
+        for inner in range(8, 320, 8):
+            need = lib.ncmb_lm_persistent_ring(192, 3, inner, 3, 301, 0, 4, sms)
+            assert (need > 0) == (inner >= sms), (sms, inner)
