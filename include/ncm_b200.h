@@ -278,6 +278,8 @@ int   ncmb_get_gemm_mode(void);
 /* The tensor-core kernels bound every barrier wait; when one runs out they record a
  * code and drain. Returns and clears that code (0 = never happened); synchronises. */
 int   ncmb_gemm_tc_check(void);
+/* Diagnostic: records `code` as a wait that ran out would, so that a caller's handling of it can be tested. */
+void  ncmb_gemm_tc_raise(int code);
 /* Entries the TMA descriptor caches keep before they start over (default 4096; diagnostic: tests
  * set 1 so that every lookup evicts the one before it). No counterpart in the reference. */
 void  ncmb_set_map_cache_limit(int entries);
@@ -390,7 +392,8 @@ void  ncmb_set_lm_persistent(int on);
  * for a shape it does not take. Host arithmetic: needs no GPU. */
 int   ncmb_lm_persistent_ring(int C, int n_kv, int I, int n_layer, int V, int gated, int elem_bytes, int sms);
 /* prompts: host int[B][np]; out: host int[B][n_new]; eos < 0 disables stopping.
- * Returns the number of ids generated per row (n_new unless every row hit eos). */
+ * Returns the number of ids generated per row (n_new unless every row hit eos); -1, with every id -1, when a bounded
+ * wait of a kernel ran out since the error word was last read (ncmb_gemm_tc_check reads and clears it too). */
 int    ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, int n_new,
                         float temp, int top_k, float top_p, unsigned long long seed,
                         int eos, int *out);

@@ -192,6 +192,7 @@ void gemm_h3_forget_range(const void *p, size_t bytes);     // cached copies of 
 void gemm_tc_forget_range(const void *p, size_t bytes);
 struct StaticWeights { StaticWeights() { ctx().w_static++; } ~StaticWeights() { ctx().w_static--; } };
 int gemm_tc_check();                    // reads + clears the tensor-core engine's timeout word
+void gemm_tc_raise(int code);           // sets it, as a wait that ran out does
 
 // ---- normalisation / elementwise (kernels_elem.cu) ----
 void layernorm(const float *x, const float *w, const float *b, float *y, int64_t rows, int C, float eps);

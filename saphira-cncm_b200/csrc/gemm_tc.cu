@@ -264,6 +264,7 @@ int gemm_tc_check() {
     if (v) CUDA_CHECK(cudaMemsetAsync(d, 0, sizeof(int), stream()));
     return v;
 }
+void gemm_tc_raise(int code) { upload(tc_err_flag(), &code, sizeof(int)); }
 
 // ---- hi / lo split for the three-pass mode: hi = rn_tf32(x), lo = x - hi (exact in fp32) ----
 __global__ void k_split_tf32(const float *__restrict__ x, int64_t ldx, float *__restrict__ hi, float *__restrict__ lo,

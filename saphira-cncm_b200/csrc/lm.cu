@@ -551,6 +551,12 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
     }
     std::vector<int> tmp((size_t)B * n_new);
     mem_d2h(tmp.data(), r.out_d, tmp.size() * 4);
+    // a bounded wait of a kernel that ran out: what came after it is not the model's
+    if (const int code = gemm_tc_check()) {
+        fprintf(stderr, "%s: a device wait ran out (code %d); no ids\n", m->is_qwen ? "qwen" : "gpt2", code);
+        std::fill(out, out + (size_t)B * n_new, -1);
+        return -1;
+    }
     for (int b = 0; b < B; b++) {
         bool ended = false;
         for (int s = 0; s < n_new; s++) {
@@ -714,7 +720,7 @@ static int lm_cmd_gen(const NCMConfig *c, const char *weights, const char *adir,
     std::vector<int> gen(n_new > 0 ? n_new : 1);
     int ngen = 0;
     if (n_new > 0) {
-        ncmb_lm_generate(m, ids.data(), 1, n, n_new, temp, top_k, top_p, seed, m->eos, gen.data());
+        if (ncmb_lm_generate(m, ids.data(), 1, n, n_new, temp, top_k, top_p, seed, m->eos, gen.data()) < 0) return 1;
         while (ngen < n_new && gen[ngen] >= 0) ngen++;
     }
     printf("ids:");

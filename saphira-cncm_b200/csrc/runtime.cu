@@ -659,6 +659,7 @@ void ncmb_sync(void) { ensure_device(); CUDA_CHECK(cudaStreamSynchronize(stream(
 void ncmb_set_gemm_mode(int mode) { ensure_device(); ctx().gemm_mode = mode; }
 int ncmb_get_gemm_mode(void) { ensure_device(); return ctx().gemm_mode; }
 int ncmb_gemm_tc_check(void) { ensure_device(); return gemm_tc_check(); }
+void ncmb_gemm_tc_raise(int code) { ensure_device(); gemm_tc_raise(code); }
 void ncmb_set_rng_mode(int mode) { ensure_device(); ctx().rng_mode = mode; }
 void ncmb_set_row_offset(long long off) { ctx().row_offset = off; }
 long long ncmb_launch_count(void) { return ctx().launches; }

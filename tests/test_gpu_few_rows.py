@@ -74,3 +74,21 @@ def test_one_row_whose_down_projection_rows_do_not_fit_the_ring_together(cuda, t
         want = om.generate(P[0], n_new, **kw)
         assert (out[0] == want).all(), (shape, kw, out[0], want)
     cuda.ncmb_lm_close(m)
+
+
+@pytest.mark.parametrize("B", [1, 3])
+def test_a_wait_that_ran_out_ends_a_generate_without_ids(cuda, models, B, capfd):
+    """The persistent step gives up at once when the error word is set and the chain's kernels run on; neither passes its ids on."""
+    import synth
+    spec, m, _ = models["qwen"]
+    cuda.ncmb_set_lm_persistent(1)
+    P = np.ascontiguousarray(synth.lm_prompts(spec, B, 35, 2))
+    out = np.zeros((B, 6), np.int32)
+    args = (m, P.ctypes.data, B, P.shape[1], 6, 0.0, 0, 1.0, 0, -1, out.ctypes.data)
+    assert cuda.ncmb_lm_generate(*args) == 6
+    want = out.copy()
+    cuda.ncmb_gemm_tc_raise(61)
+    assert cuda.ncmb_lm_generate(*args) == -1
+    assert (out == -1).all()
+    assert "code 61" in capfd.readouterr().err
+    assert cuda.ncmb_lm_generate(*args) == 6 and (out == want).all()       # the word is clear again
