@@ -399,6 +399,10 @@ int    ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, int n_new,
                         int eos, int *out);
 /* logits of one sequence: all positions ([T][V]) or the last one ([V]) to host */
 void   ncmb_lm_logits(NcmbLM *m, const int *ids, int T, int last_only, float *out_host);
+/* Logits of decode steps on given ids (the steps of ncmb_lm_generate, with a given id where it would feed back the one
+ * picked): ids host int[B][np + n_steps], of which the first np are the prompt; logits of the last n_last steps to
+ * host float[n_last][B][V]. 0, or -1 for bad arguments or when a bounded wait of a kernel ran out. */
+int    ncmb_lm_decode_logits(NcmbLM *m, const int *ids, int B, int np, int n_steps, int n_last, float *out_host);
 /* A Hugging Face .safetensors file straight into a WeightStore on the device, with the tensor rules of the
  * reference's offline converters (tools/gpt2import.c:385-417, tools/qwenimport.c:383-420, which write an NCM1
  * file instead): F16 / BF16 widened to fp32, "*.attn.bias" mask buffers dropped, names and order kept, and with

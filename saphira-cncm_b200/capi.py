@@ -154,6 +154,7 @@ _SIGS = {
     "ncmb_lm_vocab": (_I, [_P]),
     "ncmb_lm_generate": (_I, [_P, _P, _I, _I, _I, _F, _I, _F, _U64, _I, _P]),
     "ncmb_lm_persistent_ring": (_I, [_I] * 8),
+    "ncmb_lm_decode_logits": (_I, [_P, _P, _I, _I, _I, _I, _P]),
     "ncmb_lm_logits": (None, [_P, _P, _I, _I, _P]),
     "ncmb_lm_nll": (None, [_P, _P, _I, _I, _P, _P]),
     "ncmb_weights_import_safetensors": (_I, [C.POINTER(WeightStore), C.c_char_p, _I]),

@@ -446,6 +446,36 @@ void lm_sample(LMRun &r, float temp, int top_k, float top_p, int n_new) {
     LAUNCH_PDL(k_lm_finish_step, 1, 256, 0, r.pick_d, r.amax_d, greedy, r.B, n_new, r.out_d, r.ids_d, r.uni_d, r.uni_cur, r.step_d);
 }
 
+// One row (head dim 64): the whole decode step is one persistent cooperative kernel (lm_mega.cu); false where it does not apply.
+bool lm_mega_setup(LMRun &r, MegaArgs &mg) {
+    NcmbLM *m = r.m;
+    bool qk_norm = false;
+    for (auto &bw : m->blocks) qk_norm = qk_norm || bw.qnw || bw.knw;
+    const MegaShape ms = mega_shape(m, r.B);
+    if (!lm_mega_enabled() || !lm_mega_supported(ms, m->hd, qk_norm)) return false;
+    lm_mega_pack(m->mega, ms, m->blocks, m->wte, m->wte16);
+    std::vector<MegaLayer> hl(m->NL);
+    for (int li = 0; li < m->NL; li++) {
+        const BlockWeights &bw = m->blocks[li];
+        hl[li] = MegaLayer{bw.ln1w, bw.ln1b, bw.qkvb, bw.ob, bw.ln2w, bw.ln2b, bw.fcb, bw.pb, r.kv[li]};
+    }
+    upload_queued(r.mg_layers, hl.data(), sizeof(MegaLayer) * hl.size());
+    CUDA_CHECK(cudaMemsetAsync(r.mg_ll, 0, lm_mega_exchange_words(ms) * sizeof(uint2), stream()));
+    const NormSpec n1 = ln1_of(m->blocks[0]), nf = lm_last_norm(m);
+    mg.s = ms; mg.norm = n1.kind; mg.eps = n1.eps; mg.eps_f = nf.eps; mg.act = m->blocks[0].act;
+    mg.layers = r.mg_layers; mg.wte = m->wte; mg.wpe = m->is_qwen ? nullptr : m->wpe; mg.lnfw = nf.w; mg.lnfb = nf.b;
+    mg.cosb = m->cosb; mg.sinb = m->sinb; mg.logits = r.logits;
+    mg.ids = r.ids_d; mg.posmat = r.posmat; mg.step_d = r.step_d; mg.pos_base = r.np - 1;
+    mg.ll = r.mg_ll; mg.err = tc_err_flag();
+    return true;
+}
+
+// a decode step of the ids in r.ids_d, up to its logits
+void lm_step(LMRun &r, const MegaArgs *mg) {
+    if (mg) lm_mega_launch(r.m->mega, *mg);
+    else { lm_decode_step(r, r.ids_d); lm_head(r, r.x, r.B, r.logits, &r.few); }
+}
+
 } // namespace
 
 extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, int n_new,
@@ -480,28 +510,8 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
     // runs eagerly (it sizes every workspace), the second is captured, the rest are graph launches. The work
     // moves to a stream of its own for that, because the caller's stream may be the legacy default stream,
     // which cannot be captured.
-    // One row (head dim 64): the whole decode step is one persistent cooperative kernel (lm_mega.cu).
-    bool qk_norm = false;
-    for (auto &bw : m->blocks) qk_norm = qk_norm || bw.qnw || bw.knw;
-    const MegaShape ms = mega_shape(m, B);
-    const bool mega = lm_mega_enabled() && n_new >= 2 && lm_mega_supported(ms, m->hd, qk_norm);
     MegaArgs mg{};
-    if (mega) {
-        lm_mega_pack(m->mega, ms, m->blocks, m->wte, m->wte16);
-        std::vector<MegaLayer> hl(m->NL);
-        for (int li = 0; li < m->NL; li++) {
-            const BlockWeights &bw = m->blocks[li];
-            hl[li] = MegaLayer{bw.ln1w, bw.ln1b, bw.qkvb, bw.ob, bw.ln2w, bw.ln2b, bw.fcb, bw.pb, r.kv[li]};
-        }
-        upload_queued(r.mg_layers, hl.data(), sizeof(MegaLayer) * hl.size());
-        CUDA_CHECK(cudaMemsetAsync(r.mg_ll, 0, lm_mega_exchange_words(ms) * sizeof(uint2), stream()));
-        const NormSpec n1 = ln1_of(m->blocks[0]), nf = lm_last_norm(m);
-        mg.s = ms; mg.norm = n1.kind; mg.eps = n1.eps; mg.eps_f = nf.eps; mg.act = m->blocks[0].act;
-        mg.layers = r.mg_layers; mg.wte = m->wte; mg.wpe = m->is_qwen ? nullptr : m->wpe; mg.lnfw = nf.w; mg.lnfb = nf.b;
-        mg.cosb = m->cosb; mg.sinb = m->sinb; mg.logits = r.logits;
-        mg.ids = r.ids_d; mg.posmat = r.posmat; mg.step_d = r.step_d; mg.pos_base = np - 1;
-        mg.ll = r.mg_ll; mg.err = tc_err_flag();
-    }
+    const bool mega = n_new >= 2 && lm_mega_setup(r, mg);
     static const bool graphs_ok = !getenv("NCM_B200_NO_GRAPH");
     const bool use_graph = graphs_ok && eos < 0 && n_new >= 4 && !prof_enabled();
     cudaStream_t user = stream(), gs = nullptr;
@@ -529,8 +539,7 @@ extern "C" int ncmb_lm_generate(NcmbLM *m, const int *prompts, int B, int np, in
         const bool capture = use_graph && s == 1;
         long long l0 = ctx().launches;
         if (capture) CUDA_CHECK(cudaStreamBeginCapture(gs, cudaStreamCaptureModeThreadLocal));
-        if (mega) lm_mega_launch(m->mega, mg);
-        else { lm_decode_step(r, r.ids_d); lm_head(r, r.x, B, r.logits, &r.few); }
+        lm_step(r, mega ? &mg : nullptr);
         if (capture) {
             lm_sample(r, temp, top_k, top_p, n_new);
             CUDA_CHECK(cudaStreamEndCapture(gs, &graph));
@@ -585,6 +594,33 @@ extern "C" void ncmb_lm_logits(NcmbLM *m, const int *ids, int T, int last_only, 
         lm_head(r, r.x, T, r.logits);
         mem_d2h(out_host, r.logits, (size_t)T * m->V * 4);
     }
+}
+
+// Logits of decode steps on given ids: the steps of ncmb_lm_generate with the id a row has next in place of the id picked.
+extern "C" int ncmb_lm_decode_logits(NcmbLM *m, const int *ids, int B, int np, int n_steps, int n_last, float *out_host) {
+    ensure_device();
+    if (B <= 0 || np <= 0 || n_steps <= 0 || n_last <= 0 || n_last > n_steps) return -1;
+    StaticWeights sw;
+    if (np + n_steps > m->n_ctx) fatal("%s: context overflow (%d + %d > %d)", m->is_qwen ? "qwen" : "gpt2", np, n_steps, m->n_ctx);
+    const int T = np + n_steps;
+    std::vector<int> prompts((size_t)B * np), next((size_t)B);
+    for (int b = 0; b < B; b++) std::copy(ids + (size_t)b * T, ids + (size_t)b * T + np, prompts.begin() + (size_t)b * np);
+    LMRun r;
+    r.m = m; r.B = B; r.np = np; r.cap = T + 1;
+    lm_setup(r, prompts.data(), n_steps + 1, 0);
+    lm_prefill(r);
+    MegaArgs mg{};
+    const bool mega = lm_mega_setup(r, mg);
+    for (int s = 0; s < n_steps; s++) {
+        const int v = s + 1;                                   // ids finalised so far, as in ncmb_lm_generate
+        for (int b = 0; b < B; b++) next[b] = ids[(size_t)b * T + np + s];
+        upload_queued(r.ids_d, next.data(), (size_t)B * 4);
+        upload_queued(r.step_d, &v, 4);
+        lm_step(r, mega ? &mg : nullptr);
+        if (s >= n_steps - n_last) mem_d2h(out_host + (size_t)(s - (n_steps - n_last)) * B * m->V, r.logits, (size_t)B * m->V * 4);
+    }
+    CUDA_CHECK(cudaStreamSynchronize(stream()));
+    return gemm_tc_check() ? -1 : 0;
 }
 
 // ---------------------------------------------------------------------------------------------
