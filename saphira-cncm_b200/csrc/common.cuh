@@ -310,9 +310,9 @@ struct BlockWeights {
 // a norm as its consumer needs it: kind 0 none, 1 LayerNorm, 2 RMSNorm
 struct NormSpec { int kind = 0; const float *w = nullptr, *b = nullptr; float eps = 0.f; };
 static inline NormSpec ln1_of(const BlockWeights &w) { return NormSpec{w.norm == NORM_RMS ? 2 : 1, w.ln1w, w.norm == NORM_RMS ? nullptr : w.ln1b, w.norm == NORM_RMS ? 1e-6f : w.eps}; }
-// Few rows (gemm_few.cu): a chain of blocks hands the normed row over as an fp16 pair, because the kernel that closes a block
-// adds the slices of its last product and holds whole rows. `on` is set by the chain's owner; run_block() writes the pair of
-// `next` applied to its output and sets ready.
+// Few rows (gemm_few.cu): a chain of blocks hands the normed row over as an fp16 pair (y2 null: in fp32), because the kernel that closes
+// a block adds the slices of its last product and holds whole rows. `on` is set by the chain's owner; run_block() writes `next`
+// applied to its output and sets ready.
 struct FewChain { bool on = false, ready = false; NormSpec next; void *y1 = nullptr, *y2 = nullptr; };
 struct BlockBufs { float *ln, *qkv, *ctx, *mlp, *h; };   // [n][C], [n][C+2kvd], [n][C], [n][Hh or 2Hh], [n][Hh]
 struct AttnPlan {

@@ -268,11 +268,11 @@ void lm_embed(LMRun &r, const int *ids_d, const int *pos_d, int64_t n) {
 
 NormSpec lm_last_norm(const NcmbLM *m) { return NormSpec{m->is_qwen ? 2 : 1, m->lnfw, m->is_qwen ? nullptr : m->lnfb, m->is_qwen ? 1e-6f : 1e-5f}; }
 
-// few: the rows' final norm as a pair, when a few-row chain left it behind
+// few: the rows' final norm, when a few-row chain left it behind
 void lm_head(LMRun &r, const float *h, int64_t rows, float *logits, const FewChain *few = nullptr) {
     NcmbLM *m = r.m;
     if (few && few->on && few->ready) {
-        few_head(few->y1, few->y2, (int)rows, m->wte, nullptr, m->V, m->C, logits);
+        few_head(few->y1, few->y2, (int)rows, m->wte, m->wte16, nullptr, m->V, m->C, logits);
         return;
     }
     GemmArgs g;
@@ -346,7 +346,7 @@ void lm_decode_step(LMRun &r, const int *ids_d) {
     p.kv_pitch = 2 * kvd; p.kv_rows_per_seq = 1; p.kv_seq_pitch = (int64_t)r.cap * 2 * kvd;
     p.kv_store_step = 2 * kvd;
     r.few = FewChain();
-    r.few.on = few_chain_supported(r.B, m->C, m->H, m->nkv, m->blocks[0]) && gemm_few_supported(r.B, m->V, m->C);
+    r.few.on = few_chain_supported(r.B, m->C, m->H, m->nkv, m->blocks[0]) && gemm_few_supported(r.B, m->V, m->C, m->wte);
     p.few = &r.few;
     for (int li = 0; li < m->NL; li++) {
         p.k1 = r.kv[li]; p.v1 = r.kv[li] + kvd;

@@ -268,11 +268,11 @@ extern "C" VQState *ncp_vq(NCPState *m) { return m->vq; }
 
 // ------------------------------------------------------------------ shared pieces
 
-// ln_f of the stack's output x, then head k. few: the normed rows as a pair, when a few-row chain left them behind.
+// ln_f of the stack's output x, then head k. few: the normed rows, when a few-row chain left them behind.
 static void final_logits(NCPState *m, int k, const float *x, int64_t rows, const BlockBufs &bufs, float *lg, const FewChain &few) {
     const HeadW &h = m->heads[k];
-    if (few.on && few.ready && !h.proj && gemm_few_supported(rows, h.V, m->C)) {
-        few_head(few.y1, few.y2, (int)rows, h.W, h.b, h.V, m->C, lg);
+    if (few.on && few.ready && !h.proj && gemm_few_supported(rows, h.V, m->C, h.W)) {
+        few_head(few.y1, few.y2, (int)rows, h.W, nullptr, h.b, h.V, m->C, lg);
         return;
     }
     layernorm(x, m->lnfw, m->lnfb, bufs.ln, rows, m->C, 1e-6f);

@@ -107,7 +107,9 @@ static int few_max_slices(int64_t M) { return M <= 64 ? 24 : (M <= 128 ? 8 : 4);
 bool few_chain_supported(int64_t ntok, int C, int H, int nkv, const BlockWeights &w) {
     static const bool off = getenv("NCM_B200_NO_FEW") != nullptr;
     const int hd = C / H;
-    return !off && gemm_few_supported(ntok, C + 2 * nkv * hd, C) && gemm_few_supported(ntok, w.Hh, w.Hh) && C % 8 == 0 && C <= 4096 && hd % 2 == 0 &&
+    // (the fp32 products read the matrices in place, by TMA)
+    const void *at = (const void *)((uintptr_t)w.qkvw | (uintptr_t)w.ow | (uintptr_t)w.fcw | (uintptr_t)w.pw);
+    return !off && gemm_few_supported(ntok, C + 2 * nkv * hd, C, at) && gemm_few_supported(ntok, w.Hh, w.Hh, at) && C % 8 == 0 && C <= 4096 && hd % 2 == 0 &&
            !w.qnw && !w.knw && (!w.gated || w.fcw_il);
 }
 
@@ -123,43 +125,43 @@ static void run_block_few(float *x, int64_t ntok, int C, int H, int nkv, const B
     const size_t need = part_fl * 4 + (size_t)M * (2 * C + w.Hh) * 4 + 4096;
     if (need > ws.cap) { ws.reserve(need + need / 4); fc.ready = false; }
     ws.reset();
-    // (the chain's pair comes first: it lies in the same place for every block, written by the previous block's last kernel)
-    unsigned short *n1 = ws.get<unsigned short>((size_t)M * C), *n2 = ws.get<unsigned short>((size_t)M * C);
+    // (the chain's rows come first: they lie in the same place for every block, written by the previous block's last kernel)
+    const bool f32 = M <= FEW_F32_ROWS;                      // rows between the kernels: fp32, or fp16 pairs
+    unsigned short *n1 = ws.get<unsigned short>((size_t)M * C * (f32 ? 2 : 1)), *n2 = f32 ? nullptr : ws.get<unsigned short>((size_t)M * C);
     float *part = ws.get<float>(part_fl);
-    float *ctx_lo = ws.get<float>((size_t)M * C / 2 + 8), *h_lo = ws.get<float>((size_t)M * w.Hh / 2 + 8);
+    float *ctx_lo = f32 ? nullptr : ws.get<float>((size_t)M * C / 2 + 8), *h_lo = f32 ? nullptr : ws.get<float>((size_t)M * w.Hh / 2 + 8);
     if (!fc.ready) few_reduce_norm(x, nullptr, 0, nullptr, M, C, ln1_of(w).kind, w.ln1w, ln1_of(w).b, ln1_of(w).eps, n1, n2);
     const NormSpec ln2{ln1_of(w).kind, w.ln2w, w.norm == NORM_RMS ? nullptr : w.ln2b, ln1_of(w).eps};
-    FewGemm g{n1, n2, C, w.qkvw, M, Wq, C};
-    g.part = part; g.max_slices = ms;
-    gemm_few(g);
+    auto product = [&](const void *x1, const void *x2, const float *W, const unsigned short *W16, int N, int K) {
+        FewGemm g{x1, x2, K, W, M, N, K};
+        g.W16 = W16; g.part = part; g.max_slices = ms;
+        return g;
+    };
+    gemm_few(product(n1, n2, w.qkvw, w.qkvw16, Wq, C));
     FewQkv q{part, Sq, M, H, nkv, w.qkvb};
     q.cos_t = p.cos_t; q.sin_t = p.sin_t; q.pos = p.pos; q.step_d = p.step_d; q.pos_step = p.pos_step;
     q.q = b.qkv; q.ldq = Wq; q.kv_self = (!p.k1 || p.self_is_k2 || p.kv_store == nullptr) ? 1 : 0;
     q.kv = p.kv_store; q.rps = p.kv_rows_per_seq > 0 ? p.kv_rows_per_seq : M; q.seq_pitch = p.kv_seq_pitch; q.pitch = p.kv_pitch; q.step = p.kv_store_step;
     q.hd = hd;
-    const AttnArgs at = attention_args(b, p, ntok, C, H, nkv, ctx_lo, SPLIT_H16);
+    const AttnArgs at = attention_args(b, p, ntok, C, H, nkv, ctx_lo, f32 ? SPLIT_NONE : SPLIT_H16);
     if (!q.kv_self && p.kv_rows_per_seq == 1 && p.rows == M && attention_fused_supported(at)) attention_fused(at, q);
     else {
         few_reduce_qkv(q);
         if (p.kv_only) return;
         attention(at);
     }
-    g = FewGemm{b.ctx, ctx_lo, C, w.ow, M, C, C};
-    g.part = part; g.max_slices = ms;
-    gemm_few(g);
+    gemm_few(product(b.ctx, ctx_lo, w.ow, w.ow16, C, C));
     few_reduce_norm(x, part, So, w.ob, M, C, ln2.kind, ln2.w, ln2.b, ln2.eps, n1, n2);
-    g = FewGemm{n1, n2, C, w.gated ? w.fcw_il : w.fcw, M, Nu, C};
+    FewGemm g = product(n1, n2, w.gated && !f32 ? w.fcw_il : w.fcw, w.fcw16, Nu, C);
+    g.glu = w.gated;
     if (Su > 1) {
-        g.part = part; g.max_slices = ms;
         gemm_few(g);
         few_reduce_act(part, Su, M, Nu, w.gated ? w.fcb_il : w.fcb, w.act, w.gated, b.h, h_lo);
     } else {
-        g.bias = w.gated ? w.fcb_il : w.fcb; g.act = w.act; g.glu = w.gated; g.y = b.h; g.y_lo = h_lo; g.ldy = w.Hh;
+        g.part = nullptr; g.bias = w.gated && !f32 ? w.fcb_il : w.fcb; g.act = w.act; g.y = b.h; g.y_lo = h_lo; g.ldy = w.Hh;
         gemm_few(g);
     }
-    g = FewGemm{b.h, h_lo, w.Hh, w.pw, M, C, w.Hh};
-    g.part = part; g.max_slices = ms;
-    gemm_few(g);
+    gemm_few(product(b.h, h_lo, w.pw, w.pw16, C, w.Hh));
     few_reduce_norm(x, part, Sd, w.pb, M, C, fc.next.kind, fc.next.w, fc.next.b, fc.next.eps, n1, n2);
     fc.ready = fc.next.kind != 0; fc.y1 = n1; fc.y2 = n2;
 }

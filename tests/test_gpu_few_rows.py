@@ -51,19 +51,15 @@ def test_greedy_ids(cuda, models, kind, B):
     assert cuda.ncmb_gemm_tc_check() == 0
 
 
-@pytest.mark.parametrize("shape", ["qwen_896x4864", "gpt2_768x8192"])
-def test_one_row_whose_down_projection_rows_do_not_fit_the_ring_together(cuda, tmp_path, shape):
+@pytest.mark.parametrize("C,H,inner", [(896, 14, 4864), (768, 12, 8192)])
+def test_one_row_whose_down_projection_rows_do_not_fit_the_ring_together(cuda, tmp_path, C, H, inner):
     """fp32: 7 x 4864 and 6 x 8192 floats a CTA against a ring of 32768; the rows are given back in groups."""
     import orc
     import synth
-    qwen = shape.startswith("qwen")
-    if qwen:
-        spec = synth.LMSpec(shape, "qwen", 3, 896, 14, 2, 4864, 301, 64, rope_theta=1e6, rand_affine=1)
-    else:
-        spec = synth.LMSpec(shape, "gpt2", 3, 768, 12, 12, 8192, 301, 64, rand_affine=1)
+    spec = synth.LMSpec("ring", "qwen", 3, C, H, 2, inner, 301, 64, rope_theta=1e6, rand_affine=1)
     conf, w = synth.write_lm(spec, str(tmp_path))
-    m = cuda.ncmb_lm_open(cuda.load_config(conf), w.encode(), int(qwen), 0)
-    om = orc.LM(conf, w, qwen)
+    m = cuda.ncmb_lm_open(cuda.load_config(conf), w.encode(), 1, 0)
+    om = orc.LM(conf, w, True)
     cuda.ncmb_set_lm_persistent(1)
     n_new = 12
     P = np.ascontiguousarray(synth.lm_prompts(spec, 1, 35, 4))
@@ -72,7 +68,7 @@ def test_one_row_whose_down_projection_rows_do_not_fit_the_ring_together(cuda, t
         cuda.ncmb_lm_generate(m, P.ctypes.data, 1, P.shape[1], n_new, kw["temp"], kw["top_k"], kw["top_p"], kw["seed"], -1, out.ctypes.data)
         assert cuda.ncmb_gemm_tc_check() == 0
         want = om.generate(P[0], n_new, **kw)
-        assert (out[0] == want).all(), (shape, kw, out[0], want)
+        assert (out[0] == want).all(), (C, kw, out[0], want)
     cuda.ncmb_lm_close(m)
 
 
