@@ -534,9 +534,11 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         at += b_dn;
         ms_bar();
         if (tid < ncr) {
-            float y = one(L.pb, true, c0 + tid) + sm->xres[tid];
+            // the product first, then the residual: added one by one to the larger residual, sixteen partial sums lose its last bits
+            float q4[4];
 #pragma unroll
-            for (int q = 0; q < MS_WARPS; q++) y += part[tid * MS_WARPS + q];
+            for (int q = 0; q < 4; q++) { const float4 p = *(const float4 *)(part + tid * MS_WARPS + 4 * q); q4[q] = (p.x + p.y) + (p.z + p.w); }
+            const float y = ((q4[0] + q4[1]) + (q4[2] + q4[3])) + one(L.pb, true, c0 + tid) + sm->xres[tid];
             ll_store(Lx + c0 + tid, y, tag);
         }
         st.release(at, warp, lane);

@@ -103,3 +103,21 @@ def test_inner_activations_beyond_the_pair_range_keep_their_value(cuda, tmp_path
     print(f"{kind} B={B}: relative error max {e.max():.2e}, plain fp32 {plain.max():.2e}")
     # rows whose large terms cancel amplify every rounding: plain fp32 shows by how much (clipped values are off by 1e-2 and more)
     assert e.max() < 4 * plain.max() + FP32_BOUND
+
+
+@pytest.mark.parametrize("B", [1, 2, 16])
+def test_partial_sums_meet_before_the_residual(cuda, tmp_path, B):
+    """A hidden state much larger than what a layer adds to it: each rounding of it counts, so a product's partial sums must not be added to
+    it one by one. Twelve layers with one rounding each are what plain fp32 has."""
+    import synth
+    spec = synth.LMSpec("gpt2_res", "gpt2", 12, 768, 12, 12, 3072, 1009, 64, rand_affine=1)
+
+    def large_state(t):
+        t["wte.weight"] *= 400
+        t["wpe.weight"] *= 400
+    t, m = _open(cuda, spec, str(tmp_path), large_state)
+    e, plain = zip(*(_errors(cuda, spec, t, m, B, 1, steps, 3, plain=True) for steps in (9, 20, 40)))
+    cuda.ncmb_lm_close(m)
+    e, plain = np.mean(e), np.mean(plain)
+    print(f"B={B}: relative error mean {e:.2e}, plain fp32 {plain:.2e}")
+    assert e < 1.5 * plain
