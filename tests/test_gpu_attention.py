@@ -110,23 +110,22 @@ DECODE_CASES = {
     # many rows: a CTA walks several 32-key chunks with a running maximum (640 row/kv-head pairs, up to 10 chunks)
     "many_rows_several_chunks_per_cta": (list(np.random.default_rng(1).integers(1, 300, 320)) + [320, 289], 8, 2),
     # enough rows to fill the GPU without splitting keys: one CTA sees all keys of its row and writes the context itself
+    # 512 (row, kv head) pairs of seven query heads: blocks of three warps
+    "three_warps_a_block": (list(np.random.default_rng(3).integers(1, 600, 256)), 14, 2),
     "one_cta_per_row_no_merge": (list(np.random.default_rng(2).integers(1, 100, 1300)), 4, 2),
 }
 
 
-@pytest.fixture(params=["chosen", "warp_per_chunk", "tensor_core_rows"])
+@pytest.fixture(params=["chosen", "tensor_core_rows"])
 def decode_kernel(request):
-    """the split-key path as dispatched, with the warp-per-chunk kernel forced for every shape it takes, and with the
-    kernel that makes the (query, head) pairs of a kv group the 16 rows of an mma.sync tile forced likewise"""
+    """the split-key path as dispatched, and with the kernel that makes the (query, head) pairs of a kv group the 16 rows
+    of an mma.sync tile forced for every shape it takes"""
     import os
-    if request.param == "warp_per_chunk":
-        os.environ["NCM_B200_ATTN_DEC_WARP"] = "1"
     if request.param == "tensor_core_rows":
         os.environ["NCM_B200_ATTN_DEC_MMA"] = "1"
     else:
         os.environ["NCM_B200_ATTN_DEC_MMA"] = "0"
     yield request.param
-    os.environ.pop("NCM_B200_ATTN_DEC_WARP", None)
     os.environ.pop("NCM_B200_ATTN_DEC_MMA", None)
 
 

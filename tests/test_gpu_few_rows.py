@@ -1,6 +1,6 @@
 """Decode steps of 1 to 641 rows (the loop of reference src/gpt2.c:179, src/qwen.c:209): the persistent kernel at one row, the
 few-row products and their folded reductions up to 640, the general path above -- at the edges of their row tiles (16, 32, 64,
-128), with widths that fill no tile. Greedy ids of a few rows against the oracle's independent runs."""
+128), with widths that fill no tile, and with two to four warps a block of the decode attention (500 rows: three). Greedy ids of a few rows against the oracle's independent runs."""
 import numpy as np
 import pytest
 
@@ -32,10 +32,10 @@ def models(cuda, tmp_path_factory):
     yield made
     for _, m, _ in made.values():
         cuda.ncmb_lm_close(m)
-    cuda.ncmb_set_lm_persistent(0)
+    cuda.ncmb_set_lm_persistent(1)                            # the default
 
 
-@pytest.mark.parametrize("B", [1, 2, 4, 5, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257, 640, 641])
+@pytest.mark.parametrize("B", [1, 2, 4, 5, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257, 500, 640, 641])
 @pytest.mark.parametrize("kind", ["gpt2", "qwen", "qwen_bf16"])
 def test_greedy_ids(cuda, models, kind, B):
     import synth

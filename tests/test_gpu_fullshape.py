@@ -6,8 +6,8 @@ with the length of the contractions, so these run the real widths and depths on 
 * config 2 at its 12 layers, sampled as configured (CFG 1.5, temp 0.8, top-k 50, top-p 0.9, frequency 0.2);
 * config 1b (ladder 1-3-9-81) at 64 sequences, greedy, codes and the 81 decoded tokens;
 * config 5's widths (d = 1024, 16 query / 4 kv heads, 16 384 codes) at 2 layers;
-* the GPT-2 124M shape: logits of a 128-id prompt, greedy ids alone and inside a batch of 64;
-* the Qwen2-0.5B shape with bf16-rounded weights: logits of a 64-id prompt, greedy ids, and sampled ids
+* the GPT-2 124M shape: logits of a 128-id prompt, greedy and sampled ids alone, greedy ones inside a batch of 64;
+* the Qwen2-0.5B shape with bf16-rounded weights, opened as bf16 and as fp32: logits of a 64-id prompt, greedy ids, sampled ids
   at temp 0.7 / top-p 0.95 over the 151 936-entry vocabulary.
 
 Bars: integer results equal the oracle's; a differing greedy id is accepted only when the oracle's two
@@ -226,15 +226,19 @@ def test_gpt2_124m_shape_logits_and_greedy_ids(cuda, tmp):
     print(f"gpt2 124M shape: logits of a {P}-id prompt, max abs err {e:.2e}")
     # one sequence (weight-streaming decode steps)
     out1 = np.zeros((1, n_new), np.int32)
+    cuda.ncmb_set_lm_persistent(1)                         # the default: one row is one persistent kernel a step
     cuda.ncmb_lm_generate(m, pr.ctypes.data, 1, P, n_new, 0.0, 0, 1.0, 0, -1, out1.ctypes.data)
     ties = _greedy_ids_or_near_tie(om, pr, out1[0], "gpt2 B=1")
+    for top_k, top_p in ((40, 0.95), (0, 0.95)):
+        cuda.ncmb_lm_generate(m, pr.ctypes.data, 1, P, n_new, 0.8, top_k, top_p, 5, -1, out1.ctypes.data)
+        ties += _sampled_ids_or_near_tie(om, pr, out1[0], 0.8, top_k, top_p, 5, f"gpt2 B=1 sampled, top-k {top_k}")
     # 64 sequences (tensor-core decode steps); three of the rows are checked
     out = np.zeros((B, n_new), np.int32)
     cuda.ncmb_lm_generate(m, prompts.ctypes.data, B, P, n_new, 0.0, 0, 1.0, 0, -1, out.ctypes.data)
     assert cuda.ncmb_gemm_tc_check() == 0
     for b in (0, 17, 63):
         ties += _greedy_ids_or_near_tie(om, prompts[b], out[b], f"gpt2 B=64 row {b}")
-    print(f"gpt2 124M shape: {n_new} greedy ids at B=1 and 3 rows of B=64, {ties} near-ties")
+    print(f"gpt2 124M shape: {n_new} greedy and {2 * n_new} sampled ids at B=1, {n_new} greedy of 3 rows of B=64, {ties} near-ties")
     cuda.ncmb_lm_close(m)
 
 
@@ -248,6 +252,7 @@ def test_qwen2_05b_shape_bf16_weights_logits_greedy_and_sampled_ids(cuda, tmp):
     m = cuda.ncmb_lm_open(cfg, w.encode(), 1, 1)
     assert m
     om = orc.LM(conf, w, True)
+    cuda.ncmb_set_lm_persistent(1)                         # the default: one row is one persistent kernel a step
     P, n_new = 64, 8
     pr = np.ascontiguousarray(synth.lm_prompts(spec, 1, P, 3)[0])
     lg = np.zeros((P, spec.vocab), np.float32)
@@ -258,13 +263,22 @@ def test_qwen2_05b_shape_bf16_weights_logits_greedy_and_sampled_ids(cuda, tmp):
     cuda.ncmb_lm_generate(m, pr.ctypes.data, 1, P, n_new, 0.0, 0, 1.0, 0, -1, out.ctypes.data)
     ties = _greedy_ids_or_near_tie(om, pr, out[0], "qwen B=1")
     print(f"qwen2 0.5B shape: {n_new} greedy ids, {ties} near-ties")
-    # the configuration's sampler over the whole vocabulary (device-wide sort of 151 936 entries): two ids
-    n_s = 2
+    # the configuration's sampler over the whole vocabulary
+    n_s = 6
     outs = np.zeros((1, n_s), np.int32)
     cuda.ncmb_lm_generate(m, pr.ctypes.data, 1, P, n_s, 0.7, 0, 0.95, 9, -1, outs.ctypes.data)
     assert cuda.ncmb_gemm_tc_check() == 0
     ties = _sampled_ids_or_near_tie(om, pr, outs[0], 0.7, 0, 0.95, 9, "qwen sampled")
     print(f"qwen2 0.5B shape: {n_s} sampled ids, {ties} near-ties")
+    cuda.ncmb_lm_close(m)
+    # the same file opened as fp32 weights, as qwen-gen does: the step streams the fp32 matrices
+    m = cuda.ncmb_lm_open(cfg, w.encode(), 1, 0)
+    out32, outs32 = np.zeros_like(out), np.zeros_like(outs)
+    assert cuda.ncmb_lm_generate(m, pr.ctypes.data, 1, P, n_new, 0.0, 0, 1.0, 0, -1, out32.ctypes.data) == n_new
+    assert cuda.ncmb_lm_generate(m, pr.ctypes.data, 1, P, n_s, 0.7, 0, 0.95, 9, -1, outs32.ctypes.data) == n_s
+    ties = 0 if (out32 == out).all() else _greedy_ids_or_near_tie(om, pr, out32[0], "qwen fp32 B=1")
+    ties += 0 if (outs32 == outs).all() else _sampled_ids_or_near_tie(om, pr, outs32[0], 0.7, 0, 0.95, 9, "qwen fp32 sampled")
+    print(f"qwen2 0.5B shape, fp32 weights: {n_new} greedy and {n_s} sampled ids, {ties} near-ties")
     cuda.ncmb_lm_close(m)
     try:
         os.remove(w)                                       # 2 GB of weights

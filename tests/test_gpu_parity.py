@@ -393,7 +393,7 @@ LM_SPECS = {
     "qwen_hd64": lambda synth: synth.LMSpec("qwen_hd64", "qwen", 2, 256, 4, 2, 384, 411, 64, rope_theta=1e6, rand_affine=1),
     # weights rounded to bf16 in the file, opened with bf16_weights = 1: decode steps stream the exact 2-byte copies
     "qwen_hd64_bf16": lambda synth: synth.LMSpec("qwen_hd64_bf16", "qwen", 2, 256, 4, 2, 384, 411, 64, rope_theta=1e6, bf16_round=1),
-    # the same two through the persistent cooperative decode kernel (rotary pairs, grouped heads, gated MLP)
+    # the same two through the persistent cooperative decode kernel (rotary pairs, grouped heads, gated MLP), row by row: it takes one
     "gpt2_hd64_persistent": lambda synth: synth.LMSpec("gpt2_hd64", "gpt2", 2, 128, 2, 2, 512, 300, 64, rand_affine=1),
     "qwen_hd64_persistent": lambda synth: synth.LMSpec("qwen_hd64", "qwen", 2, 256, 4, 2, 384, 411, 64, rope_theta=1e6, rand_affine=1),
 }
@@ -404,7 +404,8 @@ def test_decoder_lm_logits_and_generation(cuda, tmp, kind):
     import orc
     import synth
     spec = LM_SPECS[kind](synth)
-    cuda.ncmb_set_lm_persistent(int(kind.endswith("_persistent")))
+    persistent = kind.endswith("_persistent")
+    cuda.ncmb_set_lm_persistent(int(persistent))
     is_qwen = spec.kind == "qwen"
     conf, w = synth.write_lm(spec, tmp)
     cfg = cuda.load_config(conf)
@@ -425,12 +426,14 @@ def test_decoder_lm_logits_and_generation(cuda, tmp, kind):
     P = np.ascontiguousarray(prompts)
     for (t, tk, tp, sd) in ((0.0, 0, 1.0, 0), (0.9, 8, 1.0, 5), (0.7, 0, 0.95, 9)):
         out = np.zeros((P.shape[0], n_new), np.int32)
-        cuda.ncmb_lm_generate(m, P.ctypes.data, P.shape[0], P.shape[1], n_new, t, tk, tp, sd, -1, out.ctypes.data)
+        for b in range(0, P.shape[0], 1 if persistent else P.shape[0]):
+            n = 1 if persistent else P.shape[0]
+            assert cuda.ncmb_lm_generate(m, P[b:].ctypes.data, n, P.shape[1], n_new, t, tk, tp, sd, -1, out[b:].ctypes.data) == n_new
         for b in range(P.shape[0]):
             want = om.generate(P[b], n_new, temp=t, top_k=tk, top_p=tp, seed=sd)
             assert (out[b] == want).all(), (kind, t, tk, tp, b, out[b], want)
         assert cuda.ncmb_gemm_tc_check() == 0           # no bounded wait (mbarrier, grid barrier) ran out
-    cuda.ncmb_set_lm_persistent(0)
+    cuda.ncmb_set_lm_persistent(1)                      # the default
     cuda.ncmb_lm_close(m)
 
 
@@ -446,13 +449,12 @@ PPL_SPECS = {
 }
 
 
-@pytest.mark.parametrize("decode_attention", ["chosen", "tensor_core_rows"])
-@pytest.mark.parametrize("kind", ["gpt2", "qwen"])
+@pytest.mark.parametrize("kind,decode_attention", [("gpt2", "chosen"), ("qwen", "chosen"), ("qwen", "tensor_core_rows")])
 def test_batched_decode_steps_through_k_sliced_projections(cuda, tmp, kind, decode_attention, monkeypatch):
-    """20 rows per decode step at width 768: too many rows for the GEMV path, few tiles and a long K for the
-    tensor-core GEMM, so the attention-output and MLP-down projections run K in slices with a reduce kernel behind
-    them. Ids equal independent oracle runs. Run a second time with the decode attention that makes the (query, head)
-    pairs of a kv group the rows of an mma.sync tile (what large batches of the grouped-query model get)."""
+    """20 rows per decode step at width 768: every projection is cut into slices of K that the kernel behind it adds. The
+    grouped-query model has twelve query heads on its kv head, more than the decode attention that reads those slices
+    itself takes: it runs the split-key kernel and, a second time, the one that makes the (query, head) pairs of a kv group
+    the rows of an mma.sync tile. Ids equal independent oracle runs."""
     import orc
     import synth
     if decode_attention == "tensor_core_rows":
@@ -462,7 +464,7 @@ def test_batched_decode_steps_through_k_sliced_projections(cuda, tmp, kind, deco
     if kind == "gpt2":
         spec = synth.LMSpec("gpt2_w768", "gpt2", 1, 768, 12, 12, 3072, 300, 32, rand_affine=1)
     else:
-        spec = synth.LMSpec("qwen_w768", "qwen", 1, 768, 12, 2, 2048, 300, 32, rope_theta=1e6, rand_affine=1)
+        spec = synth.LMSpec("qwen_w768", "qwen", 1, 768, 12, 1, 2048, 300, 32, rope_theta=1e6, rand_affine=1)
     conf, w = synth.write_lm(spec, tmp)
     cfg = cuda.load_config(conf)
     m = cuda.ncmb_lm_open(cfg, w.encode(), int(kind == "qwen"), 0)
