@@ -493,6 +493,7 @@ constexpr int64_t NEAR_SCAN_ROWS = 256;
 static unsigned scan_grid(int64_t items) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)ctx().sm_count * 6)); }
 
 void nearest_codes(const float *x, const float *E, int64_t rows, int V, int D, int *idx_out, int out_tlen, int out_stride, int out_off) {
+    if (rows <= 0) return;
     static Workspace ws;
     const CodeBook &cb = codebook(E, V, D);
     const int ntiles = (int)cdiv(V, NC_CODES), Dp = (D + 3) & ~3;

@@ -225,6 +225,7 @@ void vq_next_input_dev(VQState *v, const int *codes_dev, int stride, int rowmod,
 }
 
 void vq_encode_dev(VQState *v, const float *z, int B, int *idx_dev, float *scratch) {
+    if (B <= 0) return;
     const int D = v->D, L = v->L, total = vq_total_codes(v);
     const size_t n = (size_t)B * L * D;
     float *z_rest = scratch + 5 * n, *down = scratch + 6 * n, *up = scratch + 4 * n;   // caller provides 7n floats
