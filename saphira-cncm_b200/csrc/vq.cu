@@ -196,10 +196,11 @@ static void level_step(VQState *v, const int *codes, int stride, int rowmod, int
                        int tnext, float *next, float *up, float *scratch) {
     const int D = v->D, L = v->L;
     const bool refined = v->has_all && level >= 1 && level <= v->n_levels - 2 && v->urefW[level];
-    const bool plain = !(level == 0 && v->has_l1) && !v->resi && !refined && D % 4 == 0;
+    // whole float4s: the rows' width, and where the caller's buffers start
+    const bool tiles = next && L % tnext == 0, vec = D % 4 == 0 && (((uintptr_t)src | (uintptr_t)dst | (uintptr_t)(tiles ? next : nullptr)) & 15) == 0;
+    const bool plain = !(level == 0 && v->has_l1) && !v->resi && !refined && vec;
     if (!plain) vq_increment_dev(v, codes, stride, rowmod, level, B, up, scratch);
-    const bool tiles = next && L % tnext == 0;
-    if (D % 4) {                                              // rows that are not whole float4s: one pass per operation
+    if (!vec) {                                               // one pass per operation
         const size_t n = (size_t)B * L * D;
         if (src != dst) {
             if (src) CUDA_CHECK(cudaMemcpyAsync(dst, src, n * 4, cudaMemcpyDeviceToDevice, stream()));

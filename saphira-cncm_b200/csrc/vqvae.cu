@@ -79,7 +79,7 @@ void vqvae_decode_dev(VQVAEState *v, const float *zhat, float *logits, int B) {
     v->work.reset();
     float *x = v->work.get<float>(n * D);
     BlockBufs bufs = vae_bufs(v->work, n, D, Hh);
-    if (vae_stack_supported(v->dec, D, c->vq_n_layers, T, 0)) {
+    if (vae_stack_supported(v->dec, D, c->vq_n_layers, T, 0) && ((uintptr_t)zhat & 15) == 0) {
         VaeStackIO io;
         io.x = zhat; io.wpe = c->dec_positional ? v->dec_wpe : nullptr; io.lnf = v->dec_lnf; io.y = bufs.ln;
         vae_stack(v->dec, c->vq_n_layers, B, T, io);
@@ -185,7 +185,8 @@ void vqvae_encode_z(VQVAEState *v, const int *ids, float *z, int B) {
     float *t1 = v->work.get<float>(n * D), *t2 = v->work.get<float>(n * D);
     BlockBufs bufs = vae_bufs(v->work, n, D, Hh);
     upload_queued(ids_dev, ids, (size_t)n * sizeof(int));
-    if (c->enc_conv_layers == 0 && c->vq_compression <= 1 && c->pre_quant_groupnorm <= 0 && vae_stack_supported(v->enc, D, c->vq_n_layers, T, c->enc_attn_window)) {
+    if (c->enc_conv_layers == 0 && c->vq_compression <= 1 && c->pre_quant_groupnorm <= 0 && vae_stack_supported(v->enc, D, c->vq_n_layers, T, c->enc_attn_window) &&
+        ((uintptr_t)z & 15) == 0) {
         VaeStackIO io;
         io.ids = ids_dev; io.wte = v->enc_wte; io.wpe = c->enc_positional ? v->enc_wpe : nullptr; io.y = z;
         io.lnf = wneed(ws, "tok.encoder.ln_e.weight")->data;

@@ -38,3 +38,42 @@ def test_no_rows(cuda, model):
     cuda.ncmb_vq_encode_dev(m.vq, z, 0, idx)
     cuda.vq_z_to_idx(m.vq, z, 0, host.ctypes.data)
     assert (cuda.to_host(idx, (64,), np.int32) == 77).all() and (host == 77).all()
+
+
+@pytest.mark.parametrize("B", [1, 5, 70])
+def test_buffers_that_start_at_any_float(cuda, model, B):
+    """Device buffers of a caller that are aligned for a float but not for 16 bytes: the results of aligned ones, to fp32 rounding (other
+    kernels take them)."""
+    spec, _, _, m = model
+    n = B * spec.L * spec.vq_dim
+    rng = np.random.default_rng(B)
+    close = lambda a, b: np.abs(a - b).max() <= 1e-5 * np.abs(b).max()
+    ids = rng.integers(2, spec.in_vocab, (B, spec.L)).astype(np.int32)
+    z, z1 = cuda.alloc(n + 4), cuda.alloc(n + 4) + 4
+    cuda.vqvae_encode_z(m.vqvae, ids.ctypes.data, z, B)
+    cuda.vqvae_encode_z(m.vqvae, ids.ctypes.data, z1, B)
+    zh = cuda.to_host(z, (n,))
+    assert close(cuda.to_host(z1, (n,)), zh)
+    zh = (zh + 0.05 * rng.standard_normal(n)).astype(np.float32)
+    cuda.mem_h2d(z, zh.ctypes.data, zh.nbytes)
+    cuda.mem_h2d(z1, zh.ctypes.data, zh.nbytes)
+    total = sum(spec.levels)
+    got, want = np.zeros((2, B, total), np.int32)
+    cuda.vq_z_to_idx(m.vq, z, B, want.ctypes.data)
+    cuda.vq_z_to_idx(m.vq, z1, B, got.ctypes.data)
+    assert (got == want).all() and np.array_equal(cuda.to_host(z1, (n,)), zh)
+    lg, lg1 = (cuda.alloc(B * spec.L * spec.in_vocab) for _ in range(2))
+    cuda.vqvae_decode(m.vqvae, z, lg, B)
+    cuda.vqvae_decode(m.vqvae, z1, lg1, B)
+    shape = (B * spec.L * spec.in_vocab,)
+    assert close(cuda.to_host(lg1, shape), cuda.to_host(lg, shape))
+    codes = np.ascontiguousarray(want[:, 1:5])
+    nx = B * spec.levels[2] * spec.vq_dim
+    out = {}
+    for dz, dx in ((0, 0), (4, 0), (0, 4), (4, 4)):
+        zb, xb = cuda.alloc(n + 4) + dz, cuda.alloc(nx + 4) + dx
+        cuda.mem_h2d(zb, zh.ctypes.data, zh.nbytes)
+        cuda.vq_next_input(m.vq, codes.ctypes.data, 1, zb, xb, B)
+        out[dz, dx] = cuda.to_host(zb, (n,)), cuda.to_host(xb, (nx,))
+    for v in out.values():
+        assert close(v[0], out[0, 0][0]) and close(v[1], out[0, 0][1])
