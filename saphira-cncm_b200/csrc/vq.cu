@@ -198,7 +198,10 @@ static void level_step(VQState *v, const int *codes, int stride, int rowmod, int
     const bool refined = v->has_all && level >= 1 && level <= v->n_levels - 2 && v->urefW[level];
     // whole float4s: the rows' width, and where the caller's buffers start
     const bool tiles = next && L % tnext == 0, vec = D % 4 == 0 && (((uintptr_t)src | (uintptr_t)dst | (uintptr_t)(tiles ? next : nullptr)) & 15) == 0;
-    const bool plain = !(level == 0 && v->has_l1) && !v->resi && !refined && vec;
+    // k_level_step's table of interpolation weights; without one (a level of one step, a finished increment) it needs none
+    const bool flat = v->levels[level] == 1 || L == 1;
+    const size_t table = flat ? 0 : (size_t)L * 16;
+    const bool plain = !(level == 0 && v->has_l1) && !v->resi && !refined && vec && table <= 48 * 1024;
     if (!plain) vq_increment_dev(v, codes, stride, rowmod, level, B, up, scratch);
     if (!vec) {                                               // one pass per operation
         const size_t n = (size_t)B * L * D;
@@ -214,7 +217,7 @@ static void level_step(VQState *v, const int *codes, int stride, int rowmod, int
         a.up_in = plain ? nullptr : up; a.src = src; a.dst = dst; a.next = tiles ? next : nullptr;
         a.sign = sign; a.L = L; a.D = D; a.tnext = tiles ? tnext : L; a.n4 = (int64_t)B * a.tnext * (D / 4);
         ProfScope ps(NCMB_K_VQ);
-        LAUNCH(k_level_step, ew(a.n4), 256, (size_t)L * 16, a);
+        LAUNCH(k_level_step, ew(a.n4), 256, plain ? table : 0, a);
         if (tiles) return;
     }
     if (next) interp_area(dst, nlc(D, L), next, nlc(D, tnext), B, D, L, tnext);

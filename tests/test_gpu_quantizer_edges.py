@@ -77,3 +77,20 @@ def test_buffers_that_start_at_any_float(cuda, model, B):
         out[dz, dx] = cuda.to_host(zb, (n,)), cuda.to_host(xb, (nx,))
     for v in out.values():
         assert close(v[0], out[0, 0][0]) and close(v[1], out[0, 0][1])
+
+
+@pytest.mark.parametrize("L", [3072, 4096])
+def test_long_contexts(cuda, tmp_path, L):
+    """A level's interpolation weights are tabled in shared memory up to 3072 positions (48 KB)."""
+    import orc
+    spec, conf, w, m = _model(cuda, str(tmp_path), levels=[1, 5, L], vocab=[300] * 3, l1_cascade=[], l1_norm=0, enc_layers=1, dec_layers=1)
+    z = (0.05 * np.random.default_rng(L).standard_normal((2, L, spec.vq_dim))).astype(np.float32)
+    idx = np.zeros((2, L + 6), np.int32)
+    cuda.vq_z_to_idx(m.vq, cuda.to_backend(z), 2, idx.ctypes.data)
+    want = orc.Model(conf, w).z_to_idx(z)
+    assert (idx != want).mean() <= 1e-3                      # codes at near-ties
+    assert (idx[:, :6] == want[:, :6]).all()
+    zh = [cuda.alloc(z.size) for _ in range(3)]
+    cuda.vq_idx_to_zhats(m.vq, want.ctypes.data, 2, (C.c_void_p * 3)(*zh))
+    for got, ref in zip(zh, orc.Model(conf, w).idx_to_zhats(want, 3)):
+        assert np.abs(cuda.to_host(got, z.shape) - ref).max() <= 1e-6 * np.abs(ref).max() + 1e-7
