@@ -205,13 +205,12 @@ __device__ __forceinline__ void ms_rows(const MsCtx &c, MsStream &st, long long 
 // Down-projection rows [r0, r0 + n), n <= 8: the warp takes 256-wide pieces `warp`, `warp + 16` of K, whose inputs its lanes poll
 // straight into registers; part[row][warp]. Rows that do not fit the ring together (seven of the Qwen2-0.5B shape in fp32 are 136 KB) are
 // given back in groups. A CTA without rows does not wait for the inputs: nothing that it writes would keep them from being overwritten.
-template <bool W16>
+template <bool W16, bool GROUPS>
 __device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long base, int n, int I, const uint2 *hw, unsigned tag, float *part, int warp, int lane) {
     if (n == 0) return;
     const int esz = W16 ? 2 : 4;
     const long long rowb = (long long)I * esz;
     const uint32_t at = (uint32_t)(base & (MS_RING - 1)), rb = (uint32_t)rowb;
-    const int hold = ms_hold(rowb);
     float acc[8], xr[2][8];
 #pragma unroll
     for (int j = 0; j < 8; j++) acc[j] = 0.f;
@@ -227,12 +226,7 @@ __device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long 
 #pragma unroll
         for (int i = 0; i < 8; i++) { xr[i >> 2][2 * (i & 3)] = v[i].x; xr[i >> 2][2 * (i & 3) + 1] = v[i].y; }
     }
-    int g0 = 0;                                              // first row of the group in use
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-        if (r >= n) break;
-        if (r == g0 + hold) { ms_bar(); st.release(base + r * rowb, warp, lane); g0 = r; }
-        if (r == g0 || (r & 3) == 0) st.ensure(c, base + min(min(r + 4, n), g0 + hold) * rowb, lane);
+    auto row = [&](int r, float &sum) {
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int k = (warp + MS_WARPS * u) * 256 + lane * 8;
@@ -240,8 +234,29 @@ __device__ __forceinline__ void ms_down(const MsCtx &c, MsStream &st, long long 
                 float w[8];
                 ms_w8<W16>(st.ring, at + r * rb + (uint32_t)(k * esz), w);
 #pragma unroll
-                for (int e = 0; e < 8; e++) acc[r] = fmaf(w[e], xr[u][e], acc[r]);
+                for (int e = 0; e < 8; e++) sum = fmaf(w[e], xr[u][e], sum);
             }
+        }
+    };
+    if (!GROUPS) {
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            if (r >= n) break;
+            if ((r & 3) == 0) st.ensure(c, base + min(r + 4, n) * rowb, lane);
+            row(r, acc[r]);
+        }
+    } else {
+        const int hold = ms_hold(rowb);
+        int g1 = 0;                                          // end of the group in use
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            if (r >= n) break;
+            if (r == g1) {
+                if (r > 0) { ms_bar(); st.release(base + r * rowb, warp, lane); }
+                g1 = min(n, r + hold);
+                st.ensure(c, base + g1 * rowb, lane);
+            }
+            row(r, acc[r]);
         }
     }
     const float s = ms_reduce8(acc, lane);
@@ -343,7 +358,8 @@ __device__ __forceinline__ void ms_attend(MsSm *sm, MsKV &f, const float *kv, in
     }
 }
 
-template <bool W16>
+// GROUPS: a CTA's down-projection rows do not fit the ring together (a variant of its own: the others keep their registers)
+template <bool W16, bool GROUPS>
 __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ MegaArgs a, const unsigned char *stream_w, const long long *stream_off, const unsigned char *head_w) {
     extern __shared__ __align__(1024) unsigned char ms_raw[];
     const MegaShape &S = a.s;
@@ -530,7 +546,7 @@ __global__ void __launch_bounds__(MS_T + 32) k_lm_step(const __grid_constant__ M
         st.release(at, warp, lane);
         ms_bar();                                             // part is rewritten by the down-projection
         // ---- down-projection, residual ----
-        ms_down<W16>(c, st, at, ncr, I, Lh, tag, part, warp, lane);
+        ms_down<W16, GROUPS>(c, st, at, ncr, I, Lh, tag, part, warp, lane);
         at += b_dn;
         ms_bar();
         if (tid < ncr) {
@@ -666,24 +682,27 @@ void lm_mega_pack(MegaModel &m, const MegaShape &s, const std::vector<BlockWeigh
 
 size_t lm_mega_exchange_words(const MegaShape &s) { return MsLL(s).total; }
 
-template <bool W16>
+template <bool W16, bool GROUPS>
 static void launch_step(const MegaModel &m, const MegaArgs &a) {
     const MegaShape &s = a.s;
     const size_t part = (size_t)std::max<int64_t>(2 * MS_HROWS, 2 * cdiv(s.I, m.grid) + 2) * 4;
     const size_t smem = MS_RING + sizeof(MsSm) + 32 + ((size_t)s.C + part) * 4 + s.NL * sizeof(MegaLayer);
     static size_t set = 0;
-    if (smem > set) { CUDA_CHECK(cudaFuncSetAttribute(k_lm_step<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = smem; }
+    if (smem > set) { CUDA_CHECK(cudaFuncSetAttribute((k_lm_step<W16, GROUPS>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = smem; }
     MegaArgs arg = a;
     const unsigned char *w = (const unsigned char *)m.stream_w, *h = (const unsigned char *)m.head_w;
     const long long *off = m.stream_off;
     void *params[] = {&arg, &w, &off, &h};
-    cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_lm_step<W16>, dim3((unsigned)m.grid), dim3(MS_T + 32), params, smem, stream());
+    cudaError_t e = cudaLaunchCooperativeKernel((const void *)(k_lm_step<W16, GROUPS>), dim3((unsigned)m.grid), dim3(MS_T + 32), params, smem, stream());
     if (e != cudaSuccess) fatal("lm_mega: cooperative launch failed: %s", cudaGetErrorString(e));
     ctx().launches++;
 }
 void lm_mega_launch(const MegaModel &m, const MegaArgs &a) {
     ProfScope ps(NCMB_K_GEMM, 0, 0);
-    if (m.w16) launch_step<true>(m, a); else launch_step<false>(m, a);
+    const bool groups = cdiv(a.s.C, m.grid) > ms_hold((long long)a.s.I * (m.w16 ? 2 : 4));
+    if (m.w16) { if (groups) launch_step<true, true>(m, a); else launch_step<true, false>(m, a); }
+    else if (groups) launch_step<false, true>(m, a);
+    else launch_step<false, false>(m, a);
 }
 
 } // namespace ncmb
