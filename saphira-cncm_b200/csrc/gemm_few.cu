@@ -195,10 +195,11 @@ __global__ void __launch_bounds__(FW_THREADS) k_gemm_few(const __grid_constant__
 // (even and odd positions of K). Sums run over at most 16 products each, then in pairs over the warps and in order over the slices.
 //
 // Bound by issue: at 16 tokens and bf16 weights a chunk takes 64 two-wide multiply-adds, 12 shared-memory reads and 32 conversions a warp,
-// and moves of registers besides. A step of the Qwen2 shape in bf16 with 2 / 4 / 8 / 16 rows takes 0.62 / 0.74 / 1.00 / 1.37 ms (on fp16 pairs
-// 0.70 / 0.71 / 0.73 / 0.74, on the GEMV kernels 1.05 / 1.55 / 2.87 / 4.66), of the GPT-2 shape in fp32 0.31 / 0.34 / 0.40 / 0.48
-// (0.34 / 0.35 / 0.36 / 0.35; 0.43 / 0.64 / 0.91 / 1.59). Error of a step's logits against 64 bits: that of the GEMV kernels or less
-// (2.9e-7 relative for GPT-2, 5.2e-7 for Qwen2; pairs 2.2e-6 and more).
+// and moves of registers besides (4 to 7% fewer with the compiler's own two-wide multiply-add than with inline PTX). A step of the Qwen2
+// shape in bf16 with 2 / 4 / 8 / 16 rows takes 0.62 / 0.73 / 0.95 / 1.28 ms (on fp16 pairs 0.70 / 0.71 / 0.73 / 0.74, on the GEMV kernels
+// 1.05 / 1.55 / 2.87 / 4.66), of the GPT-2 shape in fp32 0.30 / 0.33 / 0.40 / 0.47 (0.34 / 0.35 / 0.36 / 0.35; 0.43 / 0.64 / 0.91 / 1.59).
+// Error of a step's logits against 64 bits: that of the GEMV kernels or less (2.9e-7 relative for GPT-2, 5.2e-7 for Qwen2; pairs
+// 2.2e-6 and more).
 constexpr int FF_WARPS = 8, FF_ST = 8, FF_RUN = 32, FF_THREADS = FF_WARPS * 32 + 32;
 constexpr int ff_tile(int MT) { return MT > 8 ? 32 : 64; }
 constexpr int ff_tgroups(int MT) { return MT > 8 ? 4 : (MT > 4 ? 2 : 1); }       // groups of tokens a warp's lanes are dealt to
@@ -213,10 +214,6 @@ struct FewF32Dev {
     float *part;
     int *err;
 };
-
-__device__ __forceinline__ uint64_t ff_pack(uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; }
-// two fp32 multiply-adds, each rounded as fmaf
-__device__ __forceinline__ void ff_fma2(uint64_t &d, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
 
 template <int MT, bool W16>
 __global__ void __launch_bounds__(FF_THREADS, 2) k_few_f32(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, FewF32Dev a) {
@@ -270,17 +267,17 @@ __global__ void __launch_bounds__(FF_THREADS, 2) k_few_f32(const __grid_constant
         return;
     }
     const int rg = lane & (RG - 1), tg = lane / RG;
-    uint64_t acc[RL][TL];                                    // two sums: over even and over odd positions of K
+    float2 acc[RL][TL];                                    // two sums: over even and over odd positions of K
     float sum[RL][TL];
 #pragma unroll
     for (int r = 0; r < RL; r++)
 #pragma unroll
-        for (int t = 0; t < TL; t++) { acc[r][t] = 0; sum[r][t] = 0.f; }
+        for (int t = 0; t < TL; t++) { acc[r][t] = make_float2(0.f, 0.f); sum[r][t] = 0.f; }
     auto put_aside = [&] {
 #pragma unroll
         for (int r = 0; r < RL; r++)
 #pragma unroll
-            for (int t = 0; t < TL; t++) { sum[r][t] += __uint_as_float((uint32_t)acc[r][t]) + __uint_as_float((uint32_t)(acc[r][t] >> 32)); acc[r][t] = 0; }
+            for (int t = 0; t < TL; t++) { sum[r][t] += acc[r][t].x + acc[r][t].y; acc[r][t] = make_float2(0.f, 0.f); }
     };
     bool ok = true;
     const unsigned char *wl = smem + rg * 128 + ((warp ^ (rg & 7)) << 4);        // (row rg + RG r has the same place in its swizzle group)
@@ -299,18 +296,18 @@ __global__ void __launch_bounds__(FF_THREADS, 2) k_few_f32(const __grid_constant
         for (int r = 0; r < RL; r++) w[r] = *(const uint4 *)(wl + s * STAGE + RG * r * 128);
 #pragma unroll
         for (int h = 0; h < XN; h++) {                       // four positions of K
-            ulonglong2 x[TL];
+            float4 x[TL];
 #pragma unroll
-            for (int t = 0; t < TL; t++) x[t] = *(const ulonglong2 *)(xl + s * STAGE + xo[t % XO][h] + TG * (t / XO * XO) * 128);
+            for (int t = 0; t < TL; t++) x[t] = *(const float4 *)(xl + s * STAGE + xo[t % XO][h] + TG * (t / XO * XO) * 128);
 #pragma unroll
             for (int r = 0; r < RL; r++) {
-                uint64_t w0, w1;
+                float2 w0, w1;
                 if (W16) {
                     const uint32_t u0 = h ? w[r].z : w[r].x, u1 = h ? w[r].w : w[r].y;
-                    w0 = ff_pack(u0 << 16, u0 & 0xffff0000u); w1 = ff_pack(u1 << 16, u1 & 0xffff0000u);
-                } else { w0 = ff_pack(w[r].x, w[r].y); w1 = ff_pack(w[r].z, w[r].w); }
+                    w0 = make_float2(__uint_as_float(u0 << 16), __uint_as_float(u0 & 0xffff0000u)); w1 = make_float2(__uint_as_float(u1 << 16), __uint_as_float(u1 & 0xffff0000u));
+                } else { w0 = make_float2(__uint_as_float(w[r].x), __uint_as_float(w[r].y)); w1 = make_float2(__uint_as_float(w[r].z), __uint_as_float(w[r].w)); }
 #pragma unroll
-                for (int t = 0; t < TL; t++) { ff_fma2(acc[r][t], w0, x[t].x); ff_fma2(acc[r][t], w1, x[t].y); }
+                for (int t = 0; t < TL; t++) { acc[r][t] = __ffma2_rn(w0, make_float2(x[t].x, x[t].y), acc[r][t]); acc[r][t] = __ffma2_rn(w1, make_float2(x[t].z, x[t].w), acc[r][t]); }
             }
         }
         __syncwarp();
