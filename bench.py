@@ -502,21 +502,6 @@ def _peaks():
     return json.load(open(pk)) if os.path.exists(pk) else {}
 
 
-# Dense TF32 throughput of one B200 of this pool: torch.matmul on 8192^3 fp32 operands with TF32 allowed, best of
-# 10, measured once with a scratch script in the way the bf16 figure of MEASURED_PEAKS.json is measured (that file
-# has no TF32 entry). Used as the denominator of the quantizer sweep, whose distance GEMM runs on the TF32 pipe.
-TF32_PEAK_TFLOPS_MEASURED = 752.7      # burst; 611.5 in a 4-second loop under the power cap
-
-
-def tf32_peak():
-    p = _peaks()
-    if "tf32_tflops" in p:
-        return p["tf32_tflops"], "MEASURED_PEAKS.json tf32_tflops"
-    if TF32_PEAK_TFLOPS_MEASURED:
-        return TF32_PEAK_TFLOPS_MEASURED, "torch.matmul TF32 8192^3 on this pool (builder-measured)"
-    return p.get("bf16_tflops", 1590.0) / 2.0, "half of the measured bf16 burst peak (no TF32 measurement)"
-
-
 def lm_bytes_per_step(spec, B, mean_ctx):
     """Algorithmic bytes of one decode step: every parameter once plus the K/V cache of B sequences at the mean
     context, at the storage width the configuration states (fp32 for the GPT-2 shape; 2-byte weights and 2-byte
@@ -631,13 +616,14 @@ def measure_quantizer(lib, stream, n, steps, warmup):
     torch.cuda.synchronize()
     dev_s = e0.elapsed_time(e1) / 1000.0 / steps
     flops = 2.0 * n * 16384 * 64
-    peak, src = tf32_peak()
+    peak = _peaks().get("bf16_tflops", 1590.0)               # fp16 MMAs run at the bf16 rate; a burst of milliseconds
     line = {"metric": "quantized vectors/sec", "value": n / dev_s, "unit": "vectors/s", "n_gpus": 1,
             "steps": steps, "warmup": warmup, "ms_per_step": 1000 * dev_s, "higher_is_better": True,
-            "dtype": "3xtf32 (fp32-grade distances)", "data": "synthetic",
+            "dtype": "fp32 distances decide, fp16 coarse pass with an error bound", "data": "synthetic",
             "config": {"workload": f"c5q: {n} fp32 N(0,1) 64-d vectors vs 16384 x 64 codebook, nearest code"},
             "roofline": {"bound": "tensor", "achieved": flops / dev_s / 1e12, "peak": peak, "unit": "TFLOP/s",
-                         "frac": flops / dev_s / 1e12 / peak, "traffic": None, "peak_source": src, "mma_passes": 3}}
+                         "frac": flops / dev_s / 1e12 / peak, "traffic": None,
+                         "peak_source": "MEASURED_PEAKS.json bf16_tflops" if "bf16_tflops" in _peaks() else "fallback", "mma_passes": 1}}
     lib.ncp_free(model.ncp)
     lib.vqvae_free(model.vqvae)
     lib.weights_free(C.byref(model.ws))

@@ -942,9 +942,10 @@ void attention_decode(const AttnArgs &a) {
     const bool mma_takes = a.hd == 64 && gq_w <= AD_MAXG && ((a.ldk1 & 3) == 0) && (!a.k2 || (a.ldk2 & 3) == 0) && ((a.ldq & 3) == 0) &&
                            al16(a.q) && al16(a.k1) && al16(a.v1) && (!a.k2 || (al16(a.k2) && al16(a.v2)));
     const bool gqa_takes = gqa_shape(a) && ((a.ldq & 3) == 0) && al16(a.q) && mma_env != 1;
-    // (measured: the 4-token level of config 2 -- 16 pairs per group, 9 chunks -- 2.99 -> 2.44 ms over its 12 layers; the
-    // Qwen2 batched-decode shape -- 7 pairs, 16 - 32 chunks -- at 256 sequences 42 936 -> 44 923 tokens/s, at 32
-    // sequences 12 821 -> 12 661: with few (row, kv head) pairs the CTA-per-chunk kernels spread a row over more SMs)
+    // (measured: the 4-token level of config 2 -- 16 pairs per group, 9 chunks -- 2.99 -> 2.44 ms over its 12 layers. Up to eight
+    // pairs per group go to k_attention_dec_gqa whatever their number; what is left for the second condition, groups of 9 to 11
+    // pairs, follows the line measured for seven: gain from about 300 (row, kv head) pairs on, below the CTA-per-chunk kernels
+    // spread a row over more SMs)
     static const int mma_min_g = getenv("NCM_B200_ATTN_DEC_MMA_MIN_G") ? atoi(getenv("NCM_B200_ATTN_DEC_MMA_MIN_G")) : 12;
     static const int mma_max_ch = getenv("NCM_B200_ATTN_DEC_MMA_MAX_CHUNKS") ? atoi(getenv("NCM_B200_ATTN_DEC_MMA_MAX_CHUNKS")) : 16;
     const bool mma_pays = (gq_w >= mma_min_g && max_chunks <= mma_max_ch && pairs * 4 >= (int64_t)ctx().sm_count) ||

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(FW_THREADS) k_gemm_few(const __grid_constant__
 }
 
 // ---- 2 to 16 rows: the same products in fp32 ----
-// A CTA takes 64 weight rows (32 from nine tokens on: smaller shares leave no SM with a second wave of its own) and a slice of K. The
+// A CTA takes 64 weight rows (32 from nine tokens on: the sums of 64 would leave an SM room for one CTA) and a slice of K. The
 // weights come by TMA in chunks of 128 bytes a row (32 floats or 64 bf16 values) with the rows of x that go with them; each of eight warps
 // takes 16 bytes of every row of a chunk. A lane of it holds a block of rows x tokens (2 x 2, 2 x 4 or 4 x 4), so that a 16-byte read of
 // shared memory feeds enough multiply-adds, free of bank conflicts (128-byte swizzle) or as a broadcast; they are issued two at a time

@@ -639,10 +639,11 @@ __global__ void __launch_bounds__(SL_THREADS) k_pick_sorted(const void *__restri
 // ---- the same draw without sorting the row (top_k = 0: the nucleus is cut from the whole vocabulary) ----
 // With seeded or near-uniform logits the nucleus holds most of a 150 K vocabulary, so the sort above is the
 // sampler. Both the cut ("cum_before - p > top_p") and the draw ("u <= cum") are the first rank at which a
-// monotone predicate over cumulative probability turns true, so each can be found the way a radix select finds
-// a rank: three passes over the row's ordered 32-bit keys (11 + 11 + 10 bits), each building per-bin probability
-// mass, element counts and the smallest / largest key of a bin, descending into the bin where the predicate
-// flips. Probabilities are accumulated as 64-bit fixed point (2^-44 steps, exact and order-independent integer
+// monotone predicate over cumulative probability turns true. One sweep of the row sums its probability mass by distance
+// below the maximum (bins of 1/64), one lists the elements of the bins the cut and the draw can fall into, and one CTA
+// per row settles both on the lists. Lists that are too long (ties) are settled the way a radix select finds a rank: three
+// passes over the row's ordered 32-bit keys (11 + 11 + 10 bits), descending into the bin where the predicate flips.
+// Probabilities are accumulated as 64-bit fixed point (2^-44 steps, exact and order-independent integer
 // sums, so runs are reproducible whatever order the atomics land in); the absolute error of a cumulative sum is
 // below 1e-11 of the row's mass, which moves a draw only when it falls that close to a boundary. Ties of equal
 // logits are ranked by ascending index, like the stable sort.

@@ -47,10 +47,12 @@ def _errors(cuda, spec, t, m, B, np_, steps, n_last, plain=False):
 @pytest.fixture(scope="module")
 def models(cuda, tmp_path_factory):
     import synth
-    # the widths of the GPT-2 124M and Qwen2-0.5B shapes, two layers; a width that fills no block of K
+    # the widths of the GPT-2 124M and Qwen2-0.5B shapes, two layers; a gated projection small enough to be cut into slices of K; a width
+    # that fills no block of K
     specs = {"gpt2": synth.LMSpec("gpt2_w", "gpt2", 2, 768, 12, 12, 3072, 1009, 64, rand_affine=1),
              "qwen": synth.LMSpec("qwen_w", "qwen", 2, 896, 14, 2, 4864, 1009, 64, rand_affine=1),
              "qwen_bf16": synth.LMSpec("qwen_w16", "qwen", 2, 896, 14, 2, 4864, 1009, 64, rand_affine=1, bf16_round=1),
+             "gated_slices": synth.LMSpec("qwen_s", "qwen", 2, 512, 8, 2, 696, 301, 64, rand_affine=1),
              "ragged": synth.LMSpec("qwen_r", "qwen", 2, 80, 5, 5, 328, 301, 64, rand_affine=1)}
     made = {k: (s, *_open(cuda, s, str(tmp_path_factory.mktemp(k)))) for k, s in specs.items()}
     cuda.ncmb_set_lm_persistent(1)
@@ -70,7 +72,7 @@ def _pair_bound(spec):
 
 
 @pytest.mark.parametrize("B", [1, 2, 3, 4, 5, 8, 9, 16, 17, 33, 65, 129, 240, 256, 300, 641])
-@pytest.mark.parametrize("kind", ["gpt2", "qwen", "qwen_bf16", "ragged"])
+@pytest.mark.parametrize("kind", ["gpt2", "qwen", "qwen_bf16", "gated_slices", "ragged"])
 def test_decode_logits_against_float64(cuda, models, kind, B):
     spec, t, m = models[kind]
     for steps in (1, 40):                                     # a prompt of one id: up to 16 rows, all of it is fp32
