@@ -149,34 +149,37 @@ struct NearCount { unsigned na, nb; };
 constexpr unsigned NEAR_PAIR_MIN = 512;
 __device__ __forceinline__ bool near_pairs(const NearCount &c, int64_t rows, int64_t min_rows) { return rows >= min_rows && c.na > NEAR_PAIR_MIN; }
 
-// the undecided rows as fp16 pairs, in list order; rinfo as above
-__global__ void __launch_bounds__(256) k_near_pairs(const float *__restrict__ x, int D, const NearMeta *__restrict__ meta, const int *__restrict__ list,
-                                                    const NearCount *__restrict__ count, unsigned short *__restrict__ xh, unsigned short *__restrict__ xl,
-                                                    float2 *__restrict__ rinfo) {
-    pdl_wait();
-    const unsigned n = count->na;
-    if (n <= NEAR_PAIR_MIN) return;
+// the undecided rows as fp16 pairs, in list order; rinfo as above. Four rows of a warp in flight.
+__device__ __forceinline__ void near_make_pairs(const float *__restrict__ x, int D, float es, const int *__restrict__ list, unsigned n, unsigned short *__restrict__ xh,
+                                                unsigned short *__restrict__ xl, float2 *__restrict__ rinfo) {
+    constexpr int RW = 4;
     const int lane = threadIdx.x & 31;
-    const float es = meta->scale;
-    for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
-        const float *xr = x + (int64_t)list[i] * D;
-        float2 v[2];
-        unsigned m = 0;
+    for (unsigned i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * RW; i0 < n; i0 += ((gridDim.x * blockDim.x) >> 5) * RW) {
+        float2 v[RW][2];
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int d = lane * 2 + h * 64;
-            v[h] = d < D ? *(const float2 *)(xr + d) : make_float2(0.f, 0.f);
-            m = max(m, max(__float_as_uint(fabsf(v[h].x)), __float_as_uint(fabsf(v[h].y))));
-        }
-        const float s = pow2_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, m)), 14);
+        for (int i = 0; i < RW; i++) {
+            const float *xr = i0 + i < n ? x + (int64_t)list[i0 + i] * D : nullptr;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int d = lane * 2 + h * 64;
-            uint32_t hi, lo;
-            h16_pair2_raw(v[h].x * s, v[h].y * s, hi, lo, 1.0f);
-            if (d < D) { *(uint32_t *)(xh + (int64_t)i * D + d) = hi; *(uint32_t *)(xl + (int64_t)i * D + d) = lo; }
+            for (int h = 0; h < 2; h++) {
+                const int d = lane * 2 + h * 64;
+                v[i][h] = xr && d < D ? *(const float2 *)(xr + d) : make_float2(0.f, 0.f);
+            }
         }
-        if (lane == 0) rinfo[i] = make_float2(s * es, 0.f);
+#pragma unroll
+        for (int i = 0; i < RW; i++) {
+            unsigned m = max(max(__float_as_uint(fabsf(v[i][0].x)), __float_as_uint(fabsf(v[i][0].y))),
+                             max(__float_as_uint(fabsf(v[i][1].x)), __float_as_uint(fabsf(v[i][1].y))));
+            const float s = pow2_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, m)), 14);
+            if (i0 + i >= n) break;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int d = lane * 2 + h * 64;
+                uint32_t hi, lo;
+                h16_pair2_raw(v[i][h].x * s, v[i][h].y * s, hi, lo, 1.0f);
+                if (d < D) { *(uint32_t *)(xh + (int64_t)(i0 + i) * D + d) = hi; *(uint32_t *)(xl + (int64_t)(i0 + i) * D + d) = lo; }
+            }
+            if (lane == 0) rinfo[i0 + i] = make_float2(s * es, 0.f);
+        }
     }
 }
 
@@ -504,16 +507,21 @@ __global__ void __launch_bounds__(256) k_nearest_refine(const float *__restrict_
 }
 
 // All codes for the listed rows (list == null: for rows 0 .. n_rows - 1). Work item: 8 rows x 256 codes, one code per
-// thread; the minimum of a warp goes to best[] by atomicMin on (ordered distance, index).
+// thread; the minimum of a warp goes to best[] by atomicMin on (ordered distance, index). Undecided rows that go through the pair
+// products are only converted for them here.
 constexpr int NS_ROWS = 8, NS_CODES = 256;
 __global__ void __launch_bounds__(NS_CODES) k_nearest_scan(const float *__restrict__ x, const float *__restrict__ et, const float *__restrict__ cn,
                                                            const NearMeta *__restrict__ meta, int V, int D,
                                                            const int *__restrict__ list, const NearCount *__restrict__ count, int n_rows, int64_t pair_rows,
+                                                           unsigned short *__restrict__ xh, unsigned short *__restrict__ xl, float2 *__restrict__ rinfo,
                                                            unsigned long long *__restrict__ best) {
     extern __shared__ __align__(16) float near_xs[];                    // [Dp / 4][NS_ROWS][4]
     __shared__ int direct_s[NS_ROWS];
     const int Dp = (D + 3) & ~3;
-    const int nb = list ? (int)count->nb : 0, n = !list ? n_rows : (near_pairs(*count, n_rows, pair_rows) ? 0 : (int)count->na), nsl = (V + NS_CODES - 1) / NS_CODES;
+    pdl_wait();
+    const bool pairs = list && near_pairs(*count, n_rows, pair_rows);
+    if (pairs) near_make_pairs(x, D, meta->scale, list, count->na, xh, xl, rinfo);
+    const int nb = list ? (int)count->nb : 0, n = !list ? n_rows : (pairs ? 0 : (int)count->na), nsl = (V + NS_CODES - 1) / NS_CODES;
     const int64_t itb = (int64_t)((nb + NS_ROWS - 1) / NS_ROWS) * nsl, items = itb + (int64_t)((n + NS_ROWS - 1) / NS_ROWS) * nsl;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
@@ -590,6 +598,7 @@ __global__ void __launch_bounds__(NS_CODES) k_nearest_scan(const float *__restri
 static_assert(NS_CODES / 32 == NS_ROWS, "a warp loads a row");
 __global__ void k_near_store(const unsigned long long *__restrict__ best, const int *__restrict__ list, const NearCount *__restrict__ count, int n_rows,
                              int *__restrict__ idx_out, int out_tlen, int out_stride, int out_off) {
+    pdl_wait();
     const int na = list ? (int)count->na : n_rows, n = na + (list ? (int)count->nb : 0);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int64_t at = i < na ? i : (int64_t)n_rows - 1 - (i - na), r = list ? list[at] : at;
@@ -645,7 +654,7 @@ static unsigned scan_grid(int64_t items) { return (unsigned)std::max<int64_t>(1,
 
 // 2^20 rows against 16384 x 64 codes, by how close codes lie (three TF32 passes over everything took 9.1 to 10.1 ms for each):
 //   random, or a code plus noise           3.7 - 3.9 ms      a tenth undecided (codes about a mean three times their spread)   5.1
-//   unused codes at zero                   3.8               all undecided (repeated codes, tight clusters, a mean of 30 times   9.0 - 9.8
+//   unused codes at zero                   3.8               all undecided (repeated codes, tight clusters, a mean of 30 times   9.1 - 10.2
 //                                                            the spread, unused codes near zero)
 // With the scan alone the undecided took up to 144 ms. Calls of under 1024 rows: 42 us for 900 rows, 190 when all are undecided.
 void nearest_codes(const float *x, const float *E, int64_t rows, int V, int D, int *idx_out, int out_tlen, int out_stride, int out_off) {
@@ -664,8 +673,9 @@ void nearest_codes(const float *x, const float *E, int64_t rows, int V, int D, i
         unsigned long long *best = ws.get<unsigned long long>(rows);
         CUDA_CHECK(cudaMemsetAsync(best, 0xff, (size_t)rows * 8, stream()));
         const int64_t items = cdiv(rows, NS_ROWS) * cdiv(V, NS_CODES);
-        LAUNCH(k_nearest_scan, scan_grid(items), NS_CODES, scan_smem, x, cb.et, cb.cn, cb.meta, V, D, (const int *)nullptr, (const NearCount *)nullptr, (int)rows, NEAR_PAIR_ROWS, best);
-        LAUNCH(k_near_store, (unsigned)std::min<int64_t>(cdiv(rows, 256), ctx().sm_count * 4), 256, 0, best, (const int *)nullptr, (const NearCount *)nullptr, (int)rows,
+        LAUNCH(k_nearest_scan, scan_grid(items), NS_CODES, scan_smem, x, cb.et, cb.cn, cb.meta, V, D, (const int *)nullptr, (const NearCount *)nullptr, (int)rows, NEAR_PAIR_ROWS,
+               (unsigned short *)nullptr, (unsigned short *)nullptr, (float2 *)nullptr, best);
+        LAUNCH_PDL(k_near_store, (unsigned)std::min<int64_t>(cdiv(rows, 256), ctx().sm_count * 4), 256, 0, best, (const int *)nullptr, (const NearCount *)nullptr, (int)rows,
                idx_out, out_tlen, out_stride, out_off);
         return;
     }
@@ -727,14 +737,13 @@ void nearest_codes(const float *x, const float *E, int64_t rows, int V, int D, i
     products(false, mx, me);
     LAUNCH(k_nearest_refine, (unsigned)cdiv(rows * 32, 256), 256, 0, x, cb.et, cb.cn, V, cb.meta, rinfo, rows, D, nslice * 4, tps, id_mask, cand,
            idx_out, out_tlen, out_stride, out_off, list, count, best);
-    if (rows >= NEAR_PAIR_ROWS) {                            // (both end at once where few rows are listed)
-        LAUNCH_PDL(k_near_pairs, (unsigned)std::min<int64_t>(cdiv(rows, 8), ctx().sm_count * 8), 256, 0, x, D, (const NearMeta *)cb.meta, (const int *)list,
-                   (const NearCount *)count, xh, xl, rinfo);
-        products(true, tc_get_map_h16(xl, rows, D, D, 128), tc_get_map_h16(cb.el, V, D, D, 128));
-    }
     const int64_t max_items = cdiv(rows, NS_ROWS) * cdiv(V, NS_CODES);
-    LAUNCH(k_nearest_scan, scan_grid(max_items), NS_CODES, scan_smem, x, cb.et, cb.cn, cb.meta, V, D, list, count, (int)rows, NEAR_PAIR_ROWS, best);
-    LAUNCH(k_near_store, (unsigned)std::min<int64_t>(cdiv(rows, 256), ctx().sm_count * 4), 256, 0, best, list, count, (int)rows, idx_out, out_tlen, out_stride, out_off);
+    LAUNCH_PDL(k_nearest_scan, scan_grid(max_items), NS_CODES, scan_smem, x, cb.et, cb.cn, (const NearMeta *)cb.meta, V, D, (const int *)list, (const NearCount *)count, (int)rows,
+               NEAR_PAIR_ROWS, xh, xl, rinfo, best);
+    if (rows >= NEAR_PAIR_ROWS)                              // (ends at once where few rows are listed)
+        products(true, tc_get_map_h16(xl, rows, D, D, 128), tc_get_map_h16(cb.el, V, D, D, 128));
+    LAUNCH_PDL(k_near_store, (unsigned)std::min<int64_t>(cdiv(rows, 256), ctx().sm_count * 4), 256, 0, (const unsigned long long *)best, (const int *)list, (const NearCount *)count, (int)rows,
+               idx_out, out_tlen, out_stride, out_off);
 }
 
 } // namespace ncmb
