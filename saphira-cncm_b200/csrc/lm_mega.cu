@@ -16,9 +16,9 @@
 //   * Products. Sixteen warps: four quarters of K x four groups of rows. A lane keeps its eight elements of the input in
 //     registers; eight rows at a time meet in a reduce-scatter.
 //
-// One row only: 681 us a step for the Qwen2 shape (the kernel chain: 757) and 307 for GPT-2 in fp32 (308). What is left is the
+// One row only: 670 us a sampled step for the Qwen2 shape (the kernel chain: 757) and 306 for GPT-2 in fp32 (308). What is left is the
 // six exchanges of a layer, about 1 us each, and the reductions between them; from two rows on the few-row kernel chain is faster
-// (two rows 783 us against 837 here, four 806 against 1187), since its tensor-core products do not grow with the rows.
+// (greedy steps of two rows 620 us and of four 725, against 837 and 1187 here with the sampler).
 //
 // Hops of a layer: hidden -> q k v -> attention partials -> hidden -> MLP -> hidden. Every wait is bounded (2 s): a wait that
 // runs out records a code, the other CTAs see it and stop waiting, and the kernel ends.
